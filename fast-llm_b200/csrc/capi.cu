@@ -86,7 +86,8 @@ int fl_b200_create(int device, fl_b200_ctx **out) {
     CK(matvec_init());
     CK(matvec_tc_init());
     CK(matmul_tc_nx_init());
-    CK(cudaMalloc(&c->xq, matmul_tc_nx_scratch_bytes(18432, 8)));   // the widest activation the kernels take, 8 columns
+    CK(cudaMalloc(&c->xq, matmul_tc_nx_scratch_bytes(kNxMaxCols, kNxTgs, 3)));
+    CK(cudaMalloc(&c->nx_part, kNxPartFloats * sizeof(float)));
     CK(matmul_umma_init());
     CK(cudaMalloc(&c->xu, matmul_umma_xu_bytes(18432)));
     CK(cudaMalloc(&c->um_scratch, matmul_umma_scratch_bytes()));
@@ -102,7 +103,7 @@ void fl_b200_destroy(fl_b200_ctx *c) {
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     cudaFree(c->attn_part);
-    cudaFree(c->xq);
+    cudaFree(c->xq); cudaFree(c->nx_part);
     cudaFree(c->xu); cudaFree(c->um_scratch); cudaFree(c->um_tickets);
     for (void *p : c->retired) cudaFree(p);
     cudaFree(c->attn_tickets);
@@ -243,9 +244,9 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
     if (nx == 0) nx = 1;
     if (pitch == row_bytes(fmt, cols)) pitch = 0;   // packed rows
     uint32_t first_single = 0;   // columns from here on go through the one-column kernel
-    if (nx >= 2 && (fmt == FL_B200_Q4_K || fmt == FL_B200_Q6_K) && !expert_id && cols <= 18432) {
-        // verify batches, prompt chunks: up to 8 columns per pass over the weights on the tensor cores, either format
-        for (uint32_t p0 = 0; p0 < nx; p0 += 8) {
+    if (nx >= 2 && (fmt == FL_B200_Q4_K || fmt == FL_B200_Q6_K || fmt == FL_B200_Q8_0) && !expert_id) {
+        // Q4_K under FLB_UMMA=1: tcgen05 with the accumulator in tensor memory, 8 columns per pass
+        for (uint32_t p0 = 0; fmt == FL_B200_Q4_K && cols <= 18432 && p0 < nx; p0 += 8) {
             const uint32_t nt = nx - p0 < 8 ? nx - p0 : 8;
             if (nt < 2 && p0 > 0) break;   // a last single column goes to the one-column kernel
             NxCall nc{};
@@ -255,14 +256,40 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
             nc.skip_convert = (same_columns && nx <= 8) ? 1 : 0;   // with more than 8 columns the scratch holds the last chunk only
             nc.y = y + (size_t)p0 * ystride; nc.ystride = ystride; nc.accumulate = accumulate;
             nc.pdl = pdl;
-            // Q4_K: tcgen05 with the accumulator in tensor memory; what it does not take goes to the mma.sync kernel
-            cudaError_t e = launch_matmul_umma(nc, c->xu, c->um_scratch, c->um_tickets, c->status, c->sms, c->stream);
-            if (e == cudaErrorNotSupported) {
-                if (fmt == FL_B200_Q4_K) nc.skip_convert = 0;   // the other kernel's scratch does not hold these columns
-                e = launch_matmul_tc_nx(nc, c->xq, c->status, c->sms, c->stream);
-            }
-            if (e == cudaErrorNotSupported) break;   // the shape does not qualify (same answer for every chunk)
+            const cudaError_t e = launch_matmul_umma(nc, c->xu, c->um_scratch, c->um_tickets, c->status, c->sms, c->stream);
+            if (e == cudaErrorNotSupported) break;   // off, or not its shape (the same answer for every chunk)
             if (e != cudaSuccess) return cuda_err(e, "multi-column matmul launch");
+            first_single = p0 + nt;
+        }
+        // verify batches, prompt chunks: up to 16 columns per pass over the weights on the tensor cores
+        for (uint32_t p0 = first_single; p0 < nx; p0 += kNxMaxTokens) {
+            const uint32_t nt = nx - p0 < kNxMaxTokens ? nx - p0 : kNxMaxTokens;
+            if (nt < 2) break;   // a last single column goes to the one-column kernel
+            const NxTensor t{fmt, w, rows, pitch, y + (size_t)p0 * ystride, ystride, 0};
+            const uint32_t parts = matmul_tc_nx_parts(&t, 1, cols, nt);
+            if (parts == 0) break;   // the shape does not qualify (same answer for every chunk)
+            NxIn in{};
+            in.x = x + (size_t)p0 * xstride; in.xstride = xstride;
+            if (x2) in.x2 = x2 + (size_t)p0 * xstride;
+            cudaError_t e = cudaSuccess;
+            if (!(same_columns && nx <= kNxMaxTokens)) {   // with more columns than that the scratch holds the last chunk only
+                e = launch_nx_convert(in, &t, 1, cols, nt, c->xq, kNxTgs, c->stream, pdl != 0);
+                if (e == cudaErrorNotSupported) break;
+                if (e != cudaSuccess) return cuda_err(e, "activation conversion launch");
+            }
+            // the matmul overlaps the conversion's launch: it reads weights only until the conversion has completed
+            const uint32_t cap = (uint32_t)(kNxPartFloats / ((size_t)parts * nt)) & ~15u, slice = parts == 1 || rows <= cap ? rows : cap;
+            const size_t rb = pitch ? pitch : row_bytes(fmt, cols);
+            for (uint32_t r0 = 0; r0 < rows; r0 += slice) {
+                NxTensor ts = t;
+                ts.w = (const uint8_t *)w + (size_t)r0 * rb;
+                ts.rows = std::min(slice, rows - r0);
+                if (parts > 1) { ts.y = c->nx_part; ts.ystride = ts.rows; ts.part_stride = (size_t)nt * ts.rows; }
+                e = launch_nx_matmul(in, &ts, 1, cols, nt, parts > 1 ? 0 : accumulate, c->xq, kNxTgs, c->status, c->sms, c->stream, true);
+                if (e == cudaSuccess && parts > 1)
+                    e = launch_reduce_parts(c->nx_part, ts.part_stride, parts, t.y + r0, ts.rows, ystride, nt, accumulate, c->stream, true);
+                if (e != cudaSuccess) return cuda_err(e, "multi-column matmul launch");
+            }
             first_single = p0 + nt;
         }
     }

@@ -23,7 +23,8 @@ struct fl_b200_ctx {
     float *argmax_scratch = nullptr;
     void *small = nullptr;
     uint8_t *xq = nullptr;               // converted activations of the multi-column matmul (fixed size, see fl_b200_create)
-    uint8_t *xu = nullptr;               // the same for the tcgen05 matmul, with its split-K scratch and tickets
+    float *nx_part = nullptr;            // its planes of partial results (kNxPartFloats, see matmul)
+    uint8_t *xu = nullptr;               // the converted activations of the tcgen05 matmul, with its split-K scratch and tickets
     float *um_scratch = nullptr;
     uint32_t *um_tickets = nullptr;
     uint32_t *grid_bar = nullptr;        // barrier state of the chained matvec launches (two words, zero between launches)
@@ -33,11 +34,15 @@ struct fl_b200_ctx {
 };
 
 namespace flb {
+// Converted activations: 16 columns of the widest activation in up to three layouts. Planes of partial results of a plain
+// matmul call: 32 MB; more rows than that holds go out in slices.
+constexpr uint32_t kNxTgs = kNxMaxTokens / 4;
+constexpr size_t kNxPartFloats = (size_t)8 << 20;
 int set_err(int code, const char *fmt, ...);
 // Makes c->attn_part at least `bytes` large (never frees a buffer a recorded plan may still use).
 int grow_attn_part(fl_b200_ctx *c, size_t bytes);
 int cuda_err(cudaError_t e, const char *what);
-// y[p * ystride + r] (+)= dot(W[r], x + p * xstride), p < nx, enqueued on the context's stream: up to 8
+// y[p * ystride + r] (+)= dot(W[r], x + p * xstride), p < nx, enqueued on the context's stream: up to 16
 // columns per pass over the weights where the multi-column kernel takes the shape, one column per pass otherwise
 // (pdl: those one-column launches are programmatic dependents of the launch before them).
 int matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t cols, const float *x, uint32_t nx,
@@ -50,11 +55,11 @@ int matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t cols,
 // Hands device memory to the decoder, which frees it when it is destroyed.
 void decoder_adopt(fl_b200_decoder *d, void *dev);
 // The MoE block inside a decoder step (moe.cu): y[t] = sum over the selected experts of gate * expert(x[t]) for
-// n_tok <= the block's max_tokens rows of x, enqueued on the block's context's stream (one token: one expert walk per
-// selected expert through the expert-indexed matvec; more: every expert once through the multi-column matmul).
-// *n_launch: launches enqueued.
-// wnorm / eps / resid (one token): x is the raw hidden state, RMSNorm(x) * wnorm is taken inside the block's first
-// kernels, and y = resid + the block's output.
+// n_tok <= the block's max_tokens rows of x, enqueued on the block's context's stream (one token, and shapes the grouped
+// multi-column matmul does not take: one expert walk per token and selected expert through the expert-indexed matvec; more:
+// every expert once through the grouped multi-column matmul). *n_launch: launches enqueued.
+// wnorm / eps / resid (one GPU): x is the raw hidden state, RMSNorm(x) * wnorm is taken inside the block's first
+// kernels, and y = resid + the block's output (resid, y: n_tok rows; they may be the same).
 int moe_enqueue_tokens(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y, uint32_t *n_launch, const float *wnorm = nullptr,
                        float eps = 0.f, const float *resid = nullptr);
 fl_b200_ctx *moe_ctx(const fl_b200_moe *m);

@@ -132,20 +132,54 @@ __global__ void wmerge_kernel(const float *__restrict__ parts, const float *__re
 
 // y[t][i] = sum_q (gates[t][q] * parts[t][q][i]), the arithmetic of fl_op_wmerge (decode_params.h:274-295) without its
 // residual terms, for every token of a block in one launch. grid (ceil(n / 256), n_tok).
-__global__ void wmerge_tokens_kernel(const float *__restrict__ parts, const float *__restrict__ gates, float *__restrict__ y,
-                                     uint32_t n_parts, uint32_t n) {
+__global__ void wmerge_tokens_kernel(const float *__restrict__ parts, const float *__restrict__ gates, float *y, uint32_t n_parts,
+                                     uint32_t n, uint32_t n_planes, size_t plane_stride, const float *resid) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y;
     if (i >= n) return;
     float acc = 0.f;
-    for (uint32_t q = 0; q < n_parts; ++q)
-        acc = __fadd_rn(acc, __fmul_rn(gates[(size_t)t * n_parts + q], parts[((size_t)t * n_parts + q) * n + i]));
-    y[(size_t)t * n + i] = __fmul_rn(acc, 1.0f);
+    for (uint32_t q = 0; q < n_parts; ++q) {
+        const float *p = parts + ((size_t)t * n_parts + q) * n + i;
+        float v = p[0];
+#pragma unroll 4
+        for (uint32_t s = 1; s < n_planes; ++s) v = __fadd_rn(v, p[s * plane_stride]);
+        acc = __fadd_rn(acc, __fmul_rn(gates[(size_t)t * n_parts + q], v));
+    }
+    if (resid) acc = __fadd_rn(resid[(size_t)t * n + i], acc);
+    y[(size_t)t * n + i] = acc;
+}
+
+// The table of a grouped multi-column launch (matvec_tc_nx.cu), by one warp: active experts in ascending order, their
+// columns from col_off on (at most P) and the groups of four columns in front of them.
+__device__ __forceinline__ void nx_table_warp(const uint32_t *cnt, uint32_t n_local, uint32_t col_off, uint32_t P, uint32_t *table) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t n_act = 0, tgs = 0, most = 0;
+    for (uint32_t b = 0; b < n_local; b += 32) {
+        const uint32_t e = b + lane, c = e < n_local ? cnt[e] : 0u;
+        const uint32_t n = c > col_off ? min(c - col_off, P) : 0u, tg = (n + 3) / 4;
+        uint32_t incl = tg;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += v;
+        }
+        const uint32_t mask = __ballot_sync(0xffffffffu, n != 0);
+        if (n) reinterpret_cast<uint4 *>(table)[1 + n_act + __popc(mask & ((1u << lane) - 1u))] = make_uint4(e, n, tgs + incl - tg, 0u);
+        n_act += __popc(mask);
+        most = max(most, __reduce_max_sync(0xffffffffu, tg));
+        tgs += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) { table[0] = n_act; table[1] = most; }
+}
+__global__ void __launch_bounds__(32) nx_table_kernel(const uint32_t *__restrict__ cnt, uint32_t n_local, uint32_t col_off, uint32_t P,
+                                                      uint32_t *__restrict__ table) {
+    nx_table_warp(cnt, n_local, col_off, P, table);
 }
 
 // One warp: a stable counting sort of the pairs by local expert.
 __global__ void __launch_bounds__(32) group_by_expert_kernel(const uint32_t *__restrict__ lids, uint32_t n_pairs, uint32_t top_k,
                                                              uint32_t n_local, uint32_t cap, uint32_t *__restrict__ cnt,
-                                                             uint32_t *__restrict__ tok_list, uint32_t *__restrict__ pair_list) {
+                                                             uint32_t *__restrict__ tok_list, uint32_t *__restrict__ pair_list,
+                                                             uint32_t *__restrict__ table) {
     const uint32_t lane = threadIdx.x;
     for (uint32_t e = lane; e < n_local; e += 32) cnt[e] = 0;
     __syncwarp();
@@ -165,6 +199,7 @@ __global__ void __launch_bounds__(32) group_by_expert_kernel(const uint32_t *__r
             __syncwarp();
         }
     }
+    if (table) nx_table_warp(cnt, n_local, 0, kNxMaxTokens, table);
 }
 
 // fl_op_silu_mul, decode_params.h:267-272: (g / (1 + expf(-g))) * u
@@ -327,16 +362,21 @@ cudaError_t launch_wmerge(const float *parts, const float *gates, const float *a
 }
 
 cudaError_t launch_wmerge_tokens(const float *parts, const float *gates, float *y, uint32_t n_parts, uint32_t n, uint32_t n_tok,
-                                 cudaStream_t stream) {
+                                 cudaStream_t stream, uint32_t n_planes, size_t plane_stride, const float *resid) {
     if (n == 0 || n_parts == 0 || n_tok == 0) return cudaErrorInvalidValue;
-    wmerge_tokens_kernel<<<dim3((n + 255) / 256, n_tok), 256, 0, stream>>>(parts, gates, y, n_parts, n);
+    wmerge_tokens_kernel<<<dim3((n + 255) / 256, n_tok), 256, 0, stream>>>(parts, gates, y, n_parts, n, n_planes, plane_stride, resid);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_nx_table(const uint32_t *cnt, uint32_t n_local, uint32_t col_off, uint32_t P, uint32_t *table, cudaStream_t stream) {
+    nx_table_kernel<<<1, 32, 0, stream>>>(cnt, n_local, col_off, P, table);
     return cudaGetLastError();
 }
 
 cudaError_t launch_group_by_expert(const uint32_t *lids, uint32_t n_pairs, uint32_t top_k, uint32_t n_local, uint32_t cap,
-                                   uint32_t *cnt, uint32_t *tok_list, uint32_t *pair_list, cudaStream_t stream) {
+                                   uint32_t *cnt, uint32_t *tok_list, uint32_t *pair_list, cudaStream_t stream, uint32_t *table) {
     if (n_pairs == 0 || top_k == 0 || n_local == 0 || cap == 0) return cudaErrorInvalidValue;
-    group_by_expert_kernel<<<1, 32, 0, stream>>>(lids, n_pairs, top_k, n_local, cap, cnt, tok_list, pair_list);
+    group_by_expert_kernel<<<1, 32, 0, stream>>>(lids, n_pairs, top_k, n_local, cap, cnt, tok_list, pair_list, table);
     return cudaGetLastError();
 }
 

@@ -89,9 +89,52 @@ cudaError_t launch_matvec_tc(const MatvecArgs &a, int sms, cudaStream_t stream);
 // when a phase does not qualify: launch them one by one then. args[0].grid_bar names the barrier state.
 cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaStream_t stream);
 cudaError_t matvec_tc_init(void);
-// Several activation columns (P <= 8) in one pass over a Q4_K / Q6_K tensor on the tensor cores (matvec_tc_nx.cu):
-// y[p * ystride + r] (+)= dot(W[r], x + p * xstride). xq: device scratch of matmul_tc_nx_scratch_bytes(cols, P) bytes
-// that holds the converted activations during the call. cudaErrorNotSupported when the shape does not qualify.
+// Several activation columns (P <= 16) in one pass over up to three Q4_K / Q6_K / Q8_0 tensors on the tensor cores
+// (matvec_tc_nx.cu): y[p * ystride + r] (+)= dot(W[r], column p). Two launches: launch_nx_convert builds the activation's
+// operand image(s) in xq, launch_nx_matmul walks the weights.
+constexpr uint32_t kNxMaxTokens = 16, kNxMaxCols = 18432;
+constexpr uint32_t kAttnRecord = 132;   // floats of one split's record of one query head: context[128], maximum, sum, pad
+struct NxTensor {
+    int fmt;
+    const void *w;           // rows x cols, GGUF block layout (grouped: the experts' slices one behind the other)
+    uint32_t rows, pitch;    // pitch 0 = packed rows
+    float *y;                // output row blocks, ystride floats apart
+    uint32_t ystride;
+    size_t part_stride;      // floats between the planes of partial results (matmul_tc_nx_parts > 1)
+};
+struct NxIn {
+    const float *x;          // column p: row p, xstride floats apart
+    const float *x2;         // optional: the column is SiLU(x) * x2 (same strides)
+    uint32_t xstride, n_parts;   // n_parts planes of x (and x2), part_stride floats apart, are added in order (0 = 1)
+    size_t part_stride;
+    const float *resid;      // optional: + resid (row p, rstride apart)
+    float *x_out;            // optional: the sum is stored here too (row p, rstride apart)
+    uint32_t rstride;
+    const float *wnorm;      // optional: RMSNorm(column) * wnorm; the matmul applies the 1 / rms to its results
+    float eps;
+    const float *att;        // optional, in place of x: the columns are the attention contexts of heads of 128 whose splits'
+    uint32_t n_splits;       // records (launch_attn_decode with records_only) are added up here
+    // Grouped columns (mixture of experts): `table` (launch_nx_table) lists the active experts; column p of an expert is row
+    // col_idx[expert * list_stride + col_off + p] of x and goes to output row block out_idx[the same].
+    const uint32_t *table, *col_idx, *out_idx;
+    uint32_t list_stride, col_off, n_groups, n_experts;   // n_groups: upper bound of active experts
+    int table_ready;         // 1: the table was complete before the kernel in front of the matmul started
+};
+// Number of parts the columns are cut into (1: y is the result; more: planes of partial sums); 0: not taken. split: planes cost the
+// caller nothing extra, cut as finely as is best.
+uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split = false);
+// tgs: groups of four columns in the image(s) (grouped: of all active experts together)
+size_t matmul_tc_nx_scratch_bytes(uint32_t cols, uint32_t tgs, int layouts);
+// n = 0 tensors: only x_out is written. cudaErrorNotSupported: strides or addresses the vector loads do not take.
+cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, uint8_t *xq, uint32_t tgs_cap,
+                              cudaStream_t stream, bool pdl);
+cudaError_t launch_nx_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,
+                             uint32_t tgs_cap, uint32_t *status, int sms, cudaStream_t stream, bool pdl, bool split = false);
+cudaError_t launch_reduce_parts(const float *part, size_t part_stride, uint32_t n_parts, float *y, uint32_t rows, uint32_t ystride,
+                                uint32_t P, int accumulate, cudaStream_t stream, bool pdl);
+// The table of a grouped launch: of cnt[e] listed columns of expert e those from col_off on, at most P.
+cudaError_t launch_nx_table(const uint32_t *cnt, uint32_t n_local, uint32_t col_off, uint32_t P, uint32_t *table, cudaStream_t stream);
+// One call of the tcgen05 form below, up to 8 columns.
 struct NxCall {
     int fmt;
     const void *w;           // rows x cols, GGUF block layout
@@ -109,8 +152,6 @@ struct NxCall {
     uint32_t col_off;
     int pdl;                 // the launches of this call are programmatic dependents of the launch before them
 };
-cudaError_t launch_matmul_tc_nx(const NxCall &c, uint8_t *xq, uint32_t *status, int sms, cudaStream_t stream);
-size_t matmul_tc_nx_scratch_bytes(uint32_t cols, uint32_t P);
 cudaError_t matmul_tc_nx_init(void);
 // The same call on tcgen05 with the accumulator in tensor memory (matmul_umma.cu; Q4_K). xu: device scratch of
 // matmul_umma_xu_bytes(cols) bytes for the converted activations; scratch / tickets: split-K partial results and their
@@ -240,14 +281,14 @@ cudaError_t launch_router_sel(const float *logits, uint32_t *ids, float *gates, 
 // expert the pairs stay in ascending order): cnt[e] pairs for expert e, their tokens in tok_list[e * cap + i] and
 // their pair indices (token * top_k + slot) in pair_list[e * cap + i]. lids: local expert of every pair or kExpertSkip.
 cudaError_t launch_group_by_expert(const uint32_t *lids, uint32_t n_pairs, uint32_t top_k, uint32_t n_local, uint32_t cap,
-                                   uint32_t *cnt, uint32_t *tok_list, uint32_t *pair_list, cudaStream_t stream);
+                                   uint32_t *cnt, uint32_t *tok_list, uint32_t *pair_list, cudaStream_t stream, uint32_t *table = nullptr);
 // fl_op_wmerge (src/runtime/decode_params.h:274-295).
 cudaError_t launch_wmerge(const float *parts, const float *gates, const float *add1, const float *add2, float *y,
                           float scale, uint32_t n_parts, uint32_t n, uint32_t n_full, cudaStream_t stream);
-// fl_op_wmerge for n_tok tokens in one launch: y[t] = sum_q gates[t][q] * parts[t][q] (products and sums rounded in
-// the reference's order; no residual terms).
+// fl_op_wmerge for n_tok tokens in one launch: y[t] = (resid[t] +) sum_q gates[t][q] * parts[t][q] (products and sums
+// rounded in the reference's order); a part is the sum of n_planes planes, plane_stride floats apart.
 cudaError_t launch_wmerge_tokens(const float *parts, const float *gates, float *y, uint32_t n_parts, uint32_t n, uint32_t n_tok,
-                                 cudaStream_t stream);
+                                 cudaStream_t stream, uint32_t n_planes = 1, size_t plane_stride = 0, const float *resid = nullptr);
 cudaError_t launch_silu_mul(const float *gate, const float *up, float *h, uint32_t n, cudaStream_t stream);
 // RoPE (adjacent pairs) on q in place and on k, then store k and v as f16 at
 // row *pos of a cache laid out [n_kv_head][kv_stride][head_dim].

@@ -1,32 +1,44 @@
-// Several activation columns in one pass over a k-quant tensor: Y[p][r] (+)= dot(W[r], X[p]) for p < P <= 8,
-// the STREAM_DOT semantics of Task::nx (include/fastllm/fastllm.h:87-96; the reference's GPU form is
-// gdot_i8k_q4_K_mc, src/runtime/kernels_gpu.h:682-740, Q4_K only). Used for draft-verification batches,
-// prompt chunks and the tokens that share an expert of a mixture-of-experts block.
+// Several activation columns in one pass over k-quant tensors: Y[p][r] (+)= dot(W[r], X[p]) for p < P <= 16, the
+// STREAM_DOT semantics of Task::nx (include/fastllm/fastllm.h:87-96; the reference's GPU form is gdot_i8k_q4_K_mc,
+// src/runtime/kernels_gpu.h:682-740, Q4_K only). Used for draft-verification batches, prompt chunks, independent
+// sequences and the tokens that share an expert of a mixture-of-experts block. Formats: Q4_K, Q6_K, Q8_0.
 //
-// The pipeline is the one of the single-column tensor-core kernel (matvec_tc.cu): a unit is 16 rows, a stage is
-// the same 2048-column segment of the unit's rows (one bulk copy per row into a padded shared-memory row), a
-// producer warp keeps a ring of stages full, consumer warp w owns super-block w of the segment, a finalizer warp
-// adds the warps' partial sums in warp order and writes Y. What differs is the use of mma.sync.m16n8k16:
-//   * the 8 columns of the B operand are 4 activation columns ("tokens"), each as an f16 (hi, lo) pair, so
-//     every product of the instruction is used; two instructions serve 8 tokens from the same A registers;
-//   * the 16 k-slots of an instruction are 16 consecutive weights of ONE scale group of a row (half a Q4_K
-//     sub-block, a whole Q6_K one): lane column t unpacks word t of the group. The accumulator a lane reads
-//     back, C[g][2t], C[g][2t+1], C[g+8][2t], C[g+8][2t+1], is then the complete 16-weight dot product of rows g
-//     and g + 8 with token t of the group of four, and the scale of the group is applied in f32;
-//   * the activations are converted once, by a small kernel of their own, into exactly the register layout of
-//     the B operand (per 256-column block and group of four tokens 4096 bytes of f16 pairs, then the tokens'
-//     sub-block sums and power-of-two block scales); the matmul kernel brings that image into shared memory with
-//     bulk copies, a chunk of at most 16 blocks (4096 columns) at a time. With more columns than a chunk the
-//     kernel walks the chunks one after the other (all units of the CTA per chunk) and the finalizer keeps
-//     the units' running sums in shared memory.
-// Every weight byte still crosses HBM once per pass, whatever P is; a pass over 8 tokens costs about what a
-// single-column pass costs.
-// For the experts of a mixture-of-experts block the columns of a call are a device-side list: the number of
-// valid columns is read from device memory (a call with none returns at once and reads no weights), the
-// conversion gathers the listed tokens (optionally as SiLU(x) * x2, the input of a down projection) and the
-// finalizer scatters the results to the listed output rows.
+// A launch is a list of jobs. A job is one tensor (or one expert's slice of it) times one range of columns (a "part":
+// one or more segments of 2048 columns whose activation fits in shared memory beside the ring). The items of all jobs
+// (a job's units of 16 rows) lie on one line, weighted by their bytes, and every CTA takes an equal, contiguous piece
+// of it: one CTA loads the activation of one job, seldom of two. With more than one part the results are partial sums,
+// one plane per part, which the next activation conversion (or a small reduce kernel) adds in part order.
+//
+// Pipeline of a CTA: two groups of 8 consumer warps take the units in turn; each group has its own ring of stages
+// (16 rows x one segment, tiled TMA boxes), its own producer warp and its own finalizer warp. Consumer warp w owns the
+// 256-column block w of a segment. A warp copies its rows' packed words into registers and releases the stage before it
+// computes: two stages per CTA are enough to keep HBM busy, which leaves the shared memory to the activation.
+//
+// mma.sync m16n8k16: A = 16 rows x 16 weights as f16, the 8 columns of B = 4 tokens as (hi, lo) f16 pairs, NTG
+// instructions for 4 NTG tokens from the same A registers.
+//   Q4_K : the 6-bit scale of the sub-block goes into A exactly. A masked nibble is, as it stands, the subnormal f16
+//          q 2^-24 (q 2^-20 in the high nibble), and one multiplication by sc 2^10 (sc 2^6) makes it the f16 number
+//          q sc 2^-14 (q sc <= 945 has 10 bits; 2^14 goes onto d). A block's 256 columns are then one chain of
+//          accumulators and the super-block scale d is applied once; lane column t unpacks the 32-byte chunk t. The mins are
+//          one more instruction: bf16 (min of sub-block k) times the sub-block sums of the activation as three bf16 parts
+//          (24 bits).
+//   Q6_K : (q - 32) sc has 13 bits, so the 16 columns of an instruction are one scale group and its f32 result is
+//          scaled afterwards (both columns of a pair in one packed FMA).
+//   Q8_0 : the same with two instructions per 32-column block and the block's f16 scale.
+// Products are exact, sums f32 in a fixed order (warps, then parts): results are reproducible run to run.
+//
+// What bounds it (B200, 148 SMs): a super-block of 16 rows x 256 columns has to be done in about 100 cycles (Q4_K) to
+// keep up with HBM. Tensor pipe: 34 / 66 instructions of 2 cycles per SM for 8 / 16 tokens; shared memory: 8 / 16 KB of
+// B per super-block at 128 bytes a cycle; issue: about 400 instructions over four schedulers, which is the bound.
+//
+// The activations are converted once per call, by a small kernel of their own, into exactly the register image of the
+// B operand; the conversion also adds partial sums and a residual, takes SiLU(x) * x2, multiplies by a norm weight (the
+// 1 / rms goes onto the results) or adds up the splits of an attention. For the experts of a mixture-of-experts block the
+// columns of a job are a device-side list (expert, column count, place of its image): an expert nobody chose costs nothing.
 #include "common.cuh"
 #include "kernels.h"
+
+#include <cuda_bf16.h>
 
 #include <algorithm>
 #include <cstdlib>
@@ -36,24 +48,42 @@ namespace flb {
 
 namespace {
 
-constexpr int kCW = 8;
-constexpr uint32_t kSeg4 = 8 * 144, kSeg6 = 8 * 210;
-// A stage arrives as one tiled TMA box of 16 rows x the segment, so the row pitch in shared memory is the segment's
-// size. Q6_K: 420 words = 4 mod 32: the 32-bit loads of lanes (g, t) are conflict free as they are. Q4_K: 288 words =
-// 0 mod 32: the rows are fetched as lines of 128 bytes with the 128-byte swizzle (tensor_map_lines_swz), which
-// spreads the same 16-byte chunk of 8 consecutive rows over 8 bank groups; rows whose pitch in memory is not a
-// multiple of 128 bytes (columns not a multiple of 2048) use the plain box and pay the conflicts.
-constexpr uint32_t kPitch4 = kSeg4, kPitch6 = kSeg6;
+constexpr int kCW = 8;                                   // consumer warps per group: one per 256-column block of a segment
+constexpr uint32_t kConsumers = 2 * kCW;
+constexpr uint32_t kThreads = (kConsumers + 4) * 32;     // + two producers, two finalizers
+constexpr uint32_t kSeg4 = 8 * 144, kSeg6 = 8 * 210, kSeg8 = 64 * 34;
+// Row pitch of a stage in shared memory. Q6_K: 420 words = 4 mod 32, conflict free for lanes (g, t) as it is. Q4_K: 288
+// words = 0 mod 32: fetched as 128-byte lines with the 128-byte swizzle (tensor_map_lines_swz), which spreads the same
+// 16-byte chunk of 8 consecutive rows over 8 bank groups; rows whose pitch in memory is no multiple of 128 bytes
+// (columns no multiple of 2048) use the plain box and pay the conflicts. Q8_0: a segment is wider than a box may be, so
+// a stage is two boxes of half a segment, each 16 bytes wider than its half: 276 words = 20 mod 32.
+constexpr uint32_t kPitch4 = kSeg4, kPitch6 = kSeg6, kPitch8 = kSeg8 / 2 + 16;
 constexpr uint32_t slot_round(uint32_t b) { return (b + 1023u) & ~1023u; }   // the swizzle pattern is tied to the address
-constexpr uint32_t kSlot4 = slot_round(16 * kPitch4), kSlot6 = slot_round(16 * kPitch6);
-constexpr uint32_t kFragBytes = 4096;                    // B fragments of one (block, token group)
-constexpr uint32_t kXqBlk = kFragBytes + 128 + 16;       // + sub-block sums [4 tokens][8] + block scales [4]
-constexpr uint32_t kMaxChunkBlks = 16;                   // blocks of activation resident at a time, at most
-constexpr uint32_t kMaxChunkUnits = 16;                  // units per CTA when the columns span several chunks
+constexpr uint32_t kSlot4 = slot_round(16 * kPitch4), kSlot6 = slot_round(16 * kPitch6), kSlot8 = slot_round(32 * kPitch8);
+// Image of one 256-column block of a group of four tokens: B fragments, Q4_K: the B operand of the mins, then the
+// tokens' power-of-two block scales and the block's sums of squares (RMSNorm).
+constexpr uint32_t kFragBytes = 4096, kMinBytes = 256;
+constexpr uint32_t kXq4 = kFragBytes + kMinBytes + 32, kXq6 = kFragBytes + 32;
+__host__ __device__ constexpr uint32_t xq_bytes(int fmt) { return fmt == FMT_Q4_K ? kXq4 : kXq6; }
+__host__ __device__ constexpr uint32_t seg_bytes(int fmt) { return fmt == FMT_Q4_K ? kSeg4 : fmt == FMT_Q6_K ? kSeg6 : kSeg8; }
+__host__ __device__ constexpr uint32_t slot_of(int fmt) { return fmt == FMT_Q4_K ? kSlot4 : fmt == FMT_Q6_K ? kSlot6 : kSlot8; }
+constexpr uint32_t kSmemLimit = 227 * 1024;
+// Shared memory in front: barriers at fixed offsets (full / empty: [2 groups][kMaxSlots]), the CTA's list of pieces, red
+// = [2 groups][8 warps][4 NTG tokens][16 rows] f32, the activation, the rings.
+constexpr uint32_t kMaxSlots = 12;                       // stages per group
+constexpr uint32_t kFull = 0, kEmpty = kFull + 2 * kMaxSlots * 8, kRedFull = kEmpty + 2 * kMaxSlots * 8, kRedEmpty = kRedFull + 16,
+                   kXFull = kRedEmpty + 16, kXEmpty = kXFull + 8, kPieces = 512, kBarBytes = 1536;
+constexpr uint32_t kMaxPieces = (kBarBytes - kPieces) / 16 - 1;   // word kPieces: their number, the stages per group, the ring's offset; 16 bytes each behind it
+static_assert(kXEmpty + 8 <= kPieces, "barriers");
 
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
     return v;
 }
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
@@ -66,13 +96,30 @@ __device__ __forceinline__ uint32_t lds16(uint32_t addr) {
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
     return v;
 }
-__device__ __forceinline__ float ldsf(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-    return v;
+__device__ __forceinline__ float ldsf(uint32_t addr) { return __uint_as_float(lds32(addr)); }
+__device__ __forceinline__ void sts32(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+__device__ __forceinline__ uint64_t *bar_at(uint32_t addr) { return reinterpret_cast<uint64_t *>(__cvta_shared_to_generic(addr)); }
+__device__ __forceinline__ void bar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, uint32_t *status) {
+    return bar_try(bar, parity) || mbar_wait_bounded(bar_at(bar), parity, status);
+}
+// A warp whose wait ran out once waits for nothing any more (its results are void, the status word says so).
+__device__ __forceinline__ void bar_wait_or_die(uint32_t bar, uint32_t parity, uint32_t *status, bool &dead) {
+    if (dead || bar_try(bar, parity)) return;
+    dead = !mbar_wait_bounded(bar_at(bar), parity, status);
 }
 __device__ __forceinline__ void tma_box2(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint64_t *bar) {
     asm volatile(
@@ -86,9 +133,9 @@ __device__ __forceinline__ void tma_box3(uint32_t dst, const CUtensorMap *map, u
         "l"(map), "r"(0), "r"(line), "r"(row), "r"(smem_u32(bar))
         : "memory");
 }
-// Byte offset o of a Q4_K row as the stage holds it: as it is, or in the swizzled 128-byte lines.
+// Byte offset o (a multiple of 16) of a Q4_K row as the stage holds it: as it is, or in the swizzled 128-byte lines.
 __device__ __forceinline__ uint32_t q4_row_off(uint32_t o, uint32_t g, bool swz) {
-    return swz ? (o & ~127u) + ((((o >> 4) ^ (g + (o >> 7))) & 7u) << 4) + (o & 15u) : o;
+    return swz ? (o & ~127u) + ((((o >> 4) ^ (g + (o >> 7))) & 7u) << 4) : o;
 }
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
@@ -96,246 +143,366 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
+__device__ __forceinline__ void mma16816_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                              uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ uint32_t hsub2_u32(uint32_t h, __half2 off) {
-    const __half2 r = __hsub2(*reinterpret_cast<const __half2 *>(&h), off);
-    return *reinterpret_cast<const uint32_t *>(&r);
+__device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
+__device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
+__device__ __forceinline__ uint32_t hsub2_u32(uint32_t h, __half2 off) { return as_u32(__hsub2(as_h2(h), off)); }
+__device__ __forceinline__ uint32_t hmul2_u32(uint32_t h, __half2 m) { return as_u32(__hmul2(as_h2(h), m)); }
+// (c.x, c.y) += s * (a, b): both columns of a token in one packed FMA
+__device__ __forceinline__ void fma_pair(float2 &c, float s, float a, float b) {
+    uint64_t cc = *reinterpret_cast<uint64_t *>(&c), ss, ab;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(ss) : "f"(s));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(ab) : "f"(a), "f"(b));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(cc) : "l"(ss), "l"(ab));
+    c = *reinterpret_cast<float2 *>(&cc);
 }
-template <int K>
-__device__ __forceinline__ float u8f(uint32_t w) {
-    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650u | K)) - 8388608.0f;
-}
-__device__ __noinline__ bool mbar_wait_slow(uint64_t *bar, uint32_t parity, uint32_t *status) {
-    return mbar_wait_bounded(bar, parity, status);
-}
-// A warp whose wait ran out once waits for nothing any more (its results are void, the status word says so).
-__device__ __forceinline__ void mbar_wait_or_die(uint64_t *bar, uint32_t parity, uint32_t *status, bool &dead) {
-    if (dead || mbar_try_wait(bar, parity)) return;
-    dead = !mbar_wait_slow(bar, parity, status);
+// byte K of w, which holds s + 128, as the float s (the byte under 0x4B000000 is 2^23 + 128 + s)
+__device__ __forceinline__ float s8f(uint32_t w, int k) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + k)) - 8388736.f;
 }
 
 // ---- activations -> the B operand's register image ----------------------------------------------------------
-// Combo m of a block = one tensor-core instruction's 16 columns. Q4_K: m = column / 16 (chunk c, nibble kind,
-// half of the sub-block). Q6_K: m = ((hf * 2 + hq) * 4 + gq) for columns 128 hf + 32 gq + 16 hq + [0, 16).
-// Within a combo lane column t' holds columns 4 t' + {0, 2} (register b0) and 4 t' + {1, 3} (register b1); lane
-// = 4 * (2 p' + h) + t' for token p' of the group and part h (0 = hi, 1 = lo). Byte offset in the fragment
-// image: (m / 2) * 512 + lane * 16 + (m & 1) * 8, so that a lane's 128-bit load fetches two combos and a warp's
-// load is one contiguous 512 bytes.
-// grid (nblk, ntg), 64 threads: half-warp p' converts the block's 256 columns of token 4 tg + p'.
-// Column p of the call is row col_idx[col_off + p] of x (col_idx == nullptr: row p); columns at or past *cnt - col_off
-// (cnt == nullptr: P) are zeros. x2 != nullptr: the value is SiLU(x) * x2 (fl_op_silu_mul, src/runtime/decode_params.h:267-272).
-__global__ void __launch_bounds__(64) act_convert_nx_kernel(const float *__restrict__ x, const float *__restrict__ x2, uint32_t xstride,
-                                                            uint32_t P, int fmt, uint8_t *__restrict__ xq, uint32_t ntg,
-                                                            const uint32_t *__restrict__ cnt, uint32_t col_off,
-                                                            const uint32_t *__restrict__ col_idx) {
-    const uint32_t blk = blockIdx.x, tg = blockIdx.y;
-    const uint32_t pp = threadIdx.x >> 4, hl = threadIdx.x & 15u, p = 4 * tg + pp;
-    // launched as a programmatic dependent: the launch itself overlaps the tail of the kernel before, whose output
-    // (x, the column list) is read only after it has completed
-    griddep_launch_dependents();
-    griddep_wait();
-    uint32_t n_valid = P;
-    if (cnt) { const uint32_t c = *cnt; n_valid = c > col_off ? min(c - col_off, P) : 0u; }
-    if (n_valid == 0) return;   // the matmul of this call returns at entry too
-    float v[16];
-    if (p < n_valid) {
-        const size_t row = col_idx ? col_idx[col_off + p] : p;
-        const float4 *src = reinterpret_cast<const float4 *>(x + row * xstride + blk * 256 + hl * 16);
+// An image is [block][token group][xq_bytes]: B fragments of 8 pieces x 32 lanes x 16 bytes, lane = 4 n + t' for column
+// n = 2 p' + part (token p' of the group, part 0 = hi, 1 = lo) and lane column t'; a lane's 16 bytes are (b0, b1) of two
+// instructions, b0 = columns c + {0, 2}, b1 = c + {1, 3} of its four consecutive columns c ..:
+//   Q4_K  piece j    : c = 64 t' + 4 j (low nibbles of word j of chunk t'), then c = 64 t' + 32 + 4 j (high nibbles)
+//   Q6_K  piece m / 2: half m & 1, m = (2 hf + hq) * 4 + gq the scale group: c = 128 hf + 32 gq + 16 hq + 4 t'
+//   Q8_0  piece b    : c = 32 b + 8 t' + {0, 4}
+// Q4_K, then: (b0, b1) per lane of the mins' instruction: b0 = part h of the sums of sub-blocks 2 t', 2 t' + 1, b1 = the
+// third part (columns of the hi part) or zero. Then four block scales, four sums of squares.
+struct ConvArgs {
+    const float *x, *x2;           // column p: row p (or the listed row) of x; x2: the value is SiLU(x) * x2
+    size_t part_stride;            // n_parts planes of x (and x2), added in order
+    const float *resid;            // + resid (row p, rstride apart)
+    float *x_out;                  // the sum is also stored here (row p, rstride apart; may be resid)
+    const float *wnorm;            // the value is multiplied by wnorm, the sum of squares of the block recorded
+    uint32_t xstride, rstride, n_parts, P, nblk;
+    uint8_t *img4, *img6, *img8;   // images wanted (nullptr: not)
+    const uint32_t *table, *col_idx;   // grouped columns (see below)
+    uint32_t list_stride, col_off;
+    const float *att;              // the columns are attention contexts of heads of 128, added up here from n_splits records
+    uint32_t n_splits;             // (attn.cu: [column][head][split][132] = context, maximum, sum)
+};
+// Device-side table of a grouped launch: word 0 = number of active groups, word 1 = the most token groups of one; then four
+// words per active group: {group, number of columns, token groups in front of it, 0}.
+
+// Four consecutive columns at p, the planes added in order; all of them are requested before the first is used.
+__device__ __forceinline__ float4 sum_planes(const float *p, uint32_t n, size_t stride) {
+    constexpr int kPlanes = (kNxMaxCols / 256 + 7) / 8;   // the most parts a matmul leaves
+    float4 v[kPlanes];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float4 u = src[k];
-            v[4 * k] = u.x; v[4 * k + 1] = u.y; v[4 * k + 2] = u.z; v[4 * k + 3] = u.w;
-        }
-        if (x2) {
-            const float4 *src2 = reinterpret_cast<const float4 *>(x2 + row * xstride + blk * 256 + hl * 16);
+    for (int s = 0; s < kPlanes; ++s) v[s] = (uint32_t)s < n ? *reinterpret_cast<const float4 *>(p + s * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float4 u = src2[k];
-                v[4 * k] = (v[4 * k] / (1.0f + expf(-v[4 * k]))) * u.x;
-                v[4 * k + 1] = (v[4 * k + 1] / (1.0f + expf(-v[4 * k + 1]))) * u.y;
-                v[4 * k + 2] = (v[4 * k + 2] / (1.0f + expf(-v[4 * k + 2]))) * u.z;
-                v[4 * k + 3] = (v[4 * k + 3] / (1.0f + expf(-v[4 * k + 3]))) * u.w;
-            }
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = 0.f;
-    }
-    float amax = 0.f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    int e = (int)((__float_as_uint(amax) >> 23) & 0xFFu) - 127 - 13;
-    e = amax > 0.f ? max(-126, min(e, 114)) : 0;
-    const float inv_s = __uint_as_float((uint32_t)(127 - e) << 23);
-    uint8_t *base = xq + ((size_t)blk * ntg + tg) * kXqBlk;
-    uint32_t m;
-    if (fmt == FMT_Q4_K) m = hl;
-    else m = (((hl >> 3) * 2 + (hl & 1u)) * 4) + ((hl >> 1) & 3u);
-    float sum = 0.f;
-#pragma unroll
-    for (int tq = 0; tq < 4; ++tq) {
-        __half hh[4], ll[4];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const float s = v[4 * tq + b] * inv_s;
-            hh[b] = __float2half_rn(s);
-            ll[b] = __float2half_rn(s - __half2float(hh[b]));
-            sum += __half2float(hh[b]) + __half2float(ll[b]);
-        }
-        const uint32_t off = (m >> 1) * 512u + (m & 1u) * 8u + tq * 16u;
-        uint2 hi, lo;
-        hi.x = (uint32_t)__half_as_ushort(hh[0]) | ((uint32_t)__half_as_ushort(hh[2]) << 16);
-        hi.y = (uint32_t)__half_as_ushort(hh[1]) | ((uint32_t)__half_as_ushort(hh[3]) << 16);
-        lo.x = (uint32_t)__half_as_ushort(ll[0]) | ((uint32_t)__half_as_ushort(ll[2]) << 16);
-        lo.y = (uint32_t)__half_as_ushort(ll[1]) | ((uint32_t)__half_as_ushort(ll[3]) << 16);
-        *reinterpret_cast<uint2 *>(base + off + (4 * (2 * pp)) * 16u) = hi;        // lane = 4 * (2 p' + 0) + tq
-        *reinterpret_cast<uint2 *>(base + off + (4 * (2 * pp + 1)) * 16u) = lo;    // lane = 4 * (2 p' + 1) + tq
-    }
-    const float sum32 = sum + __shfl_xor_sync(0xffffffffu, sum, 1);
-    if ((hl & 1u) == 0) reinterpret_cast<float *>(base + kFragBytes)[pp * 8 + (hl >> 1)] = sum32;   // [token][sub-block]
-    if (hl == 0) reinterpret_cast<float *>(base + kFragBytes + 128)[pp] = __uint_as_float((uint32_t)(127 + e) << 23);
+    for (int s = 1; s < kPlanes; ++s) { v[0].x += v[s].x; v[0].y += v[s].y; v[0].z += v[s].z; v[0].w += v[s].w; }
+    return v[0];
 }
 
-struct NxArgs {
-    CUtensorMap map;               // the tiled view a stage's box is cut from
-    const uint32_t *cnt;           // optional: number of listed columns on the device
-    const uint32_t *out_idx;       // optional: output row block (in units of ystride) of listed column col_off + p
-    uint32_t col_off, swz;
-    const uint8_t *w;
-    const uint8_t *xq;
+// Four dimensions (4 lane ..) of one head's context from its splits' records (attn_decode_kernel's combine, with all lanes of
+// a warp on one head): the weights from every split's maximum and sum, then the contexts in split order, 16 in flight.
+__device__ __forceinline__ float4 combine_records(const float *part, uint32_t S, uint32_t lane) {
+    const float m0 = lane < S ? __ldcg(part + (size_t)lane * kAttnRecord + 128) : -INFINITY;
+    const float m1 = lane + 32 < S ? __ldcg(part + (size_t)(lane + 32) * kAttnRecord + 128) : -INFINITY;
+    const float l0 = lane < S ? __ldcg(part + (size_t)lane * kAttnRecord + 129) : 0.f;
+    const float l1 = lane + 32 < S ? __ldcg(part + (size_t)(lane + 32) * kAttnRecord + 129) : 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float w0 = 0.f, w1 = 0.f, L = 1.f;
+#pragma unroll 1
+    for (uint32_t s0 = 0; s0 < S; s0 += 16) {
+        float4 ov[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            ov[j] = s0 + j < S ? __ldcg(reinterpret_cast<const float4 *>(part + (size_t)(s0 + j) * kAttnRecord) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s0 == 0) {   // the first contexts are on their way meanwhile
+            const float mx = warp_max(fmaxf(m0, m1));
+            w0 = m0 == -INFINITY ? 0.f : expf(m0 - mx);
+            w1 = m1 == -INFINITY ? 0.f : expf(m1 - mx);
+            L = warp_sum(l0 * w0 + l1 * w1);
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const float w = __shfl_sync(0xffffffffu, s0 < 32 ? w0 : w1, (s0 + j) & 31u);
+            acc.x = fmaf(ov[j].x, w, acc.x); acc.y = fmaf(ov[j].y, w, acc.y);
+            acc.z = fmaf(ov[j].z, w, acc.z); acc.w = fmaf(ov[j].w, w, acc.w);
+        }
+    }
+    const float inv = 1.0f / L;
+    return make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+}
+
+// grid (blocks, columns rounded up to groups of four, groups), 64 threads: a block converts 256 values of one column, a thread
+// four consecutive ones. What bounds it is latency (a launch moves well under a megabyte): hence few values per thread, every
+// plane in flight, and as many blocks as there are (block, column) pairs.
+__global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
+    __shared__ float2 half_s[2];   // per warp: maximum, sum of squares
+    const uint32_t blk = blockIdx.x, warp = threadIdx.x >> 5;
+    const uint32_t pp = blockIdx.y & 3u, i = threadIdx.x, hl = i >> 2, tq = i & 3u;   // column of the group; values 16 hl + 4 tq ..
+    // launched as a programmatic dependent: the launch itself overlaps the tail of the kernel before, whose output
+    // (x, the table) is read only after it has completed
+    griddep_launch_dependents();
+    float4 wn = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (a.wnorm) wn = __ldg(reinterpret_cast<const float4 *>(a.wnorm + blk * 256 + 4 * i));   // a constant
+    griddep_wait();
+    uint32_t n_valid = a.P, tg = blockIdx.y >> 2, ntg = (a.P + 3) / 4, tg0 = 0, grp = 0;
+    if (a.table) {
+        if (blockIdx.z >= a.table[0]) return;
+        const uint4 e = reinterpret_cast<const uint4 *>(a.table)[1 + blockIdx.z];
+        grp = e.x; n_valid = e.y; tg0 = e.z;
+        ntg = (n_valid + 3) / 4;
+        if (tg >= ntg) return;
+    }
+    const uint32_t p = 4 * tg + pp;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    float ss = 0.f;
+    if (p < n_valid) {
+        const size_t row = a.table ? a.col_idx[(size_t)grp * a.list_stride + a.col_off + p] : p;
+        const size_t at = row * a.xstride + blk * 256 + 4 * i, rat = (size_t)p * a.rstride + blk * 256 + 4 * i;
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (a.resid) r = *reinterpret_cast<const float4 *>(a.resid + rat);
+        if (a.att) v = combine_records(a.att + ((size_t)p * (2 * a.nblk) + 2 * blk + warp) * a.n_splits * kAttnRecord, a.n_splits, threadIdx.x & 31u);
+        else v = sum_planes(a.x + at, a.n_parts, a.part_stride);
+        if (a.x2) {   // fl_op_silu_mul (src/runtime/decode_params.h:267-272)
+            const float4 u = sum_planes(a.x2 + at, a.n_parts, a.part_stride);
+            v.x = (v.x / (1.0f + expf(-v.x))) * u.x; v.y = (v.y / (1.0f + expf(-v.y))) * u.y;
+            v.z = (v.z / (1.0f + expf(-v.z))) * u.z; v.w = (v.w / (1.0f + expf(-v.w))) * u.w;
+        }
+        if (a.resid) { v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w; }
+        if (a.x_out) *reinterpret_cast<float4 *>(a.x_out + rat) = v;
+        if (a.wnorm) {
+            ss = (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+            v.x *= wn.x; v.y *= wn.y; v.z *= wn.z; v.w *= wn.w;
+        }
+    }
+    if (!a.img4 && !a.img6 && !a.img8) return;   // only the sum was asked for
+    float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+    amax = warp_max(amax);
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31u) == 0) half_s[warp] = make_float2(amax, ss);
+    __syncthreads();
+    const float2 h0 = half_s[0], h1 = half_s[1];
+    amax = fmaxf(h0.x, h1.x);
+    // block scale 2^e with amax / 2^e in [2^13, 2^14); e clamped so that both 2^e and 2^-e are normal floats
+    int e = (int)((__float_as_uint(amax) >> 23) & 0xFFu) - 127 - 13;
+    e = amax > 0.f ? max(-126, min(e, 114)) : 0;
+    const float inv_s = __uint_as_float((uint32_t)(127 - e) << 23), scale = __uint_as_float((uint32_t)(127 + e) << 23);
+    const float s0 = v.x * inv_s, s1 = v.y * inv_s, s2 = v.z * inv_s, s3 = v.w * inv_s;
+    const __half2 h02 = __floats2half2_rn(s0, s2), h13 = __floats2half2_rn(s1, s3);
+    const float2 f02 = __half22float2(h02), f13 = __half22float2(h13);
+    const __half2 l02 = __floats2half2_rn(s0 - f02.x, s2 - f02.y), l13 = __floats2half2_rn(s1 - f13.x, s3 - f13.y);
+    const float2 g02 = __half22float2(l02), g13 = __half22float2(l13);
+    const uint2 hi = make_uint2(as_u32(h02), as_u32(h13)), lo = make_uint2(as_u32(l02), as_u32(l13));
+    float sum = ((f02.x + g02.x) + (f13.x + g13.x)) + ((f02.y + g02.y) + (f13.y + g13.y));
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);   // over the 32-column sub-block
+    const size_t unit = (size_t)tg0 * a.nblk + (size_t)blk * ntg + tg;
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+        uint8_t *base = f == 0 ? a.img4 : f == 1 ? a.img6 : a.img8;
+        if (!base) continue;
+        base += unit * (f == 0 ? kXq4 : kXq6);
+        uint32_t off, t;   // byte offset but for the lane, lane column
+        if (f == 0) {
+            off = (4 * (hl & 1u) + tq) * 512u + ((hl >> 1) & 1u) * 8u; t = hl >> 2;
+        } else if (f == 1) {
+            const uint32_t m = (((hl >> 3) * 2 + (hl & 1u)) * 4) + ((hl >> 1) & 3u);
+            off = (m >> 1) * 512u + (m & 1u) * 8u; t = tq;
+        } else {
+            off = (hl >> 1) * 512u + (tq & 1) * 8u; t = 2 * (hl & 1u) + (tq >> 1);
+        }
+        *reinterpret_cast<uint2 *>(base + off + (4 * (2 * pp) + t) * 16u) = hi;
+        *reinterpret_cast<uint2 *>(base + off + (4 * (2 * pp + 1) + t) * 16u) = lo;
+        uint8_t *tail = base + kFragBytes;
+        if (f == 0) {
+            if ((i & 7u) == 0) {   // the sum of sub-block sb in three bf16 parts (exact: 24 bits)
+                const uint32_t sb = i >> 3;
+                const __nv_bfloat16 p0 = __float2bfloat16_rn(sum);
+                const float r1 = sum - __bfloat162float(p0);
+                const __nv_bfloat16 p1 = __float2bfloat16_rn(r1);
+                const __nv_bfloat16 p2 = __float2bfloat16_rn(r1 - __bfloat162float(p1));
+                uint8_t *d0 = tail + (4 * (2 * pp) + (sb >> 1)) * 8u + (sb & 1u) * 2u;
+                uint8_t *d1 = tail + (4 * (2 * pp + 1) + (sb >> 1)) * 8u + (sb & 1u) * 2u;
+                *reinterpret_cast<__nv_bfloat16 *>(d0) = p0;
+                *reinterpret_cast<__nv_bfloat16 *>(d0 + 4) = p2;
+                *reinterpret_cast<__nv_bfloat16 *>(d1) = p1;
+                *reinterpret_cast<uint16_t *>(d1 + 4) = 0;
+            }
+            tail += kMinBytes;
+        }
+        if (i == 0) {
+            reinterpret_cast<float *>(tail)[pp] = scale;
+            reinterpret_cast<float *>(tail)[4 + pp] = h0.y + h1.y;
+        }
+    }
+}
+
+// y[p][r] (+)= sum over the parts of part[s][p][r]
+__global__ void __launch_bounds__(256) reduce_parts_kernel(const float *__restrict__ part, size_t part_stride, uint32_t n_parts,
+                                                           float *y, uint32_t rows, uint32_t ystride, int accumulate) {
+    griddep_launch_dependents();
+    griddep_wait();
+    const uint32_t r = blockIdx.x * 256 + threadIdx.x, p = blockIdx.y;
+    if (r >= rows) return;
+    float v = 0.f;
+#pragma unroll 4
+    for (uint32_t s = 0; s < n_parts; ++s) v += part[s * part_stride + (size_t)p * rows + r];
+    float *dst = y + (size_t)p * ystride + r;
+    *dst = accumulate ? *dst + v : v;
+}
+
+struct NxT {
     float *y;
-    uint32_t rows, pitch, cols, ystride, P, ntg;
-    int fmt, accumulate;
-    uint32_t nslots, slot_bytes, ring_off, x_off, uacc_off, chunk_blks;   // chunk_blks: 8 or 16 blocks of activation resident at a time
+    size_t part_stride;            // floats between the planes of the parts
+    uint32_t rows, ystride, units, xoff;   // xoff: bytes from xq to the image of this format
+    int fmt, swz;
+};
+struct NxJob { uint32_t base, cost; uint16_t tensor, part, seg0, nseg; };   // base: where the job starts on the line of a group
+constexpr int kMaxJobs = 32;
+
+struct NxArgs {
+    CUtensorMap map[3];            // the tiled views a stage's boxes are cut from
+    NxT t[3];
+    NxJob job[kMaxJobs];
+    uint32_t n_jobs, group_cost, nblk, P;
+    const uint8_t *xq;
+    int accumulate, rms;
+    float eps;
+    uint32_t slot_bytes, x_off, x_blk_tg;   // x_blk_tg: bytes of a part's activation per token group
+    uint32_t red_group;            // floats between the groups' reduction buffers (for the widest piece of the launch)
+    // grouped launches: active groups from the table, output rows from the list
+    const uint32_t *table, *out_idx;
+    uint32_t list_stride, col_off;
+    int table_ready;               // the table was complete before the previous kernel started
     uint32_t *status;
 };
 
-__host__ __device__ inline size_t nx_head_bytes(uint32_t nslots, int groups) {
-    size_t n = (size_t)nslots * 16 + 64;                     // stage barriers; reduction barriers; activation barriers
-    n += (size_t)2 * groups * kCW * 128 * 4;                // red [2][warps][16 rows][8 tokens]
-    return (n + 127) & ~(size_t)127;
+__host__ __device__ constexpr uint32_t nx_ring_off(uint32_t x_off, uint32_t x_blk_tg, uint32_t ntg) {
+    return (x_off + x_blk_tg * ntg + 1023u) & ~1023u;
 }
 
-// ---- per-block math: rows g (r0) and g + 8 (r1), tokens t and t + 4 -----------------------------------------
-// out[row][tg] in units of the tokens' block scales.
-// r0: row g of the stage (row g + 8 is 8 pitches further: the same swizzle, 72 lines on); ow[c][i]: offset in the row
-// of word 4 i + t of chunk c of this warp's block, oh: of the block's header (q4_row_off).
-template <int NTG>
-__device__ __forceinline__ void q4k_block_nx(uint32_t r0, const uint32_t (&ow)[4][2], uint32_t oh, uint32_t t, uint32_t xaddr,
-                                             uint32_t lane, float (&out)[2][NTG]) {
-    const uint32_t r1 = r0 + 8 * kPitch4;
-    // all loads first
-    uint32_t w0[4][2], w1[4][2];
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            w0[c][i] = lds32(r0 + ow[c][i]);
-            w1[c][i] = lds32(r1 + ow[c][i]);
+// The pieces of this CTA, listed in shared memory by one thread at the start: {first unit, last unit, job | columns << 8 |
+// group << 16, token groups in front << 2 | same activation as the piece before << 1 | parity of the units before}.
+struct NxPiece { uint32_t u0, u1, job, n_valid, grp, tg0, same, par; };
+__device__ __forceinline__ NxPiece nx_piece(uint32_t smem, uint32_t i) {
+    const uint4 v = lds128(smem + kPieces + 16 + 16 * i);
+    return NxPiece{v.x, v.y, v.z & 0xFFu, (v.z >> 8) & 0xFFu, v.z >> 16, v.w >> 2, (v.w >> 1) & 1u, v.w & 1u};
+}
+__device__ __noinline__ void nx_list_pieces(const NxArgs &a, uint8_t *smem_raw) {
+    uint32_t *count = reinterpret_cast<uint32_t *>(smem_raw + kPieces);
+    uint4 *out = reinterpret_cast<uint4 *>(smem_raw + kPieces + 16);
+    uint32_t n = 0, kk = 0, last_g = 0, last_part = 0, last_x = 0;
+    const uint32_t n_act = a.table ? a.table[0] : 1u;
+    // the activation region is as large as the widest piece of this launch needs (grouped: known here only), the ring has the rest
+    const uint32_t ring_off = nx_ring_off(a.x_off, a.x_blk_tg, a.table ? a.table[1] : (a.P + 3) / 4);
+    count[1] = min((kSmemLimit - ring_off) / (2 * a.slot_bytes), kMaxSlots);
+    count[2] = ring_off;
+    const uint32_t W = a.group_cost * n_act;   // < 2^31 (checked on the host)
+    const uint32_t lo = (uint32_t)((uint64_t)W * blockIdx.x / gridDim.x), hi = (uint32_t)((uint64_t)W * (blockIdx.x + 1) / gridDim.x);
+    for (uint32_t g = lo / a.group_cost; g < n_act && g * a.group_cost < hi; ++g) {
+        uint4 e = make_uint4(0u, a.P, 0u, 0u);
+        if (a.table) e = reinterpret_cast<const uint4 *>(a.table)[1 + g];
+        for (uint32_t j = 0; j < a.n_jobs && n < kMaxPieces; ++j) {
+            const NxJob &jb = a.job[j];
+            const uint32_t units = a.t[jb.tensor].units, b = g * a.group_cost + jb.base, end = b + units * jb.cost;
+            if (end <= lo || b >= hi) continue;
+            const uint32_t u0 = b >= lo ? 0u : (lo - b + jb.cost - 1) / jb.cost;
+            const uint32_t u1 = end <= hi ? units : (hi - b + jb.cost - 1) / jb.cost;
+            if (u0 >= u1) continue;
+            const uint32_t same = n > 0 && last_g == g && last_part == jb.part && last_x == a.t[jb.tensor].xoff ? 1u : 0u;
+            last_g = g; last_part = jb.part; last_x = a.t[jb.tensor].xoff;
+            out[n++] = make_uint4(u0, u1, j | (e.y << 8) | (e.x << 16), (e.z << 2) | (same << 1) | (kk & 1u));
+            kk += u1 - u0;
         }
-    const uint4 h0 = lds128(r0 + oh), h1 = lds128(r1 + oh);
-    float sums[NTG][8];   // sub-block sums of token t (+ 4 tg)
+    }
+    *count = n;
+}
+
+// ---- per-block math: rows g (row 0) and g + 8 (row 1), tokens 4 tg + t ---------------------------------------------
+// acc[row][tg] += the block's contribution. `release` runs after the last read of the stage. offs: where the block's
+// header and the two halves of chunk t lie in a row, in 16 bytes, one byte each.
+template <int NTG, typename Rel>
+__device__ __forceinline__ void q4k_block_nx(uint32_t r0, uint32_t offs, uint32_t t, uint32_t xaddr, uint32_t lane, float (&acc)[2][NTG],
+                                             Rel &&release) {
+    const uint32_t r1 = r0 + 8 * kPitch4, oh = (offs & 0xFFu) * 16u, oa = ((offs >> 8) & 0xFFu) * 16u, ob = (offs >> 16) * 16u;
+    uint4 wa[2], wb[2], hd[2];
+    wa[0] = lds128(r0 + oa); wa[1] = lds128(r1 + oa);
+    hd[0] = lds128(r0 + oh); hd[1] = lds128(r1 + oh);
+    wb[0] = lds128(r0 + ob); wb[1] = lds128(r1 + ob);
+    release();
+    // 6-bit scales / mins of sub-blocks 2t, 2t+1 (packing: fl_q4k_scale_min, src/runtime/quants.h:121-129): sub-blocks
+    // 0..3 are the low six bits of bytes 0..3 (4..7 for the mins), 4..7 a nibble of bytes 8..11 under the top two bits of those
+    const uint32_t sh = 16u * (t & 1u);
+    const uint32_t shA = t >= 2 ? sh + 2u : sh, mA = t >= 2 ? 0x3030u : 0x3F3Fu, mE = t >= 2 ? 0x0F0Fu : 0u;
+    __half2 sL[2], sH[2];   // scales times 2^10 (low nibbles), 2^6 (high nibbles)
+    uint32_t am[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const uint32_t sc = ((hd[r].y >> shA) & mA) | ((hd[r].w >> sh) & mE);
+        const uint32_t mn = ((hd[r].z >> shA) & mA) | ((hd[r].w >> (sh + 4u)) & mE);
+        const __half2 k1024 = __floats2half2_rn(1024.f, 1024.f);
+        sL[r] = __hmul2(__hsub2(as_h2(__byte_perm(sc, 0x64646464u, 0x4040u)), k1024), k1024);
+        sH[r] = __hmul2(__hsub2(as_h2(__byte_perm(sc, 0x64646464u, 0x4141u)), k1024), __floats2half2_rn(64.f, 64.f));
+        // mins as bf16 (0x4300 | b is 128 + b)
+        const uint32_t mb = __byte_perm(mn, 0x43434343u, 0x4140u);
+        const __nv_bfloat162 m2 = __hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&mb), __floats2bfloat162_rn(128.f, 128.f));
+        am[r] = *reinterpret_cast<const uint32_t *>(&m2);
+    }
+    // up to 8 tokens: one accumulator chain per nibble kind (8 dependent instructions each), else one chain
+    constexpr int kChains = NTG <= 2 ? 2 : 1;
+    float c[kChains][NTG][4];
+#pragma unroll
+    for (int i = 0; i < kChains; ++i)
+#pragma unroll
+        for (int tg = 0; tg < NTG; ++tg) c[i][tg][0] = c[i][tg][1] = c[i][tg][2] = c[i][tg][3] = 0.f;
+    const uint32_t ML = 0x000F000Fu, MH = 0x00F000F0u;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const uint4 &q0 = j < 4 ? wa[0] : wb[0], &q1 = j < 4 ? wa[1] : wb[1];
+        const uint32_t W0 = (j & 3) == 0 ? q0.x : (j & 3) == 1 ? q0.y : (j & 3) == 2 ? q0.z : q0.w;
+        const uint32_t W1 = (j & 3) == 0 ? q1.x : (j & 3) == 1 ? q1.y : (j & 3) == 2 ? q1.z : q1.w;
+        const uint32_t V0 = W0 >> 8, V1 = W1 >> 8;
+        const uint32_t l0 = hmul2_u32(W0 & ML, sL[0]), l1 = hmul2_u32(W1 & ML, sL[1]), l2 = hmul2_u32(V0 & ML, sL[0]), l3 = hmul2_u32(V1 & ML, sL[1]);
+        const uint32_t h0 = hmul2_u32(W0 & MH, sH[0]), h1 = hmul2_u32(W1 & MH, sH[1]), h2 = hmul2_u32(V0 & MH, sH[0]), h3 = hmul2_u32(V1 & MH, sH[1]);
+#pragma unroll
+        for (int tg = 0; tg < NTG; ++tg) {
+            const uint4 b = lds128(xaddr + tg * kXq4 + j * 512 + lane * 16);
+            mma16816(c[0][tg], l0, l1, l2, l3, b.x, b.y);
+            mma16816(c[kChains - 1][tg], h0, h1, h2, h3, b.z, b.w);
+        }
+    }
+    const float d0 = 16384.f * h2f_bits((uint16_t)(hd[0].x & 0xFFFFu)), e0 = h2f_bits((uint16_t)(hd[0].x >> 16));
+    const float d1 = 16384.f * h2f_bits((uint16_t)(hd[1].x & 0xFFFFu)), e1 = h2f_bits((uint16_t)(hd[1].x >> 16));
 #pragma unroll
     for (int tg = 0; tg < NTG; ++tg) {
-        const uint32_t sa = xaddr + tg * kXqBlk + kFragBytes + t * 32;
-        const uint4 s0 = lds128(sa), s1 = lds128(sa + 16);
-        sums[tg][0] = __uint_as_float(s0.x); sums[tg][1] = __uint_as_float(s0.y); sums[tg][2] = __uint_as_float(s0.z); sums[tg][3] = __uint_as_float(s0.w);
-        sums[tg][4] = __uint_as_float(s1.x); sums[tg][5] = __uint_as_float(s1.y); sums[tg][6] = __uint_as_float(s1.z); sums[tg][7] = __uint_as_float(s1.w);
-    }
-    // the eight 6-bit scales and mins of both rows (packing: fl_q4k_scale_min, src/runtime/quants.h:121-129)
-    uint32_t scw[2][2], mnw[2][2];   // [row][sub-blocks 0..3 | 4..7], one byte each
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const uint4 hdr = r ? h1 : h0;
-        scw[r][0] = hdr.y & 0x3F3F3F3Fu;
-        mnw[r][0] = hdr.z & 0x3F3F3F3Fu;
-        scw[r][1] = (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
-        mnw[r][1] = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
-    }
-    float accq[2][NTG], accm[2][NTG];
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int tg = 0; tg < NTG; ++tg) accq[r][tg] = accm[r][tg] = 0.f;
-    // the mins against the sub-block sums first: the sums' registers are free again before the unpacking starts
-#pragma unroll
-    for (int sb = 0; sb < 8; ++sb)
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const uint32_t mw = mnw[r][sb >> 2];
-            const float mnf = (sb & 3) == 0 ? u8f<0>(mw) : (sb & 3) == 1 ? u8f<1>(mw) : (sb & 3) == 2 ? u8f<2>(mw) : u8f<3>(mw);
-#pragma unroll
-            for (int tg = 0; tg < NTG; ++tg) accm[r][tg] = fmaf(mnf, sums[tg][sb], accm[r][tg]);
-        }
-    const uint32_t ML = 0x000F000Fu, KL = 0x64006400u, MH = 0x00F000F0u, KH = 0x54005400u;
-    const __half2 oL = __floats2half2_rn(1024.f, 1024.f), oH = __floats2half2_rn(64.f, 64.f);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        // A registers of the chunk's four instructions: (low nibbles, i = 0, 1), (high nibbles, i = 0, 1)
-        uint32_t aL[2][4], aH[2][4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const uint32_t W0 = w0[c][i], W1 = w1[c][i], V0 = W0 >> 8, V1 = W1 >> 8;
-            aL[i][0] = hsub2_u32(and_or(W0, ML, KL), oL); aL[i][1] = hsub2_u32(and_or(W1, ML, KL), oL);
-            aL[i][2] = hsub2_u32(and_or(V0, ML, KL), oL); aL[i][3] = hsub2_u32(and_or(V1, ML, KL), oL);
-            aH[i][0] = hsub2_u32(and_or(W0, MH, KH), oH); aH[i][1] = hsub2_u32(and_or(W1, MH, KH), oH);
-            aH[i][2] = hsub2_u32(and_or(V0, MH, KH), oH); aH[i][3] = hsub2_u32(and_or(V1, MH, KH), oH);
-        }
-#pragma unroll
-        for (int sub = 0; sub < 2; ++sub) {
-            const int sb = 2 * c + sub;
-            // scale of sub-block sb for both rows, as floats
-            float scf[2];
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const uint32_t sw = scw[r][sb >> 2];
-                scf[r] = (sb & 3) == 0 ? u8f<0>(sw) : (sb & 3) == 1 ? u8f<1>(sw) : (sb & 3) == 2 ? u8f<2>(sw) : u8f<3>(sw);
-            }
-#pragma unroll
-            for (int tg = 0; tg < NTG; ++tg) {
-                // combos m = 2 sb, 2 sb + 1 (i = 0, 1) sit in one 16-byte piece: q = sb
-                const uint4 bx = lds128(xaddr + tg * kXqBlk + sb * 512 + lane * 16);
-                float cc[4] = {0.f, 0.f, 0.f, 0.f};
-                if (sub == 0) {
-                    mma16816(cc, aL[0][0], aL[0][1], aL[0][2], aL[0][3], bx.x, bx.y);
-                    mma16816(cc, aL[1][0], aL[1][1], aL[1][2], aL[1][3], bx.z, bx.w);
-                } else {
-                    mma16816(cc, aH[0][0], aH[0][1], aH[0][2], aH[0][3], bx.x, bx.y);
-                    mma16816(cc, aH[1][0], aH[1][1], aH[1][2], aH[1][3], bx.z, bx.w);
-                }
-                accq[0][tg] = fmaf(scf[0], cc[0] + cc[1], accq[0][tg]);
-                accq[1][tg] = fmaf(scf[1], cc[2] + cc[3], accq[1][tg]);
-            }
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const uint4 hdr = r ? h1 : h0;
-        const float d = h2f_bits((uint16_t)(hdr.x & 0xFFFFu)), dmin = h2f_bits((uint16_t)(hdr.x >> 16));
-#pragma unroll
-        for (int tg = 0; tg < NTG; ++tg) out[r][tg] = d * accq[r][tg] - dmin * accm[r][tg];
+        float m[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint2 b = lds64(xaddr + tg * kXq4 + kFragBytes + lane * 8);
+        mma16816_bf16(m, am[0], am[1], am[0], am[1], b.x, b.y);
+        const float xs = ldsf(xaddr + tg * kXq4 + kFragBytes + kMinBytes + t * 4);
+        float q0 = c[0][tg][0] + c[0][tg][1], q1 = c[0][tg][2] + c[0][tg][3];
+        if (kChains == 2) { q0 += c[kChains - 1][tg][0] + c[kChains - 1][tg][1]; q1 += c[kChains - 1][tg][2] + c[kChains - 1][tg][3]; }
+        acc[0][tg] = fmaf(xs, d0 * q0 - e0 * (m[0] + m[1]), acc[0][tg]);
+        acc[1][tg] = fmaf(xs, d1 * q1 - e1 * (m[2] + m[3]), acc[1][tg]);
     }
 }
 
 // Q6_K (q = nibble | two high bits << 4, value d * sc * (q - 32); fl_dot_row_q6_K, src/runtime/quants.h:194-230): an
 // instruction covers the 16 columns of one int8 scale; lane column t unpacks bytes 4 t .. 4 t + 3 of the 16-byte runs.
-// ODD: the block starts 2 bytes past a word boundary (r0, r1 are the aligned addresses 2 bytes in front of it).
-template <int NTG, bool ODD>
-__device__ __forceinline__ void q6k_block_nx(uint32_t r0, uint32_t r1, uint32_t t, uint32_t xaddr, uint32_t lane, float (&out)[2][NTG]) {
+// ODD: the block starts 2 bytes past a word boundary (r0 is the aligned address 2 bytes in front of it).
+template <int NTG, bool ODD, typename Rel>
+__device__ __forceinline__ void q6k_block_nx(uint32_t r0, uint32_t t, uint32_t xaddr, uint32_t lane, float (&acc)[2][NTG], Rel &&release) {
     uint32_t wa[2][4], wb[2][4], wh[2][4];   // [row][(hf, hq)]
+    uint32_t sw[2][4];                       // the 16 int8 scales as (s + 128) bytes
+    float dd[2];
 #pragma unroll
-    for (int hh = 0; hh < 4; ++hh) {
-        const uint32_t hf = hh >> 1, hq = hh & 1;
-        const uint32_t oa = 64 * hf + 16 * hq + 4 * t, oh = 128 + 32 * hf + 16 * hq + 4 * t;
+    for (int r = 0; r < 2; ++r) {
+        const uint32_t rb = r0 + r * 8 * kPitch6;
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const uint32_t rb = r ? r1 : r0;
+        for (int hh = 0; hh < 4; ++hh) {
+            const uint32_t hf = hh >> 1, hq = hh & 1;
+            const uint32_t oa = 64 * hf + 16 * hq + 4 * t, oh = 128 + 32 * hf + 16 * hq + 4 * t;
             if (ODD) {
                 wa[r][hh] = __byte_perm(lds32(rb + oa), lds32(rb + oa + 4), 0x5432u);
                 wb[r][hh] = __byte_perm(lds32(rb + oa + 32), lds32(rb + oa + 36), 0x5432u);
@@ -346,30 +513,25 @@ __device__ __forceinline__ void q6k_block_nx(uint32_t r0, uint32_t r1, uint32_t 
                 wh[r][hh] = lds32(rb + oh);
             }
         }
-    }
-    // the 16 int8 scales of both rows as (s + 128) bytes, d at byte 208
-    uint32_t sw[2][4];
-    float dd[2];
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const uint32_t rb = r ? r1 : r0;
         if (ODD) {
             uint32_t s[5];
 #pragma unroll
             for (int k = 0; k < 5; ++k) s[k] = lds32(rb + 192 + 4 * k);
 #pragma unroll
             for (int k = 0; k < 4; ++k) sw[r][k] = __byte_perm(s[k], s[k + 1], 0x5432u) ^ 0x80808080u;
+            dd[r] = h2f_bits((uint16_t)(lds32(rb + 208) >> 16));
         } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k) sw[r][k] = lds32(rb + 192 + 4 * k) ^ 0x80808080u;
+            dd[r] = h2f_bits((uint16_t)lds16(rb + 208));
         }
-        dd[r] = h2f_bits((uint16_t)lds16(rb + (ODD ? 2u : 0u) + 208));
     }
-    float acc[2][NTG];
+    release();
+    float2 s2[2][NTG];
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
-        for (int tg = 0; tg < NTG; ++tg) acc[r][tg] = 0.f;
+        for (int tg = 0; tg < NTG; ++tg) s2[r][tg] = make_float2(0.f, 0.f);
     const __half2 off = __floats2half2_rn(1056.f, 1056.f);
 #pragma unroll
     for (int hh = 0; hh < 4; ++hh) {
@@ -384,288 +546,476 @@ __device__ __forceinline__ void q6k_block_nx(uint32_t r0, uint32_t r1, uint32_t 
             q[r][3] = ((b >> 4) & 0x0F0F0F0Fu) | ((h >> 2) & 0x30303030u);
         }
 #pragma unroll
-        for (int gq = 0; gq < 4; ++gq) {
-            const uint32_t a0 = hsub2_u32(__byte_perm(q[0][gq], 0x64646464u, 0x4240u), off), a1 = hsub2_u32(__byte_perm(q[1][gq], 0x64646464u, 0x4240u), off);
-            const uint32_t a2 = hsub2_u32(__byte_perm(q[0][gq], 0x64646464u, 0x4341u), off), a3 = hsub2_u32(__byte_perm(q[1][gq], 0x64646464u, 0x4341u), off);
-            // scale index 8 hf + 2 gq + hq: byte (2 gq + hq) of word (2 hf + (gq >> 1)) ... as one index into 16 bytes
-            const int si = 8 * hf + 2 * gq + hq;
-            float scf[2];
+        for (int gp = 0; gp < 2; ++gp) {   // groups 2 gp, 2 gp + 1: one 16-byte piece of B
+            float c[2][NTG][4];
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const uint32_t w = sw[r][si >> 2];
-                scf[r] = ((si & 3) == 0 ? u8f<0>(w) : (si & 3) == 1 ? u8f<1>(w) : (si & 3) == 2 ? u8f<2>(w) : u8f<3>(w)) - 128.f;
+            for (int i = 0; i < 2; ++i) {
+                const int gq = 2 * gp + i;
+                // bytes 0, 2 / 1, 3 under 0x64: f16 1024 + q; minus 1056 is q - 32, exact
+                const uint32_t a0 = hsub2_u32(__byte_perm(q[0][gq], 0x64646464u, 0x4240u), off), a1 = hsub2_u32(__byte_perm(q[1][gq], 0x64646464u, 0x4240u), off);
+                const uint32_t a2 = hsub2_u32(__byte_perm(q[0][gq], 0x64646464u, 0x4341u), off), a3 = hsub2_u32(__byte_perm(q[1][gq], 0x64646464u, 0x4341u), off);
+#pragma unroll
+                for (int tg = 0; tg < NTG; ++tg) {
+                    const uint2 b = lds64(xaddr + tg * kXq6 + (hh * 2 + gp) * 512 + lane * 16 + i * 8);
+                    c[i][tg][0] = c[i][tg][1] = c[i][tg][2] = c[i][tg][3] = 0.f;
+                    mma16816(c[i][tg], a0, a1, a2, a3, b.x, b.y);
+                }
             }
-            const int m = hh * 4 + gq;   // combo: 16-byte piece m / 2, half m & 1
 #pragma unroll
-            for (int tg = 0; tg < NTG; ++tg) {
-                const uint4 bx = lds128(xaddr + tg * kXqBlk + (m >> 1) * 512 + lane * 16);
-                float cc[4] = {0.f, 0.f, 0.f, 0.f};
-                if (m & 1) mma16816(cc, a0, a1, a2, a3, bx.z, bx.w);
-                else mma16816(cc, a0, a1, a2, a3, bx.x, bx.y);
-                acc[0][tg] = fmaf(scf[0], cc[0] + cc[1], acc[0][tg]);
-                acc[1][tg] = fmaf(scf[1], cc[2] + cc[3], acc[1][tg]);
+            for (int i = 0; i < 2; ++i) {
+                const int si = 8 * hf + 2 * (2 * gp + i) + hq;
+                const float f0 = s8f(sw[0][si >> 2], si & 3), f1 = s8f(sw[1][si >> 2], si & 3);
+#pragma unroll
+                for (int tg = 0; tg < NTG; ++tg) {
+                    fma_pair(s2[0][tg], f0, c[i][tg][0], c[i][tg][1]);
+                    fma_pair(s2[1][tg], f1, c[i][tg][2], c[i][tg][3]);
+                }
             }
         }
     }
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int tg = 0; tg < NTG; ++tg) out[r][tg] = dd[r] * acc[r][tg];
+    for (int tg = 0; tg < NTG; ++tg) {
+        const float xs = ldsf(xaddr + tg * kXq6 + kFragBytes + t * 4);
+        acc[0][tg] = fmaf(xs, dd[0] * (s2[0][tg].x + s2[0][tg].y), acc[0][tg]);
+        acc[1][tg] = fmaf(xs, dd[1] * (s2[1][tg].x + s2[1][tg].y), acc[1][tg]);
+    }
 }
 
-// Warps: G groups of 8 consumers (group i takes stages i, i + G, ... of the CTA's stage sequence), the producer, the finalizer.
-template <int NTG, int G>
-__global__ void __launch_bounds__((G * kCW + 2) * 32) matmul_tc_nx_kernel(const __grid_constant__ NxArgs a) {
+// Q8_0 (blocks of 32 int8 with one f16 d, 34 bytes; fl_dot_row_q8_0, src/runtime/quants.h:132-142): lane column t takes
+// bytes 8 t .. 8 t + 7 of a block, two instructions per block. Even blocks start on a word boundary, so their quants
+// are 2 bytes past one; odd blocks' quants are aligned. An int8 s becomes f16 through (s ^ 0x80) under 0x64: 1024 + 128 + s.
+template <int NTG, typename Rel>
+__device__ __forceinline__ void q80_block_nx(uint32_t r0, uint32_t t, uint32_t xaddr, uint32_t lane, float (&acc)[2][NTG], Rel &&release) {
+    uint32_t w[2][8][2];
+    uint32_t dw[2][4];   // scales of blocks 2 b, 2 b + 1 as a pair of halves
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const uint32_t rb = r0 + r * 8 * kPitch8;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {   // pairs of blocks: 68 bytes
+            const uint32_t p = rb + 68 * b, q = p + 8 * t;
+            const uint32_t x0 = lds32(q), x1 = lds32(q + 4), x2 = lds32(q + 8);
+            w[r][2 * b][0] = __byte_perm(x0, x1, 0x5432u) ^ 0x80808080u;
+            w[r][2 * b][1] = __byte_perm(x1, x2, 0x5432u) ^ 0x80808080u;
+            w[r][2 * b + 1][0] = lds32(q + 36) ^ 0x80808080u;
+            w[r][2 * b + 1][1] = lds32(q + 40) ^ 0x80808080u;
+            dw[r][b] = lds16(p) | (lds32(p + 32) & 0xFFFF0000u);
+        }
+    }
+    release();
+    float2 s2[2][NTG];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int tg = 0; tg < NTG; ++tg) s2[r][tg] = make_float2(0.f, 0.f);
+    const __half2 off = __floats2half2_rn(1152.f, 1152.f);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        uint32_t a[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            a[i][0] = hsub2_u32(__byte_perm(w[0][b][i], 0x64646464u, 0x4240u), off);
+            a[i][1] = hsub2_u32(__byte_perm(w[1][b][i], 0x64646464u, 0x4240u), off);
+            a[i][2] = hsub2_u32(__byte_perm(w[0][b][i], 0x64646464u, 0x4341u), off);
+            a[i][3] = hsub2_u32(__byte_perm(w[1][b][i], 0x64646464u, 0x4341u), off);
+        }
+        const uint32_t h0 = dw[0][b >> 1], h1 = dw[1][b >> 1];
+        const float f0 = h2f_bits((uint16_t)((b & 1) ? h0 >> 16 : h0 & 0xFFFFu)), f1 = h2f_bits((uint16_t)((b & 1) ? h1 >> 16 : h1 & 0xFFFFu));
+#pragma unroll
+        for (int tg = 0; tg < NTG; ++tg) {
+            const uint4 x = lds128(xaddr + tg * kXq6 + b * 512 + lane * 16);
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
+            mma16816(c, a[0][0], a[0][1], a[0][2], a[0][3], x.x, x.y);
+            mma16816(c, a[1][0], a[1][1], a[1][2], a[1][3], x.z, x.w);
+            fma_pair(s2[0][tg], f0, c[0], c[1]);
+            fma_pair(s2[1][tg], f1, c[2], c[3]);
+        }
+    }
+#pragma unroll
+    for (int tg = 0; tg < NTG; ++tg) {
+        const float xs = ldsf(xaddr + tg * kXq6 + kFragBytes + t * 4);
+        acc[0][tg] = fmaf(xs, s2[0][tg].x + s2[0][tg].y, acc[0][tg]);
+        acc[1][tg] = fmaf(xs, s2[1][tg].x + s2[1][tg].y, acc[1][tg]);
+    }
+}
+
+struct NxRing { uint32_t slot, par, slots, base; };   // a group's next stage and its parity, carried from piece to piece; its ring
+
+// One consumer warp's share of a piece: units u0, u0 + 2, ... of format FMT with NTG token groups.
+template <int FMT, int NTG>
+__device__ __forceinline__ void consume(const NxArgs &a, uint32_t smem, const NxJob &jb, uint32_t u0, uint32_t u1, uint32_t grp8,
+                                        uint32_t w, uint32_t lane, NxRing &rg, uint32_t &red_par, bool &dead) {
+    const uint32_t xs_addr = smem + a.x_off;
+    const uint32_t g = lane >> 2, t = lane & 3u;
+    const uint32_t nblk_p = min(a.nblk - jb.seg0 * 8u, jb.nseg * 8u);   // blocks of the part
+    const bool swz = FMT == FMT_Q4_K && a.t[jb.tensor].swz != 0;
+    uint32_t offs = 0;   // see q4k_block_nx
+    if (FMT == FMT_Q4_K)
+        offs = (q4_row_off(w * 144u, g, swz) >> 4) | (q4_row_off(w * 144u + 16u + 32u * t, g, swz) << 4) |
+               (q4_row_off(w * 144u + 32u + 32u * t, g, swz) << 12);
+    for (uint32_t u = u0; u < u1; u += 2) {
+        float acc[2][NTG];
+#pragma unroll
+        for (int tg = 0; tg < NTG; ++tg) acc[0][tg] = acc[1][tg] = 0.f;
+#pragma unroll 1
+        for (uint32_t seg = 0; seg < jb.nseg; ++seg) {
+            const uint32_t blk = seg * 8 + w, bar = smem + (grp8 * kMaxSlots + rg.slot) * 8;
+            bar_wait_or_die(bar + kFull, rg.par, a.status, dead);
+            auto release = [&]() {
+                __syncwarp();
+                if (lane == 0) bar_arrive(bar + kEmpty);
+            };
+            const uint32_t st = rg.base + rg.slot * a.slot_bytes, xaddr = xs_addr + blk * (NTG * xq_bytes(FMT));
+            if (blk >= nblk_p) release();
+            else if (FMT == FMT_Q4_K) q4k_block_nx<NTG>(st + g * kPitch4, offs, t, xaddr, lane, acc, release);
+            else if (FMT == FMT_Q6_K) {
+                const uint32_t r0 = st + g * kPitch6 + w * 210u;
+                if (w & 1u) q6k_block_nx<NTG, true>(r0 - 2, t, xaddr, lane, acc, release);
+                else q6k_block_nx<NTG, false>(r0, t, xaddr, lane, acc, release);
+            } else q80_block_nx<NTG>(st + (w >> 2) * 16 * kPitch8 + g * kPitch8 + (w & 3u) * 272u, t, xaddr, lane, acc, release);
+            if (++rg.slot == rg.slots) { rg.slot = 0; rg.par ^= 1u; }
+        }
+        // this warp's share of the unit: rows g, g + 8 x tokens 4 tg + t (the rows' halves trade places for odd pairs of
+        // tokens, which makes the stores conflict free)
+        bar_wait_or_die(smem + kRedEmpty + grp8 * 8, red_par ^ 1u, a.status, dead);
+        const uint32_t pp = smem + kBarBytes + (grp8 * a.red_group + w * (NTG * 64)) * 4;
+#pragma unroll
+        for (int tg = 0; tg < NTG; ++tg) {
+            const uint32_t o = (4 * tg + t) * 16u, x = (t & 2u) << 2;
+            sts32(pp + (o + (g ^ x)) * 4, acc[0][tg]);
+            sts32(pp + (o + ((g + 8) ^ x)) * 4, acc[1][tg]);
+        }
+        __syncwarp();
+        if (lane == 0) bar_arrive(smem + kRedFull + grp8 * 8);
+        red_par ^= 1u;
+    }
+}
+
+// FM: the formats an instance carries (bit 0 Q4_K, 1 Q6_K, 2 Q8_0): with all three in one kernel, what is live across the
+// choice of the body does not fit in the registers beside the largest of them (204 bytes of spills against 0..48).
+template <int FM>
+__global__ void __launch_bounds__(kThreads, 1) matmul_nx_kernel(const __grid_constant__ NxArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    constexpr uint32_t kConsumers = G * kCW, kProducer = kConsumers, kFinal = kConsumers + 1;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t S = a.nslots;
-    uint64_t *full = (uint64_t *)smem_raw, *empty = full + S;
-    uint64_t *red_full = empty + S, *red_empty = red_full + 2, *x_full = red_empty + 2, *x_empty = x_full + 1;
-    float *red = (float *)(smem_raw + S * 16 + 64);
-    const uint32_t nblk = a.cols / 256, nseg = (nblk + 7) / 8;
-    const uint32_t kChunkBlks = a.chunk_blks;
-    const uint32_t nchunk = (nblk + kChunkBlks - 1) / kChunkBlks;
-    const uint32_t units = (a.rows + 15) / 16;
-    const uint32_t my_units = blockIdx.x < units ? (units - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-    // Launched as a programmatic dependent. With a device-side column list the list decides whether any weight is read at
-    // all, so everything waits for the kernels before; without one the producer starts streaming the weights (constants)
-    // at once and only the finalizer, which fetches the converted activations and touches y, waits.
+    const uint32_t smem = smem_u32(smem_raw);
+    // Launched as a programmatic dependent. With a table that the kernels in front write, it decides what is read at all
+    // and everything waits for them; otherwise the producers start streaming the weights (constants) at once and only
+    // the finalizers, which fetch the converted activations and touch y, wait.
     griddep_launch_dependents();
-    if (a.cnt) griddep_wait();
-    uint32_t n_valid = a.P;   // listed columns of this call
-    if (a.cnt) { const uint32_t c = *a.cnt; n_valid = c > a.col_off ? min(c - a.col_off, a.P) : 0u; }
-    if (n_valid == 0) return;   // nothing routed here: no weights are read
-    if (tid == 0) {
-        for (uint32_t s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], kCW); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&red_full[i], kConsumers); mbar_init(&red_empty[i], 1); }
-        mbar_init(x_full, 1);
-        mbar_init(x_empty, kConsumers);
+    if (a.table && !a.table_ready) griddep_wait();
+    if (warp == 2) {   // (the second warp lists the pieces)
+        if (lane < 2 * kMaxSlots) { mbar_init(bar_at(smem + kFull + 8 * lane), 1); mbar_init(bar_at(smem + kEmpty + 8 * lane), kCW); }
         fence_barrier_init();
     }
+    if (tid == 0) {
+        for (uint32_t i = 0; i < 2; ++i) { mbar_init(bar_at(smem + kRedFull + 8 * i), kCW); mbar_init(bar_at(smem + kRedEmpty + 8 * i), 1); }
+        mbar_init(bar_at(smem + kXFull), 1);
+        mbar_init(bar_at(smem + kXEmpty), kConsumers);
+        fence_barrier_init();
+    }
+    if (tid == 32) nx_list_pieces(a, smem_raw);
     __syncthreads();
-    const uint32_t ring = smem_u32(smem_raw) + a.ring_off, xs_addr = smem_u32(smem_raw) + a.x_off;
-    const uint32_t segb = a.fmt == FMT_Q4_K ? kSeg4 : kSeg6;
+    const uint32_t n_pieces = lds32(smem + kPieces), slots = lds32(smem + kPieces + 4), ring = smem + lds32(smem + kPieces + 8);
+    // 640 threads start with 96 registers each: the last warpgroup (producers, finalizers) gives up 32 of them, the four
+    // of the consumers take 8 more (128 x 64 + 512 x 104 = 640 x 96)
+    if (warp >= kConsumers) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
 
-    if (warp == kProducer) {
-        uint32_t slot = 0, par = 1;
-        for (uint32_t ch = 0; ch < nchunk; ++ch) {
-            const uint32_t seg0 = ch * (kChunkBlks / 8), seg1 = min(seg0 + kChunkBlks / 8, nseg);
-            for (uint32_t k = 0; k < my_units; ++k) {
-                const uint32_t u = blockIdx.x + k * gridDim.x;
-                for (uint32_t seg = seg0; seg < seg1; ++seg) {
-                    const uint32_t off = seg * segb;
-                    if (!mbar_wait_bounded(&empty[slot], par, a.status)) return;
-                    fence_proxy_async_smem();
-                    if (lane == 0) {
-                        // one box of 16 rows x the segment; rows past the end of the tensor and blocks past the end of a
-                        // row arrive as zeros and count as bytes all the same
-                        mbar_arrive_expect_tx(&full[slot], 16 * segb);
-                        if (a.swz) tma_box3(ring + slot * a.slot_bytes, &a.map, off / 128, 16 * u, &full[slot]);
-                        else tma_box2(ring + slot * a.slot_bytes, &a.map, off / 8, 16 * u, &full[slot]);
+    if (warp >= kConsumers + 2) {
+        // ---- finalizers: group `grp8`'s units; the first one also brings the activation of a piece ----
+        const uint32_t grp8 = warp - (kConsumers + 2);
+        uint32_t red_par = 0, x_par = 1;
+        griddep_wait();   // the converted activations and y come from the kernels before
+#pragma unroll 1
+        for (uint32_t pi = 0; pi < n_pieces; ++pi) {
+            const NxPiece pc = nx_piece(smem, pi);
+            const NxJob &jb = a.job[pc.job];
+            const uint32_t grp = pc.grp, n_valid = pc.n_valid, tg0 = pc.tg0;
+            const NxT &t = a.t[jb.tensor];
+            const uint32_t ntg = (n_valid + 3) / 4, xb = xq_bytes(t.fmt), blk_bytes = ntg * xb;
+            const uint8_t *img = a.xq + t.xoff + (size_t)tg0 * a.nblk * xb;
+            if (grp8 == 0 && !pc.same) {   // one bulk copy per block, after the consumers left the activation before
+                const uint32_t b0 = jb.seg0 * 8u, nb = min(a.nblk - b0, jb.nseg * 8u);
+                if (!bar_wait(smem + kXEmpty, x_par, a.status)) return;
+                fence_proxy_async_smem();
+                if (lane == 0) mbar_arrive_expect_tx(bar_at(smem + kXFull), nb * blk_bytes);
+                __syncwarp();
+                for (uint32_t b = lane; b < nb; b += 32)
+                    bulk_g2s_addr(smem + a.x_off + b * blk_bytes, img + (size_t)(b0 + b) * blk_bytes, blk_bytes, bar_at(smem + kXFull));
+            }
+            if (!pc.same) x_par ^= 1u;
+            float inv = 1.f;   // lane p: 1 / rms of token p
+            if (a.rms) {
+                float ss = 0.f;
+                if (lane < 4 * ntg) {
+                    const uint8_t *src = img + (lane >> 2) * xb + (xb - 16) + (lane & 3u) * 4u;
+#pragma unroll 8
+                    for (uint32_t b = 0; b < a.nblk; ++b) ss += __ldcg(reinterpret_cast<const float *>(src + (size_t)b * blk_bytes));
+                }
+                inv = 1.0f / sqrtf(ss / (float)(a.nblk * 256u) + a.eps);
+            }
+            const float *mine = reinterpret_cast<const float *>(smem_raw + kBarBytes) + (size_t)grp8 * a.red_group;
+            const bool vec = ((t.rows | t.ystride) & 3u) == 0 && ((((uintptr_t)t.y) & 15u) == 0) && (t.part_stride & 3u) == 0;
+            for (uint32_t u = pc.u0 + (pc.par ^ grp8); u < pc.u1; u += 2) {
+                if (!bar_wait(smem + kRedFull + grp8 * 8, red_par, a.status)) return;
+                red_par ^= 1u;
+                float4 v[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t o = lane + 32 * i;   // outputs 4 o ..: token o / 4, rows 4 (o & 3) ..
+                    v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (o < 16 * ntg) {
+                        const float *src = mine + 16 * (o >> 2) + ((4 * (o & 3u)) ^ (((o >> 2) & 2u) << 2));
+#pragma unroll
+                        for (uint32_t w = 0; w < kCW; ++w) {
+                            const float4 p = *reinterpret_cast<const float4 *>(src + w * (ntg * 64));
+                            v[i].x += p.x; v[i].y += p.y; v[i].z += p.z; v[i].w += p.w;
+                        }
                     }
-                    if (++slot == S) { slot = 0; par ^= 1u; }
+                }
+                __syncwarp();
+                if (lane == 0) bar_arrive(smem + kRedEmpty + grp8 * 8);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t o = lane + 32 * i, tok = o >> 2, row = 16 * u + 4 * (o & 3u);
+                    const float s = __shfl_sync(0xffffffffu, inv, tok & 31u);
+                    if (tok >= n_valid || row >= t.rows) continue;
+                    if (a.rms) { v[i].x *= s; v[i].y *= s; v[i].z *= s; v[i].w *= s; }
+                    const size_t orow = a.out_idx ? a.out_idx[(size_t)grp * a.list_stride + a.col_off + tok] : tok;
+                    float *dst = t.y + jb.part * t.part_stride + orow * t.ystride + row;
+                    if (vec) {
+                        if (a.accumulate) {
+                            const float4 y = *reinterpret_cast<const float4 *>(dst);
+                            v[i].x += y.x; v[i].y += y.y; v[i].z += y.z; v[i].w += y.w;
+                        }
+                        *reinterpret_cast<float4 *>(dst) = v[i];
+                    } else {
+                        const float q[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+                        for (int r = 0; r < 4; ++r)
+                            if (row + r < t.rows) dst[r] = a.accumulate ? dst[r] + q[r] : q[r];
+                    }
                 }
             }
         }
         return;
     }
 
-    if (warp == kFinal) {
-        // ---- finalizer: 16 rows x 8 tokens per unit; lane <-> outputs 4 lane .. 4 lane + 3 (row = o / 8, token = o % 8) ----
-        float *uacc = (float *)(smem_raw + a.uacc_off);   // running sums of the units while the chunks go by
-        uint32_t kk = 0;
-        if (!a.cnt) griddep_wait();   // the converted activations and y come from the kernels before
-        for (uint32_t ch = 0; ch < nchunk; ++ch) {
-            {   // the chunk's activation image: one bulk copy per block (lanes in parallel), after the consumers left the last one
-                const uint32_t b0 = ch * kChunkBlks, nb = min(kChunkBlks, nblk - b0);
-                if (!mbar_wait_bounded(x_empty, (ch & 1u) ^ 1u, a.status)) return;
-                fence_proxy_async_smem();
-                const uint32_t blk_bytes = a.ntg * kXqBlk;
-                if (lane == 0) mbar_arrive_expect_tx(x_full, nb * blk_bytes);
-                __syncwarp();
-                if (lane < nb) bulk_g2s_addr(xs_addr + lane * blk_bytes, a.xq + (size_t)(b0 + lane) * blk_bytes, blk_bytes, x_full);
-            }
-            for (uint32_t k = 0; k < my_units; ++k, ++kk) {
-                const uint32_t u = blockIdx.x + k * gridDim.x, buf = kk & 1u;
-                if (!mbar_wait_bounded(&red_full[buf], (kk >> 1) & 1u, a.status)) return;
-                float v[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (uint32_t w = 0; w < kConsumers; ++w) {
-                    const float4 p = *reinterpret_cast<const float4 *>(red + (buf * kConsumers + w) * 128 + lane * 4);
-                    v[0] += p.x; v[1] += p.y; v[2] += p.z; v[3] += p.w;
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&red_empty[buf]);
-                if (nchunk > 1) {
-                    float4 *ua = reinterpret_cast<float4 *>(uacc + k * 128 + lane * 4);
-                    if (ch > 0) { const float4 p = *ua; v[0] += p.x; v[1] += p.y; v[2] += p.z; v[3] += p.w; }
-                    if (ch + 1 < nchunk) { *ua = make_float4(v[0], v[1], v[2], v[3]); continue; }
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint32_t o = lane * 4 + i, row = 16 * u + (o >> 3), tok = o & 7u;
-                    if (row < a.rows && tok < n_valid) {
-                        const size_t orow = a.out_idx ? a.out_idx[a.col_off + tok] : tok;
-                        float *dst = a.y + orow * a.ystride + row;
-                        *dst = a.accumulate ? *dst + v[i] : v[i];
+    if (warp >= kConsumers) {
+        // ---- producers: the stages of group `grp8` ----
+        const uint32_t grp8 = warp - kConsumers;
+        uint32_t slot = 0, par = 1;   // a fresh barrier passes a wait on parity 1
+#pragma unroll 1
+        for (uint32_t pi = 0; pi < n_pieces; ++pi) {
+            const NxPiece pc = nx_piece(smem, pi);
+            const NxJob &jb = a.job[pc.job];
+            const NxT &t = a.t[jb.tensor];
+            const CUtensorMap *map = &a.map[jb.tensor];
+            const uint32_t segb = seg_bytes(t.fmt);
+            for (uint32_t u = pc.u0 + (pc.par ^ grp8); u < pc.u1; u += 2)
+                for (uint32_t seg = 0; seg < jb.nseg; ++seg) {
+                    const uint32_t off = (jb.seg0 + seg) * segb, row0 = pc.grp * t.rows + 16 * u;
+                    const uint32_t bar = smem + (grp8 * kMaxSlots + slot) * 8;
+                    if (!bar_wait(bar + kEmpty, par, a.status)) return;
+                    fence_proxy_async_smem();
+                    if (lane == 0) {
+                        // 16 rows x the segment; rows past the end of the tensor and blocks past the end of a row arrive
+                        // as zeros (or as another expert's rows, whose results are dropped) and count as bytes all the same
+                        const uint32_t dst = ring + (grp8 * slots + slot) * a.slot_bytes;
+                        uint64_t *full = bar_at(bar + kFull);
+                        if (t.fmt == FMT_Q8_0) {
+                            mbar_arrive_expect_tx(full, 32 * kPitch8);
+                            tma_box2(dst, map, off / 8, row0, full);
+                            tma_box2(dst + 16 * kPitch8, map, (off + segb / 2) / 8, row0, full);
+                        } else {
+                            mbar_arrive_expect_tx(full, 16 * segb);
+                            if (t.swz) tma_box3(dst, map, off / 128, row0, full);
+                            else tma_box2(dst, map, off / 8, row0, full);
+                        }
                     }
+                    if (++slot == slots) { slot = 0; par ^= 1u; }
                 }
-            }
         }
         return;
     }
 
     // ---- consumers ----
-    {
-        const uint32_t w = warp % kCW, g = lane >> 2, t = lane & 3u;
-        uint32_t ow[4][2];
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int i = 0; i < 2; ++i) ow[c][i] = q4_row_off(w * 144u + 16u + 32u * c + 16u * i + 4u * t, g, a.swz != 0);
-        const uint32_t oh = q4_row_off(w * 144u, g, a.swz != 0);
-        // this group's next stage (index over the CTA's whole stage sequence), its ring slot and parity
-        uint32_t c_it = warp / kCW, c_slot = c_it % S, c_par = 0, kk = 0, it0 = 0;
-        bool dead = false;
-        for (uint32_t ch = 0; ch < nchunk; ++ch) {
-            const uint32_t seg0 = ch * (kChunkBlks / 8), seg1 = min(seg0 + kChunkBlks / 8, nseg);
-            mbar_wait_or_die(x_full, ch & 1u, a.status, dead);
-            for (uint32_t k = 0; k < my_units; ++k, ++kk) {
-                float acc[2][NTG];
-#pragma unroll
-                for (int r = 0; r < 2; ++r)
-#pragma unroll
-                    for (int tg = 0; tg < NTG; ++tg) acc[r][tg] = 0.f;
-                const uint32_t it1 = it0 + (seg1 - seg0);
-                for (; c_it < it1; c_it += G) {
-                    const uint32_t blk = (seg0 + (c_it - it0)) * 8 + w;
-                    mbar_wait_or_die(&full[c_slot], c_par, a.status, dead);
-                    if (blk < nblk) {
-                        const uint32_t xaddr = xs_addr + (blk - ch * kChunkBlks) * (NTG * kXqBlk);
-                        float o[2][NTG];
-                        if (a.fmt == FMT_Q4_K) {
-                            const uint32_t r0 = ring + c_slot * a.slot_bytes + g * kPitch4;
-                            q4k_block_nx<NTG>(r0, ow, oh, t, xaddr, lane, o);
-                        } else {
-                            const uint32_t r0 = ring + c_slot * a.slot_bytes + g * kPitch6 + w * 210u;
-                            if (w & 1u) q6k_block_nx<NTG, true>(r0 - 2, r0 + 8 * kPitch6 - 2, t, xaddr, lane, o);
-                            else q6k_block_nx<NTG, false>(r0, r0 + 8 * kPitch6, t, xaddr, lane, o);
-                        }
-#pragma unroll
-                        for (int tg = 0; tg < NTG; ++tg) {
-                            const float xs = ldsf(xaddr + tg * kXqBlk + kFragBytes + 128 + t * 4);   // block scale of token 4 tg + t
-                            acc[0][tg] = fmaf(xs, o[0][tg], acc[0][tg]);
-                            acc[1][tg] = fmaf(xs, o[1][tg], acc[1][tg]);
-                        }
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&empty[c_slot]);
-                    c_slot += G;
-                    if (c_slot >= S) { c_slot -= S; c_par ^= 1u; }
-                }
-                it0 = it1;
-                // this warp's share of the unit: rows g, g + 8 x tokens t, t + 4 (complete over the warp's columns)
-                const uint32_t buf = kk & 1u;
-                mbar_wait_or_die(&red_empty[buf], ((kk >> 1) & 1u) ^ 1u, a.status, dead);
-                float *pp = red + (buf * kConsumers + warp) * 128;
-#pragma unroll
-                for (int tg = 0; tg < NTG; ++tg) {
-                    pp[g * 8 + 4 * tg + t] = acc[0][tg];
-                    pp[(g + 8) * 8 + 4 * tg + t] = acc[1][tg];
-                }
-                if (NTG == 1) { pp[g * 8 + 4 + t] = 0.f; pp[(g + 8) * 8 + 4 + t] = 0.f; }
+    const uint32_t grp8 = warp / kCW, w = warp % kCW;
+    NxRing rg{0, 0, slots, ring + grp8 * slots * a.slot_bytes};
+    uint32_t red_par = 0, x_par = 0;
+    bool dead = false;
+#pragma unroll 1
+    for (uint32_t pi = 0; pi < n_pieces; ++pi) {
+        const NxPiece pc = nx_piece(smem, pi);
+        const NxJob &jb = a.job[pc.job];
+        const uint32_t u0 = pc.u0 + (pc.par ^ grp8), u1 = pc.u1;   // this group's units: every other one
+        if (!pc.same) {
+            if (pi) {   // done with the activation before
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&red_full[buf]);
+                if (lane == 0) bar_arrive(smem + kXEmpty);
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(x_empty);   // done with this chunk of the activation
+            bar_wait_or_die(smem + kXFull, x_par, a.status, dead);
+            x_par ^= 1u;
         }
+        const int fmt = a.t[jb.tensor].fmt;
+        const uint32_t ntg = (pc.n_valid + 3) / 4;
+#define FLB_CONSUME(F, N) consume<F, N>(a, smem, jb, u0, u1, grp8, w, lane, rg, red_par, dead)
+#define FLB_CONSUME_F(F)                                                                                             \
+    (ntg == 1 ? FLB_CONSUME(F, 1) : ntg == 2 ? FLB_CONSUME(F, 2) : ntg == 3 ? FLB_CONSUME(F, 3) : FLB_CONSUME(F, 4))
+        if ((FM & 1) && (FM == 1 || fmt == FMT_Q4_K)) FLB_CONSUME_F(FMT_Q4_K);
+        else if ((FM & 2) && (FM == 2 || fmt == FMT_Q6_K)) FLB_CONSUME_F(FMT_Q6_K);
+        else if (FM & 4) FLB_CONSUME_F(FMT_Q8_0);
+#undef FLB_CONSUME_F
+#undef FLB_CONSUME
     }
 }
 
-} // namespace
-
-// Consumer groups per CTA (FLB_NX_GROUPS=1 selects the single-group instantiation for comparison).
-static int nx_groups() {
-    static const int v = getenv("FLB_NX_GROUPS") ? atoi(getenv("FLB_NX_GROUPS")) : 2;
-    return v == 1 ? 1 : 2;
+// How a launch over tensors of these formats is cut along the columns, and its shared memory. `split`: the caller adds the
+// planes of the parts on the fly, so the columns are cut to one segment per part, which halves (4096 columns) the activation
+// that every CTA has to load before it starts, leaves room for more stages, and doubles the number of items that are shared
+// out; otherwise all columns are one part where they fit with one stage per group, or as many segments as leave two.
+struct NxPlan { uint32_t parts, segs, slot_bytes, x_off, x_blk_tg; };
+bool nx_plan(const int *fmts, int n, uint32_t cols, uint32_t ntg, bool split, NxPlan &p) {
+    uint32_t xb = 0, slot = 0;
+    for (int i = 0; i < n; ++i) { xb = std::max(xb, xq_bytes(fmts[i])); slot = std::max(slot, slot_of(fmts[i])); }
+    const uint32_t nblk = cols / 256, nseg = (nblk + 7) / 8;
+    p.x_off = kBarBytes + 2 * kCW * ntg * 64 * 4;
+    auto fit = [&](uint32_t segs) {   // stages per group beside the activation of `segs` segments
+        p.x_blk_tg = std::min(nblk, segs * 8) * xb;
+        const uint32_t off = nx_ring_off(p.x_off, p.x_blk_tg, ntg);
+        return off + 2 * slot <= kSmemLimit ? (kSmemLimit - off) / (2 * slot) : 0u;
+    };
+    uint32_t segs = split ? 1 : nseg;
+    if (!split && fit(segs) < 1) {
+        segs = 1;
+        while (segs + 1 < nseg && fit(segs + 1) >= 2) ++segs;
+        const uint32_t parts = (nseg + segs - 1) / segs;
+        segs = (nseg + parts - 1) / parts;
+    }
+    if (fit(segs) < 1) return false;
+    p.segs = segs;
+    p.parts = (nseg + segs - 1) / segs;
+    p.slot_bytes = slot;
+    return true;
 }
 
+bool nx_tensor_ok(const NxTensor &t, uint32_t cols) {
+    if ((t.fmt != FMT_Q4_K && t.fmt != FMT_Q6_K && t.fmt != FMT_Q8_0) || t.rows == 0) return false;
+    const uint64_t rb = row_bytes(t.fmt, cols), pitch = t.pitch ? t.pitch : rb;
+    return (pitch & 15u) == 0 && pitch >= rb && (((uintptr_t)t.w) & 15u) == 0;
+}
+
+size_t nx_image_bytes(int fmt, uint32_t cols, uint32_t tgs) { return (size_t)(cols / 256) * tgs * xq_bytes(fmt); }
+
+// The images of a call lie one behind the other: Q4_K, Q6_K, Q8_0 (those wanted). Returns the offset of `fmt`'s.
+uint32_t nx_image_off(int fmt, bool q4, bool q6, uint32_t cols, uint32_t tgs) {
+    size_t o = 0;
+    if (fmt != FMT_Q4_K && q4) o += nx_image_bytes(FMT_Q4_K, cols, tgs);
+    if (fmt == FMT_Q8_0 && q6) o += nx_image_bytes(FMT_Q6_K, cols, tgs);
+    return (uint32_t)o;
+}
+
+void (*const kNxKernels[5])(const NxArgs) = {matmul_nx_kernel<1>, matmul_nx_kernel<2>, matmul_nx_kernel<3>, matmul_nx_kernel<4>,
+                                             matmul_nx_kernel<7>};
+
+} // namespace
+
 cudaError_t matmul_tc_nx_init(void) {
-    const void *ks[] = {(const void *)matmul_tc_nx_kernel<1, 1>, (const void *)matmul_tc_nx_kernel<2, 1>,
-                        (const void *)matmul_tc_nx_kernel<1, 2>, (const void *)matmul_tc_nx_kernel<2, 2>};
-    for (const void *k : ks) {
-        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
+    for (auto k : kNxKernels) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
-// Bytes of device scratch the converted activations of one call need (cols <= 18432, up to 8 columns).
-size_t matmul_tc_nx_scratch_bytes(uint32_t cols, uint32_t P) {
-    return (size_t)(cols / 256) * ((P + 3) / 4) * kXqBlk;
+// Bytes of device scratch the converted activations of `tgs` groups of four columns need, one image per layout.
+size_t matmul_tc_nx_scratch_bytes(uint32_t cols, uint32_t tgs, int layouts) {
+    return (size_t)(cols / 256) * tgs * (kXq4 + (layouts > 1 ? kXq6 : 0) + (layouts > 2 ? kXq6 : 0));
 }
 
-// Y[c.out row of column p][r] (+)= dot(W[r], column p), P <= 8 columns, Q4_K or Q6_K, cols a multiple of 256, rows
-// 16-byte pitched. xq: scratch of matmul_tc_nx_scratch_bytes(cols, P). cudaErrorNotSupported for other shapes.
-cudaError_t launch_matmul_tc_nx(const NxCall &c, uint8_t *xq, uint32_t *status, int sms, cudaStream_t stream) {
+uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split) {
     static const bool off = getenv("FLB_TC_NX") && getenv("FLB_TC_NX")[0] == '0';
-    const int fmt = c.fmt;
-    const uint32_t rows = c.rows, cols = c.cols, P = c.P;
-    if (off || (fmt != FMT_Q4_K && fmt != FMT_Q6_K) || cols % 256 != 0 || cols < 256 || P == 0 || P > 8 || rows == 0) return cudaErrorNotSupported;
-    const uint32_t rb = (uint32_t)row_bytes(fmt, cols);
-    const uint32_t pitch = c.pitch ? c.pitch : rb;
-    if ((pitch & 15u) || pitch < rb || (((uintptr_t)c.w) & 15u) || (((uintptr_t)c.x) & 15u) || (((uintptr_t)c.x2) & 15u) || (c.xstride & 3u) || !xq)
-        return cudaErrorNotSupported;
-    const uint32_t nblk = cols / 256, ntg = (P + 3) / 4;
-    const uint32_t units = (rows + 15) / 16;
-    const uint32_t grid = units < (uint32_t)sms ? units : (uint32_t)sms;
-    // a chunk of 16 blocks of 8 tokens leaves room for two Q6_K stages only: 8 blocks then
-    const uint32_t kChunkBlks = (ntg == 2 && fmt == FMT_Q6_K && nblk > 8) ? 8u : kMaxChunkBlks;
-    const uint32_t nchunk = (nblk + kChunkBlks - 1) / kChunkBlks;
-    const uint32_t my_units_max = (units + grid - 1) / grid;
-    if (nchunk > 1 && my_units_max > kMaxChunkUnits) return cudaErrorNotSupported;
+    if (off || n < 1 || n > 3 || cols % 256 != 0 || cols < 256 || cols > kNxMaxCols || P == 0 || P > kNxMaxTokens) return 0;
+    int fmts[3];
+    for (int i = 0; i < n; ++i) {
+        if (!nx_tensor_ok(t[i], cols)) return 0;
+        fmts[i] = t[i].fmt;
+    }
+    NxPlan p;
+    return nx_plan(fmts, n, cols, (P + 3) / 4, split, p) ? p.parts : 0;
+}
+
+cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, uint8_t *xq, uint32_t tgs_cap,
+                              cudaStream_t stream, bool pdl) {
+    if (cols % 256 != 0 || P == 0 || P > kNxMaxTokens || (in.xstride & 3u) || (in.rstride & 3u) || (in.part_stride & 3u)) return cudaErrorNotSupported;
+    if ((((uintptr_t)in.x) | ((uintptr_t)in.x2) | ((uintptr_t)in.resid) | ((uintptr_t)in.x_out) | ((uintptr_t)in.wnorm)) & 15u) return cudaErrorNotSupported;
+    bool q4 = false, q6 = false, q8 = false;
+    for (int i = 0; i < n; ++i) (t[i].fmt == FMT_Q4_K ? q4 : t[i].fmt == FMT_Q6_K ? q6 : q8) = true;
+    ConvArgs c{};
+    c.x = in.x; c.x2 = in.x2; c.part_stride = in.part_stride; c.resid = in.resid; c.x_out = in.x_out; c.wnorm = in.wnorm;
+    c.xstride = in.xstride; c.rstride = in.rstride; c.n_parts = in.n_parts ? in.n_parts : 1; c.P = P; c.nblk = cols / 256;
+    if (q4) c.img4 = xq;
+    if (q6) c.img6 = xq + nx_image_off(FMT_Q6_K, q4, q6, cols, tgs_cap);
+    if (q8) c.img8 = xq + nx_image_off(FMT_Q8_0, q4, q6, cols, tgs_cap);
+    c.att = in.att; c.n_splits = in.n_splits;
+    c.table = in.table; c.col_idx = in.col_idx; c.list_stride = in.list_stride; c.col_off = in.col_off;
+    return launch_kernel(act_convert_nx_kernel, dim3(cols / 256, (P + 3) / 4 * 4, in.table ? in.n_groups : 1), dim3(64), 0, stream, pdl, c);
+}
+
+cudaError_t launch_nx_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,
+                             uint32_t tgs_cap, uint32_t *status, int sms, cudaStream_t stream, bool pdl, bool split) {
+    if (matmul_tc_nx_parts(t, n, cols, P, split) == 0) return cudaErrorNotSupported;
+    static_assert(sizeof(NxArgs) <= 4000, "kernel arguments");
     NxArgs k;
     memset(&k, 0, sizeof(k));
-    const uint32_t segb = fmt == FMT_Q4_K ? kSeg4 : kSeg6;
-    k.swz = (fmt == FMT_Q4_K && pitch % 128 == 0) ? 1 : 0;
-    cudaError_t e = k.swz ? tensor_map_lines_swz(&k.map, c.w, rows, pitch, segb / 128, 16)
-                          : tensor_map_2d(&k.map, 8, c.w, pitch / 8, rows, pitch, segb / 8, 16, false);
-    if (e != cudaSuccess) return e;
-    if (!c.skip_convert) {
-        e = launch_kernel(act_convert_nx_kernel, dim3(nblk, ntg), dim3(64), 0, stream, c.pdl != 0, c.x, c.x2, c.xstride, P, fmt, xq, ntg,
-                          c.cnt, c.col_off, c.col_idx);
+    int fmts[3];
+    bool q4 = false, q6 = false, q8 = false;
+    for (int i = 0; i < n; ++i) {
+        fmts[i] = t[i].fmt;
+        (t[i].fmt == FMT_Q4_K ? q4 : t[i].fmt == FMT_Q6_K ? q6 : q8) = true;
+    }
+    const auto kernel = kNxKernels[q8 ? (q4 || q6 ? 4 : 3) : (q4 ? 1 : 0) + (q6 ? 2 : 0) - 1];
+    NxPlan p;
+    if (!nx_plan(fmts, n, cols, (P + 3) / 4, split, p) || p.parts * n > (uint32_t)kMaxJobs) return cudaErrorNotSupported;
+    const uint32_t nblk = cols / 256, nseg = (nblk + 7) / 8;
+    for (int i = 0; i < n; ++i) {
+        NxT &d = k.t[i];
+        const uint32_t pitch = t[i].pitch ? t[i].pitch : (uint32_t)row_bytes(t[i].fmt, cols);
+        const uint64_t all_rows = (uint64_t)t[i].rows * (in.table ? in.n_experts : 1);
+        d.y = t[i].y; d.part_stride = p.parts > 1 ? t[i].part_stride : 0; d.rows = t[i].rows; d.ystride = t[i].ystride; d.fmt = t[i].fmt;
+        d.units = (t[i].rows + 15) / 16;
+        d.xoff = nx_image_off(t[i].fmt, q4, q6, cols, tgs_cap);
+        d.swz = (t[i].fmt == FMT_Q4_K && pitch % 128 == 0) ? 1 : 0;
+        const cudaError_t e = d.swz ? tensor_map_lines_swz(&k.map[i], t[i].w, all_rows, pitch, kSeg4 / 128, 16)
+                                    : tensor_map_2d(&k.map[i], 8, t[i].w, pitch / 8, all_rows, pitch,
+                                                    (t[i].fmt == FMT_Q8_0 ? kPitch8 : seg_bytes(t[i].fmt)) / 8, 16, false);
         if (e != cudaSuccess) return e;
     }
-    k.w = (const uint8_t *)c.w; k.xq = xq; k.y = c.y; k.rows = rows; k.pitch = pitch; k.cols = cols; k.ystride = c.ystride; k.P = P; k.ntg = ntg;
-    k.fmt = fmt; k.accumulate = c.accumulate; k.status = status; k.chunk_blks = kChunkBlks;
-    k.cnt = c.cnt; k.col_off = c.col_off; k.out_idx = c.out_idx;
-    k.slot_bytes = fmt == FMT_Q4_K ? kSlot4 : kSlot6;
-    const size_t limit = 227 * 1024 - 1024;
-    const int groups = nx_groups();
-    const size_t xbytes = (size_t)std::min(nblk, kChunkBlks) * ntg * kXqBlk;
-    const size_t uacc = nchunk > 1 ? (size_t)my_units_max * 128 * 4 : 0;
-    auto layout = [&](uint32_t ns, size_t &x_off, size_t &uacc_off, size_t &ring_off) {
-        x_off = nx_head_bytes(ns, groups);
-        uacc_off = (x_off + xbytes + 15) & ~(size_t)15;
-        ring_off = (uacc_off + uacc + 1023) & ~(size_t)1023;
-        return ring_off + (size_t)ns * k.slot_bytes;
-    };
-    size_t xo, uo, ro;
-    uint32_t nslots = 2;
-    if (layout(nslots, xo, uo, ro) > limit) return cudaErrorNotSupported;
-    while (nslots < 32 && layout(nslots + 1, xo, uo, ro) <= limit) ++nslots;
-    const size_t smem = layout(nslots, xo, uo, ro);
-    k.nslots = nslots; k.x_off = (uint32_t)xo; k.uacc_off = (uint32_t)uo; k.ring_off = (uint32_t)ro;
-    const dim3 block((groups * kCW + 2) * 32);
-    const bool pdl = c.pdl != 0;
-    if (groups == 2) {
-        if (ntg == 1) return launch_kernel(matmul_tc_nx_kernel<1, 2>, dim3(grid), block, smem, stream, pdl, k);
-        return launch_kernel(matmul_tc_nx_kernel<2, 2>, dim3(grid), block, smem, stream, pdl, k);
-    }
-    if (ntg == 1) return launch_kernel(matmul_tc_nx_kernel<1, 1>, dim3(grid), block, smem, stream, pdl, k);
-    return launch_kernel(matmul_tc_nx_kernel<2, 1>, dim3(grid), block, smem, stream, pdl, k);
+    uint64_t line = 0, items = 0;
+    for (uint32_t s = 0; s < p.parts; ++s)   // the tensors of a part side by side: those of one format share its activation
+        for (int i = 0; i < n; ++i) {
+            NxJob &j = k.job[k.n_jobs++];
+            j.tensor = (uint16_t)i; j.part = (uint16_t)s; j.seg0 = (uint16_t)(s * p.segs); j.nseg = (uint16_t)std::min(p.segs, nseg - s * p.segs);
+            j.base = (uint32_t)line; j.cost = (t[i].fmt == FMT_Q4_K ? 2u : t[i].fmt == FMT_Q6_K ? 3u : 4u) * j.nseg;   // as the segments' bytes, roughly
+            line += (uint64_t)k.t[i].units * j.cost;
+            items += k.t[i].units;
+        }
+    if (line * (in.table ? in.n_groups : 1) >= (1ull << 31)) return cudaErrorNotSupported;
+    k.group_cost = (uint32_t)line; k.nblk = nblk; k.P = P; k.xq = xq; k.accumulate = accumulate;
+    k.rms = in.wnorm ? 1 : 0; k.eps = in.eps;
+    k.red_group = kCW * ((P + 3) / 4) * 64;
+    k.slot_bytes = p.slot_bytes; k.x_off = p.x_off; k.x_blk_tg = p.x_blk_tg;
+    k.table = in.table; k.out_idx = in.out_idx; k.list_stride = in.list_stride; k.col_off = in.col_off; k.table_ready = in.table_ready;
+    k.status = status;
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(items * (in.table ? in.n_groups : 1), (uint64_t)sms);
+    if ((uint64_t)k.n_jobs * (in.table ? in.n_groups : 1) / grid + 2 > kMaxPieces) return cudaErrorNotSupported;
+    return launch_kernel(kernel, dim3(grid), dim3(kThreads), kSmemLimit, stream, pdl, k);
+}
+
+cudaError_t launch_reduce_parts(const float *part, size_t part_stride, uint32_t n_parts, float *y, uint32_t rows, uint32_t ystride,
+                                uint32_t P, int accumulate, cudaStream_t stream, bool pdl) {
+    return launch_kernel(reduce_parts_kernel, dim3((rows + 255) / 256, P), dim3(256), 0, stream, pdl, part, part_stride, n_parts, y, rows,
+                         ystride, accumulate);
 }
 
 } // namespace flb

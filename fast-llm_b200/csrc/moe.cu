@@ -7,10 +7,10 @@
 // (src/model/decoder.cpp:925-1045) and has no multi-GPU form.
 //
 // The tokens of a block are grouped by expert on the device (a stable counting sort of the (token, slot)
-// pairs), and each of this rank's experts is walked ONCE per block: gate, up and down run as multi-column
-// matmuls (matvec_tc_nx.cu) over the tokens that chose the expert, up to 8 per pass, with the token list
-// and its length read on the device (an expert nobody chose costs launches that return at entry, no
-// weight traffic). The reference describes the same grouping for its task graph ("one tile set per
+// pairs), and each of this rank's experts is walked ONCE per block: gate and up of all experts are one grouped
+// multi-column matmul launch (matvec_tc_nx.cu) over the tokens that chose each expert, up to 16 per expert and pass, down
+// is another, with the active experts and their token lists read on the device (an expert nobody chose costs
+// nothing). The reference describes the same grouping for its task graph ("one tile set per
 // DISTINCT expert serving every position that routed to it", src/model/decoder.cpp:927-930).
 //
 // Expert parallel: rank r of w holds experts [r * n / w, (r + 1) * n / w). The hidden states are
@@ -20,6 +20,7 @@
 // every rank ends with identical bits). That sum is the combine half.
 #include "capi_internal.h"
 
+#include <algorithm>
 #include <cstdlib>
 
 using namespace flb;
@@ -33,6 +34,9 @@ struct fl_b200_moe {
     float *logits = nullptr, *gates = nullptr, *mgates = nullptr, *g = nullptr, *u = nullptr, *part = nullptr, *partial = nullptr;
     uint32_t *ids = nullptr, *lids = nullptr;
     uint32_t *cnt = nullptr, *tok_list = nullptr, *pair_list = nullptr;   // the pairs grouped by local expert (launch_group_by_expert)
+    uint32_t *table = nullptr;                                            // active experts of a grouped launch
+    uint8_t *xq = nullptr;                                                // converted activations of all active experts
+    uint32_t tgs = 0, planes_gu = 0, planes_d = 0;                        // token groups in xq; planes of partial results in g, u / part
     uint8_t *comm = nullptr;
     uint8_t *peers[kCommMaxRanks] = {};
     bool peers_set = false;
@@ -126,12 +130,26 @@ int fl_b200_moe_create(fl_b200_ctx *ctx, const fl_b200_moe_cfg *cfg, uint32_t ra
     if (int rc = alloc((void **)&m->mgates, T * K * 4)) return fail(rc);
     if (int rc = alloc((void **)&m->ids, T * K * 4)) return fail(rc);
     if (int rc = alloc((void **)&m->lids, T * K * 4)) return fail(rc);
-    if (int rc = alloc((void **)&m->g, T * K * F * 4)) return fail(rc);   // gate / up outputs, one row per (token, slot) pair
-    if (int rc = alloc((void **)&m->u, T * K * F * 4)) return fail(rc);
+    // the most planes of partial results any number of tokens leads to (0: the per-slot form serves the shape)
+    for (uint32_t P = 1; P <= kNxMaxTokens && P <= T; ++P) {
+        const NxTensor gu{c.fmt_gate_up, nullptr, (uint32_t)F, 0, nullptr, 0, 0}, dn{c.fmt_down, nullptr, (uint32_t)E, 0, nullptr, 0, 0};
+        const NxTensor two[2] = {gu, gu};
+        const uint32_t a = matmul_tc_nx_parts(two, 2, c.n_embd, P, true), b = matmul_tc_nx_parts(&dn, 1, c.n_ff, P, true);
+        if (a == 0 || b == 0) { m->planes_gu = m->planes_d = 0; break; }
+        m->planes_gu = std::max(m->planes_gu, a);
+        m->planes_d = std::max(m->planes_d, b);
+    }
+    const size_t n_gu = std::max(1u, m->planes_gu), n_d = std::max(1u, m->planes_d);
+    if (int rc = alloc((void **)&m->g, n_gu * T * K * F * 4)) return fail(rc);   // gate / up outputs, one row per (token, slot) pair
+    if (int rc = alloc((void **)&m->u, n_gu * T * K * F * 4)) return fail(rc);
+    // every active expert has at most 16 columns in a pass, all of them together at most one per pair
+    m->tgs = (uint32_t)std::min<size_t>((size_t)m->n_local * (kNxMaxTokens / 4), T * K / 4 + std::min<size_t>(m->n_local, T * K));
+    if (int rc = alloc((void **)&m->xq, matmul_tc_nx_scratch_bytes((uint32_t)std::max(E, F), m->tgs, 1))) return fail(rc);
+    if (int rc = alloc((void **)&m->table, (1 + (size_t)m->n_local) * 16)) return fail(rc);
     if (int rc = alloc((void **)&m->cnt, (size_t)m->n_local * 4)) return fail(rc);
     if (int rc = alloc((void **)&m->tok_list, (size_t)m->n_local * T * 4)) return fail(rc);
     if (int rc = alloc((void **)&m->pair_list, (size_t)m->n_local * T * 4)) return fail(rc);
-    if (int rc = alloc((void **)&m->part, T * K * E * 4)) return fail(rc);
+    if (int rc = alloc((void **)&m->part, n_d * T * K * E * 4)) return fail(rc);
     if (world > 1) {
         if (int rc = alloc((void **)&m->partial, T * E * 4)) return fail(rc);
         if (int rc = alloc((void **)&m->comm, comm_buffer_bytes())) return fail(rc);
@@ -147,7 +165,7 @@ void fl_b200_moe_destroy(fl_b200_moe *m) {
     cudaSetDevice(m->ctx->device);
     cudaStreamSynchronize(m->ctx->stream);
     cudaFree(m->logits); cudaFree(m->gates); cudaFree(m->mgates); cudaFree(m->ids); cudaFree(m->lids); cudaFree(m->g);
-    cudaFree(m->cnt); cudaFree(m->tok_list); cudaFree(m->pair_list);
+    cudaFree(m->table); cudaFree(m->xq); cudaFree(m->cnt); cudaFree(m->tok_list); cudaFree(m->pair_list);
     cudaFree(m->u); cudaFree(m->part); cudaFree(m->partial); cudaFree(m->comm); cudaFree(m->comm_state);
     if (m->rec.exec) cudaGraphExecDestroy(m->rec.exec);
     if (m->rec.graph) cudaGraphDestroy(m->rec.graph);
@@ -182,7 +200,8 @@ int fl_b200_moe_set_peers(fl_b200_moe *m, void *const *bufs, uint32_t n) {
     return FL_B200_OK;
 }
 
-static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y);
+static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y, const float *wnorm = nullptr, float eps = 0.f,
+                       const float *resid = nullptr);
 
 int fl_b200_moe_forward(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y) {
     if (!m || !x || !y) return set_err(FL_B200_ERR_ARG, "moe_forward: null pointer");
@@ -219,7 +238,7 @@ int fl_b200_moe_forward(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y
 
 // One gate | up launch and one down launch per (token, slot) through the expert-indexed one-column matvec: the form
 // for shapes the multi-column matmul does not take (rows that are not 16-byte pitched, e.g. Q6_K with 1024 columns).
-// wnorm / resid (one token, inside a decoder step): x is the raw hidden state, normed on the fly by the router kernel
+// wnorm / resid (one GPU, inside a decoder step): x is the raw hidden state, normed on the fly by the router kernel
 // and by the gate | up launch's prologue, and y = resid + the block's output (the merge's add1 term).
 static int moe_enqueue_per_slot(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y, const float *wnorm = nullptr,
                                 float eps = 0.f, const float *resid = nullptr) {
@@ -270,7 +289,7 @@ static int moe_enqueue_per_slot(fl_b200_moe *m, const float *x, uint32_t n_tok, 
             }
         }
         float *dst = (m->world > 1 ? m->partial : y) + (size_t)t * E;
-        CKM(launch_wmerge(m->part + (size_t)t * K * E, m->mgates + (size_t)t * K, m->world > 1 ? nullptr : resid, nullptr, dst, 1.0f, K, E, K, s));
+        CKM(launch_wmerge(m->part + (size_t)t * K * E, m->mgates + (size_t)t * K, m->world > 1 || !resid ? nullptr : resid + (size_t)t * E, nullptr, dst, 1.0f, K, E, K, s));
     }
     if (m->world > 1) {
         for (uint32_t t = 0; t < n_tok; ++t) {   // the combine: sum of the ranks' partial outputs, rank order
@@ -287,48 +306,49 @@ static int moe_enqueue_per_slot(fl_b200_moe *m, const float *x, uint32_t n_tok, 
 // the multi-column launches of the block as programmatic dependents of one another (FLB_MOE_PDL=0: plain launches)
 static const int kMoePdlNx = getenv("FLB_MOE_PDL") ? atoi(getenv("FLB_MOE_PDL")) : 1;
 
-static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y) {
+// One token: the one-column kernel walks an expert faster than the multi-column one, which serves at least four columns (whole
+// Mixtral-8x7B-shape step: 3.62 against 3.69 ms).
+static bool moe_per_slot(const fl_b200_moe *m, uint32_t n_tok) { return m->planes_gu == 0 || n_tok == 1; }
+
+// wnorm / resid (one GPU): x is the raw hidden state, normed inside the router kernel and the gate | up conversion, and
+// y = resid + the block's output.
+static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y, const float *wnorm, float eps, const float *resid) {
     fl_b200_ctx *ctx = m->ctx;
     cudaStream_t s = ctx->stream;
     const fl_b200_moe_cfg &c = m->c;
     const uint32_t E = c.n_embd, F = c.n_ff, K = c.top_k, NE = c.n_expert, T = c.max_tokens;
-    const uint64_t stride_gu = (uint64_t)F * row_bytes(c.fmt_gate_up, E), stride_d = (uint64_t)E * row_bytes(c.fmt_down, F);
-    if (row_bytes(c.fmt_gate_up, E) % 16 != 0 || row_bytes(c.fmt_down, F) % 16 != 0)
-        return moe_enqueue_per_slot(m, x, n_tok, y);
-    router_logits_kernel<<<dim3(NE, n_tok), 128, 0, s>>>(m->router, x, m->logits, E, NE);
+    if (moe_per_slot(m, n_tok)) return moe_enqueue_per_slot(m, x, n_tok, y, wnorm, eps, resid);
+    router_logits_kernel<<<dim3(NE, n_tok), 128, 0, s>>>(m->router, x, m->logits, E, NE, wnorm, eps);
     CKM(cudaGetLastError());
     CKM(launch_router_sel(m->logits, m->ids, m->gates, n_tok, NE, K, c.norm, c.scale, s, m->lids, m->mgates, m->base, m->n_local));
-    CKM(launch_group_by_expert(m->lids, n_tok * K, K, m->n_local, T, m->cnt, m->tok_list, m->pair_list, s));
-    // Every local expert once: the tokens that chose it, 8 columns per pass. The lists live on the device, so the
-    // launch sequence is the same for every routing (and can be replayed as a graph); a pass without columns
-    // returns at entry.
-    for (uint32_t e = 0; e < m->n_local; ++e) {
-        const uint32_t *cnt = m->cnt + e, *toks = m->tok_list + (size_t)e * T, *pairs = m->pair_list + (size_t)e * T;
-        for (uint32_t off = 0; off < n_tok; off += 8) {
-            const uint32_t P = n_tok - off < 8 ? n_tok - off : 8;
-            NxCall g{};
-            g.fmt = c.fmt_gate_up; g.w = m->wg + (uint64_t)e * stride_gu; g.rows = F; g.cols = E;
-            g.x = x; g.P = P; g.xstride = E; g.y = m->g; g.ystride = F;
-            g.cnt = cnt; g.col_idx = toks; g.out_idx = pairs; g.col_off = off;
-            g.pdl = kMoePdlNx;
-            cudaError_t er = launch_matmul_tc_nx(g, ctx->xq, ctx->status, ctx->sms, s);
-            if (er == cudaErrorNotSupported) return set_err(FL_B200_ERR_ARG, "moe_forward: shape not taken by the multi-column matmul");
-            CKM(er);
-            NxCall u = g;
-            u.w = m->wu + (uint64_t)e * stride_gu; u.y = m->u; u.skip_convert = 1;   // the same columns, already converted
-            CKM(launch_matmul_tc_nx(u, ctx->xq, ctx->status, ctx->sms, s));
-            NxCall d{};   // down: the column of pair p is silu(g[p]) * u[p], built while it is converted
-            d.fmt = c.fmt_down; d.w = m->wd + (uint64_t)e * stride_d; d.rows = E; d.cols = F;
-            d.x = m->g; d.x2 = m->u; d.P = P; d.xstride = F; d.y = m->part; d.ystride = E;
-            d.cnt = cnt; d.col_idx = pairs; d.out_idx = pairs; d.col_off = off;
-            d.pdl = kMoePdlNx;
-            er = launch_matmul_tc_nx(d, ctx->xq, ctx->status, ctx->sms, s);
-            if (er == cudaErrorNotSupported) return set_err(FL_B200_ERR_ARG, "moe_forward: shape not taken by the multi-column matmul");
-            CKM(er);
-        }
+    CKM(launch_group_by_expert(m->lids, n_tok * K, K, m->n_local, T, m->cnt, m->tok_list, m->pair_list, s, m->table));
+    // Every local expert once for up to 16 of the tokens that chose it. The table and the lists live on the device, so the
+    // launch sequence is the same for every routing (and can be replayed as a graph).
+    uint32_t planes_d = 1;
+    const uint32_t P = std::min(n_tok, kNxMaxTokens);   // every pass is cut into the same parts, the last one too
+    for (uint32_t off = 0; off < n_tok; off += kNxMaxTokens) {
+        if (off) CKM(launch_nx_table(m->cnt, m->n_local, off, P, m->table, s));
+        const NxTensor gu[2] = {{c.fmt_gate_up, m->wg, F, 0, m->g, F, (size_t)T * K * F}, {c.fmt_gate_up, m->wu, F, 0, m->u, F, (size_t)T * K * F}};
+        NxIn in{};
+        in.x = x; in.xstride = E; in.wnorm = wnorm; in.eps = eps;
+        in.table = m->table; in.col_idx = m->tok_list; in.out_idx = m->pair_list; in.list_stride = T; in.col_off = off;
+        in.n_groups = std::min(m->n_local, n_tok * K); in.n_experts = m->n_local;
+        // the first conversion is an ordinary dependent of the kernel that wrote the table; every later launch starts after
+        // it did, so that the table is in place for all of them
+        in.table_ready = kMoePdlNx;
+        CKM(launch_nx_convert(in, gu, 1, E, P, m->xq, m->tgs, s, false));
+        CKM(launch_nx_matmul(in, gu, 2, E, P, 0, m->xq, m->tgs, ctx->status, ctx->sms, s, kMoePdlNx != 0, true));
+        const NxTensor dn{c.fmt_down, m->wd, E, 0, m->part, E, (size_t)T * K * E};   // down: the column of pair p is silu(g[p]) * u[p]
+        in.x = m->g; in.x2 = m->u; in.xstride = F; in.wnorm = nullptr;
+        in.n_parts = matmul_tc_nx_parts(gu, 2, E, P, true); in.part_stride = (size_t)T * K * F;
+        in.col_idx = m->pair_list;
+        CKM(launch_nx_convert(in, &dn, 1, F, P, m->xq, m->tgs, s, kMoePdlNx != 0));
+        CKM(launch_nx_matmul(in, &dn, 1, F, P, 0, m->xq, m->tgs, ctx->status, ctx->sms, s, kMoePdlNx != 0, true));
+        planes_d = matmul_tc_nx_parts(&dn, 1, F, P, true);
     }
     // WMERGE of every token: y[t] = sum_k gate[t][k] * part[t][k] (slots of experts held elsewhere carry gate 0)
-    CKM(launch_wmerge_tokens(m->part, m->mgates, m->world > 1 ? m->partial : y, K, E, n_tok, s));
+    CKM(launch_wmerge_tokens(m->part, m->mgates, m->world > 1 ? m->partial : y, K, E, n_tok, s, planes_d, (size_t)T * K * E,
+                             m->world > 1 ? nullptr : resid));
     if (m->world > 1) {
         for (uint32_t t = 0; t < n_tok; ++t) {   // the combine: sum of the ranks' partial outputs, rank order
             AllReduceArgs r{};
@@ -346,15 +366,13 @@ int flb::moe_enqueue_tokens(fl_b200_moe *m, const float *x, uint32_t n_tok, floa
     if (!m || !m->router || !m->wg) return set_err(FL_B200_ERR_STATE, "moe: weights not set");
     if (n_tok == 0 || n_tok > m->c.max_tokens) return set_err(FL_B200_ERR_ARG, "moe: %u tokens outside 1..%u", n_tok, m->c.max_tokens);
     const fl_b200_moe_cfg &c = m->c;
-    if (n_tok == 1) {
+    if (m->world > 1 && (wnorm || resid)) return set_err(FL_B200_ERR_ARG, "moe: the fused norm / residual form is for one GPU");
+    if (n_launch) {   // as moe_enqueue / moe_enqueue_per_slot enqueue them
         const bool down_streams = matvec_is_streaming(c.fmt_down, c.n_ff) && row_bytes(c.fmt_down, c.n_ff) % 16 == 0;
-        if (n_launch) *n_launch = 2 + c.top_k * (down_streams ? 2u : 3u) + 1 + (m->world > 1 ? 1u : 0u);
-        if (m->world > 1 && (wnorm || resid)) return set_err(FL_B200_ERR_ARG, "moe: the fused norm / residual form is for one GPU");
-        return moe_enqueue_per_slot(m, x, 1, y, wnorm, eps, resid);
+        const uint32_t passes = (n_tok + kNxMaxTokens - 1) / kNxMaxTokens;
+        *n_launch = (!moe_per_slot(m, n_tok) ? 3 + 5 * passes - 1 + 1 : 2 + n_tok * (c.top_k * (down_streams ? 2u : 3u) + 1)) + (m->world > 1 ? n_tok : 0u);
     }
-    if (wnorm || resid) return set_err(FL_B200_ERR_ARG, "moe: the fused norm / residual form takes one token");
-    if (n_launch) *n_launch = 0;   // not counted: the batch pass does not report launches
-    return moe_enqueue(m, x, n_tok, y);
+    return moe_enqueue(m, x, n_tok, y, wnorm, eps, resid);
 }
 fl_b200_ctx *flb::moe_ctx(const fl_b200_moe *m) { return m->ctx; }
 const fl_b200_moe_cfg *flb::moe_cfg(const fl_b200_moe *m) { return &m->c; }
