@@ -143,11 +143,18 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(const __gr
         tma_box(dst + 2 * kHalfBytes, &a.vmap, 0, r, &sm.full[slot]);
         tma_box(dst + 3 * kHalfBytes, &a.vmap, 64, r, &sm.full[slot]);
     };
-    // Older cache rows never change: request the first tiles while the previous kernel still runs.
-    if (tid == 0)
-        for (uint32_t i = 0; i < (uint32_t)kStages && i < n_tiles; ++i) issue(i);
+    // Older cache rows never change: request the first tiles while the previous kernel still runs. Fused, the current row
+    // is patched in later; otherwise the kernel before may be the one that appends the rows from *pos on (of the first
+    // position, where several share the cache), and tiles that hold any of them wait for it.
+    uint32_t early = 0;
+    if (tid == 0) {
+        const uint32_t old = fused ? 0xFFFFFFFFu : a.pos ? (uint32_t)a.pos[b * a.pos_stride] : 0u;   // rows known to be complete
+        for (; early < (uint32_t)kStages && early < n_tiles && (t0 + early + 1) * kTile <= old; ++early) issue(early);
+    }
 
     griddep_wait();   // q (and, fused, this token's k and v) come from the previous kernel
+    if (tid == 0)
+        for (uint32_t i = early; i < (uint32_t)kStages && i < n_tiles; ++i) issue(i);
     if (tid == 0) trace_min(a.trace, 1);
 
     // ---- q as the B operand of the score MMAs: column n = g is head g/2, part g&1 (hi / lo);
@@ -155,7 +162,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(const __gr
     uint32_t qb[8][2];
     {
         const uint32_t h = g >> 1, part = g & 1u;
-        const float *qg = a.q + ((uint64_t)b * a.n_q_head + (uint64_t)hkv * group + h) * kD;
+        const float *qg = a.q + (uint64_t)b * (a.q_stride ? a.q_stride : a.n_q_head * kD) + ((uint64_t)hkv * group + h) * kD;
 #pragma unroll
         for (int kb = 0; kb < 8; ++kb)
 #pragma unroll

@@ -101,6 +101,12 @@ struct fl_b200_decoder {
         float *x = nullptr, *xn = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *att = nullptr, *g = nullptr, *u = nullptr;
         float *logits = nullptr, *margin = nullptr, *part = nullptr;
         float *partial = nullptr, *top3 = nullptr;   // tensor parallel: this rank's partial O / down outputs, argmax records
+        // The pass over the multi-column kernel (nx): outputs as planes of partial sums (qkv: [planes][m][Q | K | V] rows; the
+        // others [planes][m][rows]), the positions' rotation tables, argmax scratch and tickets per token.
+        bool nx = false;
+        float *qkv = nullptr, *planes = nullptr, *gp = nullptr, *up = nullptr, *head = nullptr, *am = nullptr;
+        uint32_t *am_tickets = nullptr;
+        float2 *rope = nullptr;
         int32_t *io = nullptr;              // [0..8) tokens, [8..16) positions, [16..24) greedy next tokens
         uint32_t *tickets = nullptr;
         int32_t *h_io = nullptr;            // pinned image of io, then the 8 margins
@@ -444,6 +450,8 @@ void fl_b200_decoder_destroy(fl_b200_decoder *d) {
     cudaFree(d->b.x); cudaFree(d->b.xn); cudaFree(d->b.q); cudaFree(d->b.k); cudaFree(d->b.v); cudaFree(d->b.att);
     cudaFree(d->b.g); cudaFree(d->b.u); cudaFree(d->b.logits); cudaFree(d->b.margin); cudaFree(d->b.part);
     cudaFree(d->b.io); cudaFree(d->b.tickets); cudaFree(d->b.partial); cudaFree(d->b.top3);
+    cudaFree(d->b.qkv); cudaFree(d->b.planes); cudaFree(d->b.gp); cudaFree(d->b.up); cudaFree(d->b.head);
+    cudaFree(d->b.am); cudaFree(d->b.am_tickets); cudaFree(d->b.rope);
     cudaFreeHost(d->b.h_io);
     cudaFreeHost(d->h_pin);
     delete d;
@@ -679,8 +687,44 @@ int fl_b200_decoder_verify(fl_b200_decoder *d, int32_t first_token, const int32_
 // Passes of fewer tokens than this run as teacher-forced single steps (FLB_BATCH_MIN overrides; 1 = always the batch pass).
 static const uint32_t kBatchMin = getenv("FLB_BATCH_MIN") ? (uint32_t)atoi(getenv("FLB_BATCH_MIN")) : 4u;
 
+// The multi-column launches of a layer's matvec groups, without their outputs (0: Q | K | V, 1: O, 2: gate | up, 3: down) and
+// of the head (4). Returns the number of tensors.
+static int nx_group(const fl_b200_decoder *d, uint32_t layer, int group, NxTensor *t, uint32_t *cols) {
+    const uint32_t E = d->c.n_embd, D = d->c.head_dim, QD = d->Hq * D, KD = d->Hkv * D, F = d->F;
+    const Tensor *w = group == 4 ? nullptr : &d->lw[(size_t)layer * 7];
+    auto set = [&](int i, const Tensor &x, uint32_t rows) { t[i] = NxTensor{x.fmt, x.w, rows, x.pitch, nullptr, 0, 0}; };
+    *cols = group == 1 ? QD : group == 3 ? F : E;
+    switch (group) {
+    case 0: set(0, w[FL_B200_T_WQ], QD); set(1, w[FL_B200_T_WK], KD); set(2, w[FL_B200_T_WV], KD); return 3;
+    case 1: set(0, w[FL_B200_T_WO], E); return 1;
+    case 2: set(0, w[FL_B200_T_GATE], F); set(1, w[FL_B200_T_UP], F); return 2;
+    case 3: set(0, w[FL_B200_T_DOWN], E); return 1;
+    default: set(0, d->output, d->V); return 1;
+    }
+}
+
+// The pass runs on the multi-column kernel when it takes every tensor; then planes[g] is the most planes of partial results
+// any number of tokens leads to in group g.
+static bool nx_eligible(const fl_b200_decoder *d, uint32_t *planes) {
+    NxTensor t[3];
+    uint32_t cols;
+    for (int g = 0; g < 5; ++g) planes[g] = 1;
+    for (uint32_t l = 0; l < d->c.n_layer; ++l)
+        for (int g = 0; g < 5; ++g) {
+            if ((d->moe[l] && (g == 2 || g == 3)) || (g == 4 && l > 0)) continue;
+            const int n = nx_group(d, l, g, t, &cols);
+            for (uint32_t m = 1; m <= FL_B200_MAX_BATCH; ++m) {
+                const uint32_t parts = matmul_tc_nx_parts(t, n, cols, m, g != 4);
+                if (parts == 0) return false;
+                planes[g] = std::max(planes[g], parts);
+            }
+        }
+    return true;
+}
+
 static int batch_alloc(fl_b200_decoder *d) {
     if (d->b.ready) return FL_B200_OK;
+    static_assert(FL_B200_MAX_BATCH <= (int)kNxMaxTokens, "a batch pass is one multi-column pass");
     const fl_b200_llama_cfg &c = d->c;
     const size_t M = FL_B200_MAX_BATCH, E = c.n_embd, QD = (size_t)d->Hq * c.head_dim, KD = (size_t)d->Hkv * c.head_dim;
     CK(cudaMalloc(&d->b.x, M * E * 4)); CK(cudaMalloc(&d->b.xn, M * E * 4));
@@ -699,14 +743,149 @@ static int batch_alloc(fl_b200_decoder *d) {
     CK(cudaMalloc(&d->b.io, 3 * FL_B200_MAX_BATCH * sizeof(int32_t)));
     CK(cudaMalloc(&d->b.tickets, (size_t)d->Hkv * M * sizeof(uint32_t)));
     CK(cudaMemset(d->b.tickets, 0, (size_t)d->Hkv * M * sizeof(uint32_t)));
+    uint32_t pl[5];
+    d->b.nx = nx_eligible(d, pl);
+    if (d->b.nx) {
+        CK(cudaMalloc(&d->b.qkv, pl[0] * M * (QD + 2 * KD) * 4));
+        CK(cudaMalloc(&d->b.planes, std::max(pl[1], pl[3]) * M * E * 4));
+        CK(cudaMalloc(&d->b.gp, pl[2] * M * (size_t)d->F * 4));
+        CK(cudaMalloc(&d->b.up, pl[2] * M * (size_t)d->F * 4));
+        if (pl[4] > 1) CK(cudaMalloc(&d->b.head, pl[4] * M * (size_t)d->V * 4));
+        CK(cudaMalloc(&d->b.am, M * kArgmaxScratch * 4));
+        CK(cudaMalloc(&d->b.am_tickets, M * 4));
+        CK(cudaMemset(d->b.am_tickets, 0, M * 4));
+        CK(cudaMalloc(&d->b.rope, M * (c.head_dim / 2) * sizeof(float2)));
+    }
     CK(cudaMallocHost(&d->b.h_io, 4 * FL_B200_MAX_BATCH * sizeof(int32_t)));
     d->b.ready = true;
     return FL_B200_OK;
 }
 
+// The batch pass on the multi-column kernel: per layer 4 activation conversions (the first and third also add the planes of
+// the matmul before to the residual stream and take the norm's weights, the fourth adds the planes of gate and up and
+// takes SiLU(gate) * up), 4 matmuls, RoPE + append, attention; all of them programmatic dependents of one another.
+static int enqueue_batch_nx(fl_b200_decoder *d, uint32_t m, cudaStream_t s, bool seqs) {
+    const fl_b200_llama_cfg &c = d->c;
+    fl_b200_ctx *ctx = d->ctx;
+    const uint32_t E = c.n_embd, D = c.head_dim, QD = d->Hq * D, KD = d->Hkv * D, F = d->F, V = d->V, QKV = QD + 2 * KD;
+    const float theta_scale = powf(c.rope_base, -2.0f / (float)D);
+    static const bool pdl = !(getenv("FLB_BATCH_PDL") && getenv("FLB_BATCH_PDL")[0] == '0');
+    auto &b = d->b;
+    const bool tp = d->tp_size > 1;
+    const int32_t *tok = b.io, *pos = b.io + FL_B200_MAX_BATCH;
+    int32_t *next = b.io + 2 * FL_B200_MAX_BATCH;
+    uint32_t pending = 0;   // planes of the matmul before that still have to be added to b.x
+    auto normed = [&](const float *wnorm) {   // RMSNorm of the residual stream, with what is pending added to it first
+        NxIn in{};
+        in.xstride = in.rstride = E; in.wnorm = wnorm; in.eps = c.eps;
+        if (pending) { in.x = b.planes; in.n_parts = pending; in.part_stride = (size_t)m * E; in.resid = in.x_out = b.x; }
+        else in.x = b.x;
+        pending = 0;
+        return in;
+    };
+    // one matvec group: convert the activation, walk the weights
+    auto group = [&](const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t *parts, bool split = true) -> int {
+        *parts = matmul_tc_nx_parts(t, n, cols, m, split);
+        CK(launch_nx_convert(in, t, n, cols, m, ctx->xq, kNxTgs, s, pdl));
+        CK(launch_nx_matmul(in, t, n, cols, m, 0, ctx->xq, kNxTgs, ctx->status, ctx->sms, s, pdl, split));
+        return FL_B200_OK;
+    };
+    // the output of O / down: planes to be added by the next conversion; tensor parallel: summed over the ranks here
+    auto residual = [&](uint32_t parts) -> int {
+        pending = parts;
+        if (!tp) return FL_B200_OK;
+        CK(launch_reduce_parts(b.planes, (size_t)m * E, parts, b.partial, E, E, m, 0, s, pdl));
+        for (uint32_t i = 0; i < m; ++i) {
+            AllReduceArgs r{};
+            for (uint32_t p = 0; p < d->tp_size; ++p) r.peers[p] = d->peers[p];
+            r.in = b.partial + (size_t)i * E; r.resid = b.x + (size_t)i * E; r.out = b.x + (size_t)i * E; r.n = E;
+            r.rank = d->tp_rank; r.world = d->tp_size; r.st = CommState{d->comm_state}; r.status = ctx->status; r.wait_ns = ctx->wait_limit_ns;
+            CK(launch_allreduce_resid(r, s, false));
+        }
+        pending = 0;
+        return FL_B200_OK;
+    };
+    NxTensor t[3];
+    uint32_t cols, parts;
+    CK(launch_rope_table(pos, theta_scale, D, b.rope, s, m));
+    CK(launch_embed(d->tok_embd.fmt, d->tok_embd.w, tok, E, b.x, s, false, m));
+    for (uint32_t l = 0; l < c.n_layer; ++l) {
+        int n = nx_group(d, l, 0, t, &cols);
+        const uint32_t at[3] = {0, QD, QD + KD};
+        for (int i = 0; i < n; ++i) { t[i].y = b.qkv + at[i]; t[i].ystride = QKV; t[i].part_stride = (size_t)m * QKV; }
+        if (int rc = group(normed(d->attn_norm[l]), t, n, cols, &parts)) return rc;
+        {   // rotate q and k of every token by its own position, append k and v
+            RopeAppendArgs r{};
+            r.q = b.qkv; r.k = b.qkv + QD; r.v = b.qkv + QD + KD; r.kcache = seqs ? d->sq.kc[l] : d->kc[l]; r.vcache = seqs ? d->sq.vc[l] : d->vc[l];
+            r.pos = pos; r.seq_elems = seqs ? (uint64_t)d->Hkv * c.max_kv * D : 0;
+            r.n_q_head = d->Hq; r.n_kv_head = d->Hkv; r.head_dim = D; r.kv_stride = c.max_kv; r.theta_scale = theta_scale;
+            r.n_tok = m; r.q_tok_stride = QKV; r.kv_tok_stride = QKV; r.n_planes = parts; r.plane_stride = (uint64_t)m * QKV;
+            r.table = b.rope; r.pdl = pdl;
+            CK(launch_rope_append(r, s));
+        }
+        NxIn in{};
+        {
+            AttnArgs a{};
+            a.q = b.qkv; a.q_stride = QKV; a.k = seqs ? d->sq.kc[l] : d->kc[l]; a.v = seqs ? d->sq.vc[l] : d->vc[l]; a.out = b.att; a.part = b.part;
+            a.tickets = b.tickets; a.pos = pos; a.kv_len = 0; a.kv_len_step = seqs ? 0 : 1; a.shared_kv = seqs ? 0 : 1; a.pos_stride = seqs ? 1 : 0;
+            a.kv_stride = c.max_kv; a.batch_stride = (uint64_t)d->Hkv * c.max_kv * D;
+            a.n_q_head = d->Hq; a.n_kv_head = d->Hkv; a.batch = m;
+            a.n_splits = attn_pick_splits(d->Hkv, m, c.max_kv, ctx->sms);
+            a.scale = 1.0f / sqrtf((float)D); a.status = ctx->status; a.pdl = pdl;
+            CK(attn_make_maps(a));
+            CK(launch_attn_decode(a, s));
+        }
+        in.x = b.att; in.xstride = QD;
+        n = nx_group(d, l, 1, t, &cols);
+        t[0].y = b.planes; t[0].ystride = E; t[0].part_stride = (size_t)m * E;
+        if (int rc = group(in, t, n, cols, &parts)) return rc;
+        if (int rc = residual(parts)) return rc;
+        if (d->moe[l]) {   // every expert once for the tokens that chose it, norm and residual inside the block
+            if (pending) {
+                const NxIn sum = normed(nullptr);
+                CK(launch_nx_convert(sum, t, 0, E, m, nullptr, 0, s, pdl));
+            }
+            if (!tp) {
+                if (int rc = moe_enqueue_tokens(d->moe[l], b.x, m, b.x, nullptr, d->ffn_norm[l], c.eps, b.x)) return rc;
+            } else {
+                CK(launch_rmsnorm(b.x, d->ffn_norm[l], b.xn, c.eps, E, s, m, E));
+                if (int rc = moe_enqueue_tokens(d->moe[l], b.xn, m, b.q, nullptr)) return rc;
+                CK(launch_add2(b.x, b.q, b.x, m * E, s));
+            }
+            continue;
+        }
+        n = nx_group(d, l, 2, t, &cols);
+        t[0].y = b.gp; t[1].y = b.up;
+        for (int i = 0; i < n; ++i) { t[i].ystride = F; t[i].part_stride = (size_t)m * F; }
+        if (int rc = group(normed(d->ffn_norm[l]), t, n, cols, &parts)) return rc;
+        in = NxIn{};
+        in.x = b.gp; in.x2 = b.up; in.xstride = F; in.n_parts = parts; in.part_stride = (size_t)m * F;
+        n = nx_group(d, l, 3, t, &cols);
+        t[0].y = b.planes; t[0].ystride = E; t[0].part_stride = (size_t)m * E;
+        if (int rc = group(in, t, n, cols, &parts)) return rc;
+        if (int rc = residual(parts)) return rc;
+    }
+    const int n = nx_group(d, 0, 4, t, &cols);
+    parts = matmul_tc_nx_parts(t, n, cols, m);
+    t[0].y = parts > 1 ? b.head : b.logits; t[0].ystride = V; t[0].part_stride = (size_t)m * V;
+    if (int rc = group(normed(d->out_norm), t, n, cols, &parts, false)) return rc;
+    if (parts > 1) CK(launch_reduce_parts(b.head, (size_t)m * V, parts, b.logits, V, V, m, 0, s, pdl));
+    CK(launch_argmax(b.logits, V, next, b.margin, b.am, b.am_tickets, ctx->sms, s, pdl, tp ? b.top3 : nullptr, m));
+    for (uint32_t i = 0; tp && i < m; ++i) {   // merge the ranks' (best, index, runner-up) of this position: the same token on every rank
+        TopExchangeArgs x{};
+        for (uint32_t p = 0; p < d->tp_size; ++p) x.peers[p] = d->peers[p];
+        x.top3 = b.top3 + 4 * i; x.index_base = d->tp_rank * V; x.out_idx = next + i; x.out_margin = b.margin + i;
+        x.rank = d->tp_rank; x.world = d->tp_size; x.st = CommState{d->comm_state}; x.status = ctx->status; x.wait_ns = ctx->wait_limit_ns;
+        CK(launch_argmax_exchange(x, s, false));
+    }
+    return FL_B200_OK;
+}
+
 // seqs: the m tokens belong to m independent sequences (token i -> sequence i at its own position, its own cache)
-// instead of m consecutive positions of the one sequence.
+// instead of m consecutive positions of the one sequence. The general form, tensor by tensor: for models with a tensor
+// that the multi-column kernel does not take.
 static int enqueue_batch(fl_b200_decoder *d, uint32_t m, cudaStream_t s, bool seqs = false) {
+    if (d->b.nx) return enqueue_batch_nx(d, m, s, seqs);
     const fl_b200_llama_cfg &c = d->c;
     fl_b200_ctx *ctx = d->ctx;
     const uint32_t E = c.n_embd, D = c.head_dim, QD = d->Hq * D, KD = d->Hkv * D, F = d->F, V = d->V;

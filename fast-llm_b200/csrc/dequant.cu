@@ -34,8 +34,11 @@ __global__ void __launch_bounds__(256) dequant_kernel(const uint8_t *__restrict_
     griddep_launch_dependents();
     griddep_wait();
     // Row gather (embedding lookup): start at row *sel of a table whose rows are
-    // sel_stride bytes apart.
-    if (sel != nullptr) w += (uint64_t)(*sel) * sel_stride;
+    // sel_stride bytes apart (block row y: row sel[y], output row y).
+    if (sel != nullptr) {
+        w += (uint64_t)sel[blockIdx.y] * sel_stride;
+        out += (uint64_t)blockIdx.y * n4 * 4;
+    }
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n4;
          t += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t e = t * 4;
@@ -120,20 +123,20 @@ cudaError_t launch_dequant(int fmt, const void *w, uint64_t rows, uint32_t cols,
     return cudaGetLastError();
 }
 
-// Embedding lookup: out[0..cols) = dequant(row *token of the table), the device
+// Embedding lookup: out[i][0..cols) = dequant(row token[i] of the table), i < n_tok, the device
 // version of the host step in Decoder::step_batch (src/model/decoder.cpp:1194-1201).
 cudaError_t launch_embed(int fmt, const void *table, const int32_t *token, uint32_t cols, float *out,
-                         cudaStream_t stream, bool pdl) {
+                         cudaStream_t stream, bool pdl, uint32_t n_tok) {
     const uint64_t n4 = cols / 4;
-    const int grid = (int)((n4 + 255) / 256);
+    const dim3 grid((unsigned)((n4 + 255) / 256), n_tok);
     const uint8_t *wp = static_cast<const uint8_t *>(table);
     const uint64_t rb = row_bytes(fmt, cols);
     switch (fmt) {
-    case FMT_F32: return launch_kernel(dequant_kernel<FMT_F32>, dim3(grid), dim3(256), 0, stream, pdl, wp, out, n4, token, rb);
-    case FMT_Q8_0: return launch_kernel(dequant_kernel<FMT_Q8_0>, dim3(grid), dim3(256), 0, stream, pdl, wp, out, n4, token, rb);
-    case FMT_Q5_0: return launch_kernel(dequant_kernel<FMT_Q5_0>, dim3(grid), dim3(256), 0, stream, pdl, wp, out, n4, token, rb);
-    case FMT_Q4_K: return launch_kernel(dequant_kernel<FMT_Q4_K>, dim3(grid), dim3(256), 0, stream, pdl, wp, out, n4, token, rb);
-    case FMT_Q6_K: return launch_kernel(dequant_kernel<FMT_Q6_K>, dim3(grid), dim3(256), 0, stream, pdl, wp, out, n4, token, rb);
+    case FMT_F32: return launch_kernel(dequant_kernel<FMT_F32>, grid, dim3(256), 0, stream, pdl, wp, out, n4, token, rb);
+    case FMT_Q8_0: return launch_kernel(dequant_kernel<FMT_Q8_0>, grid, dim3(256), 0, stream, pdl, wp, out, n4, token, rb);
+    case FMT_Q5_0: return launch_kernel(dequant_kernel<FMT_Q5_0>, grid, dim3(256), 0, stream, pdl, wp, out, n4, token, rb);
+    case FMT_Q4_K: return launch_kernel(dequant_kernel<FMT_Q4_K>, grid, dim3(256), 0, stream, pdl, wp, out, n4, token, rb);
+    case FMT_Q6_K: return launch_kernel(dequant_kernel<FMT_Q6_K>, grid, dim3(256), 0, stream, pdl, wp, out, n4, token, rb);
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

@@ -225,21 +225,33 @@ __global__ void __launch_bounds__(128) rope_append_kernel(const RopeAppendArgs a
     const uint32_t n_rot_heads = (a.q ? a.n_q_head : 0) + a.n_kv_head;
     const uint32_t tokn = blockIdx.y;   // token of a batch pass (0 in a single step)
     const uint32_t pos = (uint32_t)a.pos[tokn];
+    auto pair = [&](const float *v, float &x0, float &x1) {   // two neighbours, the planes added in order
+        x0 = v[0]; x1 = v[1];
+        for (uint32_t p = 1; p < a.n_planes; ++p) { x0 += v[p * a.plane_stride]; x1 += v[p * a.plane_stride + 1]; }
+    };
     if (t < n_rot_heads * half) {
         const uint32_t h = t / half, i = t % half;
-        float theta = (float)(int32_t)pos;
-        for (uint32_t k = 0; k < i; ++k) theta = __fmul_rn(theta, a.theta_scale);
-        const float c = cosf(theta), s = sinf(theta);
+        float c, s;
+        if (a.table) {
+            const float2 cs = a.table[(size_t)tokn * half + i];
+            c = cs.x; s = cs.y;
+        } else {
+            float theta = (float)(int32_t)pos;
+            for (uint32_t k = 0; k < i; ++k) theta = __fmul_rn(theta, a.theta_scale);
+            c = cosf(theta); s = sinf(theta);
+        }
         const uint32_t nq = a.q ? a.n_q_head : 0;
         if (h < nq) {
             float *v = a.q + (size_t)tokn * a.q_tok_stride + (size_t)h * a.head_dim + 2 * i;
-            const float x0 = v[0], x1 = v[1];
+            float x0, x1;
+            pair(v, x0, x1);
             v[0] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
             v[1] = __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c));
         } else {
             const uint32_t hk = h - nq;
             const float *v = a.k + (size_t)tokn * a.kv_tok_stride + (size_t)hk * a.head_dim + 2 * i;
-            const float x0 = v[0], x1 = v[1];
+            float x0, x1;
+            pair(v, x0, x1);
             __half *dst = a.kcache + (size_t)tokn * a.seq_elems + ((size_t)hk * a.kv_stride + pos) * a.head_dim + 2 * i;
             dst[0] = __float2half_rn(__fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s)));
             dst[1] = __float2half_rn(__fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c)));
@@ -249,14 +261,18 @@ __global__ void __launch_bounds__(128) rope_append_kernel(const RopeAppendArgs a
         const uint32_t hk = u / half, i = u % half;
         const float *v = a.v + (size_t)tokn * a.kv_tok_stride + (size_t)hk * a.head_dim + 2 * i;
         __half *dst = a.vcache + (size_t)tokn * a.seq_elems + ((size_t)hk * a.kv_stride + pos) * a.head_dim + 2 * i;
-        dst[0] = __float2half_rn(v[0]);
-        dst[1] = __float2half_rn(v[1]);
+        float x0, x1;
+        pair(v, x0, x1);
+        dst[0] = __float2half_rn(x0);
+        dst[1] = __float2half_rn(x1);
     }
 }
 
 __global__ void rope_table_kernel(const int32_t *pos, float theta_scale, uint32_t half, float2 *table) {
     const uint32_t i = threadIdx.x;
     if (i >= half) return;
+    pos += blockIdx.x;
+    table += (size_t)blockIdx.x * half;
     float theta = (float)*pos;
     for (uint32_t k = 0; k < i; ++k) theta = __fmul_rn(theta, theta_scale);
     table[i] = make_float2(cosf(theta), sinf(theta));
@@ -289,6 +305,11 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ l
                                                      float *out_margin, float *scratch, uint32_t *ticket, float *top3) {
     griddep_launch_dependents();
     griddep_wait();
+    const uint32_t row = blockIdx.y;   // one row of logits per block row
+    lg += (size_t)row * n;
+    out_idx += row; out_margin += row; ticket += row;
+    scratch += (size_t)row * kArgmaxScratch;
+    if (top3) top3 += 4 * row;
     __shared__ Top wtop[8];
     __shared__ uint32_t last;
     Top t{-INFINITY, 0xFFFFFFFFu, -INFINITY};
@@ -392,18 +413,19 @@ cudaError_t launch_rope_append(const RopeAppendArgs &a, cudaStream_t stream) {
     return launch_kernel(rope_append_kernel, dim3((n + 127) / 128, a.n_tok ? a.n_tok : 1), dim3(128), 0, stream, a.pdl != 0, a);
 }
 
-cudaError_t launch_rope_table(const int32_t *pos, float theta_scale, uint32_t head_dim, float2 *table, cudaStream_t stream) {
+cudaError_t launch_rope_table(const int32_t *pos, float theta_scale, uint32_t head_dim, float2 *table, cudaStream_t stream,
+                              uint32_t n_tok) {
     if (head_dim == 0 || (head_dim & 1u) || head_dim > 2048) return cudaErrorInvalidValue;
-    rope_table_kernel<<<1, head_dim / 2, 0, stream>>>(pos, theta_scale, head_dim / 2, table);
+    rope_table_kernel<<<n_tok, head_dim / 2, 0, stream>>>(pos, theta_scale, head_dim / 2, table);
     return cudaGetLastError();
 }
 
 cudaError_t launch_argmax(const float *logits, uint32_t n, int32_t *out_idx, float *out_margin,
-                          float *scratch, uint32_t *ticket, int sms, cudaStream_t stream, bool pdl, float *top3) {
+                          float *scratch, uint32_t *ticket, int sms, cudaStream_t stream, bool pdl, float *top3, uint32_t n_tok) {
     uint32_t grid = (n + 255) / 256;
     if (grid > (uint32_t)sms) grid = (uint32_t)sms;
     if (grid == 0) return cudaErrorInvalidValue;
-    return launch_kernel(argmax_kernel, dim3(grid), dim3(256), 0, stream, pdl, logits, n, out_idx, out_margin, scratch,
+    return launch_kernel(argmax_kernel, dim3(grid, n_tok), dim3(256), 0, stream, pdl, logits, n, out_idx, out_margin, scratch,
                          ticket, top3);
 }
 

@@ -171,6 +171,7 @@ cudaError_t matvec_init(void);   // sets the dynamic shared memory attribute onc
 // ---- attn.cu ------------------------------------------------------------
 struct AttnArgs {
     const float *q;        // [batch][n_q_head][128] f32 (post-RoPE unless rope fused)
+    uint32_t q_stride;     // floats between the sequences' queries (0: n_q_head * 128)
     const __half *k;       // [batch][n_kv_head][kv_stride][128] f16
     const __half *v;       // same layout
     float *out;            // [batch][n_q_head][128]
@@ -304,18 +305,24 @@ struct RopeAppendArgs {
     // batch pass: n_tok tokens (0 = 1), token i at q + i * q_tok_stride, k / v + i * kv_tok_stride, position pos[i]
     uint32_t n_tok, q_tok_stride, kv_tok_stride;
     uint64_t seq_elems;    // independent sequences: token i appends to the cache of sequence i, seq_elems halves further (0: one cache)
+    uint32_t n_planes;     // q, k and v are the sums of n_planes planes, plane_stride floats apart (0 = 1); the rotated q goes to the first
+    uint64_t plane_stride;
+    const float2 *table;   // optional: (cos, sin) of token i's angles, head_dim / 2 per token (launch_rope_table)
 };
 cudaError_t launch_rope_append(const RopeAppendArgs &a, cudaStream_t stream);
 // (cos, sin) of pos * theta_scale^i, i < head_dim / 2, with the angle built by repeated multiplication exactly as
 // fl_op_rope_ds2 does (src/runtime/decode_params.h:124-160); table: head_dim / 2 float2.
-cudaError_t launch_rope_table(const int32_t *pos, float theta_scale, uint32_t head_dim, float2 *table, cudaStream_t stream);
+cudaError_t launch_rope_table(const int32_t *pos, float theta_scale, uint32_t head_dim, float2 *table, cudaStream_t stream,
+                              uint32_t n_tok = 1);   // n_tok positions, one table row each
 // Greedy argmax with the reference's tie rule (lowest index) and the
 // top1 - top2 margin. out_idx: int32, out_margin: float; scratch: 2*blocks*2 floats.
 cudaError_t launch_argmax(const float *logits, uint32_t n, int32_t *out_idx, float *out_margin,
                           float *scratch, uint32_t *ticket, int sms, cudaStream_t stream, bool pdl = false,
-                          float *top3 = nullptr);   // top3: optional {best, index bits, runner-up}
-// Embedding row gather + dequant: out[0..cols) = dequant(table row *token).
+                          float *top3 = nullptr,    // top3: optional {best, index bits, runner-up}
+                          uint32_t n_tok = 1);      // rows of logits (n apart); scratch, ticket, outputs and top3 per row
+constexpr uint32_t kArgmaxScratch = 3 * 1024;   // floats of scratch per row
+// Embedding row gather + dequant: out[i][0..cols) = dequant(table row token[i]), i < n_tok.
 cudaError_t launch_embed(int fmt, const void *table, const int32_t *token, uint32_t cols, float *out,
-                         cudaStream_t stream, bool pdl = false);
+                         cudaStream_t stream, bool pdl = false, uint32_t n_tok = 1);
 
 } // namespace flb
