@@ -53,7 +53,8 @@ constexpr int kAttnWarps = 4;        // warp w <-> positions 16w .. 16w+15 of a 
 constexpr int kAttnThreads = kAttnWarps * 32;
 constexpr uint32_t kHalfBytes = kTile * 128;        // one box: 64 rows x 64 f16 (128 bytes), swizzled
 constexpr uint32_t kStageBytes = 4 * kHalfBytes;    // K lo, K hi, V lo, V hi = 32 KB
-constexpr int kPartStride = kD + 4;  // o[128], m, l, pad (keeps o 16-byte aligned)
+constexpr int kPartStride = kAttnRecord;  // o[128], m, l, pad (keeps o 16-byte aligned)
+static_assert(kPartStride == kD + 4, "record");
 
 struct AttnSmem {
     uint8_t ring[kStages][kStageBytes];   // 1024-byte aligned (swizzle atom)
@@ -370,6 +371,201 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(const __gr
     }
 }
 
+// ---- several positions of one sequence (draft verification, prompt chunks): one cache, up to 8 positions per CTA ----
+// Grid = (n_splits, n_kv_head, groups of 8 positions), 8 warps: warp w serves position 8 z + w with its 4 query heads over
+// ALL keys of the CTA's tiles, so that a tile crosses from L2 to an SM once for 8 positions. (One CTA per position, the
+// form above, moved every key 8 times: 25 us per layer at 8 positions over 4096 keys, L2 bound; this one takes 8 us.)
+// Position b attends kv_len + b * kv_len_step keys: keys past its own are masked. The arithmetic is that of
+// attn_decode_kernel; a warp walks a tile's 64 keys as four blocks of 16 with one maximum and one rescaling per tile. No
+// merge between warps: every warp writes the records of its 4 heads. The splits are added by attn_combine_kernel or by the
+// activation conversion of the matmul that reads the contexts (matvec_tc_nx.cu).
+constexpr int kShWarps = 8;
+struct AttnShSmem {
+    uint8_t ring[kStages][kStageBytes];   // 1024-byte aligned (swizzle atom)
+    uint64_t full[kStages];
+};
+
+__global__ void __launch_bounds__(kShWarps * 32, 2) attn_shared_kernel(const __grid_constant__ AttnArgs a) {
+    extern __shared__ uint8_t smem_dyn[];
+    AttnShSmem &sm = *reinterpret_cast<AttnShSmem *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t g = lane >> 2, t = lane & 3u;
+    const uint32_t split = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z * kShWarps + warp;
+    const uint32_t b_last = min(blockIdx.z * kShWarps + kShWarps, a.batch) - 1;
+    griddep_launch_dependents();
+    const uint32_t kv0 = a.pos ? (uint32_t)a.pos[0] + 1u : a.kv_len;
+    const uint32_t kv_max = kv0 + b_last * a.kv_len_step;         // keys the CTA's last position attends
+    const uint32_t kv_len = kv0 + b * a.kv_len_step;              // ... this warp's
+    const uint32_t tiles_total = (kv_max + kTile - 1) / kTile;
+    const uint32_t tps = (tiles_total + a.n_splits - 1) / a.n_splits;
+    const uint32_t t0 = split * tps, t1 = min(t0 + tps, tiles_total), n_tiles = t1 > t0 ? t1 - t0 : 0;
+    const uint32_t row0 = hkv * a.kv_stride;
+
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s) mbar_init(&sm.full[s], 1);
+        fence_barrier_init();
+    }
+    __syncthreads();
+    const uint32_t ring = smem_u32(&sm.ring[0][0]);
+    auto issue = [&](uint32_t i) {   // thread 0 only: tile t0 + i into slot i % kStages
+        const uint32_t slot = i % kStages, r = row0 + (t0 + i) * kTile, dst = ring + slot * kStageBytes;
+        mbar_arrive_expect_tx(&sm.full[slot], kStageBytes);
+        tma_box(dst, &a.kmap, 0, r, &sm.full[slot]);
+        tma_box(dst + kHalfBytes, &a.kmap, 64, r, &sm.full[slot]);
+        tma_box(dst + 2 * kHalfBytes, &a.vmap, 0, r, &sm.full[slot]);
+        tma_box(dst + 3 * kHalfBytes, &a.vmap, 64, r, &sm.full[slot]);
+    };
+    // rows in front of the first position are complete; the kernel before may be the one that appends the others
+    uint32_t early = 0;
+    if (tid == 0) {
+        const uint32_t old = a.pos ? (uint32_t)a.pos[0] : 0u;
+        for (; early < (uint32_t)kStages && early < n_tiles && (t0 + early + 1) * kTile <= old; ++early) issue(early);
+    }
+    griddep_wait();
+    if (tid == 0)
+        for (uint32_t i = early; i < (uint32_t)kStages && i < n_tiles; ++i) issue(i);
+
+    // q as the B operand of the score MMAs, as in attn_decode_kernel
+    uint32_t qb[8][2];
+    {
+        const uint32_t h = g >> 1, part = g & 1u, bq = min(b, b_last);
+        const float *qg = a.q + (uint64_t)bq * (a.q_stride ? a.q_stride : a.n_q_head * kD) + ((uint64_t)hkv * kGroup + h) * kD;
+#pragma unroll
+        for (int kb = 0; kb < 8; ++kb)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float2 v = *reinterpret_cast<const float2 *>(qg + kb * 16 + 2 * t + 8 * j);
+                qb[kb][j] = pack_h2(split_part(v.x * a.scale, part), split_part(v.y * a.scale, part));
+            }
+    }
+    float o[8][4];
+#pragma unroll
+    for (int dt = 0; dt < 8; ++dt) o[dt][0] = o[dt][1] = o[dt][2] = o[dt][3] = 0.f;
+    float m_run = -INFINITY, l_run = 0.f;   // of head t (replicated over g)
+
+    for (uint32_t it = 0; it < n_tiles; ++it) {
+        const uint32_t slot = it % kStages, p0 = (t0 + it) * kTile;
+        const uint32_t st = ring + slot * kStageBytes;
+        if (!mbar_wait_bounded(&sm.full[slot], (it / kStages) & 1u, a.status)) return;
+        if (kv_max - p0 < (uint32_t)kTile) {
+            // ragged end: rows past every position's keys may hold anything (even NaN): clear them in V so that 0 * V stays 0
+            for (uint32_t k = (kv_max - p0) * 16 + tid; k < kTile * 16; k += kShWarps * 32) {
+                const uint32_t r = k >> 4, c = k & 15u;
+                *reinterpret_cast<uint4 *>(&sm.ring[slot][2 * kHalfBytes + (c >> 3) * kHalfBytes + swz(r, c & 7u)]) = make_uint4(0, 0, 0, 0);
+            }
+            __syncthreads();   // CTA-uniform
+        }
+        if (b <= b_last && kv_len > p0) {
+            // ---- scores: 4 x S[16 keys][8 columns]; lane (g, t): head t, keys 16 k + g and 16 k + g + 8 ----
+            float s[4][2];
+            {
+                float sc[4][4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) sc[k][0] = sc[k][1] = sc[k][2] = sc[k][3] = 0.f;
+                const uint32_t r = ((lane >> 3) & 1u) * 8 + (lane & 7u);
+#pragma unroll
+                for (int kb = 0; kb < 8; ++kb)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        uint32_t ka[4];
+                        ldsm_x4(st + (kb >> 2) * kHalfBytes + swz(16 * k + r, 2 * (kb & 3) + (lane >> 4)), ka);
+                        mma_f16(sc[k], ka, qb[kb][0], qb[kb][1]);
+                    }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    s[k][0] = p0 + 16 * k + g < kv_len ? sc[k][0] + sc[k][1] : -INFINITY;
+                    s[k][1] = p0 + 16 * k + g + 8 < kv_len ? sc[k][2] + sc[k][3] : -INFINITY;
+                }
+            }
+            float mt = fmaxf(fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1])), fmaxf(fmaxf(s[2][0], s[2][1]), fmaxf(s[3][0], s[3][1])));
+            mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 4));
+            mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 8));
+            mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 16));
+            const float m_new = fmaxf(m_run, mt);   // finite: key p0 is valid
+            const float al = expf(m_run - m_new);   // 0 on the first tile (m_run = -inf)
+            float ps = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                s[k][0] = expf(s[k][0] - m_new);
+                s[k][1] = expf(s[k][1] - m_new);
+                ps += s[k][0] + s[k][1];
+            }
+            ps += __shfl_xor_sync(0xffffffffu, ps, 4);
+            ps += __shfl_xor_sync(0xffffffffu, ps, 8);
+            ps += __shfl_xor_sync(0xffffffffu, ps, 16);
+            l_run = l_run * al + ps;
+            m_run = m_new;
+#pragma unroll
+            for (int dt = 0; dt < 8; ++dt) { o[dt][0] *= al; o[dt][1] *= al; o[dt][2] *= al; o[dt][3] *= al; }
+            const uint32_t srcA = (2 * t) * 4 + (g >> 1), srcB = srcA + 4, part = g & 1u, mi = lane >> 3;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float a0 = __shfl_sync(0xffffffffu, s[k][0], srcA), b0 = __shfl_sync(0xffffffffu, s[k][0], srcB);
+                const float a1 = __shfl_sync(0xffffffffu, s[k][1], srcA), b1 = __shfl_sync(0xffffffffu, s[k][1], srcB);
+                const uint32_t pb0 = pack_h2(split_part(a0, part), split_part(b0, part)), pb1 = pack_h2(split_part(a1, part), split_part(b1, part));
+                const uint32_t r = 16 * k + (mi >> 1) * 8 + (lane & 7u);
+#pragma unroll
+                for (int dt = 0; dt < 8; ++dt) {
+                    uint32_t va[4];
+                    ldsm_x4_trans(st + 2 * kHalfBytes + (dt >> 2) * kHalfBytes + swz(r, 2 * (dt & 3) + (mi & 1u)), va);
+                    mma_f16(o[dt], va, pb0, pb1);
+                }
+            }
+        }
+        __syncthreads();   // tile fully consumed by all warps: the slot can be refilled
+        if (tid == 0 && it + kStages < n_tiles) issue(it + kStages);
+    }
+    if (b > b_last) return;
+    float *part = a.part + (((uint64_t)b * a.n_q_head + (uint64_t)hkv * kGroup + t) * a.n_splits + split) * kPartStride;
+#pragma unroll
+    for (int dt = 0; dt < 8; ++dt) {
+        part[16 * dt + g] = o[dt][0] + o[dt][1];
+        part[16 * dt + g + 8] = o[dt][2] + o[dt][3];
+    }
+    if (g == 0) { part[kD] = m_run; part[kD + 1] = l_run; }
+}
+
+// Adds the splits' records of one query head of one position: grid (n_q_head, batch), 4 warps; warp w takes splits w, w + 4, ..
+// (16 at most: 64 splits), lane the dimensions 4 lane ..; the warps' sums are added in warp order.
+__global__ void __launch_bounds__(128) attn_combine_kernel(const float *__restrict__ parts, float *__restrict__ out, float2 *lse_out, uint32_t S) {
+    griddep_launch_dependents();
+    griddep_wait();
+    __shared__ float4 acc_s[4][32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t hq = (uint64_t)blockIdx.y * gridDim.x + blockIdx.x;
+    const float *part = parts + hq * S * kPartStride;
+    const float m0 = lane < S ? __ldcg(part + (uint64_t)lane * kPartStride + kD) : -INFINITY;
+    const float m1 = lane + 32 < S ? __ldcg(part + (uint64_t)(lane + 32) * kPartStride + kD) : -INFINITY;
+    const float l0 = lane < S ? __ldcg(part + (uint64_t)lane * kPartStride + kD + 1) : 0.f;
+    const float l1 = lane + 32 < S ? __ldcg(part + (uint64_t)(lane + 32) * kPartStride + kD + 1) : 0.f;
+    float4 ov[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const uint32_t s = warp + 4 * j;
+        ov[j] = s < S ? __ldcg(reinterpret_cast<const float4 *>(part + (uint64_t)s * kPartStride) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float mx = warp_max(fmaxf(m0, m1));
+    const float w0 = m0 == -INFINITY ? 0.f : expf(m0 - mx), w1 = m1 == -INFINITY ? 0.f : expf(m1 - mx);
+    const float L = warp_sum(l0 * w0 + l1 * w1);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const float w = __shfl_sync(0xffffffffu, j < 8 ? w0 : w1, (warp + 4 * j) & 31u);
+        acc.x = fmaf(ov[j].x, w, acc.x); acc.y = fmaf(ov[j].y, w, acc.y);
+        acc.z = fmaf(ov[j].z, w, acc.z); acc.w = fmaf(ov[j].w, w, acc.w);
+    }
+    acc_s[warp][lane] = acc;
+    __syncthreads();
+    if (warp) return;
+#pragma unroll
+    for (int w = 1; w < 4; ++w) { const float4 v = acc_s[w][lane]; acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w; }
+    const float inv = 1.0f / L;
+    reinterpret_cast<float4 *>(out + hq * kD)[lane] = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+    if (lse_out && lane == 0) lse_out[hq] = make_float2(mx, L);
+}
+
+constexpr size_t kAttnShSmemBytes = sizeof(AttnShSmem) + 1024;
+
 constexpr size_t kAttnSmemBytes = sizeof(AttnSmem) + 1024;   // + slack to align the ring to the swizzle atom
 
 } // namespace
@@ -384,12 +580,14 @@ cudaError_t attn_make_maps(AttnArgs &a) {
 }
 
 cudaError_t attn_init(void) {
+    const cudaError_t e = cudaFuncSetAttribute(attn_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnShSmemBytes);
+    if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemBytes);
 }
 
-uint32_t attn_pick_splits(uint32_t n_kv_head, uint32_t batch, uint32_t kv_len, int sms) {
+uint32_t attn_pick_splits(uint32_t n_kv_head, uint32_t batch, uint32_t kv_len, int sms, bool shared_kv) {
     const uint32_t tiles = (kv_len + kTile - 1) / kTile;
-    const uint32_t heads = n_kv_head * batch;
+    const uint32_t heads = n_kv_head * (shared_kv && batch > 1 ? (batch + kShWarps - 1) / kShWarps : batch);
     uint32_t s = (2u * (uint32_t)sms + heads - 1) / heads;   // two resident CTAs per SM
     if (s > tiles) s = tiles;
     if (s > 64) s = 64;   // the combine gives each lane two splits
@@ -460,11 +658,20 @@ cudaError_t launch_attn_decode_static(AttnArgs a, int device, cudaStream_t strea
 size_t attn_static_max_records(void) { return kStaticMaxRecords; }
 uint32_t attn_static_max_tickets(void) { return kStaticMaxTickets; }
 
+bool attn_uses_records(const AttnArgs &a) { return a.shared_kv && a.batch > 1 && !a.rope_k && a.pos_stride == 0 && a.n_splits <= 64; }
+
 cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t stream) {
     if (a.n_kv_head == 0 || a.n_q_head != a.n_kv_head * kGroup || a.n_splits == 0 || a.batch == 0)
         return cudaErrorInvalidValue;
     if (a.pos == nullptr && a.kv_len == 0) return cudaErrorInvalidValue;
     if (a.rope_k && (!a.rope_v || !a.k_append || !a.v_append || !a.pos)) return cudaErrorInvalidValue;
+    if (attn_uses_records(a)) {   // positions of one sequence
+        const dim3 sgrid(a.n_splits, a.n_kv_head, (a.batch + kShWarps - 1) / kShWarps);
+        const cudaError_t e = launch_kernel(attn_shared_kernel, sgrid, dim3(kShWarps * 32), kAttnShSmemBytes, stream, a.pdl != 0, a);
+        if (e != cudaSuccess || a.records_only) return e;
+        return launch_kernel(attn_combine_kernel, dim3(a.n_q_head, a.batch), dim3(128), 0, stream, true, (const float *)a.part, a.out, a.lse_out,
+                             a.n_splits);
+    }
     const dim3 grid(a.n_splits, a.n_kv_head, a.batch);
     return launch_kernel(attn_decode_kernel, grid, dim3(kAttnThreads), kAttnSmemBytes, stream, a.pdl != 0, a);
 }

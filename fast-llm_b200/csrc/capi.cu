@@ -396,7 +396,7 @@ static int attn_impl(fl_b200_ctx *c, const float *q, const uint16_t *k, const ui
     a.n_q_head = n_q;
     a.n_kv_head = n_kv;
     a.batch = batch;
-    a.n_splits = attn_pick_splits(n_kv, batch, pos_dev ? kv_stride : kv_len + (verify ? batch - 1 : 0), c->sms);
+    a.n_splits = attn_pick_splits(n_kv, batch, pos_dev ? kv_stride : kv_len + (verify ? batch - 1 : 0), c->sms, verify);
     a.lse_out = reinterpret_cast<float2 *>(lse_out);
     a.kv_len_step = verify ? 1u : 0u;
     a.shared_kv = verify ? 1u : 0u;

@@ -734,7 +734,8 @@ static int batch_alloc(fl_b200_decoder *d) {
     CK(cudaMalloc(&d->b.logits, M * (size_t)d->V * 4)); CK(cudaMalloc(&d->b.margin, M * 4));
     size_t part = 0;
     for (uint32_t m = 1; m <= M; ++m)
-        part = std::max(part, attn_part_floats(d->Hq, m, attn_pick_splits(d->Hkv, m, c.max_kv, d->ctx->sms)));
+        for (const bool shared : {false, true})
+            part = std::max(part, attn_part_floats(d->Hq, m, attn_pick_splits(d->Hkv, m, c.max_kv, d->ctx->sms, shared)));
     CK(cudaMalloc(&d->b.part, part * sizeof(float)));
     if (d->tp_size > 1) {
         CK(cudaMalloc(&d->b.partial, M * E * 4));
@@ -830,10 +831,12 @@ static int enqueue_batch_nx(fl_b200_decoder *d, uint32_t m, cudaStream_t s, bool
             a.tickets = b.tickets; a.pos = pos; a.kv_len = 0; a.kv_len_step = seqs ? 0 : 1; a.shared_kv = seqs ? 0 : 1; a.pos_stride = seqs ? 1 : 0;
             a.kv_stride = c.max_kv; a.batch_stride = (uint64_t)d->Hkv * c.max_kv * D;
             a.n_q_head = d->Hq; a.n_kv_head = d->Hkv; a.batch = m;
-            a.n_splits = attn_pick_splits(d->Hkv, m, c.max_kv, ctx->sms);
+            a.n_splits = attn_pick_splits(d->Hkv, m, c.max_kv, ctx->sms, !seqs);
             a.scale = 1.0f / sqrtf((float)D); a.status = ctx->status; a.pdl = pdl;
+            a.records_only = attn_uses_records(a);   // O's conversion adds the splits
             CK(attn_make_maps(a));
             CK(launch_attn_decode(a, s));
+            if (a.records_only) { in.att = b.part; in.n_splits = a.n_splits; }
         }
         in.x = b.att; in.xstride = QD;
         n = nx_group(d, l, 1, t, &cols);
@@ -931,7 +934,7 @@ static int enqueue_batch(fl_b200_decoder *d, uint32_t m, cudaStream_t s, bool se
             a.pos = pos; a.kv_len = 0; a.kv_len_step = seqs ? 0 : 1; a.shared_kv = seqs ? 0 : 1; a.pos_stride = seqs ? 1 : 0;
             a.kv_stride = c.max_kv; a.batch_stride = (uint64_t)d->Hkv * c.max_kv * D;
             a.n_q_head = d->Hq; a.n_kv_head = d->Hkv; a.batch = m;
-            a.n_splits = attn_pick_splits(d->Hkv, m, c.max_kv, ctx->sms);
+            a.n_splits = attn_pick_splits(d->Hkv, m, c.max_kv, ctx->sms, !seqs);
             a.scale = 1.0f / sqrtf((float)D); a.status = ctx->status;
             CK(attn_make_maps(a));
             CK(launch_attn_decode(a, s));

@@ -188,6 +188,7 @@ struct AttnArgs {
     float scale;
     uint32_t *status;
     int pdl;
+    int records_only;      // several positions of one cache (attn_uses_records): leave the splits' records in part, out is not written
     unsigned long long *trace;   // optional 4-entry timeline record (diagnostics)
     // Fused RoPE + KV append (the decoder's launch plan): q arrives un-rotated; rope_k / rope_v are this
     // token's k and v ([batch][n_kv_head][128] f32, k un-rotated); the kernel rotates q and k by the angle
@@ -201,6 +202,7 @@ struct AttnArgs {
     CUtensorMap kmap, vmap;         // filled by attn_make_maps
 };
 cudaError_t attn_make_maps(AttnArgs &a);
+bool attn_uses_records(const AttnArgs &a);   // the launch is one of several positions over one cache (attn_shared_kernel)
 cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t stream);
 // Same kernel with the split-KV scratch in a fixed file-scope device array
 // (no allocation at call time); cudaErrorMemoryAllocation when the launch needs
@@ -210,7 +212,7 @@ cudaError_t launch_attn_decode_static(AttnArgs a, int device, cudaStream_t strea
 size_t attn_static_max_records(void);
 uint32_t attn_static_max_tickets(void);
 cudaError_t attn_init(void);
-uint32_t attn_pick_splits(uint32_t n_kv_head, uint32_t batch, uint32_t kv_len, int sms);
+uint32_t attn_pick_splits(uint32_t n_kv_head, uint32_t batch, uint32_t kv_len, int sms, bool shared_kv = false);
 size_t attn_part_floats(uint32_t n_q_head, uint32_t batch, uint32_t n_splits);
 
 // ---- comm.cu: exchange steps of the tensor-parallel step ----------------------
