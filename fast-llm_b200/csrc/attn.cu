@@ -588,7 +588,9 @@ cudaError_t attn_init(void) {
 uint32_t attn_pick_splits(uint32_t n_kv_head, uint32_t batch, uint32_t kv_len, int sms, bool shared_kv) {
     const uint32_t tiles = (kv_len + kTile - 1) / kTile;
     const uint32_t heads = n_kv_head * (shared_kv && batch > 1 ? (batch + kShWarps - 1) / kShWarps : batch);
-    uint32_t s = (2u * (uint32_t)sms + heads - 1) / heads;   // two resident CTAs per SM
+    // two resident CTAs per SM, all of them in one wave: rounded down, since the CTAs of a second wave, however few, take as long
+    // as the first (4 sequences of 65000 keys, 8 heads: 9 splits 164 us, 10 splits = 320 CTAs 195 us)
+    uint32_t s = 2u * (uint32_t)sms / heads;
     if (s > tiles) s = tiles;
     if (s > 64) s = 64;   // the combine gives each lane two splits
     if (s < 1) s = 1;
