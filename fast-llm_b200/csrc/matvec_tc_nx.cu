@@ -17,11 +17,12 @@
 // mma.sync m16n8k16: A = 16 rows x 16 weights as f16, the 8 columns of B = 4 tokens as (hi, lo) f16 pairs, NTG
 // instructions for 4 NTG tokens from the same A registers.
 //   Q4_K : the 6-bit scale of the sub-block goes into A exactly. A masked nibble is, as it stands, the subnormal f16
-//          q 2^-24 (q 2^-20 in the high nibble), and one multiplication by sc 2^10 (sc 2^6) makes it the f16 number
-//          q sc 2^-14 (q sc <= 945 has 10 bits; 2^14 goes onto d). A block's 256 columns are then one chain of
-//          accumulators and the super-block scale d is applied once; lane column t unpacks the 32-byte chunk t. The mins are
-//          one more instruction: bf16 (min of sub-block k) times the sub-block sums of the activation as three bf16 parts
-//          (24 bits).
+//          q 2^-24 (q 2^-20 in the high nibble), and one FMA with sc 2^10 (sc 2^6) and -8 sc 2^-14 makes it the f16
+//          number (q - 8) sc 2^-14 (|(q - 8) sc| <= 504: exact). A block's 256 columns are then one chain of accumulators
+//          per nibble kind and the super-block scale d is applied once; lane column t unpacks the 32-byte chunk t. The mins
+//          and the 8 sc are two more instructions: bf16 (min, scale of sub-block k) times the sub-block sums of the
+//          activation as three bf16 parts (24 bits). (q sc instead of (q - 8) sc: larger sums, whose truncation in the
+//          tensor core showed: 3.2e-7 relative error against the 2.1e-7 of a chain per sub-block.)
 //   Q6_K : (q - 32) sc has 13 bits, so the 16 columns of an instruction are one scale group and its f32 result is
 //          scaled afterwards (both columns of a pair in one packed FMA).
 //   Q8_0 : the same with two instructions per 32-column block and the block's f16 scale.
@@ -152,7 +153,13 @@ __device__ __forceinline__ void mma16816_bf16(float (&c)[4], uint32_t a0, uint32
 __device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
 __device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
 __device__ __forceinline__ uint32_t hsub2_u32(uint32_t h, __half2 off) { return as_u32(__hsub2(as_h2(h), off)); }
-__device__ __forceinline__ uint32_t hmul2_u32(uint32_t h, __half2 m) { return as_u32(__hmul2(as_h2(h), m)); }
+__device__ __forceinline__ uint32_t hfma2_u32(uint32_t h, __half2 m, __half2 c) { return as_u32(__hfma2(as_h2(h), m, c)); }
+// the two low bytes (< 64) of w as a pair of bf16 (0x4300 | b is 128 + b)
+__device__ __forceinline__ uint32_t bytes_bf16(uint32_t w) {
+    const uint32_t b = __byte_perm(w, 0x43434343u, 0x4140u);
+    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&b), __floats2bfloat162_rn(128.f, 128.f));
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
 // (c.x, c.y) += s * (a, b): both columns of a token in one packed FMA
 __device__ __forceinline__ void fma_pair(float2 &c, float s, float a, float b) {
     uint64_t cc = *reinterpret_cast<uint64_t *>(&c), ss, ab;
@@ -436,22 +443,23 @@ __device__ __forceinline__ void q4k_block_nx(uint32_t r0, uint32_t offs, uint32_
     // 0..3 are the low six bits of bytes 0..3 (4..7 for the mins), 4..7 a nibble of bytes 8..11 under the top two bits of those
     const uint32_t sh = 16u * (t & 1u);
     const uint32_t shA = t >= 2 ? sh + 2u : sh, mA = t >= 2 ? 0x3030u : 0x3F3Fu, mE = t >= 2 ? 0x0F0Fu : 0u;
-    __half2 sL[2], sH[2];   // scales times 2^10 (low nibbles), 2^6 (high nibbles)
-    uint32_t am[2];
+    __half2 sL[2], sH[2], kL[2], kH[2];   // scales times 2^10 (low nibbles), 2^6 (high nibbles); -8 2^-14 times the scales
+    uint32_t sm[2];                       // the two sub-blocks' scales and mins, a byte each
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         const uint32_t sc = ((hd[r].y >> shA) & mA) | ((hd[r].w >> sh) & mE);
         const uint32_t mn = ((hd[r].z >> shA) & mA) | ((hd[r].w >> (sh + 4u)) & mE);
         const __half2 k1024 = __floats2half2_rn(1024.f, 1024.f);
-        sL[r] = __hmul2(__hsub2(as_h2(__byte_perm(sc, 0x64646464u, 0x4040u)), k1024), k1024);
-        sH[r] = __hmul2(__hsub2(as_h2(__byte_perm(sc, 0x64646464u, 0x4141u)), k1024), __floats2half2_rn(64.f, 64.f));
-        // mins as bf16 (0x4300 | b is 128 + b)
-        const uint32_t mb = __byte_perm(mn, 0x43434343u, 0x4140u);
-        const __nv_bfloat162 m2 = __hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&mb), __floats2bfloat162_rn(128.f, 128.f));
-        am[r] = *reinterpret_cast<const uint32_t *>(&m2);
+        const __half2 s0 = __hsub2(as_h2(__byte_perm(sc, 0x64646464u, 0x4040u)), k1024), s1 = __hsub2(as_h2(__byte_perm(sc, 0x64646464u, 0x4141u)), k1024);
+        const __half2 km8 = __floats2half2_rn(-0.00048828125f, -0.00048828125f);   // -8 2^-14
+        sL[r] = __hmul2(s0, k1024); kL[r] = __hmul2(s0, km8);
+        sH[r] = __hmul2(s1, __floats2half2_rn(64.f, 64.f)); kH[r] = __hmul2(s1, km8);
+        sm[r] = sc | (mn << 16);
     }
-    // up to 8 tokens: one accumulator chain per nibble kind (8 dependent instructions each), else one chain
+    // Chains of 8 dependent instructions (16: twice the error of the sums): up to 8 tokens one per nibble kind, side by side;
+    // else one after the other, the first one's sums put aside half-way (the registers of two do not fit).
     constexpr int kChains = NTG <= 2 ? 2 : 1;
+    float half[2][NTG];
     float c[kChains][NTG][4];
 #pragma unroll
     for (int i = 0; i < kChains; ++i)
@@ -460,12 +468,21 @@ __device__ __forceinline__ void q4k_block_nx(uint32_t r0, uint32_t offs, uint32_
     const uint32_t ML = 0x000F000Fu, MH = 0x00F000F0u;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
+        if (kChains == 1 && j == 4)
+#pragma unroll
+            for (int tg = 0; tg < NTG; ++tg) {
+                half[0][tg] = c[0][tg][0] + c[0][tg][1];
+                half[1][tg] = c[0][tg][2] + c[0][tg][3];
+                c[0][tg][0] = c[0][tg][1] = c[0][tg][2] = c[0][tg][3] = 0.f;
+            }
         const uint4 &q0 = j < 4 ? wa[0] : wb[0], &q1 = j < 4 ? wa[1] : wb[1];
         const uint32_t W0 = (j & 3) == 0 ? q0.x : (j & 3) == 1 ? q0.y : (j & 3) == 2 ? q0.z : q0.w;
         const uint32_t W1 = (j & 3) == 0 ? q1.x : (j & 3) == 1 ? q1.y : (j & 3) == 2 ? q1.z : q1.w;
         const uint32_t V0 = W0 >> 8, V1 = W1 >> 8;
-        const uint32_t l0 = hmul2_u32(W0 & ML, sL[0]), l1 = hmul2_u32(W1 & ML, sL[1]), l2 = hmul2_u32(V0 & ML, sL[0]), l3 = hmul2_u32(V1 & ML, sL[1]);
-        const uint32_t h0 = hmul2_u32(W0 & MH, sH[0]), h1 = hmul2_u32(W1 & MH, sH[1]), h2 = hmul2_u32(V0 & MH, sH[0]), h3 = hmul2_u32(V1 & MH, sH[1]);
+        const uint32_t l0 = hfma2_u32(W0 & ML, sL[0], kL[0]), l1 = hfma2_u32(W1 & ML, sL[1], kL[1]);
+        const uint32_t l2 = hfma2_u32(V0 & ML, sL[0], kL[0]), l3 = hfma2_u32(V1 & ML, sL[1], kL[1]);
+        const uint32_t h0 = hfma2_u32(W0 & MH, sH[0], kH[0]), h1 = hfma2_u32(W1 & MH, sH[1], kH[1]);
+        const uint32_t h2 = hfma2_u32(V0 & MH, sH[0], kH[0]), h3 = hfma2_u32(V1 & MH, sH[1], kH[1]);
 #pragma unroll
         for (int tg = 0; tg < NTG; ++tg) {
             const uint4 b = lds128(xaddr + tg * kXq4 + j * 512 + lane * 16);
@@ -473,16 +490,24 @@ __device__ __forceinline__ void q4k_block_nx(uint32_t r0, uint32_t offs, uint32_
             mma16816(c[kChains - 1][tg], h0, h1, h2, h3, b.z, b.w);
         }
     }
-    const float d0 = 16384.f * h2f_bits((uint16_t)(hd[0].x & 0xFFFFu)), e0 = h2f_bits((uint16_t)(hd[0].x >> 16));
-    const float d1 = 16384.f * h2f_bits((uint16_t)(hd[1].x & 0xFFFFu)), e1 = h2f_bits((uint16_t)(hd[1].x >> 16));
+    if (kChains == 2)
+#pragma unroll
+        for (int tg = 0; tg < NTG; ++tg) {
+            half[0][tg] = c[kChains - 1][tg][0] + c[kChains - 1][tg][1];
+            half[1][tg] = c[kChains - 1][tg][2] + c[kChains - 1][tg][3];
+        }
+    const float d0 = h2f_bits((uint16_t)(hd[0].x & 0xFFFFu)), e0 = h2f_bits((uint16_t)(hd[0].x >> 16));
+    const uint32_t as[2] = {bytes_bf16(sm[0]), bytes_bf16(sm[1])}, am[2] = {bytes_bf16(sm[0] >> 16), bytes_bf16(sm[1] >> 16)};
+    const float d1 = h2f_bits((uint16_t)(hd[1].x & 0xFFFFu)), e1 = h2f_bits((uint16_t)(hd[1].x >> 16));
 #pragma unroll
     for (int tg = 0; tg < NTG; ++tg) {
-        float m[4] = {0.f, 0.f, 0.f, 0.f};
+        float m[4] = {0.f, 0.f, 0.f, 0.f}, s[4] = {0.f, 0.f, 0.f, 0.f};
         const uint2 b = lds64(xaddr + tg * kXq4 + kFragBytes + lane * 8);
         mma16816_bf16(m, am[0], am[1], am[0], am[1], b.x, b.y);
+        mma16816_bf16(s, as[0], as[1], as[0], as[1], b.x, b.y);
         const float xs = ldsf(xaddr + tg * kXq4 + kFragBytes + kMinBytes + t * 4);
-        float q0 = c[0][tg][0] + c[0][tg][1], q1 = c[0][tg][2] + c[0][tg][3];
-        if (kChains == 2) { q0 += c[kChains - 1][tg][0] + c[kChains - 1][tg][1]; q1 += c[kChains - 1][tg][2] + c[kChains - 1][tg][3]; }
+        const float q0 = fmaf(8.f, s[0] + s[1], 16384.f * ((c[0][tg][0] + c[0][tg][1]) + half[0][tg]));
+        const float q1 = fmaf(8.f, s[2] + s[3], 16384.f * ((c[0][tg][2] + c[0][tg][3]) + half[1][tg]));
         acc[0][tg] = fmaf(xs, d0 * q0 - e0 * (m[0] + m[1]), acc[0][tg]);
         acc[1][tg] = fmaf(xs, d1 * q1 - e1 * (m[2] + m[3]), acc[1][tg]);
     }
