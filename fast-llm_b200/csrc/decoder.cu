@@ -218,8 +218,9 @@ static int enqueue_step(fl_b200_decoder *d, cudaStream_t s, uint32_t *n_launch, 
         a.t[1] = {w[FL_B200_T_UP].w, d->u, nullptr, d->F, w[FL_B200_T_UP].fmt, 0};
         a.x = d->xb; a.wnorm = d->ffn_norm[l]; a.eps = c.eps; a.cols = E;
         a.x_mode = MV_X_RMSNORM; a.status = ctx->status; a.pdl = kPdl;
-        // (Q8_0 streams without the fused product: the down projection then takes silu(g) * u on load)
-        a.swiglu = (w[FL_B200_T_GATE].fmt == w[FL_B200_T_UP].fmt && w[FL_B200_T_GATE].fmt != FL_B200_Q8_0) ? 1 : 0;
+        a.swiglu = w[FL_B200_T_GATE].fmt == w[FL_B200_T_UP].fmt ? 1 : 0;
+        // (Q8_0 has the fused product on the tensor-core kernel only: without it the down projection takes silu(g) * u on load)
+        if (w[FL_B200_T_GATE].fmt == FL_B200_Q8_0 && !matvec_tc_eligible(a)) a.swiglu = 0;
         a.issue_late = (issue_late() >> 1) & 1;
         return a;
     };

@@ -59,11 +59,14 @@ constexpr uint32_t kSeg4 = 8 * 144, kSeg6 = 8 * 210, kSeg8 = 64 * 34;
 // with the 128-byte swizzle (tensor_map_lines_swz), which spreads the same 16-byte chunk of 8 consecutive rows
 // over 8 bank groups; the consumer addresses chunk c of line l at l * 128 + ((c ^ (l & 7)) << 4). Rows whose
 // pitch in memory is not a multiple of 128 bytes (columns not a multiple of 2048) fall back to the plain box.
-// Q8_0 (a segment is wider than a box may be): one bulk copy per row, pitch + 16 (548 words = 4 mod 32).
-constexpr uint32_t kPitch4 = kSeg4, kPitch6 = kSeg6, kPitch8 = kSeg8 + 16;
+// Q8_0: a segment is wider than a box may be, so a stage is two boxes of half a segment, one behind the other, each 16 bytes
+// wider than its half: 276 words = 20 mod 32, conflict free for the 32-bit loads of lanes (g, t) at 17 t words. (One bulk
+// copy per row, the form before: 2176 bytes per some 130 cycles of the TMA unit, 4.7 TB/s at most; the 3B-class 8-bit model's
+// step 5.8 ms.)
+constexpr uint32_t kPitch4 = kSeg4, kPitch6 = kSeg6, kPitch8 = kSeg8 / 2 + 16;
 // ring slots are multiples of 1024 bytes: the swizzle pattern of a Q4_K stage is tied to the address
 constexpr uint32_t slot_round(uint32_t b) { return (b + 1023u) & ~1023u; }
-constexpr uint32_t kSlot4 = slot_round(16 * kPitch4), kSlot6 = slot_round(16 * kPitch6), kSlot8 = slot_round(16 * kPitch8);
+constexpr uint32_t kSlot4 = slot_round(16 * kPitch4), kSlot6 = slot_round(16 * kPitch6), kSlot8 = slot_round(32 * kPitch8);
 // 256-column blocks a half-warp of the prologue converts (bounds the column count: see matvec_tc_eligible)
 __host__ __device__ constexpr int max_blk_per_half_warp(int groups) { return groups == 1 ? 4 : 2; }
 
@@ -152,6 +155,13 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 __device__ __forceinline__ void imma16832(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                           uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// The same with signed 8-bit weights
+__device__ __forceinline__ void imma16832_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                             uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -608,6 +618,37 @@ __device__ __forceinline__ void q6k_block_i8(uint32_t r0, uint32_t r1, uint32_t 
 // from `r0` / `r1` (4-byte aligned). The first block's quants start 2 bytes into a word and are realigned with
 // byte permutes; the second block's are aligned. An int8 s becomes f16 through (s ^ 0x80) under 0x64: 1024 + 128 + s,
 // minus 1152, exact. The activation uses the Q4_K layout (64 consecutive columns per lane column, words of 4).
+// Integer form (q8_0_block_i8): the int8 quants are signed 8-bit operands as they are, the activation is the fixed-point image
+// of the Q4_K integer form (the same 64 columns per lane column, words of 4, one scale per 32 columns = one Q8_0 block; the
+// 1 / 16 that Q4_K's high nibbles want in the odd sub-blocks' scales is taken off again). No unpacking at all.
+__device__ __forceinline__ void q8_0_block_i8(uint32_t r0, uint32_t xaddr, uint32_t xstride, float2 xs2, float &out0, float &out1) {
+    const uint32_t r1 = r0 + 8 * kPitch8;
+    uint32_t w0[17], w1[17];
+#pragma unroll
+    for (int i = 0; i < 17; ++i) { w0[i] = lds32(r0 + 4 * i); w1[i] = lds32(r1 + 4 * i); }
+    int cA[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, cB[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const uint4 bA = lds128(xaddr + (2 * m) * xstride), bB = lds128(xaddr + (2 * m + 1) * xstride);
+        // the first block's quants start 2 bytes into a word, the second block's are aligned
+        const uint32_t a0 = __byte_perm(w0[2 * m], w0[2 * m + 1], 0x5432u), a2 = __byte_perm(w0[2 * m + 1], w0[2 * m + 2], 0x5432u);
+        const uint32_t a1 = __byte_perm(w1[2 * m], w1[2 * m + 1], 0x5432u), a3 = __byte_perm(w1[2 * m + 1], w1[2 * m + 2], 0x5432u);
+        imma16832_s8(cA[0], a0, a1, a2, a3, bA.x, bA.y);
+        imma16832_s8(cB[0], w0[9 + 2 * m], w1[9 + 2 * m], w0[10 + 2 * m], w1[10 + 2 * m], bB.x, bB.y);
+        imma16832_s8(cA[1], a0, a1, a2, a3, bA.z, bA.w);
+        imma16832_s8(cB[1], w0[9 + 2 * m], w1[9 + 2 * m], w0[10 + 2 * m], w1[10 + 2 * m], bB.z, bB.w);
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const uint32_t wa = r ? w1[0] : w0[0], wb = r ? w1[8] : w0[8];
+        const float dA = h2f_bits((uint16_t)(wa & 0xFFFFu)), dB = h2f_bits((uint16_t)(wb >> 16));
+        // the four plane sums of a block as one number: two exact integer steps (|.| < 2^28), then f32
+        const float ta = fmaf((float)(cA[0][2 * r] * 256 + cA[0][2 * r + 1]), 65536.f, (float)(cA[1][2 * r] * 256 + cA[1][2 * r + 1]));
+        const float tb = fmaf((float)(cB[0][2 * r] * 256 + cB[0][2 * r + 1]), 65536.f, (float)(cB[1][2 * r] * 256 + cB[1][2 * r + 1]));
+        (r ? out1 : out0) = dA * (xs2.x * ta) + dB * (16.f * xs2.y * tb);
+    }
+}
+
 __device__ __forceinline__ void q8_0_block(uint32_t r0, uint32_t r1, uint32_t xaddr, uint32_t xstride, float &out0, float &out1) {
     uint32_t w0[17], w1[17];
 #pragma unroll
@@ -679,8 +720,8 @@ __device__ __forceinline__ bool grid_barrier(GridBar *b, uint32_t nblocks, uint3
 // then the finalizer warp. A launch runs its phases one after the other with a grid-wide barrier in
 // between; the producer does not take part in the barriers: the weights of the next phase are already
 // streaming into the ring while the current phase drains and the next activation is built.
-// F: 0 = every format and form, decided per phase at run time (f16 forms, Q8_0, several phases); 1 / 2 / 3 = one phase
-// on the integer forms holding Q4_K tensors only / Q6_K only / both: what a decode step launches. The specialised
+// F: 0 = every format and form, decided per phase at run time (f16 forms, Q8_0 beside K-quants, several phases); 1 / 2 / 3 / 4 =
+// one phase on the integer forms holding Q4_K tensors only / Q6_K only / both / Q8_0 only: what a decode step launches. The specialised
 // instances carry only their own code (the whole kernel is some 7000 instructions, and a launch that has to fetch its
 // path out of that from L2 starts later) and get their own register allocation.
 // R: 256-column blocks a half-warp of the prologue converts (F != 0: 1 up to 34 blocks = 8704 columns, else 2; the
@@ -719,39 +760,31 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
             const uint32_t my_units = blockIdx.x < ph.total_units ? (ph.total_units - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
             for (uint32_t k = 0; k < my_units; ++k) {
                 const uint32_t u = blockIdx.x + k * gridDim.x;
-                const uint8_t *src = nullptr;
-                uint32_t pitch = 0, fmt;
-                bool valid = false;
-                if (ph.swiglu) {
-                    const TcTensor &t = ph.t[(lane >> 3) & 1u];
-                    const uint32_t row = 8 * u + (lane & 7u);
-                    fmt = (uint32_t)ph.t[0].fmt;
-                    valid = lane < 16 && row < t.rows;
-                    pitch = t.pitch;
-                    src = t.w + (size_t)row * t.pitch;
-                } else {
-                    const TcTensor &t = ph.t[unit_tensor(ph, u)];
-                    const uint32_t row = 16 * (u - t.unit0) + lane;
-                    fmt = (uint32_t)t.fmt;
-                    valid = lane < 16 && row < t.rows;
-                    pitch = t.pitch;
-                    src = t.w + (size_t)row * t.pitch;
-                }
-                const uint32_t segb = fmt == FMT_Q4_K ? kSeg4 : fmt == FMT_Q6_K ? kSeg6 : kSeg8;
-                const uint32_t rp = fmt == FMT_Q4_K ? kPitch4 : fmt == FMT_Q6_K ? kPitch6 : kPitch8;
-                const uint32_t nvalid = __popc(__ballot_sync(0xffffffffu, valid));
+                uint32_t fmt;
+                bool valid;
+                if (ph.swiglu) { fmt = (uint32_t)ph.t[0].fmt; valid = 8 * u + (lane & 7u) < ph.t[0].rows; }
+                else { const TcTensor &t = ph.t[unit_tensor(ph, u)]; fmt = (uint32_t)t.fmt; valid = 16 * (u - t.unit0) + lane < t.rows; }
+                // never empty (a unit has a row); without the vote ptxas lays out the Q6_K instance with spills (step + 1.2 %)
+                if (__ballot_sync(0xffffffffu, valid) == 0) continue;
                 const int ti = ph.swiglu ? 0 : unit_tensor(ph, u);
+                const uint32_t segb = fmt == FMT_Q4_K ? kSeg4 : fmt == FMT_Q6_K ? kSeg6 : kSeg8;
                 const uint32_t row0 = ph.swiglu ? 8 * u : 16 * (u - ph.t[ti].unit0);
                 for (uint32_t seg = 0; seg < nseg; ++seg) {
                     const uint32_t off = seg * segb;
                     if (!mbar_wait_bounded(&sm.empty[slot], par, a.status)) return;
                     fence_proxy_async_smem();
                     const uint32_t dst = ring + slot * a.slot_bytes;
-                    if (F == 0 && fmt == FMT_Q8_0) {   // one bulk copy per row
-                        const uint32_t bytes = min(segb, pitch - off);   // pitch and off are multiples of 16
-                        if (lane == 0) mbar_arrive_expect_tx(&sm.full[slot], nvalid * bytes);
-                        __syncwarp();
-                        if (valid) bulk_g2s_addr(dst + lane * rp, src + off, bytes, &sm.full[slot]);
+                    if ((F == 0 || F == 4) && fmt == FMT_Q8_0) {
+                        if (lane == 0) {   // two boxes of half the segment (SwiGLU: four, 8 gate rows then 8 up rows in each half)
+                            mbar_arrive_expect_tx(&sm.full[slot], 32 * kPitch8);
+                            const uint64_t pol8 = pol ? pol : l2_policy_evict_first();
+                            for (uint32_t h = 0; h < 2; ++h)
+                                for (uint32_t j = 0; j < (ph.swiglu ? 2u : 1u); ++j) {
+                                    const uint32_t d8 = dst + (16 * h + 8 * j) * kPitch8, x8 = (off + h * (kSeg8 / 2)) / 8;
+                                    if (a.l2_hints) tma_box2_hint(d8, &ph.t[ti + j].map, x8, row0, &sm.full[slot], pol8);
+                                    else tma_box2(d8, &ph.t[ti + j].map, x8, row0, &sm.full[slot]);
+                                }
+                        }
                     } else if (lane == 0) {
                         // one box of 16 rows x the segment (SwiGLU: 8 gate rows, then 8 up rows); rows past the end of the
                         // tensor and blocks past the end of a row arrive as zeros and count as bytes all the same
@@ -787,7 +820,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
     for (int p = 0; p < a.n_phases; ++p) {
         const TcPhase &ph = a.ph[p];
         const uint32_t nblk = ph.cols / 256, nseg = (nblk + 7) / 8;
-        const bool I8 = F ? true : ph.q4_i8 != 0, UQ4 = F ? (F & 1) != 0 : ph.use_q4 != 0, UQ6 = F ? (F & 2) != 0 : ph.use_q6 != 0;
+        const bool I8 = F ? true : ph.q4_i8 != 0, UQ4 = F ? (F & 5) != 0 : ph.use_q4 != 0, UQ6 = F ? (F & 2) != 0 : ph.use_q6 != 0;
         const TcSmem sm = tc_carve<G>(smem_raw, ph.cols, UQ4, UQ6, I8, S, a.ring_off);
         const uint32_t my_units = blockIdx.x < ph.total_units ? (ph.total_units - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
         const bool late = F == 0 && p > 0;   // the activation was written by the previous phase of this launch: read it past L1
@@ -1082,8 +1115,26 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                 // this group's stages of unit k: those of its stage sequence (grp, grp + G, ... over the whole launch)
                 // that fall into [it_base + k nseg, it_base + (k + 1) nseg)
                 const uint32_t it0 = it_base + k * nseg, it1 = it0 + nseg;
-                const bool is4 = F == 1 ? true : F == 2 ? false : fmt == FMT_Q4_K;
-                if (is4 && I8) {
+                const bool is4 = F == 1 ? true : F == 2 || F == 4 ? false : fmt == FMT_Q4_K;
+                if (F == 4) {
+#pragma unroll 1
+                    for (; c_it < it1; c_it += G) {
+                        const uint32_t blk = (c_it - it0) * 8 + w;
+                        mbar_wait_or_die(&sm.full[c_slot], c_par, a.status, dead);
+                        if (blk < nblk) {
+                            const uint32_t r0 = ring + c_slot * a.slot_bytes + ((w >> 2) * 16 + g) * kPitch8 + (w & 3u) * 272u + t * 68u;
+                            const float2 xs2 = *reinterpret_cast<const float2 *>(sm.xs8 + blk * 8 + 2 * t);
+                            float o0, o1;
+                            q8_0_block_i8(r0, xa4 + blk * xb, xstride, xs2, o0, o1);
+                            acc0 += o0;
+                            acc1 += o1;
+                        }
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&sm.empty[c_slot]);
+                        c_slot += G;
+                        if (c_slot >= S) { c_slot -= S; c_par ^= 1u; }
+                    }
+                } else if (is4 && I8) {
 #pragma unroll 1
                     for (; c_it < it1; c_it += G) {
                         const uint32_t blk = (c_it - it0) * 8 + w;
@@ -1127,7 +1178,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                         const uint32_t blk = (c_it - it0) * 8 + w;
                         mbar_wait_or_die(&sm.full[c_slot], c_par, a.status, dead);
                         if (blk < nblk) {
-                            const uint32_t r0 = ring + c_slot * a.slot_bytes + g * kPitch8 + w * 272u + t * 68u;
+                            const uint32_t r0 = ring + c_slot * a.slot_bytes + ((w >> 2) * 16 + g) * kPitch8 + (w & 3u) * 272u + t * 68u;
                             float o0, o1;
                             q8_0_block(r0, r0 + 8 * kPitch8, xa4 + blk * xb, xstride, o0, o1);
                             const float xs = sm.xs[blk];
@@ -1216,6 +1267,8 @@ cudaError_t matvec_tc_init(void) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     return e;
@@ -1223,11 +1276,17 @@ cudaError_t matvec_tc_init(void) {
 
 // True when the launch can run on the tensor-core kernel: Q4_K / Q6_K / Q8_0 tensors only, whole 256-column
 // blocks, 16-byte aligned rows, no expert indirection and no exchange prologue.
-// Q4_K and Q6_K on the integer forms (q4k_block_i8, q6k_block_i8) unless FLB_TC_I8=0; a launch that holds a Q8_0
-// tensor stays on the f16 forms (Q8_0 reads the f16 image of the activation).
+// Q4_K and Q6_K on the integer forms (q4k_block_i8, q6k_block_i8) unless FLB_TC_I8=0, Q8_0 too where a launch holds nothing else
+// and runs on a specialised instance; a launch that mixes it with K-quants stays on the f16 forms.
 bool tc_q4_i8() {
     static const bool on = !(getenv("FLB_TC_I8") && getenv("FLB_TC_I8")[0] == '0');
     return on;
+}
+
+// The specialised instances (two consumer groups only); FLB_TC_GENERIC=1: the run-time form for every launch (A/B)
+static bool tc_special() {
+    static const bool generic = getenv("FLB_TC_GENERIC") && getenv("FLB_TC_GENERIC")[0] == '1';
+    return !generic && tc_groups() == 2;
 }
 
 bool matvec_tc_eligible(const MatvecArgs &a) {
@@ -1249,7 +1308,7 @@ bool matvec_tc_eligible(const MatvecArgs &a) {
     }
     if (a.swiglu && (a.n_tensors != 2 || a.t[0].rows != a.t[1].rows || a.t[0].fmt != a.t[1].fmt || a.accumulate)) return false;
     const uint32_t slot = q8 ? kSlot8 : q6 ? kSlot6 : kSlot4;
-    return tc_head_bytes(2, groups) + tc_x_bytes(a.cols, q4, q6, !q8 && tc_q4_i8()) + 1024 + 2u * slot <= 227 * 1024 - 1024;
+    return tc_head_bytes(2, groups) + tc_x_bytes(a.cols, q4, q6, tc_q4_i8()) + 1024 + 2u * slot <= 227 * 1024 - 1024;
 }
 
 // One launch of n dependent matvecs (phase i + 1 consumes what phase i writes). n = 1: a plain launch.
@@ -1268,7 +1327,7 @@ cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaS
         if (!matvec_tc_eligible(a)) return cudaErrorNotSupported;
         if (p > 0 && (a.trace || a.issue_late)) { /* per-launch diagnostics apply to the first phase only */ }
         TcPhase &ph = k.ph[p];
-        bool q4 = false, q6 = false, q8 = false;
+        bool q4 = false, q6 = false, q8 = false, only8 = true;
         uint32_t units = 0;
         ph.n_tensors = a.n_tensors;
         for (int i = 0; i < a.n_tensors; ++i) {
@@ -1277,8 +1336,8 @@ cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaS
             ph.t[i].pitch = t.pitch ? t.pitch : (uint32_t)row_bytes(t.fmt, a.cols);
             ph.t[i].unit0 = units;
             units += (t.rows + 15) / 16;
-            if (t.fmt != FMT_Q8_0) {   // the tiled view the stages' boxes are cut from (16 rows; SwiGLU: 8 + 8)
-                const uint32_t segb = t.fmt == FMT_Q4_K ? kSeg4 : kSeg6, brows = a.swiglu ? 8 : 16;
+            {   // the tiled view the stages' boxes are cut from (16 rows; SwiGLU: 8 + 8)
+                const uint32_t segb = t.fmt == FMT_Q4_K ? kSeg4 : t.fmt == FMT_Q6_K ? kSeg6 : kPitch8, brows = a.swiglu ? 8 : 16;
                 ph.t[i].swz = (t.fmt == FMT_Q4_K && ph.t[i].pitch % 128 == 0) ? 1 : 0;
                 const cudaError_t e = ph.t[i].swz ? tensor_map_lines_swz(&ph.t[i].map, t.w, t.rows, ph.t[i].pitch, segb / 128, brows)
                                                   : tensor_map_2d(&ph.t[i].map, 8, t.w, ph.t[i].pitch / 8, t.rows, ph.t[i].pitch,
@@ -1288,12 +1347,14 @@ cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaS
             (t.fmt == FMT_Q6_K ? q6 : q4) = true;   // Q8_0 uses the Q4_K layout of the activation
             any8 = any8 || t.fmt == FMT_Q8_0;
             q8 = q8 || t.fmt == FMT_Q8_0;
+            only8 = only8 && t.fmt == FMT_Q8_0;
         }
         if (a.swiglu) units = (a.t[0].rows + 7) / 8;
         ph.x = a.x; ph.x2 = a.x2; ph.wnorm = a.wnorm; ph.eps = a.eps; ph.cols = a.cols; ph.x_mode = a.x_mode;
         ph.accumulate = a.accumulate; ph.swiglu = a.swiglu; ph.total_units = units;
         ph.use_q4 = q4 ? 1 : 0; ph.use_q6 = q6 ? 1 : 0;
-        ph.q4_i8 = (!q8 && tc_q4_i8()) ? 1 : 0;
+        const bool special = n == 1 && tc_special() && a.x_mode != MV_X_SILU_MUL && a.xn_out == nullptr;
+        ph.q4_i8 = (tc_q4_i8() && (!q8 || (only8 && special))) ? 1 : 0;
         ph.xn_out = a.xn_out;
         any6 = any6 || q6;
         xmax = std::max(xmax, tc_x_bytes(a.cols, q4, q6, ph.q4_i8 != 0));
@@ -1326,17 +1387,18 @@ cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaS
     if (groups == 2) {
         const dim3 block((2 * kCW + 2) * 32);
         const bool pdl = args[0].pdl != 0;
-        static const bool generic = getenv("FLB_TC_GENERIC") && getenv("FLB_TC_GENERIC")[0] == '1';   // A/B: the run-time form for every launch
         const TcPhase &p0 = k.ph[0];
         // the specialised instances: one phase, integer forms, plain or RMSNorm prologue, no copy of the activation asked for
-        const bool special = n == 1 && p0.q4_i8 && !generic && p0.x_mode != MV_X_SILU_MUL && p0.xn_out == nullptr;
-        const int f = special ? (p0.use_q4 ? 1 : 0) | (p0.use_q6 ? 2 : 0) : 0;
+        const bool special = n == 1 && p0.q4_i8 && tc_special() && p0.x_mode != MV_X_SILU_MUL && p0.xn_out == nullptr;
+        const int f = special ? (any8 ? 4 : (p0.use_q4 ? 1 : 0) | (p0.use_q6 ? 2 : 0)) : 0;
         const bool one = p0.cols / 256 <= 2u * (2 * kCW + 1);   // every half-warp of the prologue converts at most one block
         if (f == 1) return one ? launch_kernel(matvec_tc_kernel<2, 1, 1>, dim3(grid), block, smem, stream, pdl, k)
                                : launch_kernel(matvec_tc_kernel<2, 1, 2>, dim3(grid), block, smem, stream, pdl, k);
         // Q6_K only: the two-block instance for every width (the one-block instance spills in its consume loop: with 18
         // warps a thread can have 96 registers, five warps share a quarter of the register file)
         if (f == 2) return launch_kernel(matvec_tc_kernel<2, 2, 2>, dim3(grid), block, smem, stream, pdl, k);
+        if (f == 4) return one ? launch_kernel(matvec_tc_kernel<2, 4, 1>, dim3(grid), block, smem, stream, pdl, k)
+                               : launch_kernel(matvec_tc_kernel<2, 4, 2>, dim3(grid), block, smem, stream, pdl, k);
         if (f == 3) return one ? launch_kernel(matvec_tc_kernel<2, 3, 1>, dim3(grid), block, smem, stream, pdl, k)
                                : launch_kernel(matvec_tc_kernel<2, 3, 2>, dim3(grid), block, smem, stream, pdl, k);
         return launch_kernel(matvec_tc_kernel<2, 0, 0>, dim3(grid), block, smem, stream, pdl, k);
