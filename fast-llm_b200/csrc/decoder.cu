@@ -15,6 +15,7 @@
 
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
 #include <vector>
 
 using namespace flb;
@@ -114,6 +115,7 @@ struct fl_b200_decoder {
         cudaGraphExec_t exec[FL_B200_MAX_BATCH + 1] = {};
         uint32_t last_m = 0;
         bool ready = false;
+        uint8_t *arena = nullptr;           // the one allocation that holds all of the above but h_io
     } b;
     // Independent sequences decoded in lock step (fl_b200_decoder_seqs_*): per layer one cache [n_seq][n_kv_head][max_kv][128]
     // for K and one for V, a position per sequence, and one CUDA graph of the pass (the batch pass's buffers serve it).
@@ -448,11 +450,7 @@ void fl_b200_decoder_destroy(fl_b200_decoder *d) {
         if (d->b.exec[m]) cudaGraphExecDestroy(d->b.exec[m]);
         if (d->b.graph[m]) cudaGraphDestroy(d->b.graph[m]);
     }
-    cudaFree(d->b.x); cudaFree(d->b.xn); cudaFree(d->b.q); cudaFree(d->b.k); cudaFree(d->b.v); cudaFree(d->b.att);
-    cudaFree(d->b.g); cudaFree(d->b.u); cudaFree(d->b.logits); cudaFree(d->b.margin); cudaFree(d->b.part);
-    cudaFree(d->b.io); cudaFree(d->b.tickets); cudaFree(d->b.partial); cudaFree(d->b.top3);
-    cudaFree(d->b.qkv); cudaFree(d->b.planes); cudaFree(d->b.gp); cudaFree(d->b.up); cudaFree(d->b.head);
-    cudaFree(d->b.am); cudaFree(d->b.am_tickets); cudaFree(d->b.rope);
+    cudaFree(d->b.arena);
     cudaFreeHost(d->b.h_io);
     cudaFreeHost(d->h_pin);
     delete d;
@@ -728,36 +726,35 @@ static int batch_alloc(fl_b200_decoder *d) {
     static_assert(FL_B200_MAX_BATCH <= (int)kNxMaxTokens, "a batch pass is one multi-column pass");
     const fl_b200_llama_cfg &c = d->c;
     const size_t M = FL_B200_MAX_BATCH, E = c.n_embd, QD = (size_t)d->Hq * c.head_dim, KD = (size_t)d->Hkv * c.head_dim;
-    CK(cudaMalloc(&d->b.x, M * E * 4)); CK(cudaMalloc(&d->b.xn, M * E * 4));
-    CK(cudaMalloc(&d->b.q, M * QD * 4)); CK(cudaMalloc(&d->b.k, M * KD * 4)); CK(cudaMalloc(&d->b.v, M * KD * 4));
-    CK(cudaMalloc(&d->b.att, M * QD * 4));
-    CK(cudaMalloc(&d->b.g, M * (size_t)d->F * 4)); CK(cudaMalloc(&d->b.u, M * (size_t)d->F * 4));
-    CK(cudaMalloc(&d->b.logits, M * (size_t)d->V * 4)); CK(cudaMalloc(&d->b.margin, M * 4));
+    auto &w = d->b;
     size_t part = 0;
     for (uint32_t m = 1; m <= M; ++m)
         for (const bool shared : {false, true})
             part = std::max(part, attn_part_floats(d->Hq, m, attn_pick_splits(d->Hkv, m, c.max_kv, d->ctx->sms, shared)));
-    CK(cudaMalloc(&d->b.part, part * sizeof(float)));
-    if (d->tp_size > 1) {
-        CK(cudaMalloc(&d->b.partial, M * E * 4));
-        CK(cudaMalloc(&d->b.top3, M * 16));
-    }
-    CK(cudaMalloc(&d->b.io, 3 * FL_B200_MAX_BATCH * sizeof(int32_t)));
-    CK(cudaMalloc(&d->b.tickets, (size_t)d->Hkv * M * sizeof(uint32_t)));
-    CK(cudaMemset(d->b.tickets, 0, (size_t)d->Hkv * M * sizeof(uint32_t)));
     uint32_t pl[5];
-    d->b.nx = nx_eligible(d, pl);
-    if (d->b.nx) {
-        CK(cudaMalloc(&d->b.qkv, pl[0] * M * (QD + 2 * KD) * 4));
-        CK(cudaMalloc(&d->b.planes, std::max(pl[1], pl[3]) * M * E * 4));
-        CK(cudaMalloc(&d->b.gp, pl[2] * M * (size_t)d->F * 4));
-        CK(cudaMalloc(&d->b.up, pl[2] * M * (size_t)d->F * 4));
-        if (pl[4] > 1) CK(cudaMalloc(&d->b.head, pl[4] * M * (size_t)d->V * 4));
-        CK(cudaMalloc(&d->b.am, M * kArgmaxScratch * 4));
-        CK(cudaMalloc(&d->b.am_tickets, M * 4));
-        CK(cudaMemset(d->b.am_tickets, 0, M * 4));
-        CK(cudaMalloc(&d->b.rope, M * (c.head_dim / 2) * sizeof(float2)));
-    }
+    w.nx = nx_eligible(d, pl);
+    // one allocation for all buffers: a dozen of them were most of the time of a decoder's first pass
+    size_t total = 0;
+    auto layout = [&](auto &&take) {
+        take(w.x, M * E); take(w.att, M * QD); take(w.logits, M * (size_t)d->V); take(w.margin, M); take(w.part, part);
+        take(w.io, 3 * M); take(w.tickets, (size_t)d->Hkv * M);
+        if (d->tp_size > 1) { take(w.partial, M * E); take(w.top3, M * 4); }
+        if (!w.nx || d->tp_size > 1) { take(w.xn, M * E); take(w.q, M * std::max(QD, E)); }
+        if (w.nx) {
+            take(w.qkv, pl[0] * M * (QD + 2 * KD)); take(w.planes, std::max(pl[1], pl[3]) * M * E);
+            take(w.gp, pl[2] * M * (size_t)d->F); take(w.up, pl[2] * M * (size_t)d->F);
+            if (pl[4] > 1) take(w.head, pl[4] * M * (size_t)d->V);
+            take(w.am, M * kArgmaxScratch); take(w.am_tickets, M); take(w.rope, M * (c.head_dim / 2));
+        } else {
+            take(w.k, M * KD); take(w.v, M * KD); take(w.g, M * (size_t)d->F); take(w.u, M * (size_t)d->F);
+        }
+    };
+    layout([&](auto *&p, size_t n) { total += (n * sizeof(*p) + 255) & ~(size_t)255; });
+    if (!w.arena) CK(cudaMalloc(&w.arena, total));
+    uint8_t *at = w.arena;
+    layout([&](auto *&p, size_t n) { p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(at); at += (n * sizeof(*p) + 255) & ~(size_t)255; });
+    CK(cudaMemsetAsync(w.tickets, 0, (size_t)d->Hkv * M * sizeof(uint32_t), d->ctx->stream));
+    if (w.nx) CK(cudaMemsetAsync(w.am_tickets, 0, M * sizeof(uint32_t), d->ctx->stream));
     CK(cudaMallocHost(&d->b.h_io, 4 * FL_B200_MAX_BATCH * sizeof(int32_t)));
     d->b.ready = true;
     return FL_B200_OK;
