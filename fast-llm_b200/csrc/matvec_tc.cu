@@ -61,8 +61,7 @@ constexpr uint32_t kSeg4 = 8 * 144, kSeg6 = 8 * 210, kSeg8 = 64 * 34;
 // pitch in memory is not a multiple of 128 bytes (columns not a multiple of 2048) fall back to the plain box.
 // Q8_0: a segment is wider than a box may be, so a stage is two boxes of half a segment, one behind the other, each 16 bytes
 // wider than its half: 276 words = 20 mod 32, conflict free for the 32-bit loads of lanes (g, t) at 17 t words. (One bulk
-// copy per row, the form before: 2176 bytes per some 130 cycles of the TMA unit, 4.7 TB/s at most; the 3B-class 8-bit model's
-// step 5.8 ms.)
+// copy per row, the form before: 2176 bytes per some 130 cycles of the TMA unit, 4.7 TB/s at most.)
 constexpr uint32_t kPitch4 = kSeg4, kPitch6 = kSeg6, kPitch8 = kSeg8 / 2 + 16;
 // ring slots are multiples of 1024 bytes: the swizzle pattern of a Q4_K stage is tied to the address
 constexpr uint32_t slot_round(uint32_t b) { return (b + 1023u) & ~1023u; }
@@ -155,13 +154,6 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 __device__ __forceinline__ void imma16832(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                           uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// The same with signed 8-bit weights
-__device__ __forceinline__ void imma16832_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                             uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -618,37 +610,6 @@ __device__ __forceinline__ void q6k_block_i8(uint32_t r0, uint32_t r1, uint32_t 
 // from `r0` / `r1` (4-byte aligned). The first block's quants start 2 bytes into a word and are realigned with
 // byte permutes; the second block's are aligned. An int8 s becomes f16 through (s ^ 0x80) under 0x64: 1024 + 128 + s,
 // minus 1152, exact. The activation uses the Q4_K layout (64 consecutive columns per lane column, words of 4).
-// Integer form (q8_0_block_i8): the int8 quants are signed 8-bit operands as they are, the activation is the fixed-point image
-// of the Q4_K integer form (the same 64 columns per lane column, words of 4, one scale per 32 columns = one Q8_0 block; the
-// 1 / 16 that Q4_K's high nibbles want in the odd sub-blocks' scales is taken off again). No unpacking at all.
-__device__ __forceinline__ void q8_0_block_i8(uint32_t r0, uint32_t xaddr, uint32_t xstride, float2 xs2, float &out0, float &out1) {
-    const uint32_t r1 = r0 + 8 * kPitch8;
-    uint32_t w0[17], w1[17];
-#pragma unroll
-    for (int i = 0; i < 17; ++i) { w0[i] = lds32(r0 + 4 * i); w1[i] = lds32(r1 + 4 * i); }
-    int cA[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, cB[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        const uint4 bA = lds128(xaddr + (2 * m) * xstride), bB = lds128(xaddr + (2 * m + 1) * xstride);
-        // the first block's quants start 2 bytes into a word, the second block's are aligned
-        const uint32_t a0 = __byte_perm(w0[2 * m], w0[2 * m + 1], 0x5432u), a2 = __byte_perm(w0[2 * m + 1], w0[2 * m + 2], 0x5432u);
-        const uint32_t a1 = __byte_perm(w1[2 * m], w1[2 * m + 1], 0x5432u), a3 = __byte_perm(w1[2 * m + 1], w1[2 * m + 2], 0x5432u);
-        imma16832_s8(cA[0], a0, a1, a2, a3, bA.x, bA.y);
-        imma16832_s8(cB[0], w0[9 + 2 * m], w1[9 + 2 * m], w0[10 + 2 * m], w1[10 + 2 * m], bB.x, bB.y);
-        imma16832_s8(cA[1], a0, a1, a2, a3, bA.z, bA.w);
-        imma16832_s8(cB[1], w0[9 + 2 * m], w1[9 + 2 * m], w0[10 + 2 * m], w1[10 + 2 * m], bB.z, bB.w);
-    }
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const uint32_t wa = r ? w1[0] : w0[0], wb = r ? w1[8] : w0[8];
-        const float dA = h2f_bits((uint16_t)(wa & 0xFFFFu)), dB = h2f_bits((uint16_t)(wb >> 16));
-        // the four plane sums of a block as one number: two exact integer steps (|.| < 2^28), then f32
-        const float ta = fmaf((float)(cA[0][2 * r] * 256 + cA[0][2 * r + 1]), 65536.f, (float)(cA[1][2 * r] * 256 + cA[1][2 * r + 1]));
-        const float tb = fmaf((float)(cB[0][2 * r] * 256 + cB[0][2 * r + 1]), 65536.f, (float)(cB[1][2 * r] * 256 + cB[1][2 * r + 1]));
-        (r ? out1 : out0) = dA * (xs2.x * ta) + dB * (16.f * xs2.y * tb);
-    }
-}
-
 __device__ __forceinline__ void q8_0_block(uint32_t r0, uint32_t r1, uint32_t xaddr, uint32_t xstride, float &out0, float &out1) {
     uint32_t w0[17], w1[17];
 #pragma unroll
@@ -721,7 +682,7 @@ __device__ __forceinline__ bool grid_barrier(GridBar *b, uint32_t nblocks, uint3
 // between; the producer does not take part in the barriers: the weights of the next phase are already
 // streaming into the ring while the current phase drains and the next activation is built.
 // F: 0 = every format and form, decided per phase at run time (f16 forms, Q8_0 beside K-quants, several phases); 1 / 2 / 3 / 4 =
-// one phase on the integer forms holding Q4_K tensors only / Q6_K only / both / Q8_0 only: what a decode step launches. The specialised
+// one phase holding Q4_K tensors only / Q6_K only / both (integer forms) / Q8_0 only (f16 form): what a decode step launches. The specialised
 // instances carry only their own code (the whole kernel is some 7000 instructions, and a launch that has to fetch its
 // path out of that from L2 starts later) and get their own register allocation.
 // R: 256-column blocks a half-warp of the prologue converts (F != 0: 1 up to 34 blocks = 8704 columns, else 2; the
@@ -820,7 +781,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
     for (int p = 0; p < a.n_phases; ++p) {
         const TcPhase &ph = a.ph[p];
         const uint32_t nblk = ph.cols / 256, nseg = (nblk + 7) / 8;
-        const bool I8 = F ? true : ph.q4_i8 != 0, UQ4 = F ? (F & 5) != 0 : ph.use_q4 != 0, UQ6 = F ? (F & 2) != 0 : ph.use_q6 != 0;
+        const bool I8 = F ? F != 4 : ph.q4_i8 != 0, UQ4 = F ? (F & 5) != 0 : ph.use_q4 != 0, UQ6 = F ? (F & 2) != 0 : ph.use_q6 != 0;
         const TcSmem sm = tc_carve<G>(smem_raw, ph.cols, UQ4, UQ6, I8, S, a.ring_off);
         const uint32_t my_units = blockIdx.x < ph.total_units ? (ph.total_units - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
         const bool late = F == 0 && p > 0;   // the activation was written by the previous phase of this launch: read it past L1
@@ -1006,7 +967,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                 }
                 const float sum32 = sum + __shfl_xor_sync(0xffffffffu, sum, 1);
                 if (live) {
-                    if (F == 0 && UQ4 && !I8) {
+                    if ((F == 0 || F == 4) && UQ4 && !I8) {
                         // columns 16 hl .. 16 hl + 15: chunk c = hl / 4, sub-block half (hl / 2) & 1, words 4 (hl & 1) + j
                         const uint32_t c = hl >> 2, sub = (hl >> 1) & 1u, j0 = 4 * (hl & 1u);
                         const uint32_t base = smem_u32(sm.x4) + blk * 1024u;
@@ -1123,11 +1084,11 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                         mbar_wait_or_die(&sm.full[c_slot], c_par, a.status, dead);
                         if (blk < nblk) {
                             const uint32_t r0 = ring + c_slot * a.slot_bytes + ((w >> 2) * 16 + g) * kPitch8 + (w & 3u) * 272u + t * 68u;
-                            const float2 xs2 = *reinterpret_cast<const float2 *>(sm.xs8 + blk * 8 + 2 * t);
                             float o0, o1;
-                            q8_0_block_i8(r0, xa4 + blk * xb, xstride, xs2, o0, o1);
-                            acc0 += o0;
-                            acc1 += o1;
+                            q8_0_block(r0, r0 + 8 * kPitch8, xa4 + blk * xb, xstride, o0, o1);
+                            const float xs = sm.xs[blk];
+                            acc0 = fmaf(xs, o0, acc0);
+                            acc1 = fmaf(xs, o1, acc1);
                         }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&sm.empty[c_slot]);
@@ -1267,7 +1228,6 @@ cudaError_t matvec_tc_init(void) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(matvec_tc_kernel<2, 3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1276,8 +1236,8 @@ cudaError_t matvec_tc_init(void) {
 
 // True when the launch can run on the tensor-core kernel: Q4_K / Q6_K / Q8_0 tensors only, whole 256-column
 // blocks, 16-byte aligned rows, no expert indirection and no exchange prologue.
-// Q4_K and Q6_K on the integer forms (q4k_block_i8, q6k_block_i8) unless FLB_TC_I8=0, Q8_0 too where a launch holds nothing else
-// and runs on a specialised instance; a launch that mixes it with K-quants stays on the f16 forms.
+// Q4_K and Q6_K on the integer forms (q4k_block_i8, q6k_block_i8) unless FLB_TC_I8=0; a launch that holds a Q8_0
+// tensor stays on the f16 forms (Q8_0 reads the f16 image of the activation).
 bool tc_q4_i8() {
     static const bool on = !(getenv("FLB_TC_I8") && getenv("FLB_TC_I8")[0] == '0');
     return on;
@@ -1308,7 +1268,7 @@ bool matvec_tc_eligible(const MatvecArgs &a) {
     }
     if (a.swiglu && (a.n_tensors != 2 || a.t[0].rows != a.t[1].rows || a.t[0].fmt != a.t[1].fmt || a.accumulate)) return false;
     const uint32_t slot = q8 ? kSlot8 : q6 ? kSlot6 : kSlot4;
-    return tc_head_bytes(2, groups) + tc_x_bytes(a.cols, q4, q6, tc_q4_i8()) + 1024 + 2u * slot <= 227 * 1024 - 1024;
+    return tc_head_bytes(2, groups) + tc_x_bytes(a.cols, q4, q6, !q8 && tc_q4_i8()) + 1024 + 2u * slot <= 227 * 1024 - 1024;
 }
 
 // One launch of n dependent matvecs (phase i + 1 consumes what phase i writes). n = 1: a plain launch.
@@ -1319,7 +1279,7 @@ cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaS
     TcArgs k;
     memset(&k, 0, sizeof(k));
     const int groups = tc_groups();
-    bool any6 = false, any8 = false;
+    bool any6 = false, any8 = false, all8 = true;
     size_t xmax = 0;
     uint32_t max_units = 0;
     for (int p = 0; p < n; ++p) {
@@ -1353,8 +1313,8 @@ cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaS
         ph.x = a.x; ph.x2 = a.x2; ph.wnorm = a.wnorm; ph.eps = a.eps; ph.cols = a.cols; ph.x_mode = a.x_mode;
         ph.accumulate = a.accumulate; ph.swiglu = a.swiglu; ph.total_units = units;
         ph.use_q4 = q4 ? 1 : 0; ph.use_q6 = q6 ? 1 : 0;
-        const bool special = n == 1 && tc_special() && a.x_mode != MV_X_SILU_MUL && a.xn_out == nullptr;
-        ph.q4_i8 = (tc_q4_i8() && (!q8 || (only8 && special))) ? 1 : 0;
+        ph.q4_i8 = (!q8 && tc_q4_i8()) ? 1 : 0;
+        all8 = all8 && only8;
         ph.xn_out = a.xn_out;
         any6 = any6 || q6;
         xmax = std::max(xmax, tc_x_bytes(a.cols, q4, q6, ph.q4_i8 != 0));
@@ -1388,17 +1348,16 @@ cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaS
         const dim3 block((2 * kCW + 2) * 32);
         const bool pdl = args[0].pdl != 0;
         const TcPhase &p0 = k.ph[0];
-        // the specialised instances: one phase, integer forms, plain or RMSNorm prologue, no copy of the activation asked for
-        const bool special = n == 1 && p0.q4_i8 && tc_special() && p0.x_mode != MV_X_SILU_MUL && p0.xn_out == nullptr;
-        const int f = special ? (any8 ? 4 : (p0.use_q4 ? 1 : 0) | (p0.use_q6 ? 2 : 0)) : 0;
+        // the specialised instances: one phase, integer forms or Q8_0 alone, plain or RMSNorm prologue, no copy of the activation asked for
+        const bool special = n == 1 && (p0.q4_i8 || all8) && tc_special() && p0.x_mode != MV_X_SILU_MUL && p0.xn_out == nullptr;
+        const int f = special ? (all8 ? 4 : (p0.use_q4 ? 1 : 0) | (p0.use_q6 ? 2 : 0)) : 0;
         const bool one = p0.cols / 256 <= 2u * (2 * kCW + 1);   // every half-warp of the prologue converts at most one block
         if (f == 1) return one ? launch_kernel(matvec_tc_kernel<2, 1, 1>, dim3(grid), block, smem, stream, pdl, k)
                                : launch_kernel(matvec_tc_kernel<2, 1, 2>, dim3(grid), block, smem, stream, pdl, k);
         // Q6_K only: the two-block instance for every width (the one-block instance spills in its consume loop: with 18
         // warps a thread can have 96 registers, five warps share a quarter of the register file)
         if (f == 2) return launch_kernel(matvec_tc_kernel<2, 2, 2>, dim3(grid), block, smem, stream, pdl, k);
-        if (f == 4) return one ? launch_kernel(matvec_tc_kernel<2, 4, 1>, dim3(grid), block, smem, stream, pdl, k)
-                               : launch_kernel(matvec_tc_kernel<2, 4, 2>, dim3(grid), block, smem, stream, pdl, k);
+        if (f == 4) return launch_kernel(matvec_tc_kernel<2, 4, 2>, dim3(grid), block, smem, stream, pdl, k);   // (one block: spills)
         if (f == 3) return one ? launch_kernel(matvec_tc_kernel<2, 3, 1>, dim3(grid), block, smem, stream, pdl, k)
                                : launch_kernel(matvec_tc_kernel<2, 3, 2>, dim3(grid), block, smem, stream, pdl, k);
         return launch_kernel(matvec_tc_kernel<2, 0, 0>, dim3(grid), block, smem, stream, pdl, k);
