@@ -407,7 +407,8 @@ __device__ __noinline__ void nx_list_pieces(const NxArgs &a, uint8_t *smem_raw) 
     count[1] = min((kSmemLimit - ring_off) / (2 * a.slot_bytes), kMaxSlots);
     count[2] = ring_off;
     const uint32_t W = a.group_cost * n_act;   // < 2^31 (checked on the host)
-    const uint32_t lo = (uint32_t)((uint64_t)W * blockIdx.x / gridDim.x), hi = (uint32_t)((uint64_t)W * (blockIdx.x + 1) / gridDim.x);
+    const uint32_t wq = W / gridDim.x, wr = W % gridDim.x;   // equal shares, W x / gridDim.x without 64-bit divisions
+    const uint32_t lo = wq * blockIdx.x + wr * blockIdx.x / gridDim.x, hi = wq * (blockIdx.x + 1) + wr * (blockIdx.x + 1) / gridDim.x;
     for (uint32_t g = lo / a.group_cost; g < n_act && g * a.group_cost < hi; ++g) {
         uint4 e = make_uint4(0u, a.P, 0u, 0u);
         if (a.table) e = reinterpret_cast<const uint4 *>(a.table)[1 + g];
@@ -717,8 +718,9 @@ __device__ __forceinline__ void consume(const NxArgs &a, uint32_t smem, const Nx
 }
 
 // FM: the formats an instance carries (bit 0 Q4_K, 1 Q6_K, 2 Q8_0): with all three in one kernel, what is live across the
-// choice of the body does not fit in the registers beside the largest of them (204 bytes of spills against 0..48).
-template <int FM>
+// choice of the body does not fit in the registers beside the largest of them (204 bytes of spills against 0..48). T: the
+// most token groups a piece can have, 2 or 4, for the same reason (Q4_K: no spills against 60 bytes).
+template <int FM, int T>
 __global__ void __launch_bounds__(kThreads, 1) matmul_nx_kernel(const __grid_constant__ NxArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -738,6 +740,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_nx_kernel(const __grid_con
         mbar_init(bar_at(smem + kXEmpty), kConsumers);
         fence_barrier_init();
     }
+    if (warp == 3 && lane < 3 && a.t[lane].units) asm volatile("prefetch.tensormap [%0];" ::"l"(&a.map[lane]) : "memory");
     if (tid == 32) nx_list_pieces(a, smem_raw);
     __syncthreads();
     const uint32_t n_pieces = lds32(smem + kPieces), slots = lds32(smem + kPieces + 4), ring = smem + lds32(smem + kPieces + 8);
@@ -886,7 +889,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_nx_kernel(const __grid_con
         const uint32_t ntg = (pc.n_valid + 3) / 4;
 #define FLB_CONSUME(F, N) consume<F, N>(a, smem, jb, u0, u1, grp8, w, lane, rg, red_par, dead)
 #define FLB_CONSUME_F(F)                                                                                             \
-    (ntg == 1 ? FLB_CONSUME(F, 1) : ntg == 2 ? FLB_CONSUME(F, 2) : ntg == 3 ? FLB_CONSUME(F, 3) : FLB_CONSUME(F, 4))
+    (ntg == 1 ? FLB_CONSUME(F, 1) : T == 2 || ntg == 2 ? FLB_CONSUME(F, 2) : ntg == 3 ? FLB_CONSUME(F, 3) : FLB_CONSUME(F, 4))
         if ((FM & 1) && (FM == 1 || fmt == FMT_Q4_K)) FLB_CONSUME_F(FMT_Q4_K);
         else if ((FM & 2) && (FM == 2 || fmt == FMT_Q6_K)) FLB_CONSUME_F(FMT_Q6_K);
         else if (FM & 4) FLB_CONSUME_F(FMT_Q8_0);
@@ -940,16 +943,18 @@ uint32_t nx_image_off(int fmt, bool q4, bool q6, uint32_t cols, uint32_t tgs) {
     return (uint32_t)o;
 }
 
-void (*const kNxKernels[5])(const NxArgs) = {matmul_nx_kernel<1>, matmul_nx_kernel<2>, matmul_nx_kernel<3>, matmul_nx_kernel<4>,
-                                             matmul_nx_kernel<7>};
+void (*const kNxKernels[2][5])(const NxArgs) = {
+    {matmul_nx_kernel<1, 2>, matmul_nx_kernel<2, 2>, matmul_nx_kernel<3, 2>, matmul_nx_kernel<4, 2>, matmul_nx_kernel<7, 2>},
+    {matmul_nx_kernel<1, 4>, matmul_nx_kernel<2, 4>, matmul_nx_kernel<3, 4>, matmul_nx_kernel<4, 4>, matmul_nx_kernel<7, 4>}};
 
 } // namespace
 
 cudaError_t matmul_tc_nx_init(void) {
-    for (auto k : kNxKernels) {
-        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
-        if (e != cudaSuccess) return e;
-    }
+    for (const auto &row : kNxKernels)
+        for (auto k : row) {
+            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
+            if (e != cudaSuccess) return e;
+        }
     return cudaSuccess;
 }
 
@@ -999,7 +1004,7 @@ cudaError_t launch_nx_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t 
         fmts[i] = t[i].fmt;
         (t[i].fmt == FMT_Q4_K ? q4 : t[i].fmt == FMT_Q6_K ? q6 : q8) = true;
     }
-    const auto kernel = kNxKernels[q8 ? (q4 || q6 ? 4 : 3) : (q4 ? 1 : 0) + (q6 ? 2 : 0) - 1];
+    const auto kernel = kNxKernels[P > 8 ? 1 : 0][q8 ? (q4 || q6 ? 4 : 3) : (q4 ? 1 : 0) + (q6 ? 2 : 0) - 1];
     NxPlan p;
     if (!nx_plan(fmts, n, cols, (P + 3) / 4, split, p) || p.parts * n > (uint32_t)kMaxJobs) return cudaErrorNotSupported;
     const uint32_t nblk = cols / 256, nseg = (nblk + 7) / 8;
