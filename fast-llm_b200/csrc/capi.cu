@@ -272,7 +272,10 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
             in.x = x + (size_t)p0 * xstride; in.xstride = xstride;
             if (x2) in.x2 = x2 + (size_t)p0 * xstride;
             cudaError_t e = cudaSuccess;
-            if (!(same_columns && nx <= kNxMaxTokens)) {   // with more columns than that the scratch holds the last chunk only
+            // the scratch holds these columns already: not with more of them than a chunk (it has the last one only), nor where
+            // the call before may have gone to the tcgen05 kernel, which has a scratch of its own
+            const bool reuse = same_columns && nx <= kNxMaxTokens && !(fmt == FL_B200_Q4_K && getenv("FLB_UMMA"));
+            if (!reuse) {
                 e = launch_nx_convert(in, &t, 1, cols, nt, c->xq, kNxTgs, c->stream, pdl != 0);
                 if (e == cudaErrorNotSupported) break;
                 if (e != cudaSuccess) return cuda_err(e, "activation conversion launch");
