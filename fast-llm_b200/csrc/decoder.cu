@@ -13,6 +13,8 @@
 // then [RMSNorm + head matvec] -> [argmax] -> [advance].
 #include "capi_internal.h"
 
+#include <algorithm>
+
 #include <cmath>
 #include <cstdlib>
 #include <type_traits>
@@ -680,11 +682,18 @@ int fl_b200_decoder_verify(fl_b200_decoder *d, int32_t first_token, const int32_
 }
 
 // ---- Decoder::step_batch (src/model/decoder.h:64-70): m tokens at positions n_past .. n_past + m - 1 in one
-// pass. Every weight tensor is walked once per pass where the multi-column kernel takes it (Q4_K, up to 8
-// columns) and once per token otherwise; the attention launch covers all m positions, position b attending
+// pass. Every weight tensor is walked once per pass where the multi-column kernel takes it and once per token otherwise; the attention launch covers all m positions, position b attending
 // n_past + b + 1 keys of the one cache (the rows of this pass are appended first). ----
-// Passes of fewer tokens than this run as teacher-forced single steps (FLB_BATCH_MIN overrides; 1 = always the batch pass).
-static const uint32_t kBatchMin = getenv("FLB_BATCH_MIN") ? (uint32_t)atoi(getenv("FLB_BATCH_MIN")) : 4u;
+// Passes of fewer tokens than this run as teacher-forced single steps (FLB_BATCH_MIN overrides; 1 = always the batch pass): the
+// fused single-token step against the batch pass, measured at the 8B shape over 4096 positions: one token 1.81 ms; two 3.62
+// against 2.95 ms, three 5.37 against 2.97 ms. Models with a tensor that the multi-column kernel does not take, with experts
+// (where every further token brings experts of its own) or split over several GPUs: from four tokens on.
+static uint32_t batch_min(const fl_b200_decoder *d) {
+    static const uint32_t env = getenv("FLB_BATCH_MIN") ? (uint32_t)atoi(getenv("FLB_BATCH_MIN")) : 0u;
+    if (env) return env;
+    const bool moe = std::any_of(d->moe.begin(), d->moe.end(), [](const fl_b200_moe *x) { return x != nullptr; });
+    return d->b.nx && !moe && d->tp_size == 1 ? 2u : 4u;
+}
 
 // The multi-column launches of a layer's matvec groups, without their outputs (0: Q | K | V, 1: O, 2: gate | up, 3: down) and
 // of the head (4). Returns the number of tensors.
@@ -992,9 +1001,8 @@ int fl_b200_decoder_step_batch(fl_b200_decoder *d, const int32_t *toks, uint32_t
     cudaStream_t s = d->ctx->stream;
     CK(cudaSetDevice(d->ctx->device));
     if (int rc = batch_alloc(d)) return rc;
-    if (m < kBatchMin) {
-        // Few tokens: the fused single-token step, teacher-forced m times on the device, is faster than the batch
-        // pass (measured at the 8B shape: 2.1 / 4.3 / 6.4 ms against 3.5 / 5.4 / 6.6 ms for m = 1 / 2 / 3).
+    if (m < batch_min(d)) {
+        // few tokens: the fused single-token step, teacher-forced m times on the device
         if (m > 1) CK(cudaMemcpyAsync(d->d_forced, toks + 1, (size_t)(m - 1) * 4, cudaMemcpyHostToDevice, s));   // forced[k] follows input k
         d->h_pin[0] = toks[0]; d->h_pin[1] = 0; d->h_pin[2] = d->n_past; d->h_pin[3] = 0; d->h_pin[4] = 0; d->h_pin[5] = 1;
         CK(cudaMemcpyAsync(d->d_token, d->h_pin, 24, cudaMemcpyHostToDevice, s));

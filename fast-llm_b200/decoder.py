@@ -97,7 +97,7 @@ class Decoder:
         return k.value, v.value
 
     def step_batch(self, tokens):
-        """Decoder::step_batch: feeds len(tokens) <= 8 tokens in one pass; returns
+        """Decoder::step_batch: feeds len(tokens) <= 16 tokens in one pass; returns
         (greedy token after each position, its top1 - top2 margin)."""
         m = len(tokens)
         toks = (C.c_int32 * m)(*[int(t) for t in tokens])

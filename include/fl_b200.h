@@ -360,9 +360,10 @@ int fl_b200_decoder_verify(fl_b200_decoder *dec, int32_t first_token, const int3
  * greedy token after position i, margins_host[i] (optional) its top1 - top2
  * margin (Decoder::last_margins, :73); n_past advances by m, and rewind_to
  * (fl_b200_decoder_set_n_past) commits or discards the rows as in the
- * reference. One pass over a tensor serves up to 8 tokens where the multi-column
- * kernel takes its shape (Q4_K and Q6_K; 9 to 16 tokens: two passes); other
- * tensors are walked once per token; passes of fewer than 4 tokens run as
+ * reference. One pass over a tensor serves all tokens where the multi-column
+ * kernel takes its shape (Q4_K, Q6_K, Q8_0); other tensors are walked once per
+ * token; a pass of one token (of up to three for models with experts, with a
+ * tensor that kernel does not take, or over several GPUs) runs as
  * teacher-forced single steps on the device. Used for draft verification and for
  * prompt ingestion in chunks. On a tensor-parallel decoder all ranks make
  * the same call; the partial O / down outputs and the argmax records are
