@@ -1,0 +1,183 @@
+"""GPU tests of the multi-column matmul (csrc/matvec_tc_nx.cu), of its grouped form and of the attention of several positions
+over one cache (csrc/attn.cu: attn_shared_kernel) at the edges of their dispatch, against f64 arithmetic on the same
+quantised weights (dequantisation itself is tested bit for bit elsewhere).
+
+Tolerance of a matmul: a result is a sum of n = columns / 256 super-blocks, each a chain of f32 additions (at most 16
+tensor-core steps, which truncate, and about ten rounded ones), with operands exact to 2^-22. The error of a sum is that
+of its terms' size, not of the result's: 16 * 2^-23 + 2^-22 per super-block, the super-blocks' errors independent, hence
+about 2.2e-6 * sum |w x| / sqrt(n) at worst; measured 1e-7 .. 6e-7 of the result's root mean square. The bound used is
+1e-5 of the root mean square of the exact result, below what a single wrong weight of a row changes."""
+import math
+
+import numpy as np
+import pytest
+
+from fast_llm_b200 import capi, synth
+from fast_llm_b200.moe import MoeBlock
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def weights(ctx, fmt, rows, cols, seed):
+    w = torch.from_numpy(synth.quant_tensor(fmt, np.random.default_rng(seed), rows, cols)).cuda()
+    f = torch.empty((rows, cols), device="cuda")
+    torch.cuda.synchronize()
+    ctx.dequant(fmt, w, rows, cols, f)
+    ctx.sync()
+    return w, f.double()
+
+
+def close(got, want, tol=1e-5):
+    want = want.double()
+    return float((got.double() - want).abs().max() / (want.pow(2).mean().sqrt() + 1e-300)) <= tol
+
+
+CASES = [(fmt, 100, 4096, nx) for fmt in (capi.Q4_K, capi.Q6_K, capi.Q8_0) for nx in (2, 4, 5, 8, 9, 12, 13, 16, 17, 33)]
+CASES += [
+    (capi.Q4_K, 1, 256, 2), (capi.Q6_K, 15, 2048, 3), (capi.Q8_0, 17, 256, 16),      # fewer rows than a unit, one block
+    (capi.Q4_K, 33, 768, 7), (capi.Q8_0, 33, 768, 7), (capi.Q4_K, 50, 2304, 16),     # rows that are no whole swizzle lines
+    (capi.Q8_0, 40, 3072, 11), (capi.Q8_0, 40, 1280, 6),                             # second half of a Q8_0 segment empty
+    (capi.Q4_K, 64, 18432, 16), (capi.Q6_K, 64, 18432, 16), (capi.Q8_0, 64, 18432, 16),   # the most parts
+    (capi.Q4_K, 64, 8192, 4), (capi.Q6_K, 48, 14336, 8), (capi.Q8_0, 48, 14336, 3),
+    (capi.Q4_K, 131072, 4352, 16),   # more rows than the planes of partial results hold: slices
+]
+
+
+@pytest.mark.parametrize("fmt,rows,cols,nx", CASES)
+def test_multi_column_edges(ctx, fmt, rows, cols, nx):
+    w, f = weights(ctx, fmt, rows, cols, rows + cols + nx)
+    gen = torch.Generator(device="cuda").manual_seed(nx)
+    x = torch.full((nx, cols + 8), float("nan"), device="cuda")   # the gap between columns is never read
+    x[:, :cols] = torch.randn((nx, cols), device="cuda", generator=gen) * torch.logspace(-3, 3, nx, device="cuda")[:, None]
+    y = torch.randn((nx, rows + 3), device="cuda", generator=gen)   # rows of no multiple of 16 bytes
+    want = y.double()
+    want[:, :rows] += x[:, :cols].double() @ f.T
+    torch.cuda.synchronize()
+    ctx.matvec(fmt, w, rows, cols, x, y, nx=nx, xstride=cols + 8, ystride=rows + 3)
+    ctx.sync()
+    assert ctx.status() == 0
+    for p in range(nx):
+        assert close(y[p, :rows], want[p, :rows]), "column %d" % p
+        assert torch.equal(y[p, rows:].double(), want[p, rows:]), "written past the rows of column %d" % p
+
+
+@pytest.mark.parametrize("fmt", [capi.Q4_K, capi.Q6_K, capi.Q8_0])
+def test_multi_column_special_values(ctx, fmt):
+    """Zero columns, the smallest and largest magnitudes, one outlier per column; a column that holds an infinity or a NaN
+    spoils its own results only."""
+    rows, cols, nx = 64, 2048, 8
+    w, f = weights(ctx, fmt, rows, cols, 3)
+    x = torch.randn((nx, cols), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    x[1] = 0
+    x[2] *= 1e-30
+    x[3] *= 1e25
+    x[4, 700] = 1e6
+    x[5, 9] = float("inf")
+    x[6, 2047] = float("nan")
+    y = torch.zeros((nx, rows), device="cuda")
+    torch.cuda.synchronize()
+    ctx.matvec(fmt, w, rows, cols, x, y, nx=nx, xstride=cols, ystride=rows)
+    ctx.sync()
+    assert torch.equal(y[1], torch.zeros_like(y[1]))
+    for p in (0, 2, 3, 4, 7):
+        assert close(y[p], f @ x[p].double()), "column %d" % p
+    assert not torch.isfinite(y[5]).any() and torch.isnan(y[6]).all()
+
+
+@pytest.mark.parametrize("fmt_gu,fmt_d,n_expert,top_k,n_tok,max_tokens", [
+    (capi.Q4_K, capi.Q4_K, 8, 2, 16, 16), (capi.Q4_K, capi.Q6_K, 16, 1, 3, 16), (capi.Q6_K, capi.Q4_K, 4, 4, 16, 16),
+    (capi.Q4_K, capi.Q4_K, 4, 3, 45, 64),    # more tokens per expert than a pass takes
+    (capi.Q4_K, capi.Q4_K, 64, 1, 2, 16),    # most experts idle
+])
+def test_grouped_experts(ctx, fmt_gu, fmt_d, n_expert, top_k, n_tok, max_tokens):
+    E, F = 2048, 4096
+    blk = MoeBlock(ctx, E, F, n_expert, top_k, norm=1, scale=1.0, fmt_gate_up=fmt_gu, fmt_down=fmt_d, max_tokens=max_tokens)
+    (wg, fg), (wu, fu), (wd, fd) = (weights(ctx, fmt, n_expert * r, c, s)
+                                    for fmt, r, c, s in ((fmt_gu, F, E, 1), (fmt_gu, F, E, 2), (fmt_d, E, F, 3)))
+    gen = torch.Generator(device="cuda").manual_seed(n_tok)
+    router = torch.randn((n_expert, E), device="cuda", generator=gen)
+    x = torch.randn((n_tok, E), device="cuda", generator=gen)
+    y = torch.zeros_like(x)
+    blk.set_weights(router, wg, wu, wd)
+    torch.cuda.synchronize()
+    for _ in range(3):   # direct, recorded, replayed
+        y.zero_()
+        torch.cuda.synchronize()
+        blk.forward(x, n_tok, y)
+        ctx.sync()
+        assert ctx.status() == 0
+    p = torch.softmax(x.double() @ router.double().T, dim=-1)
+    top, ids = torch.topk(p, top_k, dim=-1)
+    top = top / top.sum(-1, keepdim=True)
+    want = torch.zeros((n_tok, E), dtype=torch.float64, device="cuda")
+    for t in range(n_tok):
+        for g, e in zip(top[t], ids[t].tolist()):
+            h = torch.nn.functional.silu(fg[e * F:(e + 1) * F] @ x[t].double()) * (fu[e * F:(e + 1) * F] @ x[t].double())
+            want[t] += g * (fd[e * E:(e + 1) * E] @ h)
+    # silu and the products multiply the relative errors of three matmuls and of the gate
+    assert close(y, want, 1e-4)
+
+
+@pytest.mark.parametrize("n_draft", [2, 3, 7, 8, 9, 16])
+@pytest.mark.parametrize("base", [1, 40, 63, 64, 65, 500, 4100])
+def test_shared_cache_positions(ctx, base, n_draft):
+    """Position b attends base + b keys; the cache rows behind the last one hold NaN."""
+    H, stride = 3, base + n_draft + 70
+    gen = torch.Generator(device="cuda").manual_seed(base * 31 + n_draft)
+    k, v = (torch.full((H, stride, 128), float("nan"), dtype=torch.float16, device="cuda") for _ in "kv")
+    n = base + n_draft - 1
+    for c in (k, v):
+        c[:, :n] = torch.randn((H, n, 128), device="cuda", generator=gen).half()
+    q = torch.randn((n_draft, 4 * H, 128), device="cuda", generator=gen) * 2
+    out = torch.zeros_like(q)
+    torch.cuda.synchronize()
+    ctx.attn_verify(q, k, v, 4 * H, H, 128, base, stride, n_draft, 1 / math.sqrt(128), out)
+    ctx.sync()
+    assert ctx.status() == 0
+    for b in range(n_draft):
+        kk, vv = (c[:, :base + b].double().repeat_interleave(4, dim=0) for c in (k, v))
+        p = torch.softmax(torch.einsum("hd,hkd->hk", q[b].double(), kk) / math.sqrt(128), dim=-1)
+        want = torch.einsum("hk,hkd->hd", p, vv)
+        # probabilities and q are exact to 2^-22, sums f32; expf is within 2 ulp: a few 1e-6 of the context's size
+        assert float((out[b].double() - want).abs().max()) <= 2e-5
+
+
+@pytest.mark.parametrize("rows,cols", [(16, 256), (512, 2304), (48, 14336)])
+def test_expert_rows_one_column(ctx, rows, cols):
+    """One column of a device-side expert: the last expert of the stack, and the mark that makes the launch leave its output
+    alone."""
+    n = 5
+    w, f = weights(ctx, capi.Q4_K, n * rows, cols, rows + cols)
+    x = torch.randn(cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    idx = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for e in (n - 1, 0, -1):
+        y = torch.full((rows,), 3.0, device="cuda")
+        idx.fill_(e)
+        torch.cuda.synchronize()
+        ctx.matvec_expert(capi.Q4_K, w, rows, cols, idx, rows * capi.row_bytes(capi.Q4_K, cols), x, y)
+        ctx.sync()
+        assert ctx.status() == 0
+        if e < 0:
+            assert torch.equal(y, torch.full_like(y, 3.0))
+        else:
+            assert close(y - 3.0, f[e * rows:(e + 1) * rows] @ x.double(), 2e-5)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 256), (33, 1024), (100, 2304), (64, 3072), (40, 14336)])
+def test_q8_0_one_column(ctx, rows, cols):
+    """Q8_0 on the tensor-core kernel, with extreme quants and one outlier in the activation."""
+    w, _ = weights(ctx, capi.Q8_0, rows, cols, rows + cols)
+    blk = w.view(-1, 34)
+    blk[0, 2:] = 0x80                        # -128
+    blk[-1, 2:] = 0x7F
+    f = torch.empty((rows, cols), device="cuda")
+    torch.cuda.synchronize()
+    ctx.dequant(capi.Q8_0, w, rows, cols, f)
+    x = torch.randn(cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(4))
+    x[cols // 2] = 1e4
+    y = torch.zeros(rows, device="cuda")
+    torch.cuda.synchronize()
+    ctx.matvec_assign(capi.Q8_0, w, rows, cols, x, y)
+    ctx.sync()
+    assert close(y, f.double() @ x.double())
