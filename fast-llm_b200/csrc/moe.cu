@@ -37,6 +37,7 @@ struct fl_b200_moe {
     uint32_t *table = nullptr;                                            // active experts of a grouped launch
     uint8_t *xq = nullptr;                                                // converted activations of all active experts
     uint32_t tgs = 0, planes_gu = 0, planes_d = 0;                        // token groups in xq; planes of partial results in g, u / part
+    uint8_t *arena = nullptr;                                             // the one allocation that holds the buffers above
     uint8_t *comm = nullptr;
     uint8_t *peers[kCommMaxRanks] = {};
     bool peers_set = false;
@@ -124,12 +125,6 @@ int fl_b200_moe_create(fl_b200_ctx *ctx, const fl_b200_moe_cfg *cfg, uint32_t ra
         if (cudaError_t e = cudaMemsetAsync(*p, 0, bytes, ctx->stream)) return cuda_err(e, "cudaMemsetAsync (moe)");
         return FL_B200_OK;
     };
-    // zero-filled: a slot that is skipped leaves its buffer as it was, and what is there is then multiplied by gate 0
-    if (int rc = alloc((void **)&m->logits, T * c.n_expert * 4)) return fail(rc);
-    if (int rc = alloc((void **)&m->gates, T * K * 4)) return fail(rc);
-    if (int rc = alloc((void **)&m->mgates, T * K * 4)) return fail(rc);
-    if (int rc = alloc((void **)&m->ids, T * K * 4)) return fail(rc);
-    if (int rc = alloc((void **)&m->lids, T * K * 4)) return fail(rc);
     // the most planes of partial results any number of tokens leads to (0: the per-slot form serves the shape)
     for (uint32_t P = 1; P <= kNxMaxTokens && P <= T; ++P) {
         const NxTensor gu{c.fmt_gate_up, nullptr, (uint32_t)F, 0, nullptr, 0, 0}, dn{c.fmt_down, nullptr, (uint32_t)E, 0, nullptr, 0, 0};
@@ -140,18 +135,26 @@ int fl_b200_moe_create(fl_b200_ctx *ctx, const fl_b200_moe_cfg *cfg, uint32_t ra
         m->planes_d = std::max(m->planes_d, b);
     }
     const size_t n_gu = std::max(1u, m->planes_gu), n_d = std::max(1u, m->planes_d);
-    if (int rc = alloc((void **)&m->g, n_gu * T * K * F * 4)) return fail(rc);   // gate / up outputs, one row per (token, slot) pair
-    if (int rc = alloc((void **)&m->u, n_gu * T * K * F * 4)) return fail(rc);
     // every active expert has at most 16 columns in a pass, all of them together at most one per pair
     m->tgs = (uint32_t)std::min<size_t>((size_t)m->n_local * (kNxMaxTokens / 4), T * K / 4 + std::min<size_t>(m->n_local, T * K));
-    if (int rc = alloc((void **)&m->xq, matmul_tc_nx_scratch_bytes((uint32_t)std::max(E, F), m->tgs, 1))) return fail(rc);
-    if (int rc = alloc((void **)&m->table, (1 + (size_t)m->n_local) * 16)) return fail(rc);
-    if (int rc = alloc((void **)&m->cnt, (size_t)m->n_local * 4)) return fail(rc);
-    if (int rc = alloc((void **)&m->tok_list, (size_t)m->n_local * T * 4)) return fail(rc);
-    if (int rc = alloc((void **)&m->pair_list, (size_t)m->n_local * T * 4)) return fail(rc);
-    if (int rc = alloc((void **)&m->part, n_d * T * K * E * 4)) return fail(rc);
-    if (world > 1) {
-        if (int rc = alloc((void **)&m->partial, T * E * 4)) return fail(rc);
+    // One allocation, zero-filled: a slot that is skipped leaves its buffer as it was, and what is there is then multiplied by gate 0.
+    const struct { void **p; size_t bytes; } bufs[] = {
+        {(void **)&m->logits, T * c.n_expert * 4}, {(void **)&m->gates, T * K * 4}, {(void **)&m->mgates, T * K * 4},
+        {(void **)&m->ids, T * K * 4}, {(void **)&m->lids, T * K * 4},
+        {(void **)&m->g, n_gu * T * K * F * 4}, {(void **)&m->u, n_gu * T * K * F * 4},   // gate / up outputs, one row per (token, slot) pair
+        {(void **)&m->xq, matmul_tc_nx_scratch_bytes((uint32_t)std::max(E, F), m->tgs, 1)}, {(void **)&m->table, (1 + (size_t)m->n_local) * 16},
+        {(void **)&m->cnt, (size_t)m->n_local * 4}, {(void **)&m->tok_list, (size_t)m->n_local * T * 4},
+        {(void **)&m->pair_list, (size_t)m->n_local * T * 4}, {(void **)&m->part, n_d * T * K * E * 4},
+        {(void **)&m->partial, world > 1 ? T * E * 4 : 0}};
+    size_t total = 0;
+    for (const auto &x : bufs) total += (x.bytes + 255) & ~(size_t)255;
+    if (int rc = alloc((void **)&m->arena, total)) return fail(rc);
+    uint8_t *at = m->arena;
+    for (const auto &x : bufs) {
+        if (x.bytes) *x.p = at;
+        at += (x.bytes + 255) & ~(size_t)255;
+    }
+    if (world > 1) {   // mapped by the peers: allocations of their own
         if (int rc = alloc((void **)&m->comm, comm_buffer_bytes())) return fail(rc);
         if (int rc = alloc((void **)&m->comm_state, 64)) return fail(rc);
     }
@@ -164,9 +167,7 @@ void fl_b200_moe_destroy(fl_b200_moe *m) {
     if (!m) return;
     cudaSetDevice(m->ctx->device);
     cudaStreamSynchronize(m->ctx->stream);
-    cudaFree(m->logits); cudaFree(m->gates); cudaFree(m->mgates); cudaFree(m->ids); cudaFree(m->lids); cudaFree(m->g);
-    cudaFree(m->table); cudaFree(m->xq); cudaFree(m->cnt); cudaFree(m->tok_list); cudaFree(m->pair_list);
-    cudaFree(m->u); cudaFree(m->part); cudaFree(m->partial); cudaFree(m->comm); cudaFree(m->comm_state);
+    cudaFree(m->arena); cudaFree(m->comm); cudaFree(m->comm_state);
     if (m->rec.exec) cudaGraphExecDestroy(m->rec.exec);
     if (m->rec.graph) cudaGraphDestroy(m->rec.graph);
     delete m;
