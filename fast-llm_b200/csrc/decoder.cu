@@ -741,7 +741,9 @@ static int batch_alloc(fl_b200_decoder *d) {
         for (const bool shared : {false, true})
             part = std::max(part, attn_part_floats(d->Hq, m, attn_pick_splits(d->Hkv, m, c.max_kv, d->ctx->sms, shared)));
     uint32_t pl[5];
-    w.nx = nx_eligible(d, pl);
+    // FLB_UMMA=1 sends the pass tensor by tensor, where Q4_K goes to the tcgen05 kernel
+    const char *umma = getenv("FLB_UMMA");
+    w.nx = !(umma && umma[0] == '1') && nx_eligible(d, pl);
     // one allocation for all buffers: a dozen of them were most of the time of a decoder's first pass
     size_t total = 0;
     auto layout = [&](auto &&take) {
