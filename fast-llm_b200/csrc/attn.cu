@@ -41,6 +41,8 @@
 #include "common.cuh"
 #include "kernels.h"
 
+#include <type_traits>
+
 namespace flb {
 
 namespace {
@@ -375,7 +377,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(const __gr
 // Grid = (n_splits, n_kv_head, groups of 8 positions), 8 warps: warp w serves position 8 z + w with its 4 query heads over
 // ALL keys of the CTA's tiles, so that a tile crosses from L2 to an SM once for 8 positions. (One CTA per position, the
 // form above, moved every key 8 times: 25 us per layer at 8 positions over 4096 keys, L2 bound; this one takes 8 us.)
-// Position b attends kv_len + b * kv_len_step keys: keys past its own are masked. The arithmetic is that of
+// Position b attends kv_len + b * kv_len_step keys: keys past its own are masked, scores and values. The arithmetic is that of
 // attn_decode_kernel; a warp walks a tile's 64 keys as four blocks of 16 with one maximum and one rescaling per tile. No
 // merge between warps: every warp writes the records of its 4 heads. The splits are added by attn_combine_kernel or by the
 // activation conversion of the matmul that reads the contexts (matvec_tc_nx.cu).
@@ -384,6 +386,9 @@ struct AttnShSmem {
     uint8_t ring[kStages][kStageBytes];   // 1024-byte aligned (swizzle atom)
     uint64_t full[kStages];
 };
+
+// Mask of the pair of halves that belong to keys p and p + 1: those below n.
+__device__ __forceinline__ uint32_t keys_below(uint32_t p, uint32_t n) { return (p < n ? 0xFFFFu : 0u) | (p + 1 < n ? 0xFFFF0000u : 0u); }
 
 __global__ void __launch_bounds__(kShWarps * 32, 2) attn_shared_kernel(const __grid_constant__ AttnArgs a) {
     extern __shared__ uint8_t smem_dyn[];
@@ -447,14 +452,6 @@ __global__ void __launch_bounds__(kShWarps * 32, 2) attn_shared_kernel(const __g
         const uint32_t slot = it % kStages, p0 = (t0 + it) * kTile;
         const uint32_t st = ring + slot * kStageBytes;
         if (!mbar_wait_bounded(&sm.full[slot], (it / kStages) & 1u, a.status)) return;
-        if (kv_max - p0 < (uint32_t)kTile) {
-            // ragged end: rows past every position's keys may hold anything (even NaN): clear them in V so that 0 * V stays 0
-            for (uint32_t k = (kv_max - p0) * 16 + tid; k < kTile * 16; k += kShWarps * 32) {
-                const uint32_t r = k >> 4, c = k & 15u;
-                *reinterpret_cast<uint4 *>(&sm.ring[slot][2 * kHalfBytes + (c >> 3) * kHalfBytes + swz(r, c & 7u)]) = make_uint4(0, 0, 0, 0);
-            }
-            __syncthreads();   // CTA-uniform
-        }
         if (b <= b_last && kv_len > p0) {
             // ---- scores: 4 x S[16 keys][8 columns]; lane (g, t): head t, keys 16 k + g and 16 k + g + 8 ----
             float s[4][2];
@@ -498,19 +495,28 @@ __global__ void __launch_bounds__(kShWarps * 32, 2) attn_shared_kernel(const __g
 #pragma unroll
             for (int dt = 0; dt < 8; ++dt) { o[dt][0] *= al; o[dt][1] *= al; o[dt][2] *= al; o[dt][3] *= al; }
             const uint32_t srcA = (2 * t) * 4 + (g >> 1), srcB = srcA + 4, part = g & 1u, mi = lane >> 3;
+            auto add_values = [&](auto ragged) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float a0 = __shfl_sync(0xffffffffu, s[k][0], srcA), b0 = __shfl_sync(0xffffffffu, s[k][0], srcB);
-                const float a1 = __shfl_sync(0xffffffffu, s[k][1], srcA), b1 = __shfl_sync(0xffffffffu, s[k][1], srcB);
-                const uint32_t pb0 = pack_h2(split_part(a0, part), split_part(b0, part)), pb1 = pack_h2(split_part(a1, part), split_part(b1, part));
-                const uint32_t r = 16 * k + (mi >> 1) * 8 + (lane & 7u);
+                for (int k = 0; k < 4; ++k) {
+                    const float a0 = __shfl_sync(0xffffffffu, s[k][0], srcA), b0 = __shfl_sync(0xffffffffu, s[k][0], srcB);
+                    const float a1 = __shfl_sync(0xffffffffu, s[k][1], srcA), b1 = __shfl_sync(0xffffffffu, s[k][1], srcB);
+                    const uint32_t pb0 = pack_h2(split_part(a0, part), split_part(b0, part)), pb1 = pack_h2(split_part(a1, part), split_part(b1, part));
+                    const uint32_t r = 16 * k + (mi >> 1) * 8 + (lane & 7u);
+                    uint32_t keep0 = 0, keep1 = 0;   // of keys 16 k + 2 t, + 1 (va[0], va[1]) and of those 8 further (va[2], va[3])
+                    if (decltype(ragged)::value) { keep0 = keys_below(p0 + 16 * k + 2 * t, kv_len); keep1 = keys_below(p0 + 16 * k + 8 + 2 * t, kv_len); }
 #pragma unroll
-                for (int dt = 0; dt < 8; ++dt) {
-                    uint32_t va[4];
-                    ldsm_x4_trans(st + 2 * kHalfBytes + (dt >> 2) * kHalfBytes + swz(r, 2 * (dt & 3) + (mi & 1u)), va);
-                    mma_f16(o[dt], va, pb0, pb1);
+                    for (int dt = 0; dt < 8; ++dt) {
+                        uint32_t va[4];
+                        ldsm_x4_trans(st + 2 * kHalfBytes + (dt >> 2) * kHalfBytes + swz(r, 2 * (dt & 3) + (mi & 1u)), va);
+                        if (decltype(ragged)::value) { va[0] &= keep0; va[1] &= keep0; va[2] &= keep1; va[3] &= keep1; }
+                        mma_f16(o[dt], va, pb0, pb1);
+                    }
                 }
-            }
+            };
+            // The tile this position's keys end in: the rows behind them have probability 0 but may hold anything (rows of later
+            // positions with an infinity or a NaN, rows never written), and 0 * inf is NaN, so their values are cleared.
+            if (kv_len - p0 < (uint32_t)kTile) add_values(std::true_type{});
+            else add_values(std::false_type{});
         }
         __syncthreads();   // tile fully consumed by all warps: the slot can be refilled
         if (tid == 0 && it + kStages < n_tiles) issue(it + kStages);

@@ -143,6 +143,31 @@ def test_shared_cache_positions(ctx, base, n_draft):
         assert float((out[b].double() - want).abs().max()) <= 2e-5
 
 
+@pytest.mark.parametrize("base,n_draft,bad", [(60, 4, 2), (1, 8, 3), (58, 8, 5), (500, 16, 9), (4090, 16, 7), (4090, 2, 1)])
+def test_shared_cache_rows_of_later_positions(ctx, base, n_draft, bad):
+    """The rows of positions `bad` and later hold infinities and NaN: the positions in front of them, which do not attend those
+    rows, are what they are without."""
+    H, n = 2, base + n_draft - 1
+    gen = torch.Generator(device="cuda").manual_seed(base + n_draft)
+    k, v = (torch.randn((H, n, 128), device="cuda", generator=gen).half() for _ in "kv")
+    q = torch.randn((n_draft, 4 * H, 128), device="cuda", generator=gen) * 2
+    want, out = torch.zeros_like(q), torch.zeros_like(q)
+    torch.cuda.synchronize()
+    ctx.attn_verify(q, k, v, 4 * H, H, 128, base, n, n_draft, 1 / math.sqrt(128), want)
+    ctx.sync()
+    row = base + bad - 1   # the first row that position `bad` attends and position bad - 1 does not
+    v[:, row] = float("inf")
+    v[:, row + 1:] = float("nan")
+    k[:, row, ::2] = float("-inf")
+    k[:, row + 1:] = float("nan")
+    torch.cuda.synchronize()
+    ctx.attn_verify(q, k, v, 4 * H, H, 128, base, n, n_draft, 1 / math.sqrt(128), out)
+    ctx.sync()
+    assert ctx.status() == 0
+    assert torch.isfinite(want).all()
+    assert torch.equal(out[:bad], want[:bad])   # the same sums in the same order, bit for bit
+
+
 @pytest.mark.parametrize("rows,cols", [(16, 256), (512, 2304), (48, 14336)])
 def test_expert_rows_one_column(ctx, rows, cols):
     """One column of a device-side expert: the last expert of the stack, and the mark that makes the launch leave its output
