@@ -518,26 +518,31 @@ __global__ void __launch_bounds__(kShWarps * 32, 2) attn_shared_kernel(const __g
                     const float p = __shfl_sync(0xffffffffu, s[k][j], srcA), q = __shfl_sync(0xffffffffu, s[k][j], srcB);
                     pb[k][j] = pack_h2(split_part(p, part), split_part(q, part));
                 }
-            // The tile's context from zero in two chains, then onto the running one with rounding: the tensor core truncates its
-            // sum towards zero at every instruction, an error with the sum's own sign, so that a sum carried through it shrinks
-            // with the number of keys (8 positions over 65536 keys, 8 KV heads: relative error 2.3e-6; like this 4.7e-7, as at
-            // 4096 keys, for 1 to 2 % of the time).
+            // The tile's context from zero in two chains (two dimension blocks at a time: four in flight), then onto the running
+            // one with rounding: the tensor core truncates its sum towards zero at every instruction, an error with the sum's own
+            // sign, so that a sum carried through it shrinks with the number of keys (8 positions over 65536 keys, 8 KV heads:
+            // relative error 2.3e-6; like this 4.7e-7, as at 4096 keys, in the same 90 us).
 #pragma unroll
-            for (int dt = 0; dt < 8; ++dt) {
-                float c[2][4];
+            for (int d0 = 0; d0 < 8; d0 += 2) {
+                float c[2][2][4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    uint32_t va[4];
-                    ldsm_x4_trans(st + 2 * kHalfBytes + (dt >> 2) * kHalfBytes + swz(16 * k + (mi >> 1) * 8 + (lane & 7u), 2 * (dt & 3) + (mi & 1u)), va);
-                    if (kRagged) {
-                        const uint32_t key = p0 + 16 * k + 2 * t, keep0 = keys_below(key, kv_len), keep1 = keys_below(key + 8, kv_len);
-                        va[0] &= keep0; va[1] &= keep0; va[2] &= keep1; va[3] &= keep1;
+                for (int k = 0; k < 4; ++k)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int dt = d0 + i;
+                        uint32_t va[4];
+                        ldsm_x4_trans(st + 2 * kHalfBytes + (dt >> 2) * kHalfBytes + swz(16 * k + (mi >> 1) * 8 + (lane & 7u), 2 * (dt & 3) + (mi & 1u)), va);
+                        if (kRagged) {
+                            const uint32_t key = p0 + 16 * k + 2 * t, keep0 = keys_below(key, kv_len), keep1 = keys_below(key + 8, kv_len);
+                            va[0] &= keep0; va[1] &= keep0; va[2] &= keep1; va[3] &= keep1;
+                        }
+                        if (k < 2) mma_f16_first(c[k % 2][i], va, pb[k][0], pb[k][1]);
+                        else mma_f16(c[k % 2][i], va, pb[k][0], pb[k][1]);
                     }
-                    if (k < 2) mma_f16_first(c[k], va, pb[k][0], pb[k][1]);
-                    else mma_f16(c[k - 2], va, pb[k][0], pb[k][1]);
-                }
 #pragma unroll
-                for (int i = 0; i < 4; i += 2) scale_add_pair(o[dt][i], o[dt][i + 1], al, c[0][i], c[0][i + 1], c[1][i], c[1][i + 1]);
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; j += 2) scale_add_pair(o[d0 + i][j], o[d0 + i][j + 1], al, c[0][i][j], c[0][i][j + 1], c[1][i][j], c[1][i][j + 1]);
             }
         };
         if (b <= b_last && kv_len > p0) {
@@ -629,6 +634,19 @@ uint32_t attn_pick_splits(uint32_t n_kv_head, uint32_t batch, uint32_t kv_len, i
     return s;
 }
 
+// 65 tiles over 64 splits are two tiles each for 33 of them; the others would only add empty records to the combine (16 positions,
+// 2 KV heads, 4096 keys: 18.4 us with 64 splits, the one-position kernel 16.4).
+uint32_t attn_used_splits(uint32_t n_splits, uint32_t kv_len) {
+    const uint32_t tiles = (kv_len + kTile - 1) / kTile, tps = (tiles + n_splits - 1) / n_splits;
+    return (tiles + tps - 1) / tps;
+}
+
+// (2 KV heads: 4 positions of one tile 6.2 us against the two launches' 7.0, 8 positions 7.2 against 7.0; 2 positions of two
+// tiles 6.2 against 7.0, 3 positions 7.2 against 7.0; 8 heads: never.)
+bool attn_few_tiles(uint32_t n_kv_head, uint32_t batch, uint32_t kv_len) {
+    return (uint64_t)n_kv_head * batch * ((kv_len + kTile - 1) / kTile) <= 8;
+}
+
 size_t attn_part_floats(uint32_t n_q_head, uint32_t batch, uint32_t n_splits) {
     return (size_t)n_q_head * batch * n_splits * kPartStride;
 }
@@ -692,7 +710,7 @@ cudaError_t launch_attn_decode_static(AttnArgs a, int device, cudaStream_t strea
 size_t attn_static_max_records(void) { return kStaticMaxRecords; }
 uint32_t attn_static_max_tickets(void) { return kStaticMaxTickets; }
 
-bool attn_uses_records(const AttnArgs &a) { return a.shared_kv && a.batch > 1 && !a.rope_k && a.pos_stride == 0 && a.n_splits <= 64; }
+bool attn_uses_records(const AttnArgs &a) { return a.shared_kv && !a.per_position && a.batch > 1 && !a.rope_k && a.pos_stride == 0 && a.n_splits <= 64; }
 
 cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t stream) {
     if (a.n_kv_head == 0 || a.n_q_head != a.n_kv_head * kGroup || a.n_splits == 0 || a.batch == 0)

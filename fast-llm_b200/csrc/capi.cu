@@ -399,7 +399,10 @@ static int attn_impl(fl_b200_ctx *c, const float *q, const uint16_t *k, const ui
     a.n_q_head = n_q;
     a.n_kv_head = n_kv;
     a.batch = batch;
-    a.n_splits = attn_pick_splits(n_kv, batch, pos_dev ? kv_stride : kv_len + (verify ? batch - 1 : 0), c->sms, verify);
+    const uint32_t keys = pos_dev ? kv_stride : kv_len + (verify ? batch - 1 : 0);
+    a.per_position = verify && attn_few_tiles(n_kv, batch, keys) ? 1 : 0;
+    a.n_splits = attn_pick_splits(n_kv, batch, keys, c->sms, verify && !a.per_position);
+    if (verify) a.n_splits = attn_used_splits(a.n_splits, keys);
     a.lse_out = reinterpret_cast<float2 *>(lse_out);
     a.kv_len_step = verify ? 1u : 0u;
     a.shared_kv = verify ? 1u : 0u;

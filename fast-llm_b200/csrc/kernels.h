@@ -189,6 +189,7 @@ struct AttnArgs {
     uint32_t *status;
     int pdl;
     int records_only;      // several positions of one cache (attn_uses_records): leave the splits' records in part, out is not written
+    int per_position;      // several positions of one cache, but one CTA per position all the same (attn_few_tiles)
     unsigned long long *trace;   // optional 4-entry timeline record (diagnostics)
     // Fused RoPE + KV append (the decoder's launch plan): q arrives un-rotated; rope_k / rope_v are this
     // token's k and v ([batch][n_kv_head][128] f32, k un-rotated); the kernel rotates q and k by the angle
@@ -202,6 +203,8 @@ struct AttnArgs {
     CUtensorMap kmap, vmap;         // filled by attn_make_maps
 };
 cudaError_t attn_make_maps(AttnArgs &a);
+// Positions over one cache so few and short that the one-position kernel, a single launch, is the faster one.
+bool attn_few_tiles(uint32_t n_kv_head, uint32_t batch, uint32_t kv_len);
 bool attn_uses_records(const AttnArgs &a);   // the launch is one of several positions over one cache (attn_shared_kernel)
 cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t stream);
 // Same kernel with the split-KV scratch in a fixed file-scope device array
@@ -213,6 +216,7 @@ size_t attn_static_max_records(void);
 uint32_t attn_static_max_tickets(void);
 cudaError_t attn_init(void);
 uint32_t attn_pick_splits(uint32_t n_kv_head, uint32_t batch, uint32_t kv_len, int sms, bool shared_kv = false);
+uint32_t attn_used_splits(uint32_t n_splits, uint32_t kv_len);   // those of n_splits that hold keys when kv_len keys are cut
 size_t attn_part_floats(uint32_t n_q_head, uint32_t batch, uint32_t n_splits);
 
 // ---- comm.cu: exchange steps of the tensor-parallel step ----------------------
