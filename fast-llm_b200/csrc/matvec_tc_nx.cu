@@ -18,18 +18,18 @@
 // instructions for 4 NTG tokens from the same A registers.
 //   Q4_K : the 6-bit scale of the sub-block goes into A exactly. A masked nibble is, as it stands, the subnormal f16
 //          q 2^-24 (q 2^-20 in the high nibble), and one FMA with sc 2^10 (sc 2^6) and -8 sc 2^-14 makes it the f16
-//          number (q - 8) sc 2^-14 (|(q - 8) sc| <= 504: exact). A block's 256 columns are then one chain of accumulators
-//          per nibble kind and the super-block scale d is applied once; lane column t unpacks the 32-byte chunk t. The mins
+//          number (q - 8) sc 2^-14 (|(q - 8) sc| <= 504: exact). A block's 256 columns are then four chains of four
+//          instructions, and the super-block scale d is applied once; lane column t unpacks the 32-byte chunk t. The mins
 //          and the 8 sc are two more instructions: bf16 (min, scale of sub-block k) times the sub-block sums of the
 //          activation as three bf16 parts (24 bits). (q sc instead of (q - 8) sc: larger sums, whose truncation in the
-//          tensor core showed: 3.2e-7 relative error against the 2.1e-7 of a chain per sub-block.)
+//          tensor core showed.)
 //   Q6_K : (q - 32) sc has 13 bits, so the 16 columns of an instruction are one scale group and its f32 result is
 //          scaled afterwards (both columns of a pair in one packed FMA).
 //   Q8_0 : the same with two instructions per 32-column block and the block's f16 scale.
 // Products are exact, sums f32 in a fixed order (warps, then parts): results are reproducible run to run.
 //
 // What bounds it (B200, 148 SMs): a super-block of 16 rows x 256 columns has to be done in about 100 cycles (Q4_K) to
-// keep up with HBM. Tensor pipe: 34 / 66 instructions of 2 cycles per SM for 8 / 16 tokens; shared memory: 8 / 16 KB of
+// keep up with HBM. Tensor pipe: 36 / 72 instructions of 2 cycles per SM for 8 / 16 tokens; shared memory: 8 / 16 KB of
 // B per super-block at 128 bytes a cycle; issue: about 400 instructions over four schedulers, which is the bound.
 //
 // The activations are converted once per call, by a small kernel of their own, into exactly the register image of the
@@ -144,6 +144,13 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// The same with a zero accumulator.
+__device__ __forceinline__ void mma16816_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                               uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
 __device__ __forceinline__ void mma16816_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                               uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -159,6 +166,13 @@ __device__ __forceinline__ uint32_t bytes_bf16(uint32_t w) {
     const uint32_t b = __byte_perm(w, 0x43434343u, 0x4140u);
     const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&b), __floats2bfloat162_rn(128.f, 128.f));
     return *reinterpret_cast<const uint32_t *>(&v);
+}
+// c + (a, b): both columns of a token in one packed addition
+__device__ __forceinline__ float2 add_pair(float2 c, float a, float b) {
+    uint64_t cc = *reinterpret_cast<uint64_t *>(&c), ab;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(ab) : "f"(a), "f"(b));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(cc) : "l"(ab));
+    return *reinterpret_cast<float2 *>(&cc);
 }
 // (c.x, c.y) += s * (a, b): both columns of a token in one packed FMA
 __device__ __forceinline__ void fma_pair(float2 &c, float s, float a, float b) {
@@ -181,7 +195,7 @@ __device__ __forceinline__ float s8f(uint32_t w, int k) {
 //   Q6_K  piece m / 2: half m & 1, m = (2 hf + hq) * 4 + gq the scale group: c = 128 hf + 32 gq + 16 hq + 4 t'
 //   Q8_0  piece b    : c = 32 b + 8 t' + {0, 4}
 // Q4_K, then: (b0, b1) per lane of the mins' instruction: b0 = part h of the sums of sub-blocks 2 t', 2 t' + 1, b1 = the
-// third part (columns of the hi part) or zero. Then four block scales, four sums of squares.
+// third part (columns of the lo part) or zero. Then four block scales, four sums of squares.
 struct ConvArgs {
     const float *x, *x2;           // column p: row p (or the listed row) of x; x2: the value is SiLU(x) * x2
     size_t part_stride;            // n_parts planes of x (and x2), added in order
@@ -333,9 +347,9 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
                 uint8_t *d0 = tail + (4 * (2 * pp) + (sb >> 1)) * 8u + (sb & 1u) * 2u;
                 uint8_t *d1 = tail + (4 * (2 * pp + 1) + (sb >> 1)) * 8u + (sb & 1u) * 2u;
                 *reinterpret_cast<__nv_bfloat16 *>(d0) = p0;
-                *reinterpret_cast<__nv_bfloat16 *>(d0 + 4) = p2;
+                *reinterpret_cast<uint16_t *>(d0 + 4) = 0;
                 *reinterpret_cast<__nv_bfloat16 *>(d1) = p1;
-                *reinterpret_cast<uint16_t *>(d1 + 4) = 0;
+                *reinterpret_cast<__nv_bfloat16 *>(d1 + 4) = p2;
             }
             tail += kMinBytes;
         }
@@ -457,25 +471,19 @@ __device__ __forceinline__ void q4k_block_nx(uint32_t r0, uint32_t offs, uint32_
         sH[r] = __hmul2(s1, __floats2half2_rn(64.f, 64.f)); kH[r] = __hmul2(s1, km8);
         sm[r] = sc | (mn << 16);
     }
-    // Chains of 8 dependent instructions (16: twice the error of the sums): up to 8 tokens one per nibble kind, side by side;
-    // else one after the other, the first one's sums put aside half-way (the registers of two do not fit).
-    constexpr int kChains = NTG <= 2 ? 2 : 1;
-    float half[2][NTG];
-    float c[kChains][NTG][4];
-#pragma unroll
-    for (int i = 0; i < kChains; ++i)
-#pragma unroll
-        for (int tg = 0; tg < NTG; ++tg) c[i][tg][0] = c[i][tg][1] = c[i][tg][2] = c[i][tg][3] = 0.f;
+    // The tensor core truncates its running sum at every instruction, always towards zero: an error that grows with the length
+    // of a chain and has the sum's own sign, so that it does not average out over blocks and adds up over the matmuls of a
+    // layer (chains of 8: -1.0e-7 of every result; a block of experts 4.8e-7 off, of 4 as here 3.1e-7, a scale group at a time,
+    // the form before, 4.1e-7). Hence chains of 4 from zero, added with rounding. Up to 8 tokens (NTG <= 2) all four chains of a
+    // block side by side, added at the end, both columns of a token (hi, lo) at once: the additions wait for nothing (14336 x
+    // 4096, 4 tokens: 17.1 us as with chains of 8; added half-way 18.5). Else one at a time, their sums put aside: the
+    // registers of two do not fit (16 tokens: 30.0 against 28.9 us).
+    constexpr bool kSide = NTG <= 2;
+    constexpr int kStep = kSide ? 4 : 2;   // words (two instructions each) between two chains
+    float c[kSide ? 4 : 1][NTG][4], sum[2][NTG];
     const uint32_t ML = 0x000F000Fu, MH = 0x00F000F0u;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        if (kChains == 1 && j == 4)
-#pragma unroll
-            for (int tg = 0; tg < NTG; ++tg) {
-                half[0][tg] = c[0][tg][0] + c[0][tg][1];
-                half[1][tg] = c[0][tg][2] + c[0][tg][3];
-                c[0][tg][0] = c[0][tg][1] = c[0][tg][2] = c[0][tg][3] = 0.f;
-            }
         const uint4 &q0 = j < 4 ? wa[0] : wb[0], &q1 = j < 4 ? wa[1] : wb[1];
         const uint32_t W0 = (j & 3) == 0 ? q0.x : (j & 3) == 1 ? q0.y : (j & 3) == 2 ? q0.z : q0.w;
         const uint32_t W1 = (j & 3) == 0 ? q1.x : (j & 3) == 1 ? q1.y : (j & 3) == 2 ? q1.z : q1.w;
@@ -484,19 +492,34 @@ __device__ __forceinline__ void q4k_block_nx(uint32_t r0, uint32_t offs, uint32_
         const uint32_t l2 = hfma2_u32(V0 & ML, sL[0], kL[0]), l3 = hfma2_u32(V1 & ML, sL[1], kL[1]);
         const uint32_t h0 = hfma2_u32(W0 & MH, sH[0], kH[0]), h1 = hfma2_u32(W1 & MH, sH[1], kH[1]);
         const uint32_t h2 = hfma2_u32(V0 & MH, sH[0], kH[0]), h3 = hfma2_u32(V1 & MH, sH[1], kH[1]);
+        const int lo = kSide ? j / kStep * 2 : 0, hi = kSide ? lo + 1 : 0;   // the chains of the low and of the high nibbles
 #pragma unroll
         for (int tg = 0; tg < NTG; ++tg) {
             const uint4 b = lds128(xaddr + tg * kXq4 + j * 512 + lane * 16);
-            mma16816(c[0][tg], l0, l1, l2, l3, b.x, b.y);
-            mma16816(c[kChains - 1][tg], h0, h1, h2, h3, b.z, b.w);
+            if (j % kStep == 0) mma16816_first(c[lo][tg], l0, l1, l2, l3, b.x, b.y);
+            else mma16816(c[lo][tg], l0, l1, l2, l3, b.x, b.y);
+            if (kSide && j % kStep == 0) mma16816_first(c[hi][tg], h0, h1, h2, h3, b.z, b.w);
+            else mma16816(c[hi][tg], h0, h1, h2, h3, b.z, b.w);
         }
-    }
-    if (kChains == 2)
+        if (!kSide && j % kStep == kStep - 1)
 #pragma unroll
-        for (int tg = 0; tg < NTG; ++tg) {
-            half[0][tg] = c[kChains - 1][tg][0] + c[kChains - 1][tg][1];
-            half[1][tg] = c[kChains - 1][tg][2] + c[kChains - 1][tg][3];
-        }
+            for (int tg = 0; tg < NTG; ++tg)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const float v = c[0][tg][2 * r] + c[0][tg][2 * r + 1];
+                    sum[r][tg] = j < kStep ? v : sum[r][tg] + v;
+                }
+    }
+    if (kSide)
+#pragma unroll
+        for (int tg = 0; tg < NTG; ++tg)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                float2 v = make_float2(c[0][tg][2 * r], c[0][tg][2 * r + 1]);
+#pragma unroll
+                for (int i = 1; i < (kSide ? 4 : 1); ++i) v = add_pair(v, c[i][tg][2 * r], c[i][tg][2 * r + 1]);
+                sum[r][tg] = v.x + v.y;
+            }
     const float d0 = h2f_bits((uint16_t)(hd[0].x & 0xFFFFu)), e0 = h2f_bits((uint16_t)(hd[0].x >> 16));
     const uint32_t as[2] = {bytes_bf16(sm[0]), bytes_bf16(sm[1])}, am[2] = {bytes_bf16(sm[0] >> 16), bytes_bf16(sm[1] >> 16)};
     const float d1 = h2f_bits((uint16_t)(hd[1].x & 0xFFFFu)), e1 = h2f_bits((uint16_t)(hd[1].x >> 16));
@@ -507,10 +530,15 @@ __device__ __forceinline__ void q4k_block_nx(uint32_t r0, uint32_t offs, uint32_
         mma16816_bf16(m, am[0], am[1], am[0], am[1], b.x, b.y);
         mma16816_bf16(s, as[0], as[1], as[0], as[1], b.x, b.y);
         const float xs = ldsf(xaddr + tg * kXq4 + kFragBytes + kMinBytes + t * 4);
-        const float q0 = fmaf(8.f, s[0] + s[1], 16384.f * ((c[0][tg][0] + c[0][tg][1]) + half[0][tg]));
-        const float q1 = fmaf(8.f, s[2] + s[3], 16384.f * ((c[0][tg][2] + c[0][tg][3]) + half[1][tg]));
-        acc[0][tg] = fmaf(xs, d0 * q0 - e0 * (m[0] + m[1]), acc[0][tg]);
-        acc[1][tg] = fmaf(xs, d1 * q1 - e1 * (m[2] + m[3]), acc[1][tg]);
+        // 8 d (s) - e (m) is mostly a difference of nearly equal numbers (a min is about 8 steps of the scale): the sums over the
+        // leading parts, s[0] and m[0], carry at most 24 bits, so that theirs is formed first, without rounding the product
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const float d = r ? d1 : d0, e = r ? e1 : e0, p = __fmul_rn(e, m[2 * r]);
+            float v = fmaf(8.f * d, s[2 * r], -p) - fmaf(e, m[2 * r], -p);
+            v = fmaf(-e, m[2 * r + 1], fmaf(8.f * d, s[2 * r + 1], v));
+            acc[r][tg] = fmaf(xs, fmaf(16384.f * d, sum[r][tg], v), acc[r][tg]);
+        }
     }
 }
 

@@ -85,6 +85,37 @@ def test_multi_column_special_values(ctx, fmt):
     assert not torch.isfinite(y[5]).any() and torch.isnan(y[6]).all()
 
 
+def centred_q4k(rows, cols, seed):
+    """Q4_K as trained tensors have it: zero mean, every min 7.5 steps of its scale."""
+    gen, nb = torch.Generator(device="cuda").manual_seed(seed), rows * cols // 256
+    w = torch.randint(0, 256, (nb, 144), dtype=torch.uint8, device="cuda", generator=gen)
+    d = (torch.rand((nb, 1), device="cuda", generator=gen) * 0.4 + 0.8) / (220.0 * math.sqrt(cols))
+    w[:, 0:2], w[:, 2:4] = ((d * s).half().view(torch.uint8).reshape(nb, 2) for s in (1.0, 7.5))
+    sc = torch.randint(32, 64, (nb, 8), dtype=torch.uint8, device="cuda", generator=gen)
+    w[:, 4:8] = w[:, 8:12] = sc[:, :4] | ((sc[:, 4:] >> 4) << 6)
+    w[:, 12:16] = (sc[:, 4:] & 15) * 17
+    return w.reshape(rows, -1)
+
+
+@pytest.mark.parametrize("nx", [4, 8, 16])
+def test_q4_k_sums_are_not_truncated(ctx, nx):
+    """mma.sync truncates its running sum towards zero: half a unit, 2^-25 to 2^-24 of it, per instruction on average and
+    always towards zero. Chains of 4 from zero, whose sum reaches its size on the way only, lose some 6e-8 of every result
+    (measured 5.5e-8; chains of 8: 1.0e-7), beside errors of random sign that leave 1.2e-7 in all (chains of 8: 1.7e-7)."""
+    rows = cols = 4096
+    w = centred_q4k(rows, cols, nx)
+    f = torch.empty((rows, cols), device="cuda")
+    x = torch.randn((nx, cols), device="cuda", generator=torch.Generator(device="cuda").manual_seed(nx))
+    y = torch.zeros((nx, rows), device="cuda")
+    torch.cuda.synchronize()
+    ctx.dequant(capi.Q4_K, w, rows, cols, f)
+    ctx.matvec(capi.Q4_K, w, rows, cols, x, y, nx=nx, xstride=cols, ystride=rows)
+    ctx.sync()
+    want = x.double() @ f.double().T
+    assert abs(float((y.double() * want).sum() / want.pow(2).sum()) - 1) <= 8e-8
+    assert float((y.double() - want).norm() / want.norm()) <= 1.5e-7
+
+
 @pytest.mark.parametrize("fmt_gu,fmt_d,n_expert,top_k,n_tok,max_tokens", [
     (capi.Q4_K, capi.Q4_K, 8, 2, 16, 16), (capi.Q4_K, capi.Q6_K, 16, 1, 3, 16), (capi.Q6_K, capi.Q4_K, 4, 4, 16, 16),
     (capi.Q4_K, capi.Q4_K, 4, 3, 45, 64),    # more tokens per expert than a pass takes
@@ -117,6 +148,42 @@ def test_grouped_experts(ctx, fmt_gu, fmt_d, n_expert, top_k, n_tok, max_tokens)
             want[t] += g * (fd[e * E:(e + 1) * E] @ h)
     # silu and the products multiply the relative errors of three matmuls and of the gate
     assert close(y, want, 1e-4)
+
+
+@pytest.mark.parametrize("n_tok", [2, 16])
+@pytest.mark.parametrize("fmt", [capi.Q4_K, capi.Q6_K])
+def test_block_of_experts_precision(ctx, fmt, n_tok):
+    """A block called by itself: activations of 22 bits, f32 sums. Gate, up and down of weights of zero
+    mean are each some 1.2e-7 off (2-norm), a share of it the truncation that all three have with the same sign; the product
+    of gate and up has both errors; together 2.1e-7 to 3.7e-7."""
+    E, F, n, k = 2048, 2048, 4, 1
+    blk = MoeBlock(ctx, E, F, n, k, norm=1, scale=1.0, fmt_gate_up=fmt, fmt_down=fmt, max_tokens=16)
+    ws, fs = [], []
+    for i, (r, c) in enumerate(((n * F, E), (n * F, E), (n * E, F))):
+        if fmt == capi.Q4_K:
+            ws.append(centred_q4k(r, c, i))
+            fs.append(torch.empty((r, c), device="cuda"))
+            torch.cuda.synchronize()
+            ctx.dequant(fmt, ws[-1], r, c, fs[-1])
+            ctx.sync()
+            fs[-1] = fs[-1].double()
+        else:
+            w, f = weights(ctx, fmt, r, c, i)
+            ws.append(w)
+            fs.append(f)
+    gen = torch.Generator(device="cuda").manual_seed(n_tok)
+    router, x = torch.randn((n, E), device="cuda", generator=gen), torch.randn((n_tok, E), device="cuda", generator=gen)
+    y = torch.zeros_like(x)
+    blk.set_weights(router, *ws)
+    torch.cuda.synchronize()
+    blk.forward(x, n_tok, y)
+    ctx.sync()
+    assert ctx.status() == 0
+    want, xd = torch.zeros((n_tok, E), dtype=torch.float64, device="cuda"), x.double()
+    for t, e in enumerate((xd @ router.double().T).argmax(-1).tolist()):
+        g, u = (f[e * F:(e + 1) * F] @ xd[t] for f in fs[:2])
+        want[t] = fs[2][e * E:(e + 1) * E] @ (torch.nn.functional.silu(g) * u)
+    assert float((y.double() - want).norm() / want.norm()) <= 4.3e-7
 
 
 @pytest.mark.parametrize("n_draft", [2, 3, 7, 8, 9, 16])
