@@ -201,8 +201,11 @@ int fl_b200_moe_set_peers(fl_b200_moe *m, void *const *bufs, uint32_t n) {
     return FL_B200_OK;
 }
 
-static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y, const float *wnorm = nullptr, float eps = 0.f,
-                       const float *resid = nullptr);
+// Shapes that the grouped form does not take.
+static bool moe_per_slot(const fl_b200_moe *m) { return m->planes_gu == 0; }
+
+static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y, bool per_slot, const float *wnorm = nullptr,
+                       float eps = 0.f, const float *resid = nullptr);
 
 int fl_b200_moe_forward(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y) {
     if (!m || !x || !y) return set_err(FL_B200_ERR_ARG, "moe_forward: null pointer");
@@ -221,10 +224,10 @@ int fl_b200_moe_forward(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y
     if (rec.graph) { cudaGraphDestroy(rec.graph); rec.graph = nullptr; }
     if (!same) {   // first sight of this call: run it directly
         rec.x = x; rec.y = y; rec.n_tok = n_tok;
-        return moe_enqueue(m, x, n_tok, y);
+        return moe_enqueue(m, x, n_tok, y, moe_per_slot(m));
     }
     CKM(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    const int rc = moe_enqueue(m, x, n_tok, y);
+    const int rc = moe_enqueue(m, x, n_tok, y, moe_per_slot(m));
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(s, &g);
     if (rc) { if (g) cudaGraphDestroy(g); return rc; }
@@ -307,18 +310,15 @@ static int moe_enqueue_per_slot(fl_b200_moe *m, const float *x, uint32_t n_tok, 
 // the multi-column launches of the block as programmatic dependents of one another (FLB_MOE_PDL=0: plain launches)
 static const int kMoePdlNx = getenv("FLB_MOE_PDL") ? atoi(getenv("FLB_MOE_PDL")) : 1;
 
-// One token: the one-column kernel walks an expert faster than the multi-column one, which serves at least four columns (whole
-// Mixtral-8x7B-shape step: 3.62 against 3.69 ms).
-static bool moe_per_slot(const fl_b200_moe *m, uint32_t n_tok) { return m->planes_gu == 0 || n_tok == 1; }
-
-// wnorm / resid (one GPU): x is the raw hidden state, normed inside the router kernel and the gate | up conversion, and
-// y = resid + the block's output.
-static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y, const float *wnorm, float eps, const float *resid) {
+// per_slot: the per-slot form. wnorm / resid (one GPU): x is the raw hidden state, normed inside the router kernel and the
+// gate | up conversion, and y = resid + the block's output.
+static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y, bool per_slot, const float *wnorm, float eps,
+                       const float *resid) {
     fl_b200_ctx *ctx = m->ctx;
     cudaStream_t s = ctx->stream;
     const fl_b200_moe_cfg &c = m->c;
     const uint32_t E = c.n_embd, F = c.n_ff, K = c.top_k, NE = c.n_expert, T = c.max_tokens;
-    if (moe_per_slot(m, n_tok)) return moe_enqueue_per_slot(m, x, n_tok, y, wnorm, eps, resid);
+    if (per_slot) return moe_enqueue_per_slot(m, x, n_tok, y, wnorm, eps, resid);
     router_logits_kernel<<<dim3(NE, n_tok), 128, 0, s>>>(m->router, x, m->logits, E, NE, wnorm, eps);
     CKM(cudaGetLastError());
     CKM(launch_router_sel(m->logits, m->ids, m->gates, n_tok, NE, K, c.norm, c.scale, s, m->lids, m->mgates, m->base, m->n_local));
@@ -368,12 +368,16 @@ int flb::moe_enqueue_tokens(fl_b200_moe *m, const float *x, uint32_t n_tok, floa
     if (n_tok == 0 || n_tok > m->c.max_tokens) return set_err(FL_B200_ERR_ARG, "moe: %u tokens outside 1..%u", n_tok, m->c.max_tokens);
     const fl_b200_moe_cfg &c = m->c;
     if (m->world > 1 && (wnorm || resid)) return set_err(FL_B200_ERR_ARG, "moe: the fused norm / residual form is for one GPU");
+    // One token inside a decoder step: per slot. The one-column kernel walks an expert faster than the multi-column one, which
+    // serves at least four columns (whole Mixtral-8x7B-shape step: 3.62 against 3.69 ms); its activation has 21 bits, relative
+    // error 2.3e-6 against 3e-7 of the grouped form, which is why a block called by itself stays on that (fl_b200_moe_forward).
+    const bool per_slot = moe_per_slot(m) || n_tok == 1;
     if (n_launch) {   // as moe_enqueue / moe_enqueue_per_slot enqueue them
         const bool down_streams = matvec_is_streaming(c.fmt_down, c.n_ff) && row_bytes(c.fmt_down, c.n_ff) % 16 == 0;
         const uint32_t passes = (n_tok + kNxMaxTokens - 1) / kNxMaxTokens;
-        *n_launch = (!moe_per_slot(m, n_tok) ? 3 + 5 * passes - 1 + 1 : 2 + n_tok * (c.top_k * (down_streams ? 2u : 3u) + 1)) + (m->world > 1 ? n_tok : 0u);
+        *n_launch = (!per_slot ? 3 + 5 * passes - 1 + 1 : 2 + n_tok * (c.top_k * (down_streams ? 2u : 3u) + 1)) + (m->world > 1 ? n_tok : 0u);
     }
-    return moe_enqueue(m, x, n_tok, y, wnorm, eps, resid);
+    return moe_enqueue(m, x, n_tok, y, per_slot, wnorm, eps, resid);
 }
 fl_b200_ctx *flb::moe_ctx(const fl_b200_moe *m) { return m->ctx; }
 const fl_b200_moe_cfg *flb::moe_cfg(const fl_b200_moe *m) { return &m->c; }

@@ -150,12 +150,12 @@ def test_grouped_experts(ctx, fmt_gu, fmt_d, n_expert, top_k, n_tok, max_tokens)
     assert close(y, want, 1e-4)
 
 
-@pytest.mark.parametrize("n_tok", [2, 16])
+@pytest.mark.parametrize("n_tok", [1, 2, 16])
 @pytest.mark.parametrize("fmt", [capi.Q4_K, capi.Q6_K])
 def test_block_of_experts_precision(ctx, fmt, n_tok):
-    """A block called by itself: activations of 22 bits, f32 sums. Gate, up and down of weights of zero
+    """A block called by itself, one token like several: activations of 22 bits, f32 sums. Gate, up and down of weights of zero
     mean are each some 1.2e-7 off (2-norm), a share of it the truncation that all three have with the same sign; the product
-    of gate and up has both errors; together 2.1e-7 to 3.7e-7."""
+    of gate and up has both errors; together 2.1e-7 to 3.7e-7. (Activations of 21 bits per 256 columns: 2.3e-6.)"""
     E, F, n, k = 2048, 2048, 4, 1
     blk = MoeBlock(ctx, E, F, n, k, norm=1, scale=1.0, fmt_gate_up=fmt, fmt_down=fmt, max_tokens=16)
     ws, fs = [], []
