@@ -4,7 +4,17 @@
 #include "common.cuh"
 #include "kernels.h"
 
+#include <memory>
 #include <vector>
+
+// Device buffer that the mixture-of-experts blocks of a context share while they run (moe.cu): freed with the last of them.
+struct MoeScratch {
+    uint8_t *p = nullptr;
+    size_t bytes = 0;
+    MoeScratch() = default;
+    MoeScratch(const MoeScratch &) = delete;
+    ~MoeScratch() { cudaFree(p); }
+};
 
 struct fl_b200_ctx {
     int device = 0;
@@ -28,6 +38,7 @@ struct fl_b200_ctx {
     float *um_scratch = nullptr;
     uint32_t *um_tickets = nullptr;
     uint32_t *grid_bar = nullptr;        // barrier state of the chained matvec launches (two words, zero between launches)
+    std::weak_ptr<MoeScratch> moe_scratch;   // the newest (largest) one
     uint64_t wait_limit_ns = 0;          // limit of the exchange kernels' waits for other ranks (0 = one second)
     void *stage = nullptr;               // device staging for the *_host entry points
     size_t stage_cap = 0;

@@ -130,14 +130,16 @@ __global__ void wmerge_kernel(const float *__restrict__ parts, const float *__re
     y[i] = acc;
 }
 
-// y[t][i] = sum_q (gates[t][q] * parts[t][q][i]), the arithmetic of fl_op_wmerge (decode_params.h:274-295) without its
-// residual terms, for every token of a block in one launch. grid (ceil(n / 256), n_tok).
+// y[t][i] = (resid[t][i] +) sum_q (gates[t][q] * parts[t][q][i]), the arithmetic of fl_op_wmerge (decode_params.h:274-295)
+// with one residual term at most, for every token of a block in one launch. grid (ceil(n / 256), n_tok).
 __global__ void wmerge_tokens_kernel(const float *__restrict__ parts, const float *__restrict__ gates, float *y, uint32_t n_parts,
-                                     uint32_t n, uint32_t n_planes, size_t plane_stride, const float *resid) {
+                                     uint32_t n, uint32_t n_planes, size_t plane_stride, const float *resid,
+                                     const uint32_t *__restrict__ lids) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y;
     if (i >= n) return;
     float acc = 0.f;
     for (uint32_t q = 0; q < n_parts; ++q) {
+        if (lids && lids[(size_t)t * n_parts + q] == kExpertSkip) continue;   // another rank's: gate 0, and no part was made here
         const float *p = parts + ((size_t)t * n_parts + q) * n + i;
         float v = p[0];
 #pragma unroll 4
@@ -148,25 +150,43 @@ __global__ void wmerge_tokens_kernel(const float *__restrict__ parts, const floa
     y[(size_t)t * n + i] = acc;
 }
 
+// grid (ceil(n / 1024), P, groups): see launch_scatter_rows.
+__global__ void __launch_bounds__(256) scatter_rows_kernel(const float *__restrict__ x, uint32_t n_planes, size_t plane_stride,
+                                                           const uint32_t *__restrict__ table, const uint32_t *__restrict__ idx,
+                                                           uint32_t list_stride, uint32_t col_off, float *__restrict__ y, uint32_t n) {
+    const uint32_t i = 4 * (blockIdx.x * 256 + threadIdx.x), p = blockIdx.y;
+    if (i >= n || blockIdx.z >= table[0]) return;
+    const uint4 e = reinterpret_cast<const uint4 *>(table)[1 + blockIdx.z];
+    if (p >= e.y) return;
+    const float *src = x + (size_t)(e.w + p) * n + i;
+    float4 v = *reinterpret_cast<const float4 *>(src);
+#pragma unroll 4
+    for (uint32_t s = 1; s < n_planes; ++s) {
+        const float4 w = *reinterpret_cast<const float4 *>(src + s * plane_stride);
+        v.x = __fadd_rn(v.x, w.x); v.y = __fadd_rn(v.y, w.y); v.z = __fadd_rn(v.z, w.z); v.w = __fadd_rn(v.w, w.w);
+    }
+    *reinterpret_cast<float4 *>(y + (size_t)idx[(size_t)e.x * list_stride + col_off + p] * n + i) = v;
+}
+
 // The table of a grouped multi-column launch (matvec_tc_nx.cu), by one warp: active experts in ascending order, their
-// columns from col_off on (at most P) and the groups of four columns in front of them.
+// columns from col_off on (at most P), the groups of four columns in front of them and the columns in front of them.
 __device__ __forceinline__ void nx_table_warp(const uint32_t *cnt, uint32_t n_local, uint32_t col_off, uint32_t P, uint32_t *table) {
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t n_act = 0, tgs = 0, most = 0;
+    uint32_t n_act = 0, before = 0, most = 0;   // before: groups of four, columns << 16
     for (uint32_t b = 0; b < n_local; b += 32) {
         const uint32_t e = b + lane, c = e < n_local ? cnt[e] : 0u;
-        const uint32_t n = c > col_off ? min(c - col_off, P) : 0u, tg = (n + 3) / 4;
-        uint32_t incl = tg;
+        const uint32_t n = c > col_off ? min(c - col_off, P) : 0u, tg = (n + 3) / 4, own = tg | n << 16;
+        uint32_t incl = own;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= (uint32_t)o) incl += v;
         }
-        const uint32_t mask = __ballot_sync(0xffffffffu, n != 0);
-        if (n) reinterpret_cast<uint4 *>(table)[1 + n_act + __popc(mask & ((1u << lane) - 1u))] = make_uint4(e, n, tgs + incl - tg, 0u);
+        const uint32_t mask = __ballot_sync(0xffffffffu, n != 0), at = before + incl - own;
+        if (n) reinterpret_cast<uint4 *>(table)[1 + n_act + __popc(mask & ((1u << lane) - 1u))] = make_uint4(e, n, at & 0xFFFFu, at >> 16);
         n_act += __popc(mask);
         most = max(most, __reduce_max_sync(0xffffffffu, tg));
-        tgs += __shfl_sync(0xffffffffu, incl, 31);
+        before += __shfl_sync(0xffffffffu, incl, 31);
     }
     if (lane == 0) { table[0] = n_act; table[1] = most; }
 }
@@ -383,9 +403,17 @@ cudaError_t launch_wmerge(const float *parts, const float *gates, const float *a
 }
 
 cudaError_t launch_wmerge_tokens(const float *parts, const float *gates, float *y, uint32_t n_parts, uint32_t n, uint32_t n_tok,
-                                 cudaStream_t stream, uint32_t n_planes, size_t plane_stride, const float *resid) {
+                                 cudaStream_t stream, uint32_t n_planes, size_t plane_stride, const float *resid, const uint32_t *lids) {
     if (n == 0 || n_parts == 0 || n_tok == 0) return cudaErrorInvalidValue;
-    wmerge_tokens_kernel<<<dim3((n + 255) / 256, n_tok), 256, 0, stream>>>(parts, gates, y, n_parts, n, n_planes, plane_stride, resid);
+    wmerge_tokens_kernel<<<dim3((n + 255) / 256, n_tok), 256, 0, stream>>>(parts, gates, y, n_parts, n, n_planes, plane_stride, resid, lids);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_scatter_rows(const float *x, uint32_t n_planes, size_t plane_stride, const uint32_t *table, const uint32_t *idx,
+                                uint32_t list_stride, uint32_t col_off, uint32_t P, uint32_t n_groups, float *y, uint32_t n,
+                                cudaStream_t stream) {
+    if (n == 0 || n % 4 != 0 || plane_stride % 4 != 0 || P == 0 || n_groups == 0) return cudaErrorInvalidValue;
+    scatter_rows_kernel<<<dim3((n + 1023) / 1024, P, n_groups), 256, 0, stream>>>(x, n_planes, plane_stride, table, idx, list_stride, col_off, y, n);
     return cudaGetLastError();
 }
 

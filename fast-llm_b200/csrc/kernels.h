@@ -115,7 +115,8 @@ struct NxIn {
     const float *att;        // optional, in place of x: the columns are the attention contexts of heads of 128 whose splits'
     uint32_t n_splits;       // records (launch_attn_decode with records_only) are added up here
     // Grouped columns (mixture of experts): `table` (launch_nx_table) lists the active experts; column p of an expert is row
-    // col_idx[expert * list_stride + col_off + p] of x and goes to output row block out_idx[the same].
+    // col_idx[expert * list_stride + col_off + p] of x and goes to output row block out_idx[the same]. Without col_idx / out_idx
+    // the rows are numbered through, expert by expert in the table's order.
     const uint32_t *table, *col_idx, *out_idx;
     uint32_t list_stride, col_off, n_groups, n_experts;   // n_groups: upper bound of active experts
     int table_ready;         // 1: the table was complete before the kernel in front of the matmul started
@@ -295,7 +296,13 @@ cudaError_t launch_wmerge(const float *parts, const float *gates, const float *a
 // fl_op_wmerge for n_tok tokens in one launch: y[t] = (resid[t] +) sum_q gates[t][q] * parts[t][q] (products and sums
 // rounded in the reference's order); a part is the sum of n_planes planes, plane_stride floats apart.
 cudaError_t launch_wmerge_tokens(const float *parts, const float *gates, float *y, uint32_t n_parts, uint32_t n, uint32_t n_tok,
-                                 cudaStream_t stream, uint32_t n_planes = 1, size_t plane_stride = 0, const float *resid = nullptr);
+                                 cudaStream_t stream, uint32_t n_planes = 1, size_t plane_stride = 0, const float *resid = nullptr,
+                                 const uint32_t *lids = nullptr);   // lids: slots whose entry is kExpertSkip are left out
+// Rows numbered through by a grouped launch's table (row r of x: n_planes planes of n floats, plane_stride apart) to the rows of
+// y that their columns stand for: y[idx[expert * list_stride + col_off + p]] = the sum of the planes. n a multiple of 4.
+cudaError_t launch_scatter_rows(const float *x, uint32_t n_planes, size_t plane_stride, const uint32_t *table, const uint32_t *idx,
+                                uint32_t list_stride, uint32_t col_off, uint32_t P, uint32_t n_groups, float *y, uint32_t n,
+                                cudaStream_t stream);
 cudaError_t launch_silu_mul(const float *gate, const float *up, float *h, uint32_t n, cudaStream_t stream);
 // RoPE (adjacent pairs) on q in place and on k, then store k and v as f16 at
 // row *pos of a cache laid out [n_kv_head][kv_stride][head_dim].

@@ -210,7 +210,7 @@ struct ConvArgs {
     uint32_t n_splits;             // (attn.cu: [column][head][split][132] = context, maximum, sum)
 };
 // Device-side table of a grouped launch: word 0 = number of active groups, word 1 = the most token groups of one; then four
-// words per active group: {group, number of columns, token groups in front of it, 0}.
+// words per active group: {group, number of columns, token groups in front of it, columns in front of it}.
 
 // Four consecutive columns at p, the planes added in order; all of them are requested before the first is used.
 __device__ __forceinline__ float4 sum_planes(const float *p, uint32_t n, size_t stride) {
@@ -268,11 +268,11 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     float4 wn = make_float4(1.f, 1.f, 1.f, 1.f);
     if (a.wnorm) wn = __ldg(reinterpret_cast<const float4 *>(a.wnorm + blk * 256 + 4 * i));   // a constant
     griddep_wait();
-    uint32_t n_valid = a.P, tg = blockIdx.y >> 2, ntg = (a.P + 3) / 4, tg0 = 0, grp = 0;
+    uint32_t n_valid = a.P, tg = blockIdx.y >> 2, ntg = (a.P + 3) / 4, tg0 = 0, grp = 0, row0 = 0;
     if (a.table) {
         if (blockIdx.z >= a.table[0]) return;
         const uint4 e = reinterpret_cast<const uint4 *>(a.table)[1 + blockIdx.z];
-        grp = e.x; n_valid = e.y; tg0 = e.z;
+        grp = e.x; n_valid = e.y; tg0 = e.z; row0 = e.w;
         ntg = (n_valid + 3) / 4;
         if (tg >= ntg) return;
     }
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     float ss = 0.f;
     if (p < n_valid) {
-        const size_t row = a.table ? a.col_idx[(size_t)grp * a.list_stride + a.col_off + p] : p;
+        const size_t row = a.col_idx ? a.col_idx[(size_t)grp * a.list_stride + a.col_off + p] : row0 + p;
         const size_t at = row * a.xstride + blk * 256 + 4 * i, rat = (size_t)p * a.rstride + blk * 256 + 4 * i;
         float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
         if (a.resid) r = *reinterpret_cast<const float4 *>(a.resid + rat);
@@ -393,7 +393,7 @@ struct NxArgs {
     float eps;
     uint32_t slot_bytes, x_off, x_blk_tg;   // x_blk_tg: bytes of a part's activation per token group
     uint32_t red_group;            // floats between the groups' reduction buffers (for the widest piece of the launch)
-    // grouped launches: active groups from the table, output rows from the list
+    // grouped launches: active groups from the table, output rows from the list (or numbered through)
     const uint32_t *table, *out_idx;
     uint32_t list_stride, col_off;
     int table_ready;               // the table was complete before the previous kernel started
@@ -405,11 +405,12 @@ __host__ __device__ constexpr uint32_t nx_ring_off(uint32_t x_off, uint32_t x_bl
 }
 
 // The pieces of this CTA, listed in shared memory by one thread at the start: {first unit, last unit, job | columns << 8 |
-// group << 16, token groups in front << 2 | same activation as the piece before << 1 | parity of the units before}.
-struct NxPiece { uint32_t u0, u1, job, n_valid, grp, tg0, same, par; };
+// group << 16, columns in front << 16 | token groups in front << 2 | same activation as the piece before << 1 | parity of the
+// units before}.
+struct NxPiece { uint32_t u0, u1, job, n_valid, grp, row0, tg0, same, par; };
 __device__ __forceinline__ NxPiece nx_piece(uint32_t smem, uint32_t i) {
     const uint4 v = lds128(smem + kPieces + 16 + 16 * i);
-    return NxPiece{v.x, v.y, v.z & 0xFFu, (v.z >> 8) & 0xFFu, v.z >> 16, v.w >> 2, (v.w >> 1) & 1u, v.w & 1u};
+    return NxPiece{v.x, v.y, v.z & 0xFFu, (v.z >> 8) & 0xFFu, v.z >> 16, v.w >> 16, (v.w >> 2) & 0x3FFFu, (v.w >> 1) & 1u, v.w & 1u};
 }
 __device__ __noinline__ void nx_list_pieces(const NxArgs &a, uint8_t *smem_raw) {
     uint32_t *count = reinterpret_cast<uint32_t *>(smem_raw + kPieces);
@@ -435,7 +436,7 @@ __device__ __noinline__ void nx_list_pieces(const NxArgs &a, uint8_t *smem_raw) 
             if (u0 >= u1) continue;
             const uint32_t same = n > 0 && last_g == g && last_part == jb.part && last_x == a.t[jb.tensor].xoff ? 1u : 0u;
             last_g = g; last_part = jb.part; last_x = a.t[jb.tensor].xoff;
-            out[n++] = make_uint4(u0, u1, j | (e.y << 8) | (e.x << 16), (e.z << 2) | (same << 1) | (kk & 1u));
+            out[n++] = make_uint4(u0, u1, j | (e.y << 8) | (e.x << 16), (e.w << 16) | (e.z << 2) | (same << 1) | (kk & 1u));
             kk += u1 - u0;
         }
     }
@@ -837,7 +838,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_nx_kernel(const __grid_con
                     const float s = __shfl_sync(0xffffffffu, inv, tok & 31u);
                     if (tok >= n_valid || row >= t.rows) continue;
                     if (a.rms) { v[i].x *= s; v[i].y *= s; v[i].z *= s; v[i].w *= s; }
-                    const size_t orow = a.out_idx ? a.out_idx[(size_t)grp * a.list_stride + a.col_off + tok] : tok;
+                    const size_t orow = a.out_idx ? a.out_idx[(size_t)grp * a.list_stride + a.col_off + tok] : pc.row0 + tok;
                     float *dst = t.y + jb.part * t.part_stride + orow * t.ystride + row;
                     if (vec) {
                         if (a.accumulate) {

@@ -31,13 +31,17 @@ struct fl_b200_moe {
     uint32_t rank = 0, world = 1, n_local = 0, base = 0;
     const float *router = nullptr;
     const uint8_t *wg = nullptr, *wu = nullptr, *wd = nullptr;
-    float *logits = nullptr, *gates = nullptr, *mgates = nullptr, *g = nullptr, *u = nullptr, *part = nullptr, *partial = nullptr;
+    float *logits = nullptr, *gates = nullptr, *mgates = nullptr, *part = nullptr, *partial = nullptr;
     uint32_t *ids = nullptr, *lids = nullptr;
     uint32_t *cnt = nullptr, *tok_list = nullptr, *pair_list = nullptr;   // the pairs grouped by local expert (launch_group_by_expert)
     uint32_t *table = nullptr;                                            // active experts of a grouped launch
-    uint8_t *xq = nullptr;                                                // converted activations of all active experts
-    uint32_t tgs = 0, planes_gu = 0, planes_d = 0;                        // token groups in xq; planes of partial results in g, u / part
-    uint8_t *arena = nullptr;                                             // the one allocation that holds the buffers above
+    // Used by one call at a time and written before it is read, hence shared by all blocks of a context (their calls are in order
+    // on its stream): gate / up outputs and down outputs, planes of `rows` rows each, and the converted activations.
+    std::shared_ptr<MoeScratch> scratch;
+    float *g = nullptr, *u = nullptr, *d = nullptr;
+    uint8_t *xq = nullptr;
+    uint32_t rows = 0, tgs = 0, planes_gu = 0, planes_d = 0;              // tgs: groups of four columns in xq
+    uint8_t *arena = nullptr;                                             // the one allocation that holds the block's own buffers
     uint8_t *comm = nullptr;
     uint8_t *peers[kCommMaxRanks] = {};
     bool peers_set = false;
@@ -137,23 +141,40 @@ int fl_b200_moe_create(fl_b200_ctx *ctx, const fl_b200_moe_cfg *cfg, uint32_t ra
     const size_t n_gu = std::max(1u, m->planes_gu), n_d = std::max(1u, m->planes_d);
     // every active expert has at most 16 columns in a pass, all of them together at most one per pair
     m->tgs = (uint32_t)std::min<size_t>((size_t)m->n_local * (kNxMaxTokens / 4), T * K / 4 + std::min<size_t>(m->n_local, T * K));
-    // One allocation, zero-filled: a slot that is skipped leaves its buffer as it was, and what is there is then multiplied by gate 0.
-    const struct { void **p; size_t bytes; } bufs[] = {
-        {(void **)&m->logits, T * c.n_expert * 4}, {(void **)&m->gates, T * K * 4}, {(void **)&m->mgates, T * K * 4},
-        {(void **)&m->ids, T * K * 4}, {(void **)&m->lids, T * K * 4},
-        {(void **)&m->g, n_gu * T * K * F * 4}, {(void **)&m->u, n_gu * T * K * F * 4},   // gate / up outputs, one row per (token, slot) pair
-        {(void **)&m->xq, matmul_tc_nx_scratch_bytes((uint32_t)std::max(E, F), m->tgs, 1)}, {(void **)&m->table, (1 + (size_t)m->n_local) * 16},
-        {(void **)&m->cnt, (size_t)m->n_local * 4}, {(void **)&m->tok_list, (size_t)m->n_local * T * 4},
-        {(void **)&m->pair_list, (size_t)m->n_local * T * 4}, {(void **)&m->part, n_d * T * K * E * 4},
-        {(void **)&m->partial, world > 1 ? T * E * 4 : 0}};
-    size_t total = 0;
-    for (const auto &x : bufs) total += (x.bytes + 255) & ~(size_t)255;
-    if (int rc = alloc((void **)&m->arena, total)) return fail(rc);
-    uint8_t *at = m->arena;
-    for (const auto &x : bufs) {
-        if (x.bytes) *x.p = at;
-        at += (x.bytes + 255) & ~(size_t)255;
+    // Rows of the planes (the per-slot form: one slot at a time). Up to 16 tokens are one pass, a row per (token, slot) pair. More of them go in passes of at most 16
+    // columns per expert, whose rows are numbered through and added up to the pairs' results after each: the planes don't grow
+    // with max_tokens.
+    const size_t one_pass = std::min<size_t>(T, kNxMaxTokens) * K;
+    m->rows = m->planes_gu == 0 ? 1 : (uint32_t)std::max(one_pass, std::min<size_t>(T * K, (size_t)m->n_local * kNxMaxTokens));
+    const size_t R = m->rows, pairs = T > kNxMaxTokens || m->planes_gu == 0 ? T * K : K;   // (K: the per-slot form of one token)
+    auto lay_out = [](const auto &bufs, uint8_t *at) {   // addresses from `at` on (nullptr: none); returns the bytes
+        size_t total = 0;
+        for (const auto &x : bufs) {
+            if (at && x.bytes) *x.p = at + total;
+            total += (x.bytes + 255) & ~(size_t)255;
+        }
+        return total;
+    };
+    struct Buf { void **p; size_t bytes; };
+    const Buf shared[] = {{(void **)&m->g, n_gu * R * F * 4}, {(void **)&m->u, n_gu * R * F * 4}, {(void **)&m->d, m->planes_gu ? n_d * R * E * 4 : 0},
+                          {(void **)&m->xq, m->planes_gu ? matmul_tc_nx_scratch_bytes((uint32_t)std::max(E, F), m->tgs, 1) : 0}};
+    const size_t need = lay_out(shared, nullptr);
+    m->scratch = ctx->moe_scratch.lock();
+    if (!m->scratch || m->scratch->bytes < need) {
+        m->scratch = std::make_shared<MoeScratch>();
+        if (cudaError_t e = cudaMalloc((void **)&m->scratch->p, need)) return fail(cuda_err(e, "cudaMalloc (moe)"));
+        m->scratch->bytes = need;
+        ctx->moe_scratch = m->scratch;
     }
+    lay_out(shared, m->scratch->p);
+    // One allocation, zero-filled: the per-slot form leaves the part of a slot that is skipped as it was and multiplies it by gate 0.
+    const Buf own[] = {
+        {(void **)&m->logits, T * c.n_expert * 4}, {(void **)&m->gates, T * K * 4}, {(void **)&m->mgates, T * K * 4},
+        {(void **)&m->ids, T * K * 4}, {(void **)&m->lids, T * K * 4}, {(void **)&m->table, (1 + (size_t)m->n_local) * 16},
+        {(void **)&m->cnt, (size_t)m->n_local * 4}, {(void **)&m->tok_list, (size_t)m->n_local * T * 4},
+        {(void **)&m->pair_list, (size_t)m->n_local * T * 4}, {(void **)&m->part, pairs * E * 4}, {(void **)&m->partial, world > 1 ? T * E * 4 : 0}};
+    if (int rc = alloc((void **)&m->arena, lay_out(own, nullptr))) return fail(rc);
+    lay_out(own, m->arena);
     if (world > 1) {   // mapped by the peers: allocations of their own
         if (int rc = alloc((void **)&m->comm, comm_buffer_bytes())) return fail(rc);
         if (int rc = alloc((void **)&m->comm_state, 64)) return fail(rc);
@@ -325,31 +346,33 @@ static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y,
     CKM(launch_group_by_expert(m->lids, n_tok * K, K, m->n_local, T, m->cnt, m->tok_list, m->pair_list, s, m->table));
     // Every local expert once for up to 16 of the tokens that chose it. The table and the lists live on the device, so the
     // launch sequence is the same for every routing (and can be replayed as a graph).
-    uint32_t planes_d = 1;
     const uint32_t P = std::min(n_tok, kNxMaxTokens);   // every pass is cut into the same parts, the last one too
+    const bool one_pass = n_tok <= kNxMaxTokens;
+    const size_t R = m->rows;
+    const NxTensor gu[2] = {{c.fmt_gate_up, m->wg, F, 0, m->g, F, R * F}, {c.fmt_gate_up, m->wu, F, 0, m->u, F, R * F}};
+    const NxTensor dn{c.fmt_down, m->wd, E, 0, m->d, E, R * E};   // down: the column of pair p is silu(g[p]) * u[p]
+    const uint32_t parts_gu = matmul_tc_nx_parts(gu, 2, E, P, true), parts_d = matmul_tc_nx_parts(&dn, 1, F, P, true);
     for (uint32_t off = 0; off < n_tok; off += kNxMaxTokens) {
         if (off) CKM(launch_nx_table(m->cnt, m->n_local, off, P, m->table, s));
-        const NxTensor gu[2] = {{c.fmt_gate_up, m->wg, F, 0, m->g, F, (size_t)T * K * F}, {c.fmt_gate_up, m->wu, F, 0, m->u, F, (size_t)T * K * F}};
         NxIn in{};
         in.x = x; in.xstride = E; in.wnorm = wnorm; in.eps = eps;
-        in.table = m->table; in.col_idx = m->tok_list; in.out_idx = m->pair_list; in.list_stride = T; in.col_off = off;
+        in.table = m->table; in.col_idx = m->tok_list; in.out_idx = one_pass ? m->pair_list : nullptr; in.list_stride = T; in.col_off = off;
         in.n_groups = std::min(m->n_local, n_tok * K); in.n_experts = m->n_local;
         // the first conversion is an ordinary dependent of the kernel that wrote the table; every later launch starts after
         // it did, so that the table is in place for all of them
         in.table_ready = kMoePdlNx;
         CKM(launch_nx_convert(in, gu, 1, E, P, m->xq, m->tgs, s, false));
         CKM(launch_nx_matmul(in, gu, 2, E, P, 0, m->xq, m->tgs, ctx->status, ctx->sms, s, kMoePdlNx != 0, true));
-        const NxTensor dn{c.fmt_down, m->wd, E, 0, m->part, E, (size_t)T * K * E};   // down: the column of pair p is silu(g[p]) * u[p]
         in.x = m->g; in.x2 = m->u; in.xstride = F; in.wnorm = nullptr;
-        in.n_parts = matmul_tc_nx_parts(gu, 2, E, P, true); in.part_stride = (size_t)T * K * F;
-        in.col_idx = m->pair_list;
+        in.n_parts = parts_gu; in.part_stride = R * F;
+        in.col_idx = in.out_idx;
         CKM(launch_nx_convert(in, &dn, 1, F, P, m->xq, m->tgs, s, kMoePdlNx != 0));
         CKM(launch_nx_matmul(in, &dn, 1, F, P, 0, m->xq, m->tgs, ctx->status, ctx->sms, s, kMoePdlNx != 0, true));
-        planes_d = matmul_tc_nx_parts(&dn, 1, F, P, true);
+        if (!one_pass) CKM(launch_scatter_rows(m->d, parts_d, R * E, m->table, m->pair_list, T, off, P, in.n_groups, m->part, E, s));
     }
-    // WMERGE of every token: y[t] = sum_k gate[t][k] * part[t][k] (slots of experts held elsewhere carry gate 0)
-    CKM(launch_wmerge_tokens(m->part, m->mgates, m->world > 1 ? m->partial : y, K, E, n_tok, s, planes_d, (size_t)T * K * E,
-                             m->world > 1 ? nullptr : resid));
+    // WMERGE of every token: y[t] = sum_k gate[t][k] * part[t][k], slots of experts held elsewhere left out
+    CKM(launch_wmerge_tokens(one_pass ? m->d : m->part, m->mgates, m->world > 1 ? m->partial : y, K, E, n_tok, s, one_pass ? parts_d : 1, R * E,
+                             m->world > 1 ? nullptr : resid, m->world > 1 ? m->lids : nullptr));
     if (m->world > 1) {
         for (uint32_t t = 0; t < n_tok; ++t) {   // the combine: sum of the ranks' partial outputs, rank order
             AllReduceArgs r{};
@@ -375,7 +398,7 @@ int flb::moe_enqueue_tokens(fl_b200_moe *m, const float *x, uint32_t n_tok, floa
     if (n_launch) {   // as moe_enqueue / moe_enqueue_per_slot enqueue them
         const bool down_streams = matvec_is_streaming(c.fmt_down, c.n_ff) && row_bytes(c.fmt_down, c.n_ff) % 16 == 0;
         const uint32_t passes = (n_tok + kNxMaxTokens - 1) / kNxMaxTokens;
-        *n_launch = (!per_slot ? 3 + 5 * passes - 1 + 1 : 2 + n_tok * (c.top_k * (down_streams ? 2u : 3u) + 1)) + (m->world > 1 ? n_tok : 0u);
+        *n_launch = (!per_slot ? 3 + 4 * passes + (passes > 1 ? 2 * passes - 1 : 0) + 1 : 2 + n_tok * (c.top_k * (down_streams ? 2u : 3u) + 1)) + (m->world > 1 ? n_tok : 0u);
     }
     return moe_enqueue(m, x, n_tok, y, per_slot, wnorm, eps, resid);
 }

@@ -186,6 +186,64 @@ def test_block_of_experts_precision(ctx, fmt, n_tok):
     assert float((y.double() - want).norm() / want.norm()) <= 4.3e-7
 
 
+def test_block_of_experts_memory(ctx):
+    """What a block holds besides a row of results per (token, slot) pair does not grow with max_tokens and is shared by the
+    blocks of a context: creating one for many tokens takes less than two rows of n_ff and one of n_embd floats per pair, and
+    the sixteenth block of 16 tokens next to nothing."""
+    E, F, k = 4096, 14336, 2
+
+    def free():
+        ctx.sync()
+        return torch.cuda.mem_get_info()[0]
+    before = free()
+    big = MoeBlock(ctx, E, F, 8, k, max_tokens=2048)
+    assert before - free() <= 2048 * k * 4 * (2 * F + E)
+    big.close()
+    assert before - free() <= 1 << 21   # given back
+    blocks = [MoeBlock(ctx, E, F, 8, k, max_tokens=16) for _ in range(16)]
+    assert before - free() <= 16 * 16 * k * 4 * (2 * F + E)
+    for b in blocks:
+        b.close()
+    assert before - free() <= 1 << 21
+
+
+def test_blocks_of_experts_share_scratch(ctx):
+    """Blocks of different sizes and formats called in turn, directly and as recorded launches, and after the largest has gone:
+    every result is what the block gives alone."""
+    shapes = [(2048, 2048, 4, 2, capi.Q4_K, 16, 5), (2048, 4096, 8, 2, capi.Q6_K, 64, 40), (4096, 2048, 4, 1, capi.Q4_K, 16, 16)]
+    blocks, args, alone = [], [], []
+    for i, (E, F, n, k, fmt, max_tokens, n_tok) in enumerate(shapes):
+        ws = [weights(ctx, fmt, r, c, 10 * i + j)[0] for j, (r, c) in enumerate(((n * F, E), (n * F, E), (n * E, F)))]
+        gen = torch.Generator(device="cuda").manual_seed(i)
+        router, x = torch.randn((n, E), device="cuda", generator=gen), torch.randn((n_tok, E), device="cuda", generator=gen)
+        first = MoeBlock(ctx, E, F, n, k, fmt_gate_up=fmt, fmt_down=fmt, max_tokens=max_tokens)
+        y = torch.zeros_like(x)
+        first.set_weights(router, *ws)
+        torch.cuda.synchronize()
+        first.forward(x, n_tok, y)
+        ctx.sync()
+        first.close()
+        alone.append(y)
+        args.append((router, ws, x, n_tok))
+    for (E, F, n, k, fmt, max_tokens, n_tok), (router, ws, x, _) in zip(shapes, args):
+        blocks.append(MoeBlock(ctx, E, F, n, k, fmt_gate_up=fmt, fmt_down=fmt, max_tokens=max_tokens))
+        blocks[-1].set_weights(router, *ws)
+    outs = [torch.zeros_like(y) for y in alone]
+    for turn in range(4):
+        if turn == 3:
+            blocks.pop(1).close()
+            del outs[1], args[1], alone[1]
+        for y in outs:
+            y.zero_()
+        torch.cuda.synchronize()
+        for b, (_, _, x, n_tok), y in zip(blocks, args, outs):
+            b.forward(x, n_tok, y)
+        ctx.sync()
+        assert ctx.status() == 0
+        for y, want in zip(outs, alone):
+            assert torch.equal(y, want)
+
+
 @pytest.mark.parametrize("n_draft", [2, 3, 7, 8, 9, 16])
 @pytest.mark.parametrize("base", [1, 40, 63, 64, 65, 500, 4100])
 def test_shared_cache_positions(ctx, base, n_draft):
