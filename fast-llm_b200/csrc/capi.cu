@@ -246,7 +246,8 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
     uint32_t first_single = 0;   // columns from here on go through the one-column kernel
     if (nx >= 2 && (fmt == FL_B200_Q4_K || fmt == FL_B200_Q6_K || fmt == FL_B200_Q8_0) && !expert_id) {
         // Q4_K under FLB_UMMA=1: tcgen05 with the accumulator in tensor memory, 8 columns per pass
-        for (uint32_t p0 = 0; fmt == FL_B200_Q4_K && cols <= 18432 && p0 < nx; p0 += 8) {
+        const bool umma = fmt == FL_B200_Q4_K && matmul_umma_on();
+        for (uint32_t p0 = 0; umma && cols <= 18432 && p0 < nx; p0 += 8) {
             const uint32_t nt = nx - p0 < 8 ? nx - p0 : 8;
             if (nt < 2 && p0 > 0) break;   // a last single column goes to the one-column kernel
             NxCall nc{};
@@ -255,9 +256,8 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
             if (x2) nc.x2 = x2 + (size_t)p0 * xstride;
             nc.skip_convert = (same_columns && nx <= 8) ? 1 : 0;   // with more than 8 columns the scratch holds the last chunk only
             nc.y = y + (size_t)p0 * ystride; nc.ystride = ystride; nc.accumulate = accumulate;
-            nc.pdl = pdl;
             const cudaError_t e = launch_matmul_umma(nc, c->xu, c->um_scratch, c->um_tickets, c->status, c->sms, c->stream);
-            if (e == cudaErrorNotSupported) break;   // off, or not its shape (the same answer for every chunk)
+            if (e == cudaErrorNotSupported) break;   // not its shape (the same answer for every chunk)
             if (e != cudaSuccess) return cuda_err(e, "multi-column matmul launch");
             first_single = p0 + nt;
         }
@@ -274,7 +274,7 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
             cudaError_t e = cudaSuccess;
             // the scratch holds these columns already: not with more of them than a chunk (it has the last one only), nor where
             // the call before may have gone to the tcgen05 kernel, which has a scratch of its own
-            const bool reuse = same_columns && nx <= kNxMaxTokens && !(fmt == FL_B200_Q4_K && getenv("FLB_UMMA"));
+            const bool reuse = same_columns && nx <= kNxMaxTokens && !umma;
             if (!reuse) {
                 e = launch_nx_convert(in, &t, 1, cols, nt, c->xq, kNxTgs, c->stream, pdl != 0);
                 if (e == cudaErrorNotSupported) break;

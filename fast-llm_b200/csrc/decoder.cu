@@ -110,9 +110,9 @@ struct fl_b200_decoder {
         float *qkv = nullptr, *planes = nullptr, *gp = nullptr, *up = nullptr, *head = nullptr, *am = nullptr;
         uint32_t *am_tickets = nullptr;
         float2 *rope = nullptr;
-        int32_t *io = nullptr;              // [0..8) tokens, [8..16) positions, [16..24) greedy next tokens
+        int32_t *io = nullptr;              // FL_B200_MAX_BATCH tokens, as many positions, as many greedy next tokens
         uint32_t *tickets = nullptr;
-        int32_t *h_io = nullptr;            // pinned image of io, then the 8 margins
+        int32_t *h_io = nullptr;            // pinned image of io, then FL_B200_MAX_BATCH margins
         cudaGraph_t graph[FL_B200_MAX_BATCH + 1] = {};
         cudaGraphExec_t exec[FL_B200_MAX_BATCH + 1] = {};
         uint32_t last_m = 0;
@@ -742,8 +742,7 @@ static int batch_alloc(fl_b200_decoder *d) {
             part = std::max(part, attn_part_floats(d->Hq, m, attn_pick_splits(d->Hkv, m, c.max_kv, d->ctx->sms, shared)));
     uint32_t pl[5];
     // FLB_UMMA=1 sends the pass tensor by tensor, where Q4_K goes to the tcgen05 kernel
-    const char *umma = getenv("FLB_UMMA");
-    w.nx = !(umma && umma[0] == '1') && nx_eligible(d, pl);
+    w.nx = !matmul_umma_on() && nx_eligible(d, pl);
     // one allocation for all buffers: a dozen of them were most of the time of a decoder's first pass
     size_t total = 0;
     auto layout = [&](auto &&take) {
@@ -1054,7 +1053,8 @@ int fl_b200_decoder_step_batch(fl_b200_decoder *d, const int32_t *toks, uint32_t
 }
 
 // ---- independent sequences in lock step: one pass feeds one token to each of n sequences (each with its own cache and
-// position); every tensor is walked once per 8 sequences, the attention runs per sequence over its own keys. ----
+// position); every tensor is walked once where the multi-column kernel takes it, the attention runs per sequence over its own
+// keys. ----
 int fl_b200_decoder_seqs_init(fl_b200_decoder *d, uint32_t n_seq) {
     if (!d) return set_err(FL_B200_ERR_ARG, "decoder_seqs_init: null");
     if (n_seq < 2 || n_seq > FL_B200_MAX_BATCH) return set_err(FL_B200_ERR_ARG, "decoder_seqs_init: %u sequences outside 2..%d", n_seq, FL_B200_MAX_BATCH);

@@ -146,17 +146,13 @@ struct NxCall {
     float *y;                // output row blocks, ystride floats apart
     uint32_t ystride;
     int accumulate;
-    int skip_convert;        // 1: xq already holds exactly these columns in this format's layout (the call before used them)
-    // Device-side column list (mixture of experts): column p is row col_idx[col_off + p] of x and goes to output row
-    // block out_idx[col_off + p]; only columns col_off + p < *cnt exist. All nullptr: column p = row p -> row block p.
-    const uint32_t *cnt, *col_idx, *out_idx;
-    uint32_t col_off;
-    int pdl;                 // the launches of this call are programmatic dependents of the launch before them
+    int skip_convert;        // 1: xu already holds exactly these columns in this format's layout (the call before used them)
 };
 cudaError_t matmul_tc_nx_init(void);
-// The same call on tcgen05 with the accumulator in tensor memory (matmul_umma.cu; Q4_K). xu: device scratch of
+// Up to 8 columns on tcgen05 with the accumulator in tensor memory (matmul_umma.cu; Q4_K; matmul_umma_on). xu: device scratch of
 // matmul_umma_xu_bytes(cols) bytes for the converted activations; scratch / tickets: split-K partial results and their
 // counters (matmul_umma_scratch_bytes() bytes, matmul_umma_ticket_count() zeroed words).
+bool matmul_umma_on(void);   // FLB_UMMA=1 in the environment now
 cudaError_t launch_matmul_umma(const NxCall &c, uint8_t *xu, float *scratch, uint32_t *tickets, uint32_t *status, int sms,
                                cudaStream_t stream);
 size_t matmul_umma_xu_bytes(uint32_t cols);

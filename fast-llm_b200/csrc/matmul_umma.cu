@@ -54,8 +54,6 @@ struct UmArgs {
     uint32_t ystride, rows, nblk, P;
     uint32_t n_tiles, splits, blk_per_split;
     int accumulate;
-    const uint32_t *cnt, *out_idx;
-    uint32_t col_off;
     float *scratch;                   // [n_tiles * splits][128][8] partial results (splits > 1)
     uint32_t *tickets;                // [n_tiles][4 epilogue warps], zero between launches
     uint32_t *status;
@@ -157,15 +155,11 @@ __device__ __forceinline__ float um_u8f(uint32_t w) {
 // the block scale 2^e (x = 2^e (hi + lo)). Position k of a chunk's K axis holds column pi(k) of the chunk, the order in
 // which the unpack produces the weights: pi(8 j + e) = 4 j + {0, 2, 1, 3, 32, 34, 33, 35}[e].
 __global__ void __launch_bounds__(128) act_convert_umma_kernel(const float *__restrict__ x, const float *__restrict__ x2, uint32_t xstride,
-                                                               uint32_t P, uint8_t *__restrict__ xu, const uint32_t *__restrict__ cnt,
-                                                               uint32_t col_off, const uint32_t *__restrict__ col_idx) {
+                                                               uint32_t P, uint8_t *__restrict__ xu) {
     const uint32_t blk = blockIdx.x, p = threadIdx.x >> 4, hl = threadIdx.x & 15u;
-    uint32_t n_valid = P;
-    if (cnt) { const uint32_t c = *cnt; n_valid = c > col_off ? min(c - col_off, P) : 0u; }
-    if (n_valid == 0) return;   // the matmul of this call returns at entry too
     float v[16];
-    if (p < n_valid) {
-        const size_t row = col_idx ? col_idx[col_off + p] : p;
+    if (p < P) {
+        const size_t row = p;
         const float4 *src = reinterpret_cast<const float4 *>(x + row * xstride + blk * 256 + hl * 16);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -231,9 +225,6 @@ __global__ void __launch_bounds__(128) act_convert_umma_kernel(const float *__re
 __global__ void __launch_bounds__(kThreads, 1) matmul_umma_kernel(const __grid_constant__ UmArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    uint32_t n_valid = a.P;
-    if (a.cnt) { const uint32_t c = *a.cnt; n_valid = c > a.col_off ? min(c - a.col_off, a.P) : 0u; }
-    if (n_valid == 0) return;   // no column of this call exists (uniform over the grid)
     const UmSmem sm = um_carve(smem_raw);
     if (tid == 0) {
         for (uint32_t i = 0; i < kNS; ++i) { mbar_init(&sm.raw_full[i], 1); mbar_init(&sm.raw_empty[i], kUnpackWarps + 1); }
@@ -386,7 +377,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_umma_kernel(const __grid_c
                 mn[4] = um_u8f<0>(h.z); mn[5] = um_u8f<1>(h.z); mn[6] = um_u8f<2>(h.z); mn[7] = um_u8f<3>(h.z);
 #pragma unroll
                 for (int p = 0; p < 8; ++p) {
-                    if ((uint32_t)p < n_valid) {   // uniform
+                    if ((uint32_t)p < a.P) {   // uniform
                         const uint32_t sa = hb + kRows * 16u + p * 36u;
                         float m = 0.f;
 #pragma unroll
@@ -436,9 +427,8 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_umma_kernel(const __grid_c
             if (grow < a.rows) {
 #pragma unroll
                 for (int p = 0; p < 8; ++p) {
-                    if ((uint32_t)p < n_valid) {
-                        const size_t ob = a.out_idx ? a.out_idx[a.col_off + p] : (uint32_t)p;
-                        float *dst = a.y + ob * a.ystride + grow;
+                    if ((uint32_t)p < a.P) {
+                        float *dst = a.y + (size_t)p * a.ystride + grow;
                         *dst = a.accumulate ? *dst + acc[p] : acc[p];
                     }
                 }
@@ -454,17 +444,17 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_umma_kernel(const __grid_c
     }
 }
 
+} // namespace
+
 // Off unless FLB_UMMA=1 (read at every call, so that one process can run both kernels): on the shapes of the decode
 // step the 128-row tile makes the weight stream fetch 144-byte pieces of 128 different rows per stage, two 128-byte
 // lines each, and the TMA unit's rate of about one line per 6.5 cycles then caps the stream at 2.7 TB/s; measured on
 // the gate|up shape with 8 columns: 56 us per pass against 37 us for the mma.sync kernel (37 us already with the
 // unpack, the tensor-core instructions and the epilogue all switched off).
-bool umma_on() {
+bool matmul_umma_on(void) {
     const char *v = getenv("FLB_UMMA");
     return v && v[0] == '1';
 }
-
-} // namespace
 
 size_t matmul_umma_xu_bytes(uint32_t cols) { return (size_t)(cols / 256) * kXuBlk; }
 size_t matmul_umma_scratch_bytes(void) { return (size_t)16 << 20; }
@@ -478,7 +468,7 @@ cudaError_t matmul_umma_init(void) {
 // then takes the mma.sync kernel).
 cudaError_t launch_matmul_umma(const NxCall &c, uint8_t *xu, float *scratch, uint32_t *tickets, uint32_t *status, int sms,
                                cudaStream_t stream) {
-    if (!umma_on() || c.fmt != FMT_Q4_K || c.P < 1 || c.P > 8 || c.cols % 256 != 0 || c.cols < 256 || c.rows == 0) return cudaErrorNotSupported;
+    if (c.fmt != FMT_Q4_K || c.P < 1 || c.P > 8 || c.cols % 256 != 0 || c.cols < 256 || c.rows == 0) return cudaErrorNotSupported;
     const uint32_t pitch = c.pitch ? c.pitch : (uint32_t)row_bytes(c.fmt, c.cols);
     if ((pitch & 15u) || (((uintptr_t)c.w) & 15u) || (((uintptr_t)c.x) & 15u) || (c.xstride & 3u) || (((uintptr_t)c.x2) & 15u)) return cudaErrorNotSupported;
     UmArgs k;
@@ -502,12 +492,11 @@ cudaError_t launch_matmul_umma(const NxCall &c, uint8_t *xu, float *scratch, uin
     cudaError_t e = tensor_map_2d(&k.map, 8, c.w, pitch / 8, c.rows, pitch, 18, kRows, false);
     if (e != cudaSuccess) return e;
     if (!c.skip_convert) {
-        act_convert_umma_kernel<<<nblk, 128, 0, stream>>>(c.x, c.x2, c.xstride, c.P, xu, c.cnt, c.col_off, c.col_idx);
+        act_convert_umma_kernel<<<nblk, 128, 0, stream>>>(c.x, c.x2, c.xstride, c.P, xu);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
     k.xu = xu; k.y = c.y; k.ystride = c.ystride; k.accumulate = c.accumulate;
-    k.cnt = c.cnt; k.out_idx = c.out_idx; k.col_off = c.col_off;
     k.scratch = scratch; k.tickets = tickets; k.status = status;
     const uint32_t n_items = n_tiles * best_s;
     const uint32_t grid = n_items < (uint32_t)sms ? n_items : (uint32_t)sms;
