@@ -966,7 +966,7 @@ static int enqueue_batch(fl_b200_decoder *d, uint32_t m, cudaStream_t s, bool se
         // SiLU(g) * u is built while the down projection's activation is converted (streaming formats); other formats
         // get the product from a launch of its own
         const bool fuse_silu = (w[FL_B200_T_DOWN].fmt == FL_B200_Q4_K || w[FL_B200_T_DOWN].fmt == FL_B200_Q6_K || w[FL_B200_T_DOWN].fmt == FL_B200_Q8_0) &&
-                               row_bytes(w[FL_B200_T_DOWN].fmt, F) % 16 == 0;   // rows the streaming kernels take
+                               row_bytes(w[FL_B200_T_DOWN].fmt, F) % 16 == 0 && F <= kNxMaxCols;   // rows and widths the kernels with a prologue take
         if (!fuse_silu) CK(launch_silu_mul(b.g, b.u, b.g, m * F, s));
         const float *down_x2 = fuse_silu ? b.u : nullptr;
         if (!tp) {

@@ -10,7 +10,8 @@ from fast_llm_b200.decoder import Decoder
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-# SMALL: no tensor qualifies for the multi-column kernel (2048 columns); WIDE: wq, wk, wo, gate, up do.
+# Both run the batch pass on the multi-column kernel (SMALL: one segment of 2048 columns per row; WIDE: two); the
+# tensor-by-tensor form and other weight formats: test_gpu_batch_forms.py.
 SMALL = dict(n_layer=2, n_embd=2048, n_head=16, n_kv_head=4, head_dim=128, n_ff=4096, n_vocab=1000, max_kv=96,
              rope_base=500000.0, eps=1e-5)
 WIDE = dict(n_layer=2, n_embd=4096, n_head=32, n_kv_head=8, head_dim=128, n_ff=4096, n_vocab=1024, max_kv=96,
