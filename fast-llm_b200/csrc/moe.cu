@@ -141,9 +141,9 @@ int fl_b200_moe_create(fl_b200_ctx *ctx, const fl_b200_moe_cfg *cfg, uint32_t ra
     const size_t n_gu = std::max(1u, m->planes_gu), n_d = std::max(1u, m->planes_d);
     // every active expert has at most 16 columns in a pass, all of them together at most one per pair
     m->tgs = (uint32_t)std::min<size_t>((size_t)m->n_local * (kNxMaxTokens / 4), T * K / 4 + std::min<size_t>(m->n_local, T * K));
-    // Rows of the planes (the per-slot form: one slot at a time). Up to 16 tokens are one pass, a row per (token, slot) pair. More of them go in passes of at most 16
-    // columns per expert, whose rows are numbered through and added up to the pairs' results after each: the planes don't grow
-    // with max_tokens.
+    // Rows of the planes (the per-slot form: one slot at a time). Up to 16 tokens are one pass, a row per (token, slot) pair.
+    // More of them go in passes of at most 16 columns per expert, whose rows are numbered through and added up to the pairs'
+    // results after each: the planes don't grow with max_tokens.
     const size_t one_pass = std::min<size_t>(T, kNxMaxTokens) * K;
     m->rows = m->planes_gu == 0 ? 1 : (uint32_t)std::max(one_pass, std::min<size_t>(T * K, (size_t)m->n_local * kNxMaxTokens));
     const size_t R = m->rows, pairs = T > kNxMaxTokens || m->planes_gu == 0 ? T * K : K;   // (K: the per-slot form of one token)

@@ -364,8 +364,15 @@ int fl_b200_decoder_verify(fl_b200_decoder *dec, int32_t first_token, const int3
  * kernel takes its shape (Q4_K, Q6_K, Q8_0); other tensors are walked once per
  * token; a pass of one token (of up to three for models with experts, with a
  * tensor that kernel does not take, or over several GPUs) runs as
- * teacher-forced single steps on the device. Used for draft verification and for
- * prompt ingestion in chunks. On a tensor-parallel decoder all ranks make
+ * teacher-forced single steps on the device. A pass and single steps are not the
+ * same arithmetic, so that results agree to f32 rounding, not bit for bit, and
+ * an f16 cache value may round the other way: the multi-column kernel reads an
+ * activation as two f16 parts (22 bits of every value) and adds exact products
+ * in f32; the one-column kernel reads K-quants' activations as 30-bit fixed
+ * point per 32 columns and adds integers within a super-block, f32 beyond.
+ * Against 64 bits (2-norm, 512 to 14336 columns) a product is 0.9e-7 to 1.3e-7
+ * off in a pass of any size and 1.0e-7 to 2.9e-7 in a single step. Used for
+ * draft verification and for prompt ingestion in chunks. On a tensor-parallel decoder all ranks make
  * the same call; the partial O / down outputs and the argmax records are
  * exchanged per token, and fl_b200_decoder_batch_logits returns this rank's
  * slice. */
@@ -377,8 +384,8 @@ int fl_b200_decoder_step_batch(fl_b200_decoder *dec, const int32_t *toks_host, u
  * [n][n_kv_head][max_kv][head_dim] f16 for K and for V; fl_b200_decoder_seqs_kv returns sequence seq's part so that a
  * caller can prefill it) and a position per sequence (fl_b200_decoder_seqs_set_pos = rewind_to of that sequence).
  * fl_b200_decoder_seqs_step feeds toks_host[i] to sequence i at its own position and returns each sequence's greedy
- * token (and margin): one pass, every weight tensor walked once per 8 sequences, the attention per sequence over its own
- * keys; every position advances by one. fl_b200_decoder_batch_logits(i) then returns the logits of sequence i. The
+ * token (and margin): one pass, every weight tensor walked once where the multi-column kernel takes it, the attention per
+ * sequence over its own keys; every position advances by one. fl_b200_decoder_batch_logits(i) then returns the logits of sequence i. The
  * single-sequence calls (step, run, step_batch) keep working on their own cache. One GPU. */
 int fl_b200_decoder_seqs_init(fl_b200_decoder *dec, uint32_t n_seq);
 int fl_b200_decoder_seqs_kv(fl_b200_decoder *dec, uint32_t layer, uint32_t seq, uint16_t **k_dev_out, uint16_t **v_dev_out);
