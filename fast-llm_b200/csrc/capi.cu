@@ -269,6 +269,7 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
             const uint32_t parts = matmul_tc_nx_parts(&t, 1, cols, nt);
             if (parts == 0) break;   // the shape does not qualify (same answer for every chunk)
             NxIn in{};
+            in.tm = matmul_tc_tm(nt, false);
             in.x = x + (size_t)p0 * xstride; in.xstride = xstride;
             if (x2) in.x2 = x2 + (size_t)p0 * xstride;
             cudaError_t e = cudaSuccess;

@@ -798,8 +798,10 @@ static int enqueue_batch_nx(fl_b200_decoder *d, uint32_t m, cudaStream_t s, bool
         return in;
     };
     // one matvec group: convert the activation, walk the weights
-    auto group = [&](const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t *parts, bool split = true) -> int {
+    auto group = [&](const NxIn &from, const NxTensor *t, int n, uint32_t cols, uint32_t *parts, bool split = true) -> int {
         *parts = matmul_tc_nx_parts(t, n, cols, m, split);
+        NxIn in = from;
+        in.tm = matmul_tc_tm(m, false);
         CK(launch_nx_convert(in, t, n, cols, m, ctx->xq, kNxTgs, s, pdl));
         CK(launch_nx_matmul(in, t, n, cols, m, 0, ctx->xq, kNxTgs, ctx->status, ctx->sms, s, pdl, split));
         return FL_B200_OK;

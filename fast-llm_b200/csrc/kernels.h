@@ -120,10 +120,18 @@ struct NxIn {
     const uint32_t *table, *col_idx, *out_idx;
     uint32_t list_stride, col_off, n_groups, n_experts;   // n_groups: upper bound of active experts
     int table_ready;         // 1: the table was complete before the kernel in front of the matmul started
+    int tm;                  // 1: the form with the weights in tensor memory (matmul_tc_tm)
 };
+// ---- matmul_tm.cu: the same on tcgen05, weights and results in tensor memory ----
+constexpr uint32_t kTmUnit = 8 * 1064;   // image bytes of 256 columns of up to 8 tokens (up to 16: twice as many)
+cudaError_t matmul_tm_init(void);
+uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split, uint32_t groups, int sms);
+cudaError_t launch_tm_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,
+                             const uint32_t *xoff, uint32_t *status, int sms, cudaStream_t stream, bool pdl, bool split);
 // Number of parts the columns are cut into (1: y is the result; more: planes of partial sums); 0: not taken. split: planes cost the
 // caller nothing extra, cut as finely as is best.
-uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split = false);
+uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split = false, uint32_t groups = 1);
+int matmul_tc_tm(uint32_t P, bool grouped);
 // tgs: groups of four columns in the image(s) (grouped: of all active experts together)
 size_t matmul_tc_nx_scratch_bytes(uint32_t cols, uint32_t tgs, int layouts);
 // n = 0 tensors: only x_out is written. cudaErrorNotSupported: strides or addresses the vector loads do not take.
