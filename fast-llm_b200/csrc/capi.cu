@@ -88,11 +88,6 @@ int fl_b200_create(int device, fl_b200_ctx **out) {
     CK(matmul_tc_nx_init());
     CK(cudaMalloc(&c->xq, matmul_tc_nx_scratch_bytes(kNxMaxCols, kNxTgs, 3)));
     CK(cudaMalloc(&c->nx_part, kNxPartFloats * sizeof(float)));
-    CK(matmul_umma_init());
-    CK(cudaMalloc(&c->xu, matmul_umma_xu_bytes(18432)));
-    CK(cudaMalloc(&c->um_scratch, matmul_umma_scratch_bytes()));
-    CK(cudaMalloc(&c->um_tickets, matmul_umma_ticket_count() * sizeof(uint32_t)));
-    CK(cudaMemset(c->um_tickets, 0, matmul_umma_ticket_count() * sizeof(uint32_t)));
     CK(attn_init());
     *out = c;
     return FL_B200_OK;
@@ -104,7 +99,6 @@ void fl_b200_destroy(fl_b200_ctx *c) {
     cudaStreamSynchronize(c->stream);
     cudaFree(c->attn_part);
     cudaFree(c->xq); cudaFree(c->nx_part);
-    cudaFree(c->xu); cudaFree(c->um_scratch); cudaFree(c->um_tickets);
     for (void *p : c->retired) cudaFree(p);
     cudaFree(c->attn_tickets);
     cudaFree(c->argmax_scratch);
@@ -245,22 +239,7 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
     if (pitch == row_bytes(fmt, cols)) pitch = 0;   // packed rows
     uint32_t first_single = 0;   // columns from here on go through the one-column kernel
     if (nx >= 2 && (fmt == FL_B200_Q4_K || fmt == FL_B200_Q6_K || fmt == FL_B200_Q8_0) && !expert_id) {
-        // Q4_K under FLB_UMMA=1: tcgen05 with the accumulator in tensor memory, 8 columns per pass
-        const bool umma = fmt == FL_B200_Q4_K && matmul_umma_on();
-        for (uint32_t p0 = 0; umma && cols <= 18432 && p0 < nx; p0 += 8) {
-            const uint32_t nt = nx - p0 < 8 ? nx - p0 : 8;
-            if (nt < 2 && p0 > 0) break;   // a last single column goes to the one-column kernel
-            NxCall nc{};
-            nc.fmt = fmt; nc.w = w; nc.rows = rows; nc.cols = cols; nc.pitch = pitch;
-            nc.x = x + (size_t)p0 * xstride; nc.P = nt; nc.xstride = xstride;
-            if (x2) nc.x2 = x2 + (size_t)p0 * xstride;
-            nc.skip_convert = (same_columns && nx <= 8) ? 1 : 0;   // with more than 8 columns the scratch holds the last chunk only
-            nc.y = y + (size_t)p0 * ystride; nc.ystride = ystride; nc.accumulate = accumulate;
-            const cudaError_t e = launch_matmul_umma(nc, c->xu, c->um_scratch, c->um_tickets, c->status, c->sms, c->stream);
-            if (e == cudaErrorNotSupported) break;   // not its shape (the same answer for every chunk)
-            if (e != cudaSuccess) return cuda_err(e, "multi-column matmul launch");
-            first_single = p0 + nt;
-        }
+        const bool umma = matmul_umma_on();   // Q4_K on the tcgen05 form, whatever the shape
         // verify batches, prompt chunks: up to 16 columns per pass over the weights on the tensor cores
         for (uint32_t p0 = first_single; p0 < nx; p0 += kNxMaxTokens) {
             const uint32_t nt = nx - p0 < kNxMaxTokens ? nx - p0 : kNxMaxTokens;
@@ -269,17 +248,23 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
             const uint32_t parts = matmul_tc_nx_parts(&t, 1, cols, nt);
             if (parts == 0) break;   // the shape does not qualify (same answer for every chunk)
             NxIn in{};
-            in.tm = matmul_tc_tm(nt, false);
             in.x = x + (size_t)p0 * xstride; in.xstride = xstride;
             if (x2) in.x2 = x2 + (size_t)p0 * xstride;
             cudaError_t e = cudaSuccess;
+            in.tm = umma && fmt == FL_B200_Q4_K && matmul_tm_parts(&t, 1, cols, false) == 1;
             // the scratch holds these columns already: not with more of them than a chunk (it has the last one only), nor where
-            // the call before may have gone to the tcgen05 kernel, which has a scratch of its own
+            // this call or the one before may be on the tcgen05 form, whose image is another one
             const bool reuse = same_columns && nx <= kNxMaxTokens && !umma;
             if (!reuse) {
                 e = launch_nx_convert(in, &t, 1, cols, nt, c->xq, kNxTgs, c->stream, pdl != 0);
                 if (e == cudaErrorNotSupported) break;
                 if (e != cudaSuccess) return cuda_err(e, "activation conversion launch");
+            }
+            if (in.tm) {
+                e = launch_tm_matmul(in, &t, 1, cols, nt, accumulate, c->xq, c->status, c->stream, true, false);
+                if (e != cudaSuccess) return cuda_err(e, "multi-column matmul launch");
+                first_single = p0 + nt;
+                continue;
             }
             // the matmul overlaps the conversion's launch: it reads weights only until the conversion has completed
             const uint32_t cap = (uint32_t)(kNxPartFloats / ((size_t)parts * nt)) & ~15u, slice = parts == 1 || rows <= cap ? rows : cap;

@@ -34,9 +34,6 @@ struct fl_b200_ctx {
     void *small = nullptr;
     uint8_t *xq = nullptr;               // converted activations of the multi-column matmul (fixed size, see fl_b200_create)
     float *nx_part = nullptr;            // its planes of partial results (kNxPartFloats, see matmul)
-    uint8_t *xu = nullptr;               // the converted activations of the tcgen05 matmul, with its split-K scratch and tickets
-    float *um_scratch = nullptr;
-    uint32_t *um_tickets = nullptr;
     uint32_t *grid_bar = nullptr;        // barrier state of the chained matvec launches (two words, zero between launches)
     std::weak_ptr<MoeScratch> moe_scratch;   // the newest (largest) one
     uint64_t wait_limit_ns = 0;          // limit of the exchange kernels' waits for other ranks (0 = one second)

@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(256) scatter_rows_kernel(const float *__restri
 // columns from col_off on (at most P), the groups of four columns in front of them and the columns in front of them.
 __device__ __forceinline__ void nx_table_warp(const uint32_t *cnt, uint32_t n_local, uint32_t col_off, uint32_t P, uint32_t *table) {
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t n_act = 0, before = 0, most = 0, before8 = 0;   // before: groups of four, columns << 16; before8: groups of eight
+    uint32_t n_act = 0, before = 0, most = 0;   // before: groups of four, columns << 16
     for (uint32_t b = 0; b < n_local; b += 32) {
         const uint32_t e = b + lane, c = e < n_local ? cnt[e] : 0u;
         const uint32_t n = c > col_off ? min(c - col_off, P) : 0u, tg = (n + 3) / 4, own = tg | n << 16;
@@ -182,15 +182,8 @@ __device__ __forceinline__ void nx_table_warp(const uint32_t *cnt, uint32_t n_lo
             const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= (uint32_t)o) incl += v;
         }
-        uint32_t incl8 = (n + 7) / 8;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl8, o);
-            if (lane >= (uint32_t)o) incl8 += v;
-        }
-        const uint32_t mask = __ballot_sync(0xffffffffu, n != 0), at = before + incl - own, at8 = before8 + incl8 - (n + 7) / 8;
-        if (n) reinterpret_cast<uint4 *>(table)[1 + n_act + __popc(mask & ((1u << lane) - 1u))] = make_uint4(e, n, (at & 0xFFFFu) | at8 << 16, at >> 16);
-        before8 += __shfl_sync(0xffffffffu, incl8, 31);
+        const uint32_t mask = __ballot_sync(0xffffffffu, n != 0), at = before + incl - own;
+        if (n) reinterpret_cast<uint4 *>(table)[1 + n_act + __popc(mask & ((1u << lane) - 1u))] = make_uint4(e, n, at & 0xFFFFu, at >> 16);
         n_act += __popc(mask);
         most = max(most, __reduce_max_sync(0xffffffffu, tg));
         before += __shfl_sync(0xffffffffu, incl, 31);

@@ -120,18 +120,12 @@ struct NxIn {
     const uint32_t *table, *col_idx, *out_idx;
     uint32_t list_stride, col_off, n_groups, n_experts;   // n_groups: upper bound of active experts
     int table_ready;         // 1: the table was complete before the kernel in front of the matmul started
-    int tm;                  // 1: the form with the weights in tensor memory (matmul_tc_tm)
+    int tm;                  // 1: launch_nx_convert builds the image of the form below (Q4_K only, not grouped)
 };
-// ---- matmul_tm.cu: the same on tcgen05, weights and results in tensor memory ----
-constexpr uint32_t kTmUnit = 8 * 1064;   // image bytes of 256 columns of up to 8 tokens (up to 16: twice as many)
-cudaError_t matmul_tm_init(void);
-uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split, uint32_t groups, int sms);
-cudaError_t launch_tm_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,
-                             const uint32_t *xoff, uint32_t *status, int sms, cudaStream_t stream, bool pdl, bool split);
 // Number of parts the columns are cut into (1: y is the result; more: planes of partial sums); 0: not taken. split: planes cost the
 // caller nothing extra, cut as finely as is best.
-uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split = false, uint32_t groups = 1);
-int matmul_tc_tm(uint32_t P, bool grouped);
+// tm: launches that matmul_tm_takes are cut as that form cuts them.
+uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split = false, bool tm = false);
 // tgs: groups of four columns in the image(s) (grouped: of all active experts together)
 size_t matmul_tc_nx_scratch_bytes(uint32_t cols, uint32_t tgs, int layouts);
 // n = 0 tensors: only x_out is written. cudaErrorNotSupported: strides or addresses the vector loads do not take.
@@ -143,30 +137,16 @@ cudaError_t launch_reduce_parts(const float *part, size_t part_stride, uint32_t 
                                 uint32_t P, int accumulate, cudaStream_t stream, bool pdl);
 // The table of a grouped launch: of cnt[e] listed columns of expert e those from col_off on, at most P.
 cudaError_t launch_nx_table(const uint32_t *cnt, uint32_t n_local, uint32_t col_off, uint32_t P, uint32_t *table, cudaStream_t stream);
-// One call of the tcgen05 form below, up to 8 columns.
-struct NxCall {
-    int fmt;
-    const void *w;           // rows x cols, GGUF block layout
-    uint32_t rows, cols, pitch;   // pitch 0 = packed rows
-    const float *x;          // columns: rows of x, xstride floats apart
-    const float *x2;         // optional: the column is SiLU(x) * x2 (same stride)
-    uint32_t P, xstride;     // columns of this call (<= 8)
-    float *y;                // output row blocks, ystride floats apart
-    uint32_t ystride;
-    int accumulate;
-    int skip_convert;        // 1: xu already holds exactly these columns in this format's layout (the call before used them)
-};
+// The same on tcgen05, weights and results in tensor memory (matmul_tm.cu): Q4_K, not grouped; between launch_nx_convert with
+// in.tm set and the next conversion or reduction, as launch_nx_matmul. The image of 256 columns takes 8512 bytes up to 8 tokens,
+// else 17024: less than matmul_tc_nx_scratch_bytes provides.
+bool matmul_tm_takes(const NxTensor *t, int n, uint32_t cols, uint32_t P);   // launches with planes (split) for which it is the faster form
+uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, bool split);
+cudaError_t launch_tm_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,
+                             uint32_t *status, cudaStream_t stream, bool pdl, bool split);
+cudaError_t matmul_tm_init(void);
+bool matmul_umma_on(void);   // FLB_UMMA=1 in the environment now: every Q4_K call of several columns on that form
 cudaError_t matmul_tc_nx_init(void);
-// Up to 8 columns on tcgen05 with the accumulator in tensor memory (matmul_umma.cu; Q4_K; matmul_umma_on). xu: device scratch of
-// matmul_umma_xu_bytes(cols) bytes for the converted activations; scratch / tickets: split-K partial results and their
-// counters (matmul_umma_scratch_bytes() bytes, matmul_umma_ticket_count() zeroed words).
-bool matmul_umma_on(void);   // FLB_UMMA=1 in the environment now
-cudaError_t launch_matmul_umma(const NxCall &c, uint8_t *xu, float *scratch, uint32_t *tickets, uint32_t *status, int sms,
-                               cudaStream_t stream);
-size_t matmul_umma_xu_bytes(uint32_t cols);
-size_t matmul_umma_scratch_bytes(void);
-size_t matmul_umma_ticket_count(void);
-cudaError_t matmul_umma_init(void);
 // True when launch_matvec would take the streaming kernel for this shape.
 bool matvec_is_streaming(int fmt, uint32_t cols);
 // Dynamic shared memory the streaming kernel needs for (cols, formats used).

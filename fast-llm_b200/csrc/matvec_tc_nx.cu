@@ -208,7 +208,7 @@ struct ConvArgs {
     uint32_t list_stride, col_off;
     const float *att;              // the columns are attention contexts of heads of 128, added up here from n_splits records
     uint32_t n_splits;             // (attn.cu: [column][head][split][132] = context, maximum, sum)
-    uint32_t tm;                   // the images are those of matmul_tm.cu
+    int tm;                        // img4 is the image of matmul_tm.cu
 };
 // Device-side table of a grouped launch: word 0 = number of active groups, word 1 = the most token groups of one; then four
 // words per active group: {group, number of columns, token groups in front of it, columns in front of it}.
@@ -273,12 +273,11 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     if (a.table) {
         if (blockIdx.z >= a.table[0]) return;
         const uint4 e = reinterpret_cast<const uint4 *>(a.table)[1 + blockIdx.z];
-        grp = e.x; n_valid = e.y; tg0 = a.tm ? e.z >> 16 : e.z & 0xFFFFu; row0 = e.w;
+        grp = e.x; n_valid = e.y; tg0 = e.z; row0 = e.w;
         ntg = (n_valid + 3) / 4;
         if (tg >= ntg) return;
     }
     const uint32_t p = 4 * tg + pp;
-    if (a.tm && p >= n_valid) return;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     float ss = 0.f;
     if (p < n_valid) {
@@ -322,31 +321,19 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);   // over the 32-column sub-block
     if (a.tm) {
-        // Image of a block for NT = 8 or 16 tokens (matmul_tm.cu): four tiles of 64 columns, 2 NT rows of 128 bytes (row p the hi
-        // parts of token p, row NT + p the lo parts; 16-byte piece j of a row at j ^ (row & 7), the 128-byte swizzle), then
-        // the sub-block sums [8][NT], the block scales [NT] and the sums of squares [NT]. The order of the columns is that of
-        // the fragments above: columns c, c + 2 / c + 1, c + 3 of a thread's four are words 0 / 1 of instruction m, lane column t.
+        // Image of a block for NT = 8 or 16 tokens (matmul_tm.cu): a tile per 64 columns of 2 NT rows of 128 bytes (row p the hi parts
+        // of token p, row NT + p the lo parts; 16-byte piece j of a row at j ^ (row & 7), the 128-byte swizzle), then the
+        // sub-block sums [8][NT], the block scales [NT] and the sums of squares [NT]. Piece j: columns 4 j + {0, 2, 1, 3} of the
+        // first sub-block of the tile, then of the second. Rows of tokens that there are not are never written nor used.
+        if (p >= n_valid) return;
         const uint32_t NT = n_valid > 8 ? 16u : 8u;
-        const size_t at = ((size_t)(a.table ? tg0 : 0u) * a.nblk + (size_t)blk * (NT / 8)) * kTmUnit;
-#pragma unroll
-        for (int f = 0; f < 3; ++f) {
-            uint8_t *base = f == 0 ? a.img4 : f == 1 ? a.img6 : a.img8;
-            if (!base) continue;
-            base += at;
-            uint32_t m, t;
-            if (f == 0) { m = 2 * (i & 7u) + ((i >> 3) & 1u); t = i >> 4; }
-            else if (f == 1) { m = ((i >> 5) * 2 + ((i >> 2) & 1u)) * 4 + ((i >> 3) & 3u); t = i & 3u; }
-            else { m = 2 * (i >> 3) + (i & 1u); t = (i >> 1) & 3u; }
-            uint8_t *tile = base + (m >> 2) * (NT * 256) + 4 * t;
-            const uint32_t j0 = (m & 3u) * 2, rh = p, rl = NT + p;   // NT is a multiple of 8: both rows swizzle alike
-            *reinterpret_cast<uint32_t *>(tile + rh * 128 + ((j0 ^ (p & 7u)) << 4)) = hi.x;
-            *reinterpret_cast<uint32_t *>(tile + rh * 128 + (((j0 + 1) ^ (p & 7u)) << 4)) = hi.y;
-            *reinterpret_cast<uint32_t *>(tile + rl * 128 + ((j0 ^ (p & 7u)) << 4)) = lo.x;
-            *reinterpret_cast<uint32_t *>(tile + rl * 128 + (((j0 + 1) ^ (p & 7u)) << 4)) = lo.y;
-            float *side = reinterpret_cast<float *>(base + NT * 1024);
-            if ((i & 7u) == 0) side[(i >> 3) * NT + p] = sum;
-            if (i == 0) { side[8 * NT + p] = scale; side[9 * NT + p] = h0.y + h1.y; }
-        }
+        uint8_t *img = a.img4 + (size_t)blk * (NT * 1064u), *row = img + (i >> 4) * (NT * 256) + p * 128;
+        const uint32_t piece = (((i & 7u) ^ (p & 7u)) << 4) + (i & 8u);   // (NT is a multiple of 8: both rows swizzle alike)
+        *reinterpret_cast<uint2 *>(row + piece) = hi;
+        *reinterpret_cast<uint2 *>(row + NT * 128 + piece) = lo;
+        float *side = reinterpret_cast<float *>(img + NT * 1024);
+        if ((i & 7u) == 0) side[(i >> 3) * NT + p] = sum;
+        if (i == 0) { side[8 * NT + p] = scale; side[9 * NT + p] = h0.y + h1.y; }
         return;
     }
     const size_t unit = (size_t)tg0 * a.nblk + (size_t)blk * ntg + tg;
@@ -466,7 +453,7 @@ __device__ __noinline__ void nx_list_pieces(const NxArgs &a, uint8_t *smem_raw) 
             if (u0 >= u1) continue;
             const uint32_t same = n > 0 && last_g == g && last_part == jb.part && last_x == a.t[jb.tensor].xoff ? 1u : 0u;
             last_g = g; last_part = jb.part; last_x = a.t[jb.tensor].xoff;
-            out[n++] = make_uint4(u0, u1, j | (e.y << 8) | (e.x << 16), (e.w << 16) | ((e.z & 0xFFFFu) << 2) | (same << 1) | (kk & 1u));
+            out[n++] = make_uint4(u0, u1, j | (e.y << 8) | (e.x << 16), (e.w << 16) | (e.z << 2) | (same << 1) | (kk & 1u));
             kk += u1 - u0;
         }
     }
@@ -1020,23 +1007,10 @@ cudaError_t matmul_tc_nx_init(void) {
 
 // Bytes of device scratch the converted activations of `tgs` groups of four columns need, one image per layout.
 size_t matmul_tc_nx_scratch_bytes(uint32_t cols, uint32_t tgs, int layouts) {
-    return std::max((size_t)(cols / 256) * tgs * (kXq4 + (layouts > 1 ? kXq6 : 0) + (layouts > 2 ? kXq6 : 0)),
-                    (size_t)(cols / 256) * (layouts == 1 ? tgs : (tgs + 1) / 2) * kTmUnit * layouts);
+    return (size_t)(cols / 256) * tgs * (kXq4 + (layouts > 1 ? kXq6 : 0) + (layouts > 2 ? kXq6 : 0));
 }
 
-int matmul_tc_tm(uint32_t P, bool grouped) {
-    static const int tm = getenv("FLB_TM") ? atoi(getenv("FLB_TM")) : 0;
-    (void)grouped;
-    return tm && (int)P >= tm ? 1 : 0;
-}
-
-// Where the image of a format starts in the tm form (image of one format: of all columns and units of 8 tokens).
-static uint32_t tm_image_off(int fmt, bool q4, bool q6, uint32_t cols, uint32_t tgs) {
-    const uint32_t one = (cols / 256) * ((tgs + 1) / 2) * kTmUnit;
-    return (fmt != FMT_Q4_K && q4 ? one : 0) + (fmt == FMT_Q8_0 && q6 ? one : 0);
-}
-
-uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split, uint32_t groups) {
+uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split, bool tm) {
     static const bool off = getenv("FLB_TC_NX") && getenv("FLB_TC_NX")[0] == '0';
     if (off || n < 1 || n > 3 || cols % 256 != 0 || cols < 256 || cols > kNxMaxCols || P == 0 || P > kNxMaxTokens) return 0;
     int fmts[3];
@@ -1044,7 +1018,7 @@ uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P,
         if (!nx_tensor_ok(t[i], cols)) return 0;
         fmts[i] = t[i].fmt;
     }
-    if (matmul_tc_tm(P, groups > 1)) return matmul_tm_parts(t, n, cols, P, split, groups, 148);
+    if (split && tm && matmul_tm_takes(t, n, cols, P)) return matmul_tm_parts(t, n, cols, true);
     NxPlan p;
     return nx_plan(fmts, n, cols, (P + 3) / 4, split, p) ? p.parts : 0;
 }
@@ -1059,15 +1033,10 @@ cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t
     c.x = in.x; c.x2 = in.x2; c.part_stride = in.part_stride; c.resid = in.resid; c.x_out = in.x_out; c.wnorm = in.wnorm;
     c.xstride = in.xstride; c.rstride = in.rstride; c.n_parts = in.n_parts ? in.n_parts : 1; c.P = P; c.nblk = cols / 256;
     c.tm = in.tm;
-    if (in.tm) {
-        if (q4) c.img4 = xq;
-        if (q6) c.img6 = xq + tm_image_off(FMT_Q6_K, q4, q6, cols, tgs_cap);
-        if (q8) c.img8 = xq + tm_image_off(FMT_Q8_0, q4, q6, cols, tgs_cap);
-    } else {
+    if (in.tm && (q6 || q8 || in.table)) return cudaErrorNotSupported;
     if (q4) c.img4 = xq;
     if (q6) c.img6 = xq + nx_image_off(FMT_Q6_K, q4, q6, cols, tgs_cap);
     if (q8) c.img8 = xq + nx_image_off(FMT_Q8_0, q4, q6, cols, tgs_cap);
-    }
     c.att = in.att; c.n_splits = in.n_splits;
     c.table = in.table; c.col_idx = in.col_idx; c.list_stride = in.list_stride; c.col_off = in.col_off;
     return launch_kernel(act_convert_nx_kernel, dim3(cols / 256, (P + 3) / 4 * 4, in.table ? in.n_groups : 1), dim3(64), 0, stream, pdl, c);
@@ -1075,14 +1044,7 @@ cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t
 
 cudaError_t launch_nx_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,
                              uint32_t tgs_cap, uint32_t *status, int sms, cudaStream_t stream, bool pdl, bool split) {
-    if (matmul_tc_nx_parts(t, n, cols, P, split, in.table ? in.n_groups : 1) == 0) return cudaErrorNotSupported;
-    if (in.tm) {
-        bool h4 = false, h6 = false;
-        for (int i = 0; i < n; ++i) { h4 |= t[i].fmt == FMT_Q4_K; h6 |= t[i].fmt == FMT_Q6_K; }
-        uint32_t xoff[3];
-        for (int i = 0; i < n; ++i) xoff[i] = tm_image_off(t[i].fmt, h4, h6, cols, tgs_cap);
-        return launch_tm_matmul(in, t, n, cols, P, accumulate, xq, xoff, status, sms, stream, pdl, split);
-    }
+    if (matmul_tc_nx_parts(t, n, cols, P, split) == 0) return cudaErrorNotSupported;
     static_assert(sizeof(NxArgs) <= 4000, "kernel arguments");
     NxArgs k;
     memset(&k, 0, sizeof(k));

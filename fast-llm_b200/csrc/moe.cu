@@ -133,8 +133,7 @@ int fl_b200_moe_create(fl_b200_ctx *ctx, const fl_b200_moe_cfg *cfg, uint32_t ra
     for (uint32_t P = 1; P <= kNxMaxTokens && P <= T; ++P) {
         const NxTensor gu{c.fmt_gate_up, nullptr, (uint32_t)F, 0, nullptr, 0, 0}, dn{c.fmt_down, nullptr, (uint32_t)E, 0, nullptr, 0, 0};
         const NxTensor two[2] = {gu, gu};
-        const uint32_t groups = (uint32_t)std::min<size_t>(m->n_local, T * K);
-        const uint32_t a = matmul_tc_nx_parts(two, 2, c.n_embd, P, true, groups), b = matmul_tc_nx_parts(&dn, 1, c.n_ff, P, true, groups);
+        const uint32_t a = matmul_tc_nx_parts(two, 2, c.n_embd, P, true), b = matmul_tc_nx_parts(&dn, 1, c.n_ff, P, true);
         if (a == 0 || b == 0) { m->planes_gu = m->planes_d = 0; break; }
         m->planes_gu = std::max(m->planes_gu, a);
         m->planes_d = std::max(m->planes_d, b);
@@ -352,14 +351,13 @@ static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y,
     const size_t R = m->rows;
     const NxTensor gu[2] = {{c.fmt_gate_up, m->wg, F, 0, m->g, F, R * F}, {c.fmt_gate_up, m->wu, F, 0, m->u, F, R * F}};
     const NxTensor dn{c.fmt_down, m->wd, E, 0, m->d, E, R * E};   // down: the column of pair p is silu(g[p]) * u[p]
-    const uint32_t n_groups = std::min(m->n_local, n_tok * K);
-    const uint32_t parts_gu = matmul_tc_nx_parts(gu, 2, E, P, true, n_groups), parts_d = matmul_tc_nx_parts(&dn, 1, F, P, true, n_groups);
+    const uint32_t parts_gu = matmul_tc_nx_parts(gu, 2, E, P, true), parts_d = matmul_tc_nx_parts(&dn, 1, F, P, true);
     for (uint32_t off = 0; off < n_tok; off += kNxMaxTokens) {
         if (off) CKM(launch_nx_table(m->cnt, m->n_local, off, P, m->table, s));
         NxIn in{};
         in.x = x; in.xstride = E; in.wnorm = wnorm; in.eps = eps;
         in.table = m->table; in.col_idx = m->tok_list; in.out_idx = one_pass ? m->pair_list : nullptr; in.list_stride = T; in.col_off = off;
-        in.n_groups = n_groups; in.n_experts = m->n_local; in.tm = matmul_tc_tm(P, true);
+        in.n_groups = std::min(m->n_local, n_tok * K); in.n_experts = m->n_local;
         // the first conversion is an ordinary dependent of the kernel that wrote the table; every later launch starts after
         // it did, so that the table is in place for all of them
         in.table_ready = kMoePdlNx;
