@@ -45,11 +45,13 @@ constexpr uint32_t kSmemLimit = 227 * 1024;
 constexpr uint32_t kMaxSlots = 8, kComb = 1024;   // in front of the ring: barriers, then (kComb) the sums that one half of the epilogue hands to the other
 __host__ __device__ constexpr uint32_t head_of(uint32_t T) { return kComb + kRows * T * 4; }
 constexpr uint32_t kACol = 0, kABuf = 128, kDCol = 256, kTmemCols = 512;
-constexpr uint32_t kPitch = 144;   // bytes of a row of a step: an odd multiple of 16, so that the row-per-thread reads do not collide
+// Bytes of a row that a stage holds: odd multiples of 16, so that neither the row-per-thread reads nor the fragment reads of Q6_K
+// collide. A Q6_K super-block (210 bytes) starts on any even byte; its stage starts on the 16-byte boundary in front of it.
+__host__ __device__ constexpr uint32_t pitch_of(int fmt) { return fmt == FMT_Q4_K ? 144u : 240u; }
 
 // A stage: the rows' bytes, then the step's activation (the operand's four tiles, sub-block sums, block scales, sums of squares).
-template <int T> constexpr uint32_t kSlot = (kRows * kPitch + T * 1064 + 1023) & ~1023u;
-template <int T> constexpr uint32_t kSlots = (kSmemLimit - head_of(T)) / kSlot<T> < kMaxSlots ? (kSmemLimit - head_of(T)) / kSlot<T> : kMaxSlots;
+template <int F, int T> constexpr uint32_t kSlot = (kRows * pitch_of(F) + T * 1064 + 1023) & ~1023u;
+template <int F, int T> constexpr uint32_t kSlots = (kSmemLimit - head_of(T)) / kSlot<F, T> < kMaxSlots ? (kSmemLimit - head_of(T)) / kSlot<F, T> : kMaxSlots;
 
 struct TmT {
     float *y;
@@ -57,7 +59,7 @@ struct TmT {
     uint32_t rows, ystride, base;   // base: where the tensor starts on the line
 };
 struct TmArgs {
-    CUtensorMap map[3];   // [rows][pitch / 8] 8-byte elements, box 128 rows x kPitch
+    CUtensorMap map[3];   // [rows][pitch / 8] 8-byte elements, box 128 rows x pitch_of
     TmT t[3];
     uint32_t n, steps, nblk, P, parts, whole;   // whole: a CTA takes whole tiles only
     const uint8_t *xq;
@@ -128,6 +130,16 @@ __device__ __forceinline__ bool one_wait(uint32_t bar, uint32_t parity, uint32_t
 
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// 16 lanes x 64 columns of tensor memory from the warp: r[2 i], r[2 i + 1] = rows g, g + 8 of column 4 i + t
+__device__ __forceinline__ void tm_store64(uint32_t addr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x128b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
+        "%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(addr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]),
+        "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
 // 32 lanes x 32 columns: r[i] = column i of the thread's lane
 __device__ __forceinline__ void tm_store32(uint32_t addr, const uint32_t (&r)[32]) {
     asm volatile(
@@ -180,9 +192,12 @@ __device__ __forceinline__ bool elect_one() {
 }
 __device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
 __device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
+__device__ __forceinline__ uint32_t hsub2_u32(uint32_t h, __half2 off) { return as_u32(__hsub2(as_h2(h), off)); }
 __device__ __forceinline__ uint32_t hfma2_u32(uint32_t h, __half2 m, __half2 c) { return as_u32(__hfma2(as_h2(h), m, c)); }
 // byte k of w as a float
 __device__ __forceinline__ float u8f(uint32_t w, int k) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + k)) - 8388608.f; }
+// byte k of w, which holds s + 128, as s
+__device__ __forceinline__ float s8f(uint32_t w, int k) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + k)) - 8388736.f; }
 
 // two f32 at once
 struct F2 { uint64_t v; };
@@ -256,8 +271,47 @@ __device__ __forceinline__ void unpack_q4k(uint32_t r, uint32_t tm) {
         tm_store32(tm + 32 * c, o);
     }
 }
+// Q6_K, 16 rows at a time in the layout of an mma.sync A fragment, lane (g, t): rows g, g + 8 (r0: row g), column t of every four (a
+// thread per row would have to realign its bytes by any even number). q - 32 as f16; instruction m = (2 hf + hq) * 4 + gq covers one
+// scale group (matvec_tc_nx.cu). ODD: the block starts 2 bytes past a word boundary (r0 is 2 bytes in front of it).
+template <bool ODD>
+__device__ __forceinline__ void unpack_q6k(uint32_t r0, uint32_t t, uint32_t tm) {
+    constexpr uint32_t kPitch = pitch_of(FMT_Q6_K);
+    const __half2 off = __floats2half2_rn(1056.f, 1056.f);
+#pragma unroll 1
+    for (uint32_t hf = 0; hf < 2; ++hf) {
+        uint32_t o[32];
+#pragma unroll
+        for (int hq = 0; hq < 2; ++hq)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const uint32_t rb = r0 + r * 8 * kPitch, oa = 64 * hf + 16 * hq + 4 * t, oh = 128 + 32 * hf + 16 * hq + 4 * t;
+                uint32_t a, b, h;
+                if (ODD) {
+                    a = __byte_perm(lds32(rb + oa), lds32(rb + oa + 4), 0x5432u);
+                    b = __byte_perm(lds32(rb + oa + 32), lds32(rb + oa + 36), 0x5432u);
+                    h = __byte_perm(lds32(rb + oh), lds32(rb + oh + 4), 0x5432u);
+                } else {
+                    a = lds32(rb + oa); b = lds32(rb + oa + 32); h = lds32(rb + oh);
+                }
+                uint32_t q[4];
+                q[0] = (a & 0x0F0F0F0Fu) | ((h << 4) & 0x30303030u);
+                q[1] = (b & 0x0F0F0F0Fu) | ((h << 2) & 0x30303030u);
+                q[2] = ((a >> 4) & 0x0F0F0F0Fu) | (h & 0x30303030u);
+                q[3] = ((b >> 4) & 0x0F0F0F0Fu) | ((h >> 2) & 0x30303030u);
+#pragma unroll
+                for (int gq = 0; gq < 4; ++gq) {   // bytes 0, 2 / 1, 3 under 0x64: f16 1024 + q
+                    o[16 * hq + 4 * gq + r] = hsub2_u32(__byte_perm(q[gq], 0x64646464u, 0x4240u), off);
+                    o[16 * hq + 4 * gq + 2 + r] = hsub2_u32(__byte_perm(q[gq], 0x64646464u, 0x4341u), off);
+                }
+            }
+        tm_store64(tm + 64 * hf, o);
+    }
+}
+
 // ---- epilogue of one step: acc[i] += the step's results of tokens 2 i, 2 i + 1 -----------------------------------------
-// The four results of a step (D: 4 x N columns; N = 2 NT: hi columns of the tokens, then lo columns).
+// Four results at a time (D: 4 x N columns; N = 2 NT: hi columns of the tokens, then lo columns): Q4_K has one such unit per step, a
+// half of the epilogue every other step; Q6_K four, a half every other one.
 struct Ring { uint32_t slot, par; };
 struct Epi {
     uint32_t smem, tmem;   // tmem: this warp's lanes
@@ -296,7 +350,7 @@ __device__ __forceinline__ bool step_results(const Epi &e, Ring &d, uint32_t lan
     return true;
 }
 template <int NT, int R>
-__device__ __forceinline__ bool epi_step(const Epi &e, Ring &d, uint32_t lane, uint32_t row_addr, uint32_t side, F2 (&acc)[NT / 2]) {
+__device__ __forceinline__ bool epi_step_q4k(const Epi &e, Ring &d, uint32_t lane, uint32_t row_addr, uint32_t side, F2 (&acc)[NT / 2]) {
     const uint32_t xs = side + NT * 32;
     F2 sum[NT / 2];
     const uint4 hd = lds128(row_addr);
@@ -342,15 +396,81 @@ __device__ __forceinline__ bool epi_step(const Epi &e, Ring &d, uint32_t lane, u
     return true;
 }
 
-// The 16 instructions of a step (a: its weights, b: descriptor of its activation, dt: its four results).
-template <int N>
-__device__ __forceinline__ void tensor_step(uint32_t a, uint64_t b, uint32_t dt) {
-    constexpr uint32_t idesc = (1u << 4) | ((N >> 3) << 17) | ((128u >> 4) << 24);   // f16 x f16 -> f32, K-major, M 128
+// Row address of the block's stage, which it starts `misalign` bytes into.
+template <int NT, int R>
+__device__ __forceinline__ bool epi_step_q6k(const Epi &e, Ring &d, uint32_t half, uint32_t lane, uint32_t row_addr, uint32_t misalign, uint32_t side, F2 (&acc)[NT / 2]) {
+    // the 16 scales and d: 18 bytes from byte 192 of the block on
+    const uint4 p0 = lds128(row_addr + 192), p1 = lds128(row_addr + 208);
+    uint32_t w[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+    if (misalign & 8u) {
 #pragma unroll
-    for (int m = 0; m < 16; ++m) tm_mma(dt + (m >> 2) * N, a + 8 * m, b + (uint64_t)((m >> 2) * N * 8 + (m & 3) * 2), idesc, m & 3);
+        for (int k = 0; k < 6; ++k) w[k] = w[k + 2];
+    }
+    if (misalign & 4u) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) w[k] = w[k + 1];
+    }
+    if (misalign & 2u) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) w[k] = __byte_perm(w[k], w[k + 1], 0x5432u);
+    }
+    const F2 d2 = f2(h2f_bits((uint16_t)(w[4] & 0xFFFFu)));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[k] ^= 0x80808080u;
+    F2 sum[NT / 2];
+#pragma unroll
+    for (int i = 0; i < NT / 2; ++i) sum[i] = f2(0.f);
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {   // units 2 hf + half: the scale of group gq is 8 hf + 2 gq + half
+        const uint32_t lo = w[2 * hf] >> (8 * half), up = w[2 * hf + 1] >> (8 * half);
+        const F2 f[4] = {f2(s8f(lo, 0)), f2(s8f(lo, 2)), f2(s8f(up, 0)), f2(s8f(up, 2))};
+        const auto mul8 = [&](float (&a)[16], float (&b)[16], float (&c)[16], float (&g)[16]) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                sum[i] = fma2(f[0], f2(a[2 * i], a[2 * i + 1]), sum[i]);
+                sum[i] = fma2(f[1], f2(b[2 * i], b[2 * i + 1]), sum[i]);
+                sum[i] = fma2(f[2], f2(c[2 * i], c[2 * i + 1]), sum[i]);
+                sum[i] = fma2(f[3], f2(g[2 * i], g[2 * i + 1]), sum[i]);
+                sum[i] = fma2(f[0], f2(a[8 + 2 * i], a[9 + 2 * i]), sum[i]);
+                sum[i] = fma2(f[1], f2(b[8 + 2 * i], b[9 + 2 * i]), sum[i]);
+                sum[i] = fma2(f[2], f2(c[8 + 2 * i], c[9 + 2 * i]), sum[i]);
+                sum[i] = fma2(f[3], f2(g[8 + 2 * i], g[9 + 2 * i]), sum[i]);
+            }
+        };
+        const auto mul16 = [&](int k, float (&h)[16], float (&l)[16]) {
+#pragma unroll
+            for (int i = 0; i < NT / 2; ++i) {
+                sum[i] = fma2(f[k], f2(h[2 * i], h[2 * i + 1]), sum[i]);
+                sum[i] = fma2(f[k], f2(l[2 * i], l[2 * i + 1]), sum[i]);
+            }
+        };
+        if constexpr (NT == 8) { if (!step_results<NT, R>(e, d, lane, mul8)) return false; }
+        else { if (!step_results<NT, R>(e, d, lane, mul16)) return false; }
+    }
+#pragma unroll
+    for (int i = 0; i < NT / 2; i += 2) {
+        F2 x0, x1;
+        lds_f2x2(side + NT * 32 + i * 8, x0, x1);
+        acc[i] = fma2(x0 * d2, sum[i], acc[i]);
+        acc[i + 1] = fma2(x1 * d2, sum[i + 1], acc[i + 1]);
+    }
+    return true;
 }
 
-template <int T>
+// Instructions u .. of a step (a: its weights, b: descriptor of its activation) into a unit's four results at dt: all 16 of Q4_K, a chain
+// of four each, or 4 of Q6_K's.
+template <int F, int N>
+__device__ __forceinline__ void tensor_unit(uint32_t a, uint64_t b, uint32_t dt, int u) {
+    constexpr uint32_t idesc = (1u << 4) | ((N >> 3) << 17) | ((128u >> 4) << 24);   // f16 x f16 -> f32, K-major, M 128
+    constexpr int C = F == FMT_Q4_K ? 4 : 1;
+#pragma unroll
+    for (int i = 0; i < 4 * C; ++i) {
+        const int m = u + i;
+        tm_mma(dt + i / C * N, a + 8 * m, b + (uint64_t)((m >> 2) * N * 8 + (m & 3) * 2), idesc, i % C);
+    }
+}
+
+template <int F, int T>
 __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_constant__ TmArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     constexpr int R = T == 16 ? 2 : 4;   // D buffers (4 x N columns each)
@@ -361,7 +481,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
         for (uint32_t i = 0; i < kMaxSlots; ++i) {
             mbar_init(bar_at(smem + kRawFull + 8 * i), 1);
             mbar_init(bar_at(smem + kActFull + 8 * i), 1);
-            mbar_init(bar_at(smem + kEmpty + 8 * i), 4 + 4);   // the step's unpack warps and epilogue (which comes after the tensor core)
+            mbar_init(bar_at(smem + kEmpty + 8 * i), F == FMT_Q4_K ? 4 + 4 : 4 + 8);   // the step's unpack warps and epilogue (which comes after the tensor core)
         }
         for (uint32_t i = 0; i < 2; ++i) { mbar_init(bar_at(smem + kAFull + 8 * i), 4); mbar_init(bar_at(smem + kAEmpty + 8 * i), 1); }
         for (uint32_t i = 0; i < (uint32_t)R; ++i) { mbar_init(bar_at(smem + kDFull + 8 * i), 1); mbar_init(bar_at(smem + kDEmpty + 8 * i), 4); }
@@ -381,14 +501,14 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
     Walk wk = walk_begin(a);
     Piece pc;
     Ring st{0, 0};   // the stage ring
-    auto step_on = [&]() { if (++st.slot == kSlots<T>) { st.slot = 0; st.par ^= 1u; } };
+    auto step_on = [&]() { if (++st.slot == kSlots<F, T>) { st.slot = 0; st.par ^= 1u; } };
     bool dead = false;
     // after an abort: waits for the copies in flight, those of the last n steps of the ring's barriers at `full`
     auto drain = [&](uint32_t full, uint32_t n) {
-        for (uint32_t k = 0; dead && k < min(n, kSlots<T>); ++k) {
+        for (uint32_t k = 0; dead && k < min(n, kSlots<F, T>); ++k) {
             const uint32_t i = n - 1 - k;
             const uint64_t t0 = globaltimer_ns();
-            while (!bar_try(smem + full + 8 * (i % kSlots<T>), (i / kSlots<T>) & 1u) && globaltimer_ns() - t0 < kDefaultWaitNs) {}
+            while (!bar_try(smem + full + 8 * (i % kSlots<F, T>), (i / kSlots<F, T>) & 1u) && globaltimer_ns() - t0 < kDefaultWaitNs) {}
         }
     };
 
@@ -403,11 +523,19 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
         while (!dead && walk_next(a, wk, pc)) {
             for (uint32_t blk = pc.b0; blk < pc.b1; ++blk, turn ^= 1u) {
                 if (turn != wg) { step_on(); continue; }
-                const uint32_t raw = stages + st.slot * kSlot<T>;
+                const uint32_t raw = stages + st.slot * kSlot<F, T>;
                 if (!warp_wait(smem + kRawFull + 8 * st.slot, st.par, a.status, abort_flag) ||
                     !warp_wait(smem + kAEmpty + 8 * wg, par, a.status, abort_flag)) { dead = true; break; }
                 fence_after();
-                unpack_q4k(raw + (quad * 32 + lane) * kPitch, tmem + ((quad * 32) << 16) + kACol + wg * kABuf);
+                const uint32_t tm = tmem + ((quad * 32) << 16) + kACol + wg * kABuf;
+                if (F == FMT_Q4_K) unpack_q4k(raw + (quad * 32 + lane) * pitch_of(F), tm);
+                else
+#pragma unroll 1
+                    for (uint32_t h = 0; h < 2; ++h) {
+                        const uint32_t r0 = raw + (quad * 32 + 16 * h + (lane >> 2)) * pitch_of(F) + ((blk * 210u) & 15u);
+                        if (blk & 1u) unpack_q6k<true>(r0 - 2, lane & 3u, tm + (h << 20));
+                        else unpack_q6k<false>(r0, lane & 3u, tm + (h << 20));
+                    }
                 tm_wait_st();
                 fence_before();
                 __syncwarp();
@@ -439,11 +567,12 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
 #pragma unroll
             for (int i = 0; i < T / 2; ++i) acc[i] = f2(0.f);
             for (uint32_t blk = pc.b0; blk < pc.b1; ++blk) {
-                const uint32_t raw = stages + st.slot * kSlot<T>, side = raw + kRows * kPitch + T * 1024u;
-                if (turn++ % 2 != half) { step_on(); continue; }
+                const uint32_t raw = stages + st.slot * kSlot<F, T>, side = raw + kRows * pitch_of(F) + T * 1024u;
+                if (F == FMT_Q4_K && turn++ % 2 != half) { step_on(); continue; }
                 if (!warp_wait(smem + kRawFull + 8 * st.slot, st.par, a.status, abort_flag) ||
                     !warp_wait(smem + kActFull + 8 * st.slot, st.par, a.status, abort_flag) ||
-                    !epi_step<T, R>(e, d, lane, raw + row * kPitch, side, acc)) { dead = true; break; }
+                    !(F == FMT_Q4_K ? epi_step_q4k<T, R>(e, d, lane, raw + row * pitch_of(F), side, acc)
+                                    : epi_step_q6k<T, R>(e, d, half, lane, raw + row * pitch_of(F), (blk * 210u) & 15u, side, acc))) { dead = true; break; }
                 __syncwarp();
                 if (lane == 0) bar_arrive(smem + kEmpty + 8 * st.slot);
                 step_on();
@@ -501,12 +630,13 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
                     if (!one_wait(smem + kEmpty + 8 * st.slot, st.par, a.status, abort_flag)) { dead = true; break; }
                     fence_proxy_async_smem();
                     uint64_t *full = bar_at(smem + kRawFull + 8 * st.slot);
-                    mbar_arrive_expect_tx(full, kRows * kPitch);
+                    mbar_arrive_expect_tx(full, kRows * pitch_of(F));
+                    const uint32_t x = F == FMT_Q4_K ? blk * 18u : ((blk * 210u) & ~15u) / 8;
                     // rows past the end of the tensor arrive as zeros
                     asm volatile(
                         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                            stages + st.slot * kSlot<T>),
-                        "l"(map), "r"(blk * 18u), "r"(pc.tile * kRows), "r"(smem_u32(full))
+                            stages + st.slot * kSlot<F, T>),
+                        "l"(map), "r"(x), "r"(pc.tile * kRows), "r"(smem_u32(full))
                         : "memory");
                     step_on();
                 }
@@ -519,19 +649,27 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
         auto wait = [&](uint32_t bar, uint32_t parity) { return warp_wait(bar, parity, a.status, abort_flag); };
         while (!dead && walk_next(a, wk, pc)) {
             for (uint32_t blk = pc.b0; blk < pc.b1; ++blk) {
-                Ring &r = d[buf];
-                if (!wait(smem + kDEmpty + 8 * r.slot, r.par) || !wait(smem + kActFull + 8 * st.slot, st.par) || !wait(smem + kAFull + 8 * buf, apar)) { dead = true; break; }
+                if (!wait(smem + kActFull + 8 * st.slot, st.par) || !wait(smem + kAFull + 8 * buf, apar)) { dead = true; break; }
                 fence_after();
-                const uint64_t b = b_desc(__shfl_sync(0xffffffffu, stages + st.slot * kSlot<T> + kRows * kPitch, 0));   // (uniform)
-                const uint32_t at = __shfl_sync(0xffffffffu, tmem + kACol + buf * kABuf, 0), dt = __shfl_sync(0xffffffffu, tmem + kDCol + r.slot * (256 / R), 0);
-                if (elect_one()) {
-                    tensor_step<2 * T>(at, b, dt);
-                    tm_commit(smem + kDFull + 8 * r.slot);
-                    tm_commit(smem + kAEmpty + 8 * buf);
+                const uint64_t b = b_desc(__shfl_sync(0xffffffffu, stages + st.slot * kSlot<F, T> + kRows * pitch_of(F), 0));   // (uniform)
+                const uint32_t at = __shfl_sync(0xffffffffu, tmem + kACol + buf * kABuf, 0);
+#pragma unroll
+                for (int u = 0; u < 16; u += F == FMT_Q4_K ? 16 : 4) {
+                    Ring &r = d[F == FMT_Q4_K ? buf : (u >> 2) & 1];
+                    if (!wait(smem + kDEmpty + 8 * r.slot, r.par)) { dead = true; break; }
+                    fence_after();
+                    const uint32_t dt = __shfl_sync(0xffffffffu, tmem + kDCol + r.slot * (256 / R), 0);
+                    if (elect_one()) {
+                        tensor_unit<F, 2 * T>(at, b, dt, u);
+                        tm_commit(smem + kDFull + 8 * r.slot);
+                    }
+                    __syncwarp();
+                    if (R == 2) r.par ^= 1u;
+                    else if ((++r.slot & 1u) == 0) { r.slot -= 2; r.par ^= 1u; }
                 }
+                if (dead) break;
+                if (elect_one()) tm_commit(smem + kAEmpty + 8 * buf);
                 __syncwarp();
-                if (R == 2) r.par ^= 1u;
-                else if ((++r.slot & 1u) == 0) { r.slot -= 2; r.par ^= 1u; }
                 buf ^= 1u;
                 if (!buf) apar ^= 1u;
                 step_on();
@@ -553,7 +691,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
                 if (!one_wait(smem + kEmpty + 8 * st.slot, st.par, a.status, abort_flag)) { dead = true; break; }
                 fence_proxy_async_smem();
                 mbar_arrive_expect_tx(bar_at(smem + kActFull + 8 * st.slot), T * 1064u);
-                bulk_g2s_addr(stages + st.slot * kSlot<T> + kRows * kPitch, a.xq + (size_t)blk * (T * 1064u), T * 1064u, bar_at(smem + kActFull + 8 * st.slot));
+                bulk_g2s_addr(stages + st.slot * kSlot<F, T> + kRows * pitch_of(F), a.xq + (size_t)blk * (T * 1064u), T * 1064u, bar_at(smem + kActFull + 8 * st.slot));
                 step_on();
             }
         }
@@ -577,7 +715,7 @@ bool tm_plan(const NxTensor *t, int n, uint32_t cols, bool split, TmPlan &p) {
     const uint32_t nblk = cols / 256;
     uint64_t tiles = 0;
     for (int i = 0; i < n; ++i) {
-        if (t[i].fmt != FMT_Q4_K || t[i].rows == 0) return false;
+        if ((t[i].fmt != FMT_Q4_K && t[i].fmt != FMT_Q6_K) || t[i].fmt != t[0].fmt || t[i].rows == 0) return false;
         tiles += (t[i].rows + kRows - 1) / kRows;
     }
     if (tiles * nblk >= (1ull << 24)) return false;   // (shares are formed in 32 bits)
@@ -608,7 +746,7 @@ bool matmul_umma_on(void) {
 // against 18.0 us, and 3 us for the planes).
 bool matmul_tm_takes(const NxTensor *t, int n, uint32_t cols, uint32_t P) {
     TmPlan p;
-    return P > 4 && tm_plan(t, n, cols, true, p) && p.grid == kTmCtas && p.steps >= 8 * kTmCtas;
+    return P > 4 && tm_plan(t, n, cols, true, p) && p.grid == kTmCtas && p.steps >= (P > 8 ? 3 : 8) * kTmCtas;
 }
 
 uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, bool split) {
@@ -616,9 +754,15 @@ uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, bool split) {
     return tm_plan(t, n, cols, split, p) ? p.parts : 0;
 }
 
+static const struct { void (*k)(const TmArgs); uint32_t smem; } kTmKernels[2][2] = {
+    {{matmul_tm_kernel<FMT_Q4_K, 8>, head_of(8) + kSlots<FMT_Q4_K, 8> * kSlot<FMT_Q4_K, 8>}, {matmul_tm_kernel<FMT_Q4_K, 16>, head_of(16) + kSlots<FMT_Q4_K, 16> * kSlot<FMT_Q4_K, 16>}},
+    {{matmul_tm_kernel<FMT_Q6_K, 8>, head_of(8) + kSlots<FMT_Q6_K, 8> * kSlot<FMT_Q6_K, 8>}, {matmul_tm_kernel<FMT_Q6_K, 16>, head_of(16) + kSlots<FMT_Q6_K, 16> * kSlot<FMT_Q6_K, 16>}}};
+
 cudaError_t matmul_tm_init(void) {
-    const cudaError_t e = cudaFuncSetAttribute(matmul_tm_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(matmul_tm_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
+    for (const auto &row : kTmKernels)
+        for (const auto &k : row)
+            if (const cudaError_t e = cudaFuncSetAttribute(k.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem)) return e;
+    return cudaSuccess;
 }
 
 cudaError_t launch_tm_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,
@@ -632,15 +776,15 @@ cudaError_t launch_tm_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t 
         TmT &d = k.t[i];
         d.y = t[i].y; d.part_stride = t[i].part_stride; d.rows = t[i].rows; d.ystride = t[i].ystride;
         d.base = base;
-        const uint32_t pitch = t[i].pitch ? t[i].pitch : (uint32_t)row_bytes(FMT_Q4_K, cols);
-        const cudaError_t e = tensor_map_2d(&k.map[i], 8, t[i].w, pitch / 8, t[i].rows, pitch, kPitch / 8, kRows, false);
+        const uint32_t pitch = t[i].pitch ? t[i].pitch : (uint32_t)row_bytes(t[i].fmt, cols);
+        const cudaError_t e = tensor_map_2d(&k.map[i], 8, t[i].w, pitch / 8, t[i].rows, pitch, pitch_of(t[i].fmt) / 8, kRows, false);
         if (e != cudaSuccess) return e;
         base += (t[i].rows + kRows - 1) / kRows * (cols / 256);
     }
     k.n = n; k.steps = p.steps; k.nblk = cols / 256; k.P = P; k.parts = p.parts; k.whole = split ? 0 : 1;
     k.xq = xq; k.accumulate = accumulate; k.rms = in.wnorm ? 1 : 0; k.eps = in.eps; k.status = status;
-    if (P > 8) return launch_kernel(matmul_tm_kernel<16>, dim3(p.grid), dim3(kThreads), head_of(16) + kSlots<16> * kSlot<16>, stream, pdl, k);
-    return launch_kernel(matmul_tm_kernel<8>, dim3(p.grid), dim3(kThreads), head_of(8) + kSlots<8> * kSlot<8>, stream, pdl, k);
+    const auto &kernel = kTmKernels[t[0].fmt == FMT_Q6_K][P > 8];
+    return launch_kernel(kernel.k, dim3(p.grid), dim3(kThreads), kernel.smem, stream, pdl, k);
 }
 
 } // namespace flb

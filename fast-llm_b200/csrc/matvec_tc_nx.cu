@@ -208,7 +208,7 @@ struct ConvArgs {
     uint32_t list_stride, col_off;
     const float *att;              // the columns are attention contexts of heads of 128, added up here from n_splits records
     uint32_t n_splits;             // (attn.cu: [column][head][split][132] = context, maximum, sum)
-    int tm;                        // img4 is the image of matmul_tm.cu
+    int tm;                        // img4 or img6 is the image of matmul_tm.cu
 };
 // Device-side table of a grouped launch: word 0 = number of active groups, word 1 = the most token groups of one; then four
 // words per active group: {group, number of columns, token groups in front of it, columns in front of it}.
@@ -323,14 +323,26 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     if (a.tm) {
         // Image of a block for NT = 8 or 16 tokens (matmul_tm.cu): a tile per 64 columns of 2 NT rows of 128 bytes (row p the hi parts
         // of token p, row NT + p the lo parts; 16-byte piece j of a row at j ^ (row & 7), the 128-byte swizzle), then the
-        // sub-block sums [8][NT], the block scales [NT] and the sums of squares [NT]. Piece j: columns 4 j + {0, 2, 1, 3} of the
-        // first sub-block of the tile, then of the second. Rows of tokens that there are not are never written nor used.
+        // sub-block sums [8][NT], the block scales [NT] and the sums of squares [NT]. Q4_K, piece j: columns 4 j + {0, 2, 1, 3} of
+        // the first sub-block of the tile, then of the second. Q6_K, tile 2 hf + hq, pieces 2 gq and 2 gq + 1: columns c, c + 2
+        // and c + 1, c + 3 for c = 128 hf + 32 gq + 16 hq + 4 t, t = 0 .. 3. Rows of tokens that there are not are never written
+        // nor used.
         if (p >= n_valid) return;
         const uint32_t NT = n_valid > 8 ? 16u : 8u;
-        uint8_t *img = a.img4 + (size_t)blk * (NT * 1064u), *row = img + (i >> 4) * (NT * 256) + p * 128;
-        const uint32_t piece = (((i & 7u) ^ (p & 7u)) << 4) + (i & 8u);   // (NT is a multiple of 8: both rows swizzle alike)
-        *reinterpret_cast<uint2 *>(row + piece) = hi;
-        *reinterpret_cast<uint2 *>(row + NT * 128 + piece) = lo;
+        uint8_t *img = (a.img4 ? a.img4 : a.img6) + (size_t)blk * (NT * 1064u);
+        // (NT is a multiple of 8: the rows of both parts swizzle alike)
+        if (a.img4) {
+            uint8_t *row = img + (i >> 4) * (NT * 256) + p * 128 + (((i & 7u) ^ (p & 7u)) << 4) + (i & 8u);
+            *reinterpret_cast<uint2 *>(row) = hi;
+            *reinterpret_cast<uint2 *>(row + NT * 128) = lo;
+        } else {
+            uint8_t *row = img + ((i >> 5) * 2 + ((i >> 2) & 1u)) * (NT * 256) + p * 128 + 4 * (i & 3u);
+            const uint32_t j = 2 * ((i >> 3) & 3u), j0 = (j ^ (p & 7u)) << 4, j1 = ((j + 1) ^ (p & 7u)) << 4;
+            *reinterpret_cast<uint32_t *>(row + j0) = hi.x;
+            *reinterpret_cast<uint32_t *>(row + j1) = hi.y;
+            *reinterpret_cast<uint32_t *>(row + NT * 128 + j0) = lo.x;
+            *reinterpret_cast<uint32_t *>(row + NT * 128 + j1) = lo.y;
+        }
         float *side = reinterpret_cast<float *>(img + NT * 1024);
         if ((i & 7u) == 0) side[(i >> 3) * NT + p] = sum;
         if (i == 0) { side[8 * NT + p] = scale; side[9 * NT + p] = h0.y + h1.y; }
@@ -1033,7 +1045,7 @@ cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t
     c.x = in.x; c.x2 = in.x2; c.part_stride = in.part_stride; c.resid = in.resid; c.x_out = in.x_out; c.wnorm = in.wnorm;
     c.xstride = in.xstride; c.rstride = in.rstride; c.n_parts = in.n_parts ? in.n_parts : 1; c.P = P; c.nblk = cols / 256;
     c.tm = in.tm;
-    if (in.tm && (q6 || q8 || in.table)) return cudaErrorNotSupported;
+    if (in.tm && (q8 || q4 == q6 || in.table)) return cudaErrorNotSupported;
     if (q4) c.img4 = xq;
     if (q6) c.img6 = xq + nx_image_off(FMT_Q6_K, q4, q6, cols, tgs_cap);
     if (q8) c.img8 = xq + nx_image_off(FMT_Q8_0, q4, q6, cols, tgs_cap);
