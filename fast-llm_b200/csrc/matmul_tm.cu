@@ -1,4 +1,4 @@
-// Several activation columns in one pass over Q4_K tensors on the Blackwell tensor cores: tcgen05.mma with the unpacked
+// Several activation columns in one pass over Q4_K or Q6_K tensors on the Blackwell tensor cores: tcgen05.mma with the unpacked
 // weights (A) and the results (D) in tensor memory, the activation (B) in shared memory. The same job as matvec_tc_nx.cu
 // (Y[p][r] (+)= dot(W[r], X[p]), p < P <= 16; the STREAM_DOT semantics of Task::nx, include/fastllm/fastllm.h:87-96), whose
 // tensor instructions bring every 16 x 16 weights into registers once per 4 tokens: the more tokens and the larger the tensor,
@@ -10,16 +10,17 @@
 // are reproducible run to run.
 //
 // Roles of a CTA (20 warps), all coupled by mbarriers:
-//   unpack (2 x 4 warps)   : every other step each; thread = row: packed bytes -> f16, written to tensor memory (tcgen05.st 32x32b)
-//   epilogue (2 x 4 warps) : every other step each; thread = row: D out of tensor memory, scales and mins, sum over the steps in
-//                            f32; the second hands its sums to the first at the end of a tile, which writes the results
-//   weights (1 thread)     : the packed bytes of a step, one TMA box of 128 rows x 144 bytes, into a ring of stages
+//   unpack (2 x 4 warps)   : every other step each: packed bytes -> f16, written to tensor memory (Q4_K: thread = row)
+//   epilogue (2 x 4 warps) : every other step (Q6_K: every other four results) each; thread = row: D out of tensor memory, scales
+//                            and mins, sum over the steps in f32; the second hands its sums to the first at the end of a tile, which writes the results
+//   weights (1 thread)     : the packed bytes of a step, one TMA box of 128 rows, into a ring of stages
 //   activation (1 thread)  : the step's B operand (one bulk copy of the image that act_convert_nx_kernel built), same ring
 //   tensor (1 warp)        : 16 instructions (M 128, N 2 x 8 or 2 x 16 tokens as (hi, lo), K 16) per step
 // Every wait is bounded; a wait that runs out sets the status word and an abort flag all roles watch, the launch then drains,
 // frees its tensor memory and returns.
 //
-// Arithmetic as in matvec_tc_nx.cu: (q - 8) sc as exact f16, activation of 22 bits per 256-column block, chains of four
+// Arithmetic as in matvec_tc_nx.cu. Q6_K: q - 32 as f16, an instruction per scale group, scaled in f32 by the epilogue. Q4_K:
+// (q - 8) sc as exact f16, activation of 22 bits per 256-column block, chains of four
 // instructions (64 columns) from zero, added with rounding: tcgen05.mma truncates its running sum exactly as mma.sync does (bias of
 // a chain of 4: -5.4e-8 of the result with either, of 16: -2.1e-7). The mins: 8 d sc - dmin m of a sub-block, rounded once, times
 // the sub-block's f32 sum.
@@ -27,7 +28,9 @@
 // What bounds it (B200): issue slots. A step takes 2600 warp instructions besides the polls (324 per 16 rows; matvec_tc_nx.cu 413 for 8
 // tokens, 560 for 16), over four schedulers at 0.6 a cycle; the tensor pipe is 9 % busy (an instruction takes 15 cycles for N 16, 20
 // for N 32, with A in tensor memory; 40 with A in shared memory), the weights arrive at 5.9 TB/s when nothing else is done.
-// 28672 x 4096 with its conversion: 25.8 us for 8 tokens and 34.9 for 16 (matvec_tc_nx.cu: 28.3 and 40.5); 2 tokens 23.9 (23.4).
+// 28672 x 4096 Q4_K with its conversion: 25.8 us for 8 tokens and 34.9 for 16 (matvec_tc_nx.cu: 28.3 and 40.5); 2 tokens 23.9 (23.4).
+// Inside a pass more, since the activation arrives beside the weights instead of in front of them (70 KB per CTA): 8B shape, 16 tokens
+// 4207 us with matvec_tc_nx.cu throughout, 3886 with gate | up, 3844 with O and 3626 with down (Q6_K) in this form too.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -741,9 +744,9 @@ bool matmul_umma_on(void) {
 
 // Whether a launch whose planes are added on the fly takes this form. Time = start + steps per CTA x time of one, conversion included:
 // 8 tokens 8.9 + 0.70 us against 7.9 + 0.84 (matvec_tc_nx.cu), 16 tokens 11.4 + 0.97 against 9.2 + 1.29, equal at 7 steps per CTA.
-// Up to 4 tokens the other kernel needs half its tensor instructions and is the faster one (28672 x 4096, 2 tokens: 23.4
-// against 23.9 us). Calls whose planes would take a launch of their own to add don't take it (14336 x 4096, 8 tokens: 17.4
-// against 18.0 us, and 3 us for the planes).
+// Inside a pass of 16 tokens O (3.5 steps per CTA) gains 1.3 us a layer all the same, of 8 nothing. Up to 4 tokens the other kernel
+// needs half its tensor instructions and is the faster one (28672 x 4096, 2 tokens: 23.4 against 23.9 us). Calls whose planes
+// would take a launch of their own to add don't take it (14336 x 4096, 8 tokens: 17.4 against 18.0 us, and 3 us for the planes).
 bool matmul_tm_takes(const NxTensor *t, int n, uint32_t cols, uint32_t P) {
     TmPlan p;
     return P > 4 && tm_plan(t, n, cols, true, p) && p.grid == kTmCtas && p.steps >= (P > 8 ? 3 : 8) * kTmCtas;
