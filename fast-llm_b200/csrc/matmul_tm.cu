@@ -745,11 +745,13 @@ bool matmul_umma_on(void) {
 // Whether a launch whose planes are added on the fly takes this form. Time = start + steps per CTA x time of one, conversion included:
 // 8 tokens 8.9 + 0.70 us against 7.9 + 0.84 (matvec_tc_nx.cu), 16 tokens 11.4 + 0.97 against 9.2 + 1.29, equal at 7 steps per CTA.
 // Inside a pass of 16 tokens O (3.5 steps per CTA) gains 1.3 us a layer all the same, of 8 nothing. Up to 4 tokens the other kernel
-// needs half its tensor instructions and is the faster one (28672 x 4096, 2 tokens: 23.4 against 23.9 us). Calls whose planes
+// needs half its tensor instructions and is the faster one alone (28672 x 4096, 2 tokens: 23.4 against 23.9 us), but not inside a pass
+// (8B shape over 4096 keys, 2 / 3 / 4 tokens: 2968 / 3015 / 3060 us with it, 2938 / 2979 / 3048 with this form; 16 layers of it in
+// Q4_K over 512, 2 / 4 tokens: 1373 / 1394 and 1332 / 1350). Calls whose planes
 // would take a launch of their own to add don't take it (14336 x 4096, 8 tokens: 17.4 against 18.0 us, and 3 us for the planes).
 bool matmul_tm_takes(const NxTensor *t, int n, uint32_t cols, uint32_t P) {
     TmPlan p;
-    return P > 4 && tm_plan(t, n, cols, true, p) && p.grid == kTmCtas && p.steps >= (P > 8 ? 3 : 8) * kTmCtas;
+    return P > 1 && tm_plan(t, n, cols, true, p) && p.grid == kTmCtas && p.steps >= (P > 8 ? 3 : 8) * kTmCtas;
 }
 
 uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, bool split) {

@@ -40,7 +40,7 @@ def test_whole_tiles(ctx, monkeypatch, rows, cols, nx):
     assert torch.equal(y[:, rows:].double(), want[:, rows:])
 
 
-@pytest.mark.parametrize("m", [4, 5, 8, 9, 16])
+@pytest.mark.parametrize("m", [2, 4, 5, 8, 9, 16])
 @pytest.mark.parametrize("recipe,n_embd,n_ff", [("Q4_K", 4096, 14336), ("Q4_K", 2048, 9472), ("Q4_K", 4096, 4864), ("Q4_K_M", 4096, 14336)])
 def test_batch_pass(recipe, n_embd, n_ff, m):
     """Gate | up (two planes) and, where it is large enough, down (six planes): 9472 x 2 rows of 2048 columns are the fewest steps
