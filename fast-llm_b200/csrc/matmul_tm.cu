@@ -547,6 +547,9 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
                 step_on();
             }
         }
+        // The last arrival at the barrier of this group's weights, which nothing else waits for: it must not be in flight when the
+        // CTA gives its shared memory up to the next one, which may be there already (a programmatic dependent).
+        if (!dead) warp_wait(smem + kAEmpty + 8 * wg, par, a.status, abort_flag);
     } else if (warp < kLoadWarp) {
         // ---- epilogue ----
         const uint32_t quad = warp & 3u, row = quad * 32 + lane;

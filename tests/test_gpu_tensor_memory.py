@@ -40,6 +40,30 @@ def test_whole_tiles(ctx, monkeypatch, rows, cols, nx):
     assert torch.equal(y[:, rows:].double(), want[:, rows:])
 
 
+@pytest.mark.parametrize("nx", [8, 16])
+def test_launches_in_a_row(ctx, monkeypatch, nx):
+    """Launches whose CTAs have one to five steps, one behind the other without a wait between them: a CTA waits for the last
+    arrival at the barrier of either weight buffer (an odd number of steps leaves the second one phase behind, one step never
+    uses it) before the next CTA sets up its own in the same memory. A wait on the wrong phase runs out and says so in the
+    status; a missing one shows by reading only."""
+    monkeypatch.setenv("FLB_UMMA", "1")
+    rows, cols = 148 * 128, 256
+    w = torch.from_numpy(synth.quant_tensor(capi.Q4_K, np.random.default_rng(nx), 5 * rows, cols)).cuda()
+    f = torch.empty((5 * rows, cols), device="cuda")
+    x = torch.randn((nx, cols), device="cuda", generator=torch.Generator(device="cuda").manual_seed(nx))
+    ys = [torch.zeros((nx, k * rows), device="cuda") for k in range(1, 6)]
+    torch.cuda.synchronize()
+    ctx.dequant(capi.Q4_K, w, 5 * rows, cols, f)
+    for _ in range(6):
+        for k, y in enumerate(ys, 1):
+            ctx.matvec(capi.Q4_K, w, k * rows, cols, x, y, nx=nx, xstride=cols, ystride=k * rows)
+    ctx.sync()
+    assert ctx.status() == 0
+    want = 6 * (x.double() @ f.double().T)
+    for k, y in enumerate(ys, 1):
+        assert float((y.double() - want[:, :k * rows]).abs().max() / want.pow(2).mean().sqrt()) <= 1e-5, k
+
+
 @pytest.mark.parametrize("m", [2, 4, 5, 8, 9, 16])
 @pytest.mark.parametrize("recipe,n_embd,n_ff", [("Q4_K", 4096, 14336), ("Q4_K", 2048, 9472), ("Q4_K", 4096, 4864), ("Q4_K_M", 4096, 14336)])
 def test_batch_pass(recipe, n_embd, n_ff, m):
