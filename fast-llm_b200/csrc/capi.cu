@@ -251,7 +251,7 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
             in.x = x + (size_t)p0 * xstride; in.xstride = xstride;
             if (x2) in.x2 = x2 + (size_t)p0 * xstride;
             cudaError_t e = cudaSuccess;
-            in.tm = umma && fmt == FL_B200_Q4_K && matmul_tm_parts(&t, 1, cols, false) == 1;
+            in.tm = umma && fmt == FL_B200_Q4_K && matmul_tm_parts(&t, 1, cols, false, c->sms) == 1;
             // the scratch holds these columns already: not with more of them than a chunk (it has the last one only), nor where
             // this call or the one before may be on the tcgen05 form, whose image is another one
             const bool reuse = same_columns && nx <= kNxMaxTokens && !umma;
@@ -261,7 +261,7 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
                 if (e != cudaSuccess) return cuda_err(e, "activation conversion launch");
             }
             if (in.tm) {
-                e = launch_tm_matmul(in, &t, 1, cols, nt, accumulate, c->xq, c->status, c->stream, true, false);
+                e = launch_tm_matmul(in, &t, 1, cols, nt, accumulate, c->xq, c->status, c->sms, c->stream, true, false);
                 if (e != cudaSuccess) return cuda_err(e, "multi-column matmul launch");
                 first_single = p0 + nt;
                 continue;

@@ -727,7 +727,7 @@ static bool nx_eligible(const fl_b200_decoder *d, uint32_t *planes) {
             if ((d->moe[l] && (g == 2 || g == 3)) || (g == 4 && l > 0)) continue;
             const int n = nx_group(d, l, g, t, &cols);
             for (uint32_t m = 1; m <= FL_B200_MAX_BATCH; ++m) {
-                const uint32_t parts = matmul_tc_nx_parts(t, n, cols, m, g != 4, true);
+                const uint32_t parts = matmul_tc_nx_parts(t, n, cols, m, g != 4, d->ctx->sms);
                 if (parts == 0) return false;
                 planes[g] = std::max(planes[g], parts);
             }
@@ -799,11 +799,11 @@ static int enqueue_batch_nx(fl_b200_decoder *d, uint32_t m, cudaStream_t s, bool
     };
     // one matvec group: convert the activation, walk the weights
     auto group = [&](const NxIn &from, const NxTensor *t, int n, uint32_t cols, uint32_t *parts, bool split = true) -> int {
-        *parts = matmul_tc_nx_parts(t, n, cols, m, split, true);
+        *parts = matmul_tc_nx_parts(t, n, cols, m, split, ctx->sms);
         NxIn in = from;
-        in.tm = split && matmul_tm_takes(t, n, cols, m);
+        in.tm = split && matmul_tm_takes(t, n, cols, m, ctx->sms);
         CK(launch_nx_convert(in, t, n, cols, m, ctx->xq, kNxTgs, s, pdl));
-        if (in.tm) CK(launch_tm_matmul(in, t, n, cols, m, 0, ctx->xq, ctx->status, s, pdl, true));
+        if (in.tm) CK(launch_tm_matmul(in, t, n, cols, m, 0, ctx->xq, ctx->status, ctx->sms, s, pdl, true));
         else CK(launch_nx_matmul(in, t, n, cols, m, 0, ctx->xq, kNxTgs, ctx->status, ctx->sms, s, pdl, split));
         return FL_B200_OK;
     };

@@ -93,6 +93,7 @@ cudaError_t matvec_tc_init(void);
 // (matvec_tc_nx.cu): y[p * ystride + r] (+)= dot(W[r], column p). Two launches: launch_nx_convert builds the activation's
 // operand image(s) in xq, launch_nx_matmul walks the weights.
 constexpr uint32_t kNxMaxTokens = 16, kNxMaxCols = 18432;
+constexpr uint32_t kMaxPlanes = 9;   // planes of partial results that the next conversion adds: no form may leave more
 constexpr uint32_t kAttnRecord = 132;   // floats of one split's record of one query head: context[128], maximum, sum, pad
 struct NxTensor {
     int fmt;
@@ -120,12 +121,12 @@ struct NxIn {
     const uint32_t *table, *col_idx, *out_idx;
     uint32_t list_stride, col_off, n_groups, n_experts;   // n_groups: upper bound of active experts
     int table_ready;         // 1: the table was complete before the kernel in front of the matmul started
-    int tm;                  // 1: launch_nx_convert builds the image of the form below (Q4_K only, not grouped)
+    int tm;                  // 1: launch_nx_convert builds the image of matmul_tm.cu (Q4_K or Q6_K, one format, not grouped)
 };
 // Number of parts the columns are cut into (1: y is the result; more: planes of partial sums); 0: not taken. split: planes cost the
 // caller nothing extra, cut as finely as is best.
-// tm: launches that matmul_tm_takes are cut as that form cuts them.
-uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split = false, bool tm = false);
+// tm_sms > 0: launches that matmul_tm_takes on so many SMs are cut as that form cuts them.
+uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split = false, int tm_sms = 0);
 // tgs: groups of four columns in the image(s) (grouped: of all active experts together)
 size_t matmul_tc_nx_scratch_bytes(uint32_t cols, uint32_t tgs, int layouts);
 // n = 0 tensors: only x_out is written. cudaErrorNotSupported: strides or addresses the vector loads do not take.
@@ -137,13 +138,13 @@ cudaError_t launch_reduce_parts(const float *part, size_t part_stride, uint32_t 
                                 uint32_t P, int accumulate, cudaStream_t stream, bool pdl);
 // The table of a grouped launch: of cnt[e] listed columns of expert e those from col_off on, at most P.
 cudaError_t launch_nx_table(const uint32_t *cnt, uint32_t n_local, uint32_t col_off, uint32_t P, uint32_t *table, cudaStream_t stream);
-// The same on tcgen05, weights and results in tensor memory (matmul_tm.cu): Q4_K, not grouped; between launch_nx_convert with
+// The same on tcgen05, weights and results in tensor memory (matmul_tm.cu): Q4_K or Q6_K, one format, not grouped; between launch_nx_convert with
 // in.tm set and the next conversion or reduction, as launch_nx_matmul. The image of 256 columns takes 8512 bytes up to 8 tokens,
 // else 17024: less than matmul_tc_nx_scratch_bytes provides.
-bool matmul_tm_takes(const NxTensor *t, int n, uint32_t cols, uint32_t P);   // launches with planes (split) for which it is the faster form
-uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, bool split);
+bool matmul_tm_takes(const NxTensor *t, int n, uint32_t cols, uint32_t P, int sms);   // launches with planes (split) for which it is the faster form
+uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, bool split, int sms);
 cudaError_t launch_tm_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,
-                             uint32_t *status, cudaStream_t stream, bool pdl, bool split);
+                             uint32_t *status, int sms, cudaStream_t stream, bool pdl, bool split);
 cudaError_t matmul_tm_init(void);
 bool matmul_umma_on(void);   // FLB_UMMA=1 in the environment now: every Q4_K call of several columns on that form
 cudaError_t matmul_tc_nx_init(void);

@@ -712,12 +712,13 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
     }
 }
 
-constexpr uint32_t kMaxParts = 8, kTmCtas = 148;
+constexpr uint32_t kMaxParts = 8;
+static_assert(kMaxParts <= kMaxPlanes, "planes");
 
-// The grid and the number of planes. A share of the line holds at least one step; with planes, no more than kMaxParts shares touch
+// The grid (a CTA per SM) and the number of planes. A share of the line holds at least one step; with planes, no more than kMaxParts shares touch
 // a tile: a tile's nblk steps start within nblk - 1 of each other, so that at most (nblk - 1) / share + 2 shares do.
 struct TmPlan { uint32_t grid, parts, steps; };
-bool tm_plan(const NxTensor *t, int n, uint32_t cols, bool split, TmPlan &p) {
+bool tm_plan(const NxTensor *t, int n, uint32_t cols, bool split, int sms, TmPlan &p) {
     const uint32_t nblk = cols / 256;
     uint64_t tiles = 0;
     for (int i = 0; i < n; ++i) {
@@ -727,11 +728,11 @@ bool tm_plan(const NxTensor *t, int n, uint32_t cols, bool split, TmPlan &p) {
     if (tiles * nblk >= (1ull << 24)) return false;   // (shares are formed in 32 bits)
     p.steps = (uint32_t)tiles * nblk;
     if (!split) {
-        p.grid = (uint32_t)std::min<uint64_t>(kTmCtas, tiles);
+        p.grid = (uint32_t)std::min<uint64_t>(sms, tiles);
         p.parts = 1;
         return true;
     }
-    p.grid = std::min(kTmCtas, p.steps);
+    p.grid = std::min((uint32_t)sms, p.steps);
     if (nblk > 1) p.grid = std::max(1u, std::min(p.grid, p.steps * (kMaxParts - 2) / (nblk - 1)));
     p.parts = p.grid == 1 ? 1 : std::min(kMaxParts, (nblk - 1) / (p.steps / p.grid) + 2);
     return true;
@@ -752,14 +753,14 @@ bool matmul_umma_on(void) {
 // (8B shape over 4096 keys, 2 / 3 / 4 tokens: 2968 / 3015 / 3060 us with it, 2938 / 2979 / 3048 with this form; 16 layers of it in
 // Q4_K over 512, 2 / 4 tokens: 1373 / 1394 and 1332 / 1350). Calls whose planes
 // would take a launch of their own to add don't take it (14336 x 4096, 8 tokens: 17.4 against 18.0 us, and 3 us for the planes).
-bool matmul_tm_takes(const NxTensor *t, int n, uint32_t cols, uint32_t P) {
+bool matmul_tm_takes(const NxTensor *t, int n, uint32_t cols, uint32_t P, int sms) {
     TmPlan p;
-    return P > 1 && tm_plan(t, n, cols, true, p) && p.grid == kTmCtas && p.steps >= (P > 8 ? 3 : 8) * kTmCtas;
+    return P > 1 && tm_plan(t, n, cols, true, sms, p) && p.grid == (uint32_t)sms && p.steps >= (P > 8 ? 3 : 8) * p.grid;
 }
 
-uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, bool split) {
+uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, bool split, int sms) {
     TmPlan p;
-    return tm_plan(t, n, cols, split, p) ? p.parts : 0;
+    return tm_plan(t, n, cols, split, sms, p) ? p.parts : 0;
 }
 
 static const struct { void (*k)(const TmArgs); uint32_t smem; } kTmKernels[2][2] = {
@@ -774,9 +775,9 @@ cudaError_t matmul_tm_init(void) {
 }
 
 cudaError_t launch_tm_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,
-                             uint32_t *status, cudaStream_t stream, bool pdl, bool split) {
+                             uint32_t *status, int sms, cudaStream_t stream, bool pdl, bool split) {
     TmPlan p;
-    if (in.table || P == 0 || P > kNxMaxTokens || !tm_plan(t, n, cols, split, p) || (accumulate && p.parts > 1)) return cudaErrorNotSupported;
+    if (in.table || P == 0 || P > kNxMaxTokens || !tm_plan(t, n, cols, split, sms, p) || (accumulate && p.parts > 1)) return cudaErrorNotSupported;
     TmArgs k;
     memset(&k, 0, sizeof(k));
     uint32_t base = 0;

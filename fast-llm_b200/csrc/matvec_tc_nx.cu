@@ -215,7 +215,8 @@ struct ConvArgs {
 
 // Four consecutive columns at p, the planes added in order; all of them are requested before the first is used.
 __device__ __forceinline__ float4 sum_planes(const float *p, uint32_t n, size_t stride) {
-    constexpr int kPlanes = (kNxMaxCols / 256 + 7) / 8;   // the most parts a matmul leaves
+    constexpr int kPlanes = kMaxPlanes;
+    static_assert((kNxMaxCols / 256 + 7) / 8 <= kMaxPlanes, "planes of the finest cut, one segment each");
     float4 v[kPlanes];
 #pragma unroll
     for (int s = 0; s < kPlanes; ++s) v[s] = (uint32_t)s < n ? *reinterpret_cast<const float4 *>(p + s * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1022,7 +1023,7 @@ size_t matmul_tc_nx_scratch_bytes(uint32_t cols, uint32_t tgs, int layouts) {
     return (size_t)(cols / 256) * tgs * (kXq4 + (layouts > 1 ? kXq6 : 0) + (layouts > 2 ? kXq6 : 0));
 }
 
-uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split, bool tm) {
+uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P, bool split, int tm_sms) {
     static const bool off = getenv("FLB_TC_NX") && getenv("FLB_TC_NX")[0] == '0';
     if (off || n < 1 || n > 3 || cols % 256 != 0 || cols < 256 || cols > kNxMaxCols || P == 0 || P > kNxMaxTokens) return 0;
     int fmts[3];
@@ -1030,7 +1031,7 @@ uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P,
         if (!nx_tensor_ok(t[i], cols)) return 0;
         fmts[i] = t[i].fmt;
     }
-    if (split && tm && matmul_tm_takes(t, n, cols, P)) return matmul_tm_parts(t, n, cols, true);
+    if (split && tm_sms && matmul_tm_takes(t, n, cols, P, tm_sms)) return matmul_tm_parts(t, n, cols, true, tm_sms);
     NxPlan p;
     return nx_plan(fmts, n, cols, (P + 3) / 4, split, p) ? p.parts : 0;
 }
