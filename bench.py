@@ -39,6 +39,8 @@ N_PREFILL = 8192
 METRIC = "decode tokens/s at 8B Q4_K_M shape, 1/2/4/8 B200; HBM GB/s % of roofline"
 
 
+MATMUL_CASES = {"matmul-nx8": ("Q4_K", 28672, 4096, 8), "matmul-nx16": ("Q4_K", 28672, 4096, 16),
+                "matmul-q6k-nx8": ("Q6_K", 4096, 14336, 8), "matmul-q6k-nx16": ("Q6_K", 4096, 14336, 16)}
 NCU_TRAFFIC_RATIO = 1.0057
 TIMED_REGION_MS = 1000.0   # device time the repeated K-step loops add up to, at least
 
@@ -233,9 +235,9 @@ def main():
                     help="device time the repeated K-step loops add up to, at least (0 = one repetition: profiler captures)")
     ap.add_argument("--layers", type=int, default=32,
                     help="number of layers (32 = the benchmark; fewer = a small case of the same kernels for profiler captures, not a benchmark number)")
-    ap.add_argument("--case", default="decode", choices=["decode", "matmul-nx8", "attn-long", "moe", "moe-decode"],
-                    help="decode = the benchmark (default). matmul-nx8 = the multi-column Q4_K matmul alone (gate|up shape, 8 "
-                         "columns); attn-long = decode attention alone at 32K / 64K / 128K keys; moe = the MoE feed-forward "
+    ap.add_argument("--case", default="decode", choices=["decode", *MATMUL_CASES, "attn-long", "moe", "moe-decode"],
+                    help="decode = the benchmark (default). matmul-* = one multi-column matmul alone (nx8, nx16: Q4_K, gate|up shape, 8 / 16 "
+                         "columns; q6k-nx8, q6k-nx16: Q6_K, down); attn-long = decode attention alone at 32K / 64K / 128K keys; moe = the MoE feed-forward "
                          "block at the Mixtral shape (8 experts, top-2, 16 tokens; expert parallel under torchrun); moe-decode = greedy "
                          "decode of a whole synthetic Mixtral-8x7B-shape model (32 layers, 8 experts, top-2) on one GPU: kernel "
                          "cases for profiler captures and sweeps, each prints its own JSON line and is not the benchmark number")
@@ -322,23 +324,26 @@ def kernel_case(case, steps, warmup):
     ctx = capi.Context(0)
     gen = torch.Generator(device="cuda")
     gen.manual_seed(1)
-    if case == "matmul-nx8":
-        rows, cols, nx, copies = 28672, 4096, 8, 3
-        w = [synth.device_quant_tensor(capi.Q4_K, rows, cols, gen) for _ in range(copies)]
+    if case in MATMUL_CASES:
+        fmt, rows, cols, nx = MATMUL_CASES[case]
+        fmt, copies = getattr(capi, fmt), 3
+        w = [synth.device_quant_tensor(fmt, rows, cols, gen) for _ in range(copies)]
         x = torch.randn((nx, cols), device="cuda", generator=gen)
         y = torch.zeros((nx, rows), device="cuda")
         torch.cuda.synchronize()
 
         def run(n):
             for i in range(n):
-                ctx.matvec(capi.Q4_K, w[i % copies], rows, cols, x, y, nx=nx, xstride=cols, ystride=rows)
+                ctx.matvec(fmt, w[i % copies], rows, cols, x, y, nx=nx, xstride=cols, ystride=rows)
         run(warmup)
         ctx.sync()
         ctx.timer_start()
         run(steps)
         us = ctx.timer_stop() * 1e3 / steps
-        nbytes = rows * capi.row_bytes(capi.Q4_K, cols)
-        print(json.dumps({"case": case, "kernel": "matmul_tm_kernel (tcgen05, FLB_UMMA=1)" if os.environ.get("FLB_UMMA", "")[:1] == "1" else "matmul_nx_kernel",
+        nbytes = rows * capi.row_bytes(fmt, cols)
+        form = os.environ.get("FLB_UMMA", "")[:1]   # 1: whole tiles (Q4_K), 2: shares and planes as in a batch pass
+        tm = form == "2" or (form == "1" and fmt == capi.Q4_K)
+        print(json.dumps({"case": case, "kernel": "matmul_tm_kernel (tcgen05, FLB_UMMA=%s)" % form if tm else "matmul_nx_kernel",
                           "rows": rows, "cols": cols, "columns": nx,
                           "us_per_pass": us, "weight_bytes": nbytes, "achieved_gbs": nbytes / us / 1e3,
                           "frac_of_measured_hbm": nbytes / us / 1e3 / peak, "status": ctx.status()}))
@@ -709,8 +714,7 @@ def measure(tp_mode, args, ctx, cfg, config, dist, gloo, rank, local_rank, world
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peak_kind == "measured" else "fallback 6.65 TB/s",
                      "unit": "GB/s", "frac": achieved / peak,
                      # dram__bytes_read.sum + dram__bytes_write.sum of the four matvec launch shapes in one ncu
-                     # capture (profiles/matvec_tc_kernel_8b_layer_shapes.md) were 1.0079 x their algorithmic
-                     # bytes; traffic grows in proportion to the weights streamed, so it is scaled to this launch mix
+                     # capture were 1.0057 x their algorithmic bytes; traffic grows in proportion to the weights streamed, so it is scaled to this launch mix
                      "traffic": NCU_TRAFFIC_RATIO * w_bytes / mv_n,
                      "bytes_per_launch": w_bytes / mv_n, "launches_per_step": mv_n, "avg_launch_us": mv_ms * 1e3 / mv_n,
                      "step": {"bytes": w_bytes + kv_bytes, "achieved": (w_bytes + kv_bytes) / (ms_dev / steps * 1e-3) / 1e9,

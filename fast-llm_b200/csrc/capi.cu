@@ -239,7 +239,7 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
     if (pitch == row_bytes(fmt, cols)) pitch = 0;   // packed rows
     uint32_t first_single = 0;   // columns from here on go through the one-column kernel
     if (nx >= 2 && (fmt == FL_B200_Q4_K || fmt == FL_B200_Q6_K || fmt == FL_B200_Q8_0) && !expert_id) {
-        const bool umma = matmul_umma_on();   // Q4_K on the tcgen05 form, whatever the shape
+        const int tm = matmul_tm_switch();   // 1, 2: on the tcgen05 form, whatever the shape
         // verify batches, prompt chunks: up to 16 columns per pass over the weights on the tensor cores
         for (uint32_t p0 = first_single; p0 < nx; p0 += kNxMaxTokens) {
             const uint32_t nt = nx - p0 < kNxMaxTokens ? nx - p0 : kNxMaxTokens;
@@ -251,32 +251,32 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
             in.x = x + (size_t)p0 * xstride; in.xstride = xstride;
             if (x2) in.x2 = x2 + (size_t)p0 * xstride;
             cudaError_t e = cudaSuccess;
-            in.tm = umma && fmt == FL_B200_Q4_K && matmul_tm_parts(&t, 1, cols, false, c->sms) == 1;
+            const bool planes = tm == 2 && fmt != FL_B200_Q8_0;
+            in.tm = (planes || (tm == 1 && fmt == FL_B200_Q4_K)) && matmul_tm_parts(&t, 1, cols, planes, c->sms) != 0;
             // the scratch holds these columns already: not with more of them than a chunk (it has the last one only), nor where
             // this call or the one before may be on the tcgen05 form, whose image is another one
-            const bool reuse = same_columns && nx <= kNxMaxTokens && !umma;
+            const bool reuse = same_columns && nx <= kNxMaxTokens && tm <= 0;
             if (!reuse) {
                 e = launch_nx_convert(in, &t, 1, cols, nt, c->xq, kNxTgs, c->stream, pdl != 0);
                 if (e == cudaErrorNotSupported) break;
                 if (e != cudaSuccess) return cuda_err(e, "activation conversion launch");
             }
-            if (in.tm) {
-                e = launch_tm_matmul(in, &t, 1, cols, nt, accumulate, c->xq, c->status, c->sms, c->stream, true, false);
-                if (e != cudaSuccess) return cuda_err(e, "multi-column matmul launch");
-                first_single = p0 + nt;
-                continue;
-            }
             // the matmul overlaps the conversion's launch: it reads weights only until the conversion has completed
-            const uint32_t cap = (uint32_t)(kNxPartFloats / ((size_t)parts * nt)) & ~15u, slice = parts == 1 || rows <= cap ? rows : cap;
+            const uint32_t most = !in.tm ? parts : planes ? kMaxPlanes : 1;   // (how many planes a slice leaves then depends on its rows)
+            const uint32_t cap = (uint32_t)(kNxPartFloats / ((size_t)most * nt)) & ~15u, slice = most == 1 || rows <= cap ? rows : cap;
             const size_t rb = pitch ? pitch : row_bytes(fmt, cols);
             for (uint32_t r0 = 0; r0 < rows; r0 += slice) {
                 NxTensor ts = t;
                 ts.w = (const uint8_t *)w + (size_t)r0 * rb;
                 ts.rows = std::min(slice, rows - r0);
-                if (parts > 1) { ts.y = c->nx_part; ts.ystride = ts.rows; ts.part_stride = (size_t)nt * ts.rows; }
-                e = launch_nx_matmul(in, &ts, 1, cols, nt, parts > 1 ? 0 : accumulate, c->xq, kNxTgs, c->status, c->sms, c->stream, true);
-                if (e == cudaSuccess && parts > 1)
-                    e = launch_reduce_parts(c->nx_part, ts.part_stride, parts, t.y + r0, ts.rows, ystride, nt, accumulate, c->stream, true);
+                const uint32_t n_parts = in.tm ? matmul_tm_parts(&ts, 1, cols, planes, c->sms) : parts;
+                const int acc = n_parts > 1 ? 0 : accumulate;
+                ts.y = t.y + r0;
+                if (n_parts > 1) { ts.y = c->nx_part; ts.ystride = ts.rows; ts.part_stride = (size_t)nt * ts.rows; }
+                e = in.tm ? launch_tm_matmul(in, &ts, 1, cols, nt, acc, c->xq, c->status, c->sms, c->stream, true, planes)
+                          : launch_nx_matmul(in, &ts, 1, cols, nt, acc, c->xq, kNxTgs, c->status, c->sms, c->stream, true);
+                if (e == cudaSuccess && n_parts > 1)
+                    e = launch_reduce_parts(c->nx_part, ts.part_stride, n_parts, t.y + r0, ts.rows, ystride, nt, accumulate, c->stream, true);
                 if (e != cudaSuccess) return cuda_err(e, "multi-column matmul launch");
             }
             first_single = p0 + nt;

@@ -107,6 +107,7 @@ struct fl_b200_decoder {
         // The pass over the multi-column kernel (nx): outputs as planes of partial sums (qkv: [planes][m][Q | K | V] rows; the
         // others [planes][m][rows]), the positions' rotation tables, argmax scratch and tickets per token.
         bool nx = false;
+        int tm_sms = 0;   // SMs that matmul_tm_takes is asked for (0: it is not)
         float *qkv = nullptr, *planes = nullptr, *gp = nullptr, *up = nullptr, *head = nullptr, *am = nullptr;
         uint32_t *am_tickets = nullptr;
         float2 *rope = nullptr;
@@ -718,7 +719,7 @@ static int nx_group(const fl_b200_decoder *d, uint32_t layer, int group, NxTenso
 
 // The pass runs on the multi-column kernel when it takes every tensor; then planes[g] is the most planes of partial results
 // any number of tokens leads to in group g.
-static bool nx_eligible(const fl_b200_decoder *d, uint32_t *planes) {
+static bool nx_eligible(const fl_b200_decoder *d, int tm_sms, uint32_t *planes) {
     NxTensor t[3];
     uint32_t cols;
     for (int g = 0; g < 5; ++g) planes[g] = 1;
@@ -727,7 +728,7 @@ static bool nx_eligible(const fl_b200_decoder *d, uint32_t *planes) {
             if ((d->moe[l] && (g == 2 || g == 3)) || (g == 4 && l > 0)) continue;
             const int n = nx_group(d, l, g, t, &cols);
             for (uint32_t m = 1; m <= FL_B200_MAX_BATCH; ++m) {
-                const uint32_t parts = matmul_tc_nx_parts(t, n, cols, m, g != 4, d->ctx->sms);
+                const uint32_t parts = matmul_tc_nx_parts(t, n, cols, m, g != 4, tm_sms);
                 if (parts == 0) return false;
                 planes[g] = std::max(planes[g], parts);
             }
@@ -746,8 +747,10 @@ static int batch_alloc(fl_b200_decoder *d) {
         for (const bool shared : {false, true})
             part = std::max(part, attn_part_floats(d->Hq, m, attn_pick_splits(d->Hkv, m, c.max_kv, d->ctx->sms, shared)));
     uint32_t pl[5];
-    // FLB_UMMA=1 sends the pass tensor by tensor, where Q4_K goes to the tcgen05 kernel
-    w.nx = !matmul_umma_on() && nx_eligible(d, pl);
+    // FLB_UMMA=1 and 2 send the pass tensor by tensor, every call to matmul_tm.cu; 0 keeps it off that form
+    const int sw = matmul_tm_switch();
+    w.tm_sms = sw == 0 ? 0 : d->ctx->sms;
+    w.nx = sw <= 0 && nx_eligible(d, w.tm_sms, pl);
     // one allocation for all buffers: a dozen of them were most of the time of a decoder's first pass
     size_t total = 0;
     auto layout = [&](auto &&take) {
@@ -799,9 +802,9 @@ static int enqueue_batch_nx(fl_b200_decoder *d, uint32_t m, cudaStream_t s, bool
     };
     // one matvec group: convert the activation, walk the weights
     auto group = [&](const NxIn &from, const NxTensor *t, int n, uint32_t cols, uint32_t *parts, bool split = true) -> int {
-        *parts = matmul_tc_nx_parts(t, n, cols, m, split, ctx->sms);
+        *parts = matmul_tc_nx_parts(t, n, cols, m, split, b.tm_sms);
         NxIn in = from;
-        in.tm = split && matmul_tm_takes(t, n, cols, m, ctx->sms);
+        in.tm = split && b.tm_sms && matmul_tm_takes(t, n, cols, m, b.tm_sms);
         CK(launch_nx_convert(in, t, n, cols, m, ctx->xq, kNxTgs, s, pdl));
         if (in.tm) CK(launch_tm_matmul(in, t, n, cols, m, 0, ctx->xq, ctx->status, ctx->sms, s, pdl, true));
         else CK(launch_nx_matmul(in, t, n, cols, m, 0, ctx->xq, kNxTgs, ctx->status, ctx->sms, s, pdl, split));

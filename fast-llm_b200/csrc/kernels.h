@@ -146,7 +146,9 @@ uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, bool split, in
 cudaError_t launch_tm_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,
                              uint32_t *status, int sms, cudaStream_t stream, bool pdl, bool split);
 cudaError_t matmul_tm_init(void);
-bool matmul_umma_on(void);   // FLB_UMMA=1 in the environment now: every Q4_K call of several columns on that form
+// FLB_UMMA in the environment now (-1: not set). 1: every Q4_K call of several columns on that form, whole tiles; 2: every Q4_K and
+// Q6_K call, with planes as in a batch pass; 0: no launch of a batch pass on it.
+int matmul_tm_switch(void);
 cudaError_t matmul_tc_nx_init(void);
 // True when launch_matvec would take the streaming kernel for this shape.
 bool matvec_is_streaming(int fmt, uint32_t cols);

@@ -740,10 +740,10 @@ bool tm_plan(const NxTensor *t, int n, uint32_t cols, bool split, int sms, TmPla
 
 } // namespace
 
-// FLB_UMMA=1 (read at every call, so that one process can run both kernels): every Q4_K call of several columns takes this form.
-bool matmul_umma_on(void) {
+// Read at every call, so that one process can run both kernels.
+int matmul_tm_switch(void) {
     const char *v = getenv("FLB_UMMA");
-    return v && v[0] == '1';
+    return v && v[0] >= '0' && v[0] <= '2' ? v[0] - '0' : -1;
 }
 
 // Whether a launch whose planes are added on the fly takes this form. Time = start + steps per CTA x time of one, conversion included:

@@ -1,12 +1,14 @@
-"""GPU tests of the multi-column matmul with the weights in tensor memory (csrc/matmul_tm.cu): by itself (FLB_UMMA=1 sends every
-Q4_K call of several columns there) at the edges of its tiles of 128 rows, steps of 256 columns and 8 / 16 tokens, and with its planes
-of partial sums in a batch pass whose FFN is large enough for it.
+"""GPU tests of the multi-column matmul with the weights in tensor memory (csrc/matmul_tm.cu): by itself, in whole tiles
+(FLB_UMMA=1 sends every Q4_K call of several columns there) and in the shares and planes of partial sums that a batch pass uses
+(FLB_UMMA=2, Q4_K and Q6_K), at the edges of its tiles of 128 rows, steps of 256 columns and 8 / 16 tokens; and in batch passes at
+the edges of the rule that picks it.
 
 Tolerance of a matmul as in test_gpu_multi_column.py (the sums are the same): 1e-5 of the root mean square of the exact result.
 Batch passes against single steps as in test_gpu_batch_forms.py: 5e-4 of the logits."""
 import numpy as np
 import pytest
 
+import test_gpu_multi_column as multi_column
 from fast_llm_b200 import capi, synth
 
 pytestmark = pytest.mark.gpu
@@ -38,6 +40,56 @@ def test_whole_tiles(ctx, monkeypatch, rows, cols, nx):
     err = (y.double() - want)[:, :rows].abs().amax(1) / want[:, :rows].pow(2).mean(1).sqrt()
     assert float(err.max()) <= 1e-5
     assert torch.equal(y[:, rows:].double(), want[:, rows:])
+
+
+@pytest.mark.parametrize("fmt,rows,cols,nx", [
+    (capi.Q4_K, 1, 256, 2), (capi.Q4_K, 129, 768, 9), (capi.Q4_K, 20000, 256, 16),    # one block: a tile is one CTA's
+    (capi.Q4_K, 28672, 4096, 8), (capi.Q4_K, 28672, 4096, 16), (capi.Q4_K, 300, 2304, 33),
+    (capi.Q6_K, 100, 2048, 2), (capi.Q6_K, 4096, 14336, 8), (capi.Q6_K, 4096, 14336, 16), (capi.Q6_K, 12801, 2048, 5),
+    (capi.Q4_K, 1024, 6144, 9), (capi.Q6_K, 1000, 6144, 3),                           # the most planes, 8
+    (capi.Q4_K, 64, 18432, 16), (capi.Q6_K, 200, 18432, 8),                           # the most columns
+    (capi.Q4_K, 131072, 4352, 16),                                                    # more rows than the planes hold: slices
+])
+def test_planes(ctx, monkeypatch, fmt, rows, cols, nx):
+    """Shares that cut tiles anywhere. The memory of the planes holds NaN before: a plane that a tile has no sums for is cleared."""
+    monkeypatch.setenv("FLB_UMMA", "2")
+    w = torch.from_numpy(synth.quant_tensor(capi.Q4_K, np.random.default_rng(1), 65536, 256)).cuda()
+    x, y = torch.full((16, 256), float("nan"), device="cuda"), torch.zeros((16, 65536), device="cuda")
+    torch.cuda.synchronize()
+    ctx.matvec(capi.Q4_K, w, 65536, 256, x, y, nx=16, xstride=256, ystride=65536)
+    ctx.sync()
+    assert torch.isnan(y).all()
+    multi_column.test_multi_column_edges(ctx, fmt, rows, cols, nx)
+
+
+@pytest.mark.parametrize("form,fmt", [("1", capi.Q4_K), ("2", capi.Q4_K), ("2", capi.Q6_K)])
+def test_special_values(ctx, monkeypatch, form, fmt):
+    monkeypatch.setenv("FLB_UMMA", form)
+    multi_column.test_multi_column_special_values(ctx, fmt)
+
+
+@pytest.mark.parametrize("rows,cols", [(4096, 4096), (4096, 14336)])
+@pytest.mark.parametrize("nx", [2, 8, 9, 16])
+@pytest.mark.parametrize("form,recipe", [("1", "Q4_K"), ("2", "Q4_K"), ("2", "Q6_K")])
+def test_sums_are_not_truncated(ctx, monkeypatch, form, recipe, nx, rows, cols):
+    """Bias and 2-norm of the error as test_gpu_multi_column.py asks them of the other kernel: tcgen05.mma truncates its running sum
+    as mma.sync does, so that the chains are as short."""
+    from perf import cases
+    monkeypatch.setenv("FLB_UMMA", form)
+    fmt = cases.FMT[recipe]
+    gen = torch.Generator(device="cuda").manual_seed(nx)
+    w = cases._weights(recipe, rows, cols, gen)
+    f = torch.empty((rows, cols), device="cuda")
+    x = torch.randn((nx, cols), device="cuda", generator=gen)
+    y = torch.zeros((nx, rows), device="cuda")
+    torch.cuda.synchronize()
+    ctx.dequant(fmt, w, rows, cols, f)
+    ctx.matvec(fmt, w, rows, cols, x, y, nx=nx, xstride=cols, ystride=rows)
+    ctx.sync()
+    want = x.double() @ f.double().T
+    bias, err = float((y.double() * want).sum() / want.pow(2).sum()) - 1, float((y.double() - want).norm() / want.norm())
+    assert abs(bias) <= 8e-8, bias
+    assert err <= 1.5e-7, err
 
 
 @pytest.mark.parametrize("nx", [8, 16])
@@ -88,3 +140,33 @@ def test_batch_pass(recipe, n_embd, n_ff, m):
         assert abs(margins[i] - dec.last_margin()) <= 2 * np.abs(got[i] - single).max() + 1e-6
     assert s["ctx"].status() == 0
     dec.close()
+
+
+@pytest.mark.parametrize("recipe,n_embd,n_ff,m,taken", [
+    ("Q4_K_M", 4096, 14336, 2, True), ("Q4_K_M", 4096, 14336, 8, True), ("Q4_K_M", 4096, 10240, 5, True),   # Q6_K down with few tokens
+    ("Q4_K_M", 4096, 4096, 9, True), ("Q4_K_M", 4096, 4096, 16, True), ("Q4_K_M", 4096, 4096, 8, False),     # O and down, from 9 on
+    ("Q4_K", 2048, 9472, 8, True), ("Q4_K", 2048, 9216, 8, False),   # 8 and 7.8 steps per CTA in gate | up
+    ("Q4_K", 1024, 7168, 9, True), ("Q4_K", 1024, 6912, 9, False),   # 3.03 and 2.9
+])
+def test_pass_with_and_without(monkeypatch, recipe, n_embd, n_ff, m, taken):
+    """The pass against itself with FLB_UMMA=0, on a layer whose Q, K and V go the same way in both: K and V are then the same
+    bits and no flipped f16 rounding covers anything, so that 1 / rms per token, the planes and both formats show as sums in another
+    order. O (from 9 tokens on), gate, up, down and the head, whose input then differs, are each 1.3e-7 off (2-norm) in either
+    form, independently: sqrt(10) of that is 4.1e-7, and a tenth more for the scatter from token to token (measured 3.7e-7). Launches
+    that the rule leaves to the other kernel: the same bits."""
+    from perf import cases
+    case = dict(kind="batch", pos=70, m=m, n_layer=1, n_embd=n_embd, n_kv_head=n_embd // 512, n_ff=n_ff, n_vocab=1000, recipe=recipe,
+                rope_base=500000.0)
+    logits = []
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("FLB_UMMA", "0")
+        s = cases.prepare(case, m)
+        s["dec"].rewind_to(70)
+        s["dec"].step_batch(s["tokens"])
+        logits.append(np.stack([s["dec"].batch_logits(i) for i in range(m)]).astype(np.float64))
+        assert s["ctx"].status() == 0
+        s["dec"].close()
+    diff = np.linalg.norm(logits[0] - logits[1], axis=1) / np.linalg.norm(logits[1], axis=1)
+    assert (diff.max() > 0) == taken
+    assert diff.max() <= 4.5e-7, diff
