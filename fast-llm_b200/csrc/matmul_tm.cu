@@ -454,8 +454,9 @@ __device__ __forceinline__ bool epi_step_q6k(const Epi &e, Ring &d, uint32_t hal
     for (int i = 0; i < NT / 2; i += 2) {
         F2 x0, x1;
         lds_f2x2(side + NT * 32 + i * 8, x0, x1);
-        acc[i] = fma2(x0 * d2, sum[i], acc[i]);
-        acc[i + 1] = fma2(x1 * d2, sum[i + 1], acc[i + 1]);
+        // (never x0 d2 by itself: with an activation at either end of the range it is infinite or loses bits)
+        acc[i] = fma2(x0, d2 * sum[i], acc[i]);
+        acc[i + 1] = fma2(x1, d2 * sum[i + 1], acc[i + 1]);
     }
     return true;
 }

@@ -68,6 +68,36 @@ def test_special_values(ctx, monkeypatch, form, fmt):
     multi_column.test_multi_column_special_values(ctx, fmt)
 
 
+@pytest.mark.parametrize("form", ["0", "2"])
+@pytest.mark.parametrize("nx", [8, 16])
+def test_q6_k_smallest_and_largest_scales(ctx, monkeypatch, form, nx):
+    """The block scales of weight and activation meet in the result only: their product alone may not be a finite or a normal
+    number. Rows of scale zero under d = 40000 and an activation near the end of the range give zero; d of two bits in f16's
+    last places times an activation of 1e-35 is as exact as any other."""
+    monkeypatch.setenv("FLB_UMMA", form)
+    rows, cols = 256, 2048
+    w = torch.from_numpy(synth.quant_tensor(capi.Q6_K, np.random.default_rng(0), rows, cols)).cuda()
+    blk = w.view(-1, 210)
+    x = torch.randn((nx, cols), device="cuda", generator=torch.Generator(device="cuda").manual_seed(0))
+    f = torch.empty((rows, cols), device="cuda")
+    for d, size in ((40000.0, 1e37), (3 * 2.0 ** -24, 1e-35)):
+        blk[:, 208:210] = torch.tensor([d], dtype=torch.float16, device="cuda").view(torch.uint8)
+        xs, y = x * size, torch.zeros((nx, rows), device="cuda")
+        xs[:, 5::256] = 8.9 * size                      # the largest of every block, the same block scale everywhere
+        if d > 1:
+            blk[:, 192:208] = 0
+        else:
+            blk[:, 192:208] = 100
+        torch.cuda.synchronize()
+        ctx.dequant(capi.Q6_K, w, rows, cols, f)
+        ctx.matvec(capi.Q6_K, w, rows, cols, xs, y, nx=nx, xstride=cols, ystride=rows)
+        ctx.sync()
+        if d > 1:
+            assert torch.equal(y, torch.zeros_like(y))
+        else:
+            assert multi_column.close(y, xs.double() @ f.double().T)
+
+
 @pytest.mark.parametrize("rows,cols", [(4096, 4096), (4096, 14336)])
 @pytest.mark.parametrize("nx", [2, 8, 9, 16])
 @pytest.mark.parametrize("form,recipe", [("1", "Q4_K"), ("2", "Q4_K"), ("2", "Q6_K")])
