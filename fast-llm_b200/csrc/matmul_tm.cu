@@ -237,6 +237,12 @@ __device__ __forceinline__ bool walk_next(const TmArgs &a, Walk &w, Piece &p) {
     return true;
 }
 
+// Steps of this CTA.
+__device__ __forceinline__ uint32_t steps_of(const TmArgs &a) {
+    const Walk w = walk_begin(a);
+    return a.whole ? ((w.hi + a.nblk - 1) / a.nblk - (w.pos + a.nblk - 1) / a.nblk) * a.nblk : w.hi - w.pos;
+}
+
 // Offsets in shared memory.
 constexpr uint32_t kRawFull = 0, kActFull = kRawFull + 8 * kMaxSlots, kEmpty = kActFull + 8 * kMaxSlots, kAFull = kEmpty + 8 * kMaxSlots,
                    kAEmpty = kAFull + 16, kDFull = kAEmpty + 16, kDEmpty = kDFull + 32, kCombFull = kDEmpty + 32, kCombEmpty = kCombFull + 32,
@@ -503,6 +509,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
     fence_after();
     const uint32_t tmem = lds32(smem + kTmemPtr), stages = smem + head_of(T);
     Walk wk = walk_begin(a);
+    const uint32_t n_steps = steps_of(a);
     Piece pc;
     Ring st{0, 0};   // the stage ring
     auto step_on = [&]() { if (++st.slot == kSlots<F, T>) { st.slot = 0; st.par ^= 1u; } };
@@ -548,9 +555,6 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
                 step_on();
             }
         }
-        // The last arrival at the barrier of this group's weights, which nothing else waits for: it must not be in flight when the
-        // CTA gives its shared memory up to the next one, which may be there already (a programmatic dependent).
-        if (!dead) warp_wait(smem + kAEmpty + 8 * wg, par, a.status, abort_flag);
     } else if (warp < kLoadWarp) {
         // ---- epilogue ----
         const uint32_t quad = warp & 3u, row = quad * 32 + lane;
@@ -651,7 +655,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
             drain(kRawFull, n);
         }
     } else if (warp == kTensorWarp) {
-        uint32_t buf = 0, apar = 0;
+        uint32_t buf = 0, apar = 0, left = n_steps;
         Ring d[2] = {{0, 1}, {R / 2, 1}};   // the buffers of the epilogue's halves
         auto wait = [&](uint32_t bar, uint32_t parity) { return warp_wait(bar, parity, a.status, abort_flag); };
         while (!dead && walk_next(a, wk, pc)) {
@@ -675,7 +679,9 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_tm_kernel(const __grid_con
                     else if ((++r.slot & 1u) == 0) { r.slot -= 2; r.par ^= 1u; }
                 }
                 if (dead) break;
-                if (elect_one()) tm_commit(smem + kAEmpty + 8 * buf);
+                // (not after the last step of either buffer: an arrival that nothing waits for could still be in flight when the CTA gives
+                // its shared memory up to the next one, which may be there already as a programmatic dependent)
+                if (left-- > 2 && elect_one()) tm_commit(smem + kAEmpty + 8 * buf);
                 __syncwarp();
                 buf ^= 1u;
                 if (!buf) apar ^= 1u;

@@ -124,10 +124,9 @@ def test_sums_are_not_truncated(ctx, monkeypatch, form, recipe, nx, rows, cols):
 
 @pytest.mark.parametrize("nx", [8, 16])
 def test_launches_in_a_row(ctx, monkeypatch, nx):
-    """Launches whose CTAs have one to five steps, one behind the other without a wait between them: a CTA waits for the last
-    arrival at the barrier of either weight buffer (an odd number of steps leaves the second one phase behind, one step never
-    uses it) before the next CTA sets up its own in the same memory. A wait on the wrong phase runs out and says so in the
-    status; a missing one shows by reading only."""
+    """Launches whose CTAs have one to five steps, one behind the other without a wait between them: after the last step of either
+    weight buffer nothing arrives at its barrier any more, so that the next CTA can set up its own in the same memory. One arrival
+    too few and a wait runs out, which the status says; one too many shows by reading only."""
     monkeypatch.setenv("FLB_UMMA", "1")
     rows, cols = 148 * 128, 256
     w = torch.from_numpy(synth.quant_tensor(capi.Q4_K, np.random.default_rng(nx), 5 * rows, cols)).cuda()
