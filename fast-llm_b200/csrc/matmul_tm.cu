@@ -25,9 +25,10 @@
 // a chain of 4: -5.4e-8 of the result with either, of 16: -2.1e-7). The mins: 8 d sc - dmin m of a sub-block, rounded once, times
 // the sub-block's f32 sum.
 //
-// What bounds it (B200): issue slots. A step takes 2600 warp instructions besides the polls (324 per 16 rows; matvec_tc_nx.cu 413 for 8
-// tokens, 560 for 16), over four schedulers at 0.6 a cycle; the tensor pipe is 9 % busy (an instruction takes 15 cycles for N 16, 20
-// for N 32, with A in tensor memory; 40 with A in shared memory), the weights arrive at 5.9 TB/s when nothing else is done.
+// What bounds it (B200): issue slots. A step of Q4_K with 8 tokens takes 2600 warp instructions besides the polls (324 per 16 rows;
+// matvec_tc_nx.cu 413, 560 for 16 tokens), over four schedulers at 0.6 a cycle in the steady state; the tensor pipe is 8 % busy with 8
+// tokens and 13 % with 16 (28672 x 4096 Q4_K; Q6_K 4 and 8 %; an instruction takes 15 cycles for N 16, 20 for N 32, with A in tensor
+// memory; 40 with A in shared memory), the weights arrive at 5.9 TB/s when nothing else is done.
 // 28672 x 4096 Q4_K with its conversion: 25.8 us for 8 tokens and 34.9 for 16 (matvec_tc_nx.cu: 28.3 and 40.5); 2 tokens 23.9 (23.4).
 // Inside a pass more, since the activation arrives beside the weights instead of in front of them (70 KB per CTA): 8B shape, 16 tokens
 // 4207 us with matvec_tc_nx.cu throughout, 3886 with gate | up, 3844 with O and 3626 with down (Q6_K) in this form too.
@@ -186,8 +187,8 @@ __device__ __forceinline__ void tm_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 // One lane of the warp, the same one every time. The tensor warp runs as a whole and branches on this only around its
-// instructions: their operands stay in uniform registers (with one thread in a branch of its own, moving them there took
-// most of the 135 cycles that an instruction cost; the unit itself needs 45 for N up to 64).
+// instructions: measured, one by one from a thread in a branch of its own an instruction cost 45 cycles alone and 135 beside the other
+// roles, this way 15 (N 16).
 __device__ __forceinline__ bool elect_one() {
     uint32_t r;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
@@ -748,13 +749,18 @@ int matmul_tm_switch(void) {
     return v && v[0] >= '0' && v[0] <= '2' ? v[0] - '0' : -1;
 }
 
-// Whether a launch whose planes are added on the fly takes this form. Time = start + steps per CTA x time of one, conversion included:
-// 8 tokens 8.9 + 0.70 us against 7.9 + 0.84 (matvec_tc_nx.cu), 16 tokens 11.4 + 0.97 against 9.2 + 1.29, equal at 7 steps per CTA.
-// Inside a pass of 16 tokens O (3.5 steps per CTA) gains 1.3 us a layer all the same, of 8 nothing. Up to 4 tokens the other kernel
-// needs half its tensor instructions and is the faster one alone (28672 x 4096, 2 tokens: 23.4 against 23.9 us), but not inside a pass
-// (8B shape over 4096 keys, 2 / 3 / 4 tokens: 2968 / 3015 / 3060 us with it, 2938 / 2979 / 3048 with this form; 16 layers of it in
-// Q4_K over 512, 2 / 4 tokens: 1373 / 1394 and 1332 / 1350). Calls whose planes
-// would take a launch of their own to add don't take it (14336 x 4096, 8 tokens: 17.4 against 18.0 us, and 3 us for the planes).
+// Whether a launch whose planes are added on the fly takes this form. Time of Q4_K alone = start + steps per CTA x time of one,
+// conversion included: 8 tokens 8.9 + 0.70 us against 7.9 + 0.84 (matvec_tc_nx.cu), 16 tokens 11.4 + 0.97 against 9.2 + 1.29, equal at
+// 7 steps per CTA. Inside a pass the line lies lower from 9 tokens on, since the other kernel's instance for so many is the slower one;
+// passes of 8 layers over 512 keys (embedding / FFN) with this form over without it, 9 / 12 / 16 tokens:
+//   4096 / 4096  Q4_K_M  (O and down, Q6_K, 3.5 steps per CTA, gate | up 6.9)  0.980 / 0.998 / 0.964
+//   2048 / 8192  Q4_K    (down 3.5, gate | up 6.9)                             0.976 / 0.988 / 0.967
+//   2048 / 14336 Q4_K_M  (down, Q6_K, 6.0, gate | up 12)                       0.977 / 0.979 / 0.953
+// 5 and 8 tokens, from 8 steps on: 4096 / 10240 Q4_K_M (down, Q6_K, 8.6) 0.929 / 0.935, 2048 / 9472 Q4_K (gate | up 8.0) 0.968 / 0.969.
+// Up to 4 tokens the other kernel needs half its tensor instructions and is the faster one alone (28672 x 4096, 2 tokens: 23.4 against
+// 23.9 us), but not inside a pass (8B shape over 4096 keys, 2 / 3 / 4 tokens: 2968 / 3015 / 3060 us with it, 2938 / 2979 / 3048 with this
+// form; at 8.0 to 8.6 steps, 2048 columns, 0.983 to 1.004). Calls whose planes would take a launch of their own to add don't take it
+// (14336 x 4096, 8 tokens: 17.4 against 18.0 us, and 3 us for the planes).
 bool matmul_tm_takes(const NxTensor *t, int n, uint32_t cols, uint32_t P, int sms) {
     TmPlan p;
     return P > 1 && tm_plan(t, n, cols, true, sms, p) && p.grid == (uint32_t)sms && p.steps >= (P > 8 ? 3 : 8) * p.grid;

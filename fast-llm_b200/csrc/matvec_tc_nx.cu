@@ -777,8 +777,8 @@ __device__ __forceinline__ void consume(const NxArgs &a, uint32_t smem, const Nx
 }
 
 // FM: the formats an instance carries (bit 0 Q4_K, 1 Q6_K, 2 Q8_0): with all three in one kernel, what is live across the
-// choice of the body does not fit in the registers beside the largest of them (204 bytes of spills against 0..48). T: the
-// most token groups a piece can have, 2 or 4, for the same reason (Q4_K: no spills against 60 bytes).
+// choice of the body does not fit in the registers beside the largest of them (bytes spilled: 56 with T 2 and 96 with T 4, against 0
+// to 20 and 24 to 76). T: the most token groups a piece can have, 2 or 4, for the same reason (Q4_K: 8 bytes against 56).
 template <int FM, int T>
 __global__ void __launch_bounds__(kThreads, 1) matmul_nx_kernel(const __grid_constant__ NxArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];

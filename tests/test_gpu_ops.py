@@ -459,19 +459,20 @@ def test_stream_dot_multi_column_both_formats(ctx, checker, fmt, rows, cols, nx)
 
 
 @pytest.mark.parametrize("rows,cols,nx", [
-    (256, 14336, 8),      # two row tiles, the k range split over several work items (partial results through the ticket)
+    (256, 14336, 8),      # two tiles of rows, 56 steps each
     (4096, 4096, 8), (1029, 4096, 6), (37, 2048, 3), (64, 768, 2), (300, 14336, 9), (128, 512, 8),
 ])
 def test_stream_dot_multi_column_tcgen05(ctx, checker, monkeypatch, rows, cols, nx):
-    """The same contract on the tcgen05 kernel (accumulator in tensor memory, split-K with ordered partial sums), which
-    is off by default: FLB_UMMA=1 is read at every call."""
+    """The same contract on the tcgen05 kernel (weights and results in tensor memory), which plain calls do not take by themselves:
+    FLB_UMMA=1, read at every call, sends them there in whole tiles of 128 rows (a batch pass cuts its launches into shares that
+    leave planes of partial sums: test_gpu_tensor_memory.py)."""
     monkeypatch.setenv("FLB_UMMA", "1")
     multi_column_case(ctx, checker, capi.Q4_K, rows, cols, nx)
 
 
 def multi_column_case(ctx, checker, fmt, rows, cols, nx):
     """Task::nx > 1 on Q6_K as well as Q4_K tensors (draft verification, prompt chunks): all columns in one pass over
-    the weights (up to 8 at a time); every column equals the reference's STREAM_DOT of that column, accumulate and
+    the weights (up to 16 at a time); every column equals the reference's STREAM_DOT of that column, accumulate and
     assign-after-zero alike; ragged row counts, column counts that are not a multiple of 2048, strides with gaps."""
     rng = np.random.default_rng(7 * rows + cols + nx + fmt)
     w = synth.quant_tensor(fmt, rng, rows, cols)
