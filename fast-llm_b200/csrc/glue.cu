@@ -373,6 +373,27 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ l
 
 } // namespace
 
+// Bound by its launch: a few hundred kilobytes at most in earnest (16 bytes a thread and round).
+__global__ void __launch_bounds__(256) fill_kernel(uint8_t *dst, uint32_t v, size_t bytes, uint32_t head) {
+    griddep_launch_dependents();
+    griddep_wait();
+    uint4 *mid = reinterpret_cast<uint4 *>(dst + head);
+    const size_t n16 = (bytes - head) / 16, tail = head + 16 * n16;
+    const uint4 q = make_uint4(v, v, v, v);
+    for (size_t i = blockIdx.x * (size_t)256 + threadIdx.x; i < n16; i += (size_t)gridDim.x * 256) mid[i] = q;
+    if (blockIdx.x == 0 && threadIdx.x < 32) {   // the bytes in front of the first and behind the last whole 16
+        if (threadIdx.x < head) dst[threadIdx.x] = (uint8_t)v;
+        if (tail + threadIdx.x < bytes && threadIdx.x < 16) dst[tail + threadIdx.x] = (uint8_t)v;
+    }
+}
+
+cudaError_t launch_fill(void *dst, int value, size_t bytes, int sms, cudaStream_t stream, bool pdl) {
+    if (!dst || !bytes) return cudaErrorInvalidValue;
+    const uint32_t head = (uint32_t)std::min<size_t>((16 - ((uintptr_t)dst & 15u)) & 15u, bytes);
+    const uint32_t grid = (uint32_t)std::min<size_t>(bytes / 4096 + 1, (size_t)8 * sms);
+    return launch_kernel(fill_kernel, dim3(grid), dim3(256), 0, stream, pdl, (uint8_t *)dst, (uint32_t)(uint8_t)value * 0x01010101u, bytes, head);
+}
+
 cudaError_t launch_rmsnorm(const float *x, const float *wnorm, float *y, float eps, uint32_t n,
                            cudaStream_t stream, uint32_t rows, uint32_t stride) {
     if (rows == 0) return cudaErrorInvalidValue;

@@ -51,7 +51,8 @@ struct MatvecArgs {
     int swiglu;           // 1: t[0] = gate, t[1] = up (same shape and format): t[0].y[r] = silu(gate_r . x) * (up_r . x)
     uint32_t *status;     // device status word
     float *xn_out;        // optional: CTA 0 also writes the activation it built (nullptr: no)
-    int pdl;              // launch with programmatic dependent launch (inside the decoder's step)
+    int pdl;              // launch with programmatic dependent launch
+    int w_after;          // with pdl: nothing is read before the dependency is met, the weights neither (the kernel before may write them)
     int issue_late;       // 1: request the first weight stages after the activation loads are in flight instead of
                           // before the dependency wait (for launches whose CTAs only become resident when the previous
                           // kernel's CTAs leave, so that nothing is gained by requesting early)
@@ -121,6 +122,7 @@ struct NxIn {
     const uint32_t *table, *col_idx, *out_idx;
     uint32_t list_stride, col_off, n_groups, n_experts;   // n_groups: upper bound of active experts
     int table_ready;         // 1: the table was complete before the kernel in front of the matmul started
+    int dep_first;           // 1: the launch after the conversion starts only when what lies in front of the conversion has completed
     int tm;                  // 1: launch_nx_convert builds the image of matmul_tm.cu (Q4_K or Q6_K, one format, not grouped)
 };
 // Number of parts the columns are cut into (1: y is the result; more: planes of partial sums); 0: not taken. split: planes cost the
@@ -154,6 +156,8 @@ cudaError_t matmul_tc_nx_init(void);
 bool matvec_is_streaming(int fmt, uint32_t cols);
 // Dynamic shared memory the streaming kernel needs for (cols, formats used).
 size_t matvec_smem_bytes(uint32_t cols, bool use_q4k, bool use_q6k, int *stages_out, int *warps_out, bool use_q8_0 = false);
+// [p, p + bytes) lies in one allocation of `device` (false: elsewhere, or unknown).
+bool in_device_memory(int device, const void *p, size_t bytes);
 cudaError_t matvec_init(void);   // sets the dynamic shared memory attribute once
 
 // ---- attn.cu ------------------------------------------------------------
@@ -262,6 +266,8 @@ cudaError_t launch_argmax_exchange(const TopExchangeArgs &a, cudaStream_t stream
 
 // ---- glue.cu ------------------------------------------------------------
 // rows vectors of n floats, `stride` floats apart in x and in y (one weight vector for all).
+// dst[0 .. bytes) = value; dst of any alignment.
+cudaError_t launch_fill(void *dst, int value, size_t bytes, int sms, cudaStream_t stream, bool pdl);
 cudaError_t launch_rmsnorm(const float *x, const float *wnorm, float *y, float eps, uint32_t n,
                            cudaStream_t stream, uint32_t rows = 1, uint32_t stride = 0);
 cudaError_t launch_add2(const float *a, const float *b, float *y, uint32_t n, cudaStream_t stream);

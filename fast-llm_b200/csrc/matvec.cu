@@ -765,6 +765,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static EncodeTiledFn g_encode = nullptr;
+typedef CUresult (*PointerAttributesFn)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+static PointerAttributesFn g_pointer = nullptr;
 
 cudaError_t matvec_init(void) {
     if (!g_encode) {
@@ -774,6 +776,8 @@ cudaError_t matvec_init(void) {
         if (e != cudaSuccess) return e;
         if (qres != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
         g_encode = (EncodeTiledFn)fn;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess)
+            g_pointer = (PointerAttributesFn)fn;
     }
     const void *kernels[] = {(const void *)matvec_stream_kernel<false, false>, (const void *)matvec_stream_kernel<true, false>,
                              (const void *)matvec_stream_kernel<false, true>};
@@ -782,6 +786,20 @@ cudaError_t matvec_init(void) {
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+
+bool in_device_memory(int device, const void *p, size_t bytes) {
+    if (!g_pointer) return false;
+    unsigned type = 0;
+    int ordinal = -1;
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    CUpointer_attribute which[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                    CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *got[4] = {&type, &ordinal, &base, &size};
+    if (g_pointer(4, which, got, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+    const uint64_t off = (uint64_t)p - base;   // (0 for what the driver does not know: no size then)
+    return type == CU_MEMORYTYPE_DEVICE && ordinal == device && off <= size && bytes <= size - off;
 }
 
 // The packed tensor as [rows][row_bytes / 8] 8-byte elements, box = 4 rows x one segment.

@@ -234,6 +234,7 @@ struct TcArgs {
     uint32_t nslots, slot_bytes, ring_off;   // ring_off: bytes from the start of shared memory to the ring
     uint32_t *status;
     int l2_hints;                            // weights evict-first, norm weights evict-last in L2
+    int w_after;                             // the weights are requested after the dependency wait (MatvecArgs::w_after)
     GridBar *bar;                            // n_phases > 1
     unsigned long long *trace;
 };
@@ -713,6 +714,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
         // ---- producer: one bulk copy per row and stage; the weights do not depend on any activation ----
         const TcSmem sm = tc_carve<G>(smem_raw, 256, false, false, false, S, a.ring_off);
         uint32_t slot = 0, par = 1;   // a fresh barrier passes a wait on parity 1
+        if (a.w_after) griddep_wait();
         const uint64_t pol = a.l2_hints ? l2_policy_evict_first() : 0ull;
 #pragma unroll 1
         for (int p = 0; p < a.n_phases; ++p) {
@@ -1323,6 +1325,7 @@ cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaS
     k.n_phases = n;
     k.status = args[0].status;
     k.trace = args[0].trace;
+    k.w_after = args[0].w_after;
     static const bool hints = !(getenv("FLB_TC_L2HINT") && getenv("FLB_TC_L2HINT")[0] == '0');
     k.l2_hints = hints ? 1 : 0;
     k.slot_bytes = any8 ? kSlot8 : any6 ? kSlot6 : kSlot4;

@@ -209,6 +209,7 @@ struct ConvArgs {
     const float *att;              // the columns are attention contexts of heads of 128, added up here from n_splits records
     uint32_t n_splits;             // (attn.cu: [column][head][split][132] = context, maximum, sum)
     int tm;                        // img4 or img6 is the image of matmul_tm.cu
+    int dep_first;                 // see NxIn
 };
 // Device-side table of a grouped launch: word 0 = number of active groups, word 1 = the most token groups of one; then four
 // words per active group: {group, number of columns, token groups in front of it, columns in front of it}.
@@ -266,10 +267,11 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     const uint32_t pp = blockIdx.y & 3u, i = threadIdx.x, hl = i >> 2, tq = i & 3u;   // column of the group; values 16 hl + 4 tq ..
     // launched as a programmatic dependent: the launch itself overlaps the tail of the kernel before, whose output
     // (x, the table) is read only after it has completed
-    griddep_launch_dependents();
+    if (!a.dep_first) griddep_launch_dependents();
     float4 wn = make_float4(1.f, 1.f, 1.f, 1.f);
     if (a.wnorm) wn = __ldg(reinterpret_cast<const float4 *>(a.wnorm + blk * 256 + 4 * i));   // a constant
     griddep_wait();
+    if (a.dep_first) griddep_launch_dependents();
     uint32_t n_valid = a.P, tg = blockIdx.y >> 2, ntg = (a.P + 3) / 4, tg0 = 0, grp = 0, row0 = 0;
     if (a.table) {
         if (blockIdx.z >= a.table[0]) return;
@@ -1045,7 +1047,7 @@ cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t
     ConvArgs c{};
     c.x = in.x; c.x2 = in.x2; c.part_stride = in.part_stride; c.resid = in.resid; c.x_out = in.x_out; c.wnorm = in.wnorm;
     c.xstride = in.xstride; c.rstride = in.rstride; c.n_parts = in.n_parts ? in.n_parts : 1; c.P = P; c.nblk = cols / 256;
-    c.tm = in.tm;
+    c.tm = in.tm; c.dep_first = in.dep_first;
     if (in.tm && (q8 || q4 == q6 || in.table)) return cudaErrorNotSupported;
     if (q4) c.img4 = xq;
     if (q6) c.img6 = xq + nx_image_off(FMT_Q6_K, q4, q6, cols, tgs_cap);

@@ -1,0 +1,114 @@
+"""GPU tests of calls in a row on a context's stream: a call starts under the one before it, so that nothing may be read (weights,
+keys, activations) or written before that one has completed. Expected bits are those of the same call on an idle stream."""
+import ctypes as C
+import math
+
+import pytest
+
+from fast_llm_b200 import capi
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def inputs(fmt, rows, cols, nx, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    blocks = rows * cols // capi.BLK_ELEMS[fmt]
+    w = torch.randint(0, 256, (blocks, capi.BLK_BYTES[fmt]), dtype=torch.uint8, device="cuda", generator=g)
+    d = (torch.rand(blocks, device="cuda", generator=g) * 0.01 + 0.001).half().view(torch.uint8).reshape(-1, 2)
+    at = {capi.Q4_K: (0, 2), capi.Q6_K: (208,), capi.Q8_0: (0,)}[fmt]
+    for o in at:
+        w[:, o:o + 2] = d
+    return w.reshape(rows, -1), torch.randn((nx, cols), device="cuda", generator=g)
+
+
+@pytest.mark.parametrize("fmt", [capi.Q4_K, capi.Q6_K, capi.Q8_0])
+@pytest.mark.parametrize("rows,cols,nx", [(16, 2048, 1), (4096, 4096, 1), (2049, 14336, 1), (4096, 4096, 3), (300, 2048, 16)])
+def test_weights_written_by_the_kernel_before(ctx, fmt, rows, cols, nx):
+    pair = [inputs(fmt, rows, cols, nx, s) for s in (1, 2)]
+    w, x = torch.empty_like(pair[0][0]), torch.empty_like(pair[0][1])
+    y = torch.zeros((nx, rows), device="cuda")
+
+    def call():
+        if nx == 1:
+            ctx.matvec_assign(fmt, w, rows, cols, x, y)
+        else:
+            capi._ck(ctx.lib.fl_b200_memset(ctx._h, C.c_void_p(y.data_ptr()), 0, C.c_size_t(4 * nx * rows)))
+            ctx.matvec(fmt, w, rows, cols, x, y, nx=nx, xstride=cols, ystride=rows)
+
+    want = []
+    for a, b in pair:
+        w.copy_(a)
+        x.copy_(b)
+        torch.cuda.synchronize()
+        call()
+        ctx.sync()
+        want.append(y.clone())
+    assert not torch.equal(*want)
+    torch.cuda.synchronize()
+    got = []
+    with torch.cuda.stream(torch.cuda.ExternalStream(ctx.stream())):
+        zero = torch.zeros_like(w[:1])
+        for i in range(40):   # kernels that write weights and activation, the call, a kernel that reads its result
+            a, b = pair[i % 2]
+            torch.bitwise_or(a, zero, out=w)
+            torch.mul(b, 1.0, out=x)
+            call()
+            call()
+            got.append(y.clone())
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, want[i % 2]) for i, g in enumerate(got))
+    assert ctx.status() == 0
+
+
+@pytest.mark.parametrize("kv_len,batch", [(1, 1), (1024, 1), (4097, 3)])
+def test_cache_written_by_the_kernel_before(ctx, kv_len, batch):
+    g = torch.Generator(device="cuda").manual_seed(kv_len)
+    pair = [tuple(torch.randn(s, device="cuda", generator=g).to(t) for s, t in (((batch, 8, 128), torch.float32), ((batch, 2, kv_len, 128), torch.float16),
+                                                                              ((batch, 2, kv_len, 128), torch.float16))) for _ in range(2)]
+    q, k, v = (torch.empty_like(t) for t in pair[0])
+    out = torch.zeros_like(q)
+
+    def call():
+        ctx.attn_decode(q, k, v, 8, 2, 128, kv_len, kv_len, batch, 1.0 / math.sqrt(128), out)
+
+    want = []
+    for p in pair:
+        for dst, src in zip((q, k, v), p):
+            dst.copy_(src)
+        torch.cuda.synchronize()
+        call()
+        ctx.sync()
+        want.append(out.clone())
+    torch.cuda.synchronize()
+    got = []
+    with torch.cuda.stream(torch.cuda.ExternalStream(ctx.stream())):
+        for i in range(40):
+            for dst, src in zip((q, k, v), pair[i % 2]):
+                torch.mul(src, 1.0, out=dst)
+            call()
+            call()
+            got.append(out.clone())
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want[i % 2]) for i, o in enumerate(got))
+
+
+@pytest.mark.parametrize("offset,size", [(0, 1), (0, 16), (1, 15), (3, 14), (15, 1), (7, 4096), (16, 4099), (5, 3_000_001), (0, 64 << 20)])
+def test_memset_any_range(ctx, offset, size):
+    buf = torch.randint(0, 200, (offset + size + 40,), dtype=torch.uint8, device="cuda")
+    want = buf.clone()
+    want[offset:offset + size] = 0xAB
+    torch.cuda.synchronize()
+    capi._ck(ctx.lib.fl_b200_memset(ctx._h, C.c_void_p(buf.data_ptr() + offset), 0x1AB, C.c_size_t(size)))   # the low byte, as memset
+    ctx.sync()
+    assert torch.equal(buf, want)
+
+
+def test_memset_what_the_driver_takes_or_refuses(ctx):
+    host = torch.full((100,), 7, dtype=torch.uint8).pin_memory()
+    capi._ck(ctx.lib.fl_b200_memset(ctx._h, C.c_void_p(host.data_ptr()), 1, C.c_size_t(100)))
+    capi._ck(ctx.lib.fl_b200_memset(ctx._h, C.c_void_p(0), 0, C.c_size_t(0)))
+    ctx.sync()
+    assert bool((host == 1).all())
+    assert ctx.lib.fl_b200_memset(ctx._h, C.c_void_p(0), 0, C.c_size_t(16)) != 0   # no memory there: refused, nothing is launched
+    ctx.sync()
