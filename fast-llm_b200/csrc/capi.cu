@@ -85,6 +85,7 @@ int fl_b200_create(int device, fl_b200_ctx **out) {
     CK(cudaMalloc(&c->small, 64));
     CK(matvec_init());
     CK(matvec_tc_init());
+    CK(matvec_expert_init());
     CK(matmul_tc_nx_init());
     CK(cudaMalloc(&c->xq, matmul_tc_nx_scratch_bytes(kNxMaxCols, kNxTgs, 3)));
     CK(cudaMalloc(&c->nx_part, kNxPartFloats * sizeof(float)));

@@ -48,21 +48,16 @@ __global__ void add2_kernel(const float *__restrict__ a, const float *__restrict
 // the exponentials (ascending expert index, one lane) and the sum of the chosen weights (selection order).
 // With expert parallelism (lids != nullptr) the kernel also writes, per (token, slot), the index of the expert
 // among this rank's experts [base, base + n_local) or the skip mark, and the gate or 0.
-constexpr int kRouterWarps = 4;
-__global__ void __launch_bounds__(kRouterWarps * 32) router_sel_kernel(const float *__restrict__ logits, uint32_t *ids, float *gates,
-                                                                     uint32_t *lids, float *mgates, uint32_t n_tok,
-                                                                     uint32_t n_expert, uint32_t top_k, uint32_t norm, float scale,
-                                                                     uint32_t base, uint32_t n_local) {
-    __shared__ float w_s[kRouterWarps][256], g_s[kRouterWarps][256];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t tok = blockIdx.x * kRouterWarps + warp;
-    if (tok >= n_tok) return;
-    const float *l = logits + (size_t)tok * n_expert;
-    float *w = w_s[warp], *gk = g_s[warp];
+struct RouterOut { uint32_t *ids; float *gates; uint32_t *lids; float *mgates; uint32_t top_k, norm; float scale; uint32_t base, n_local; };
+// One warp; w, gk: n_expert and top_k floats of shared memory. The logits may come from other blocks of the launch.
+__device__ __forceinline__ void router_select(const float *l, float *w, float *gk, uint32_t lane, size_t tok, uint32_t n_expert, const RouterOut &o) {
+    uint32_t *ids = o.ids, *lids = o.lids;
+    float *gates = o.gates, *mgates = o.mgates;
+    const uint32_t top_k = o.top_k;
     float mx = -1e30f;
-    for (uint32_t i = lane; i < n_expert; i += 32) mx = fmaxf(mx, l[i]);
+    for (uint32_t i = lane; i < n_expert; i += 32) mx = fmaxf(mx, __ldcg(l + i));
     mx = warp_max(mx);
-    for (uint32_t i = lane; i < n_expert; i += 32) w[i] = expf(__fsub_rn(l[i], mx));
+    for (uint32_t i = lane; i < n_expert; i += 32) w[i] = expf(__fsub_rn(__ldcg(l + i), mx));
     __syncwarp();
     float sum = 0.f;
     if (lane == 0)
@@ -85,7 +80,7 @@ __global__ void __launch_bounds__(kRouterWarps * 32) router_sel_kernel(const flo
         }
         tsum = __fadd_rn(tsum, bw);   // every lane keeps the same running sum, in selection order
         if (lane == 0) {
-            ids[(size_t)tok * top_k + k] = best;
+            ids[tok * top_k + k] = best;
             gk[k] = bw;
             if (bw >= 0.f) w[best] = -2.f;
         }
@@ -93,16 +88,92 @@ __global__ void __launch_bounds__(kRouterWarps * 32) router_sel_kernel(const flo
     }
     for (uint32_t k = lane; k < top_k; k += 32) {
         float g = gk[k];
-        if (norm) g = __fdiv_rn(g, tsum);
-        g = __fmul_rn(g, scale);
-        gates[(size_t)tok * top_k + k] = g;
+        if (o.norm) g = __fdiv_rn(g, tsum);
+        g = __fmul_rn(g, o.scale);
+        gates[tok * top_k + k] = g;
         if (lids) {
-            const uint32_t e = ids[(size_t)tok * top_k + k];
-            const bool mine = e >= base && e - base < n_local;
-            lids[(size_t)tok * top_k + k] = mine ? e - base : kExpertSkip;
-            mgates[(size_t)tok * top_k + k] = mine ? g : 0.f;
+            const uint32_t e = ids[tok * top_k + k];
+            const bool mine = e >= o.base && e - o.base < o.n_local;
+            lids[tok * top_k + k] = mine ? e - o.base : kExpertSkip;
+            mgates[tok * top_k + k] = mine ? g : 0.f;
         }
     }
+}
+
+constexpr int kRouterWarps = 4;
+__global__ void __launch_bounds__(kRouterWarps * 32) router_sel_kernel(const float *__restrict__ logits, uint32_t n_tok, uint32_t n_expert, RouterOut o) {
+    __shared__ float w_s[kRouterWarps][256], g_s[kRouterWarps][256];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t tok = blockIdx.x * kRouterWarps + warp;
+    if (tok >= n_tok) return;
+    router_select(logits + (size_t)tok * n_expert, w_s[warp], g_s[warp], lane, tok, n_expert, o);
+}
+
+// Router of a block: logits[t][e] = dot(router[e], x[t]), one block per (expert, token), and the selection by the block that is the
+// last of its token. wnorm != nullptr: x is the raw hidden state and the logits are those of RMSNorm(x) * wnorm (fl_op_rmsnorm,
+// src/runtime/decode_params.h:101-106, fused: every block norms the token itself). Bound by latency: the router's rows and the norm
+// weights are requested before the dependency, the selection saves a launch (8 experts of 4096 columns, one token, inside a
+// step: 10.1 us in two launches -> 5.4).
+__global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
+    __shared__ float red[4], w_s[256], g_s[256];
+    __shared__ uint32_t last;
+    constexpr int kAhead = 8;   // 16-byte pieces a thread requests up front
+    const uint32_t e = blockIdx.x, t = blockIdx.y, n4 = a.n_embd / 4;
+    const float4 *w = reinterpret_cast<const float4 *>(a.router + (size_t)e * a.n_embd);
+    const float4 *v = reinterpret_cast<const float4 *>(a.x + (size_t)t * a.n_embd);
+    const float4 *gn = reinterpret_cast<const float4 *>(a.wnorm);
+    float4 wa[kAhead], ga[kAhead], xa[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+        const uint32_t i = threadIdx.x + 128 * k;
+        wa[k] = ga[k] = xa[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < n4) { wa[k] = __ldg(w + i); if (gn) ga[k] = __ldg(gn + i); }
+    }
+    griddep_wait();
+    griddep_launch_dependents();   // what starts now may take x for complete (ExpertArgs::x_ready)
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+        if (threadIdx.x + 128 * k < n4) xa[k] = v[threadIdx.x + 128 * k];
+    float inv_rms = 1.f;
+    if (gn) {
+        float ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const float4 b = xa[k];
+            ss += (b.x * b.x + b.y * b.y) + (b.z * b.z + b.w * b.w);
+        }
+        for (uint32_t i = threadIdx.x + 128 * kAhead; i < n4; i += 128) {
+            const float4 b = v[i];
+            ss += (b.x * b.x + b.y * b.y) + (b.z * b.z + b.w * b.w);
+        }
+        ss = warp_sum(ss);
+        if ((threadIdx.x & 31u) == 0) red[threadIdx.x >> 5] = ss;
+        __syncthreads();
+        inv_rms = 1.0f / sqrtf(((red[0] + red[1]) + (red[2] + red[3])) / (float)a.n_embd + a.eps);
+        __syncthreads();
+    }
+    float acc = 0.f;
+    auto add = [&](const float4 &r, float4 b, const float4 &g) {
+        if (gn) { b.x = b.x * inv_rms * g.x; b.y = b.y * inv_rms * g.y; b.z = b.z * inv_rms * g.z; b.w = b.w * inv_rms * g.w; }
+        acc = fmaf(r.x, b.x, acc); acc = fmaf(r.y, b.y, acc); acc = fmaf(r.z, b.z, acc); acc = fmaf(r.w, b.w, acc);
+    };
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+        if (threadIdx.x + 128 * k < n4) add(wa[k], xa[k], ga[k]);
+    for (uint32_t i = threadIdx.x + 128 * kAhead; i < n4; i += 128) add(w[i], v[i], gn ? gn[i] : make_float4(0.f, 0.f, 0.f, 0.f));
+    acc = warp_sum(acc);
+    if ((threadIdx.x & 31u) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        a.logits[(size_t)t * a.n_expert + e] = (red[0] + red[1]) + (red[2] + red[3]);
+        __threadfence();
+        last = atomicAdd(a.tickets + t, 1u) == a.n_expert - 1 ? 1u : 0u;
+        if (last) { __threadfence(); a.tickets[t] = 0; }   // for the next launch
+    }
+    __syncthreads();
+    if (!last || threadIdx.x >= 32) return;
+    const RouterOut o{a.ids, a.gates, a.lids, a.mgates, a.top_k, a.norm, a.scale, a.base, a.n_local};
+    router_select(a.logits + (size_t)t * a.n_expert, w_s, g_s, threadIdx.x, t, a.n_expert, o);
 }
 
 // fl_op_wmerge, decode_params.h:274-295: y = add1 + add2 + scale * sum_q gate_q * part_q,
@@ -110,6 +181,8 @@ __global__ void __launch_bounds__(kRouterWarps * 32) router_sel_kernel(const flo
 __global__ void wmerge_kernel(const float *__restrict__ parts, const float *__restrict__ gates,
                               const float *__restrict__ add1, const float *__restrict__ add2, float *__restrict__ y,
                               float scale, uint32_t n_parts, uint32_t n, uint32_t n_full) {
+    griddep_launch_dependents();
+    griddep_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float gsc = 1.0f;
@@ -412,15 +485,19 @@ cudaError_t launch_router_sel(const float *logits, uint32_t *ids, float *gates, 
     if (n_tok == 0 || n_expert == 0 || n_expert > 256 || top_k == 0 || top_k > n_expert) return cudaErrorInvalidValue;
     if ((lids == nullptr) != (mgates == nullptr)) return cudaErrorInvalidValue;
     router_sel_kernel<<<(n_tok + kRouterWarps - 1) / kRouterWarps, kRouterWarps * 32, 0, stream>>>(
-        logits, ids, gates, lids, mgates, n_tok, n_expert, top_k, norm, scale, base, n_local);
+        logits, n_tok, n_expert, RouterOut{ids, gates, lids, mgates, top_k, norm, scale, base, n_local});
     return cudaGetLastError();
 }
 
+cudaError_t launch_router(const RouterArgs &a, cudaStream_t stream) {
+    if (a.n_tok == 0 || a.n_expert == 0 || a.n_expert > 256 || a.top_k == 0 || a.top_k > a.n_expert || a.n_embd % 4) return cudaErrorInvalidValue;
+    return launch_kernel(router_kernel, dim3(a.n_expert, a.n_tok), dim3(128), 0, stream, a.pdl != 0, a);
+}
+
 cudaError_t launch_wmerge(const float *parts, const float *gates, const float *add1, const float *add2, float *y,
-                          float scale, uint32_t n_parts, uint32_t n, uint32_t n_full, cudaStream_t stream) {
+                          float scale, uint32_t n_parts, uint32_t n, uint32_t n_full, cudaStream_t stream, bool pdl) {
     if (n == 0 || n_parts == 0) return cudaErrorInvalidValue;
-    wmerge_kernel<<<(n + 255) / 256, 256, 0, stream>>>(parts, gates, add1, add2, y, scale, n_parts, n, n_full);
-    return cudaGetLastError();
+    return launch_kernel(wmerge_kernel, dim3((n + 255) / 256), dim3(256), 0, stream, pdl, parts, gates, add1, add2, y, scale, n_parts, n, n_full);
 }
 
 cudaError_t launch_wmerge_tokens(const float *parts, const float *gates, float *y, uint32_t n_parts, uint32_t n, uint32_t n_tok,

@@ -90,6 +90,23 @@ cudaError_t launch_matvec_tc(const MatvecArgs &a, int sms, cudaStream_t stream);
 // when a phase does not qualify: launch them one by one then. args[0].grid_bar names the barrier state.
 cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaStream_t stream);
 cudaError_t matvec_tc_init(void);
+// The experts that one token selected (matvec_expert.cu), slot k's being id[k]: y[k * rows + r] = silu(gate_r . h) * (up_r . h) with
+// h = RMSNorm(x) * wnorm (w[1] set), or y[k * rows + r] = w_r . (x + k * x_stride). Same bits as a streaming launch per slot.
+struct ExpertArgs {
+    int fmt;
+    const void *w[2];            // gate and up, or down and nullptr: the experts' rows one behind the other, packed
+    uint32_t rows, cols, n_experts, n_slots;   // rows: of one expert
+    const uint32_t *id;          // device; gate | up: from the launch in front; down: in place before the launch in front read anything
+    const float *x, *wnorm;
+    uint32_t x_stride;
+    float eps, *y;
+    int x_ready;                 // x was complete before the launch in front started its dependents
+    uint32_t *status;
+    int pdl;
+};
+bool matvec_expert_takes(int fmt, uint32_t cols, uint32_t rows, uint32_t n_slots, uint32_t n_experts);
+cudaError_t launch_matvec_expert(const ExpertArgs &e, int sms, cudaStream_t stream);
+cudaError_t matvec_expert_init(void);
 // Several activation columns (P <= 16) in one pass over up to three Q4_K / Q6_K / Q8_0 tensors on the tensor cores
 // (matvec_tc_nx.cu): y[p * ystride + r] (+)= dot(W[r], column p). Two launches: launch_nx_convert builds the activation's
 // operand image(s) in xq, launch_nx_matmul walks the weights.
@@ -275,6 +292,20 @@ cudaError_t launch_add2(const float *a, const float *b, float *y, uint32_t n, cu
 // softmax over n_expert logits, top_k by weight; logits [n_tok][n_expert], ids / gates [n_tok][top_k]. Expert
 // parallel (lids, mgates != nullptr): also the expert's index among this rank's experts [base, base + n_local)
 // or the skip mark, and the gate or 0.
+struct RouterArgs {
+    const float *router, *x, *wnorm;   // [n_expert][n_embd]; [n_tok][n_embd]; optional: the logits are those of RMSNorm(x) * wnorm
+    float eps;
+    uint32_t n_embd, n_expert, n_tok;
+    float *logits;                     // [n_tok][n_expert]
+    uint32_t *tickets;                 // [n_tok], zero between launches
+    uint32_t *ids, *lids;              // the rest: as launch_router_sel
+    float *gates, *mgates;
+    uint32_t top_k, norm;
+    float scale;
+    uint32_t base, n_local;
+    int pdl;
+};
+cudaError_t launch_router(const RouterArgs &a, cudaStream_t stream);
 cudaError_t launch_router_sel(const float *logits, uint32_t *ids, float *gates, uint32_t n_tok, uint32_t n_expert, uint32_t top_k,
                               uint32_t norm, float scale, cudaStream_t stream, uint32_t *lids = nullptr,
                               float *mgates = nullptr, uint32_t base = 0, uint32_t n_local = 0);
@@ -285,7 +316,7 @@ cudaError_t launch_group_by_expert(const uint32_t *lids, uint32_t n_pairs, uint3
                                    uint32_t *cnt, uint32_t *tok_list, uint32_t *pair_list, cudaStream_t stream, uint32_t *table = nullptr);
 // fl_op_wmerge (src/runtime/decode_params.h:274-295).
 cudaError_t launch_wmerge(const float *parts, const float *gates, const float *add1, const float *add2, float *y,
-                          float scale, uint32_t n_parts, uint32_t n, uint32_t n_full, cudaStream_t stream);
+                          float scale, uint32_t n_parts, uint32_t n, uint32_t n_full, cudaStream_t stream, bool pdl = false);
 // fl_op_wmerge for n_tok tokens in one launch: y[t] = (resid[t] +) sum_q gates[t][q] * parts[t][q] (products and sums
 // rounded in the reference's order); a part is the sum of n_planes planes, plane_stride floats apart.
 cudaError_t launch_wmerge_tokens(const float *parts, const float *gates, float *y, uint32_t n_parts, uint32_t n, uint32_t n_tok,

@@ -38,6 +38,7 @@
 // the form that decides everything at run time: see matvec_tc_kernel.
 #include "common.cuh"
 #include "kernels.h"
+#include "tc_ops.cuh"
 
 #include <cuda.h>
 #include <algorithm>
@@ -68,123 +69,6 @@ constexpr uint32_t slot_round(uint32_t b) { return (b + 1023u) & ~1023u; }
 constexpr uint32_t kSlot4 = slot_round(16 * kPitch4), kSlot6 = slot_round(16 * kPitch6), kSlot8 = slot_round(32 * kPitch8);
 // 256-column blocks a half-warp of the prologue converts (bounds the column count: see matvec_tc_eligible)
 __host__ __device__ constexpr int max_blk_per_half_warp(int groups) { return groups == 1 ? 4 : 2; }
-
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
-    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
-}
-__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ void sts32(uint32_t addr, uint32_t a) {
-    asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(a) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// Tiled TMA loads into shared memory (2-D: x counts 8-byte elements, a multiple of 2; 3-D: lines of 128 bytes).
-__device__ __forceinline__ void tma_box2(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ void tma_box3(uint32_t dst, const CUtensorMap *map, uint32_t line, uint32_t row, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-        "l"(map), "r"(0), "r"(line), "r"(row), "r"(smem_u32(bar))
-        : "memory");
-}
-// The same with an L2 eviction policy for the lines the copy touches (the weights pass through L2 once).
-__device__ __forceinline__ void tma_box2_hint(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint64_t *bar, uint64_t pol) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(dst),
-        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(pol)
-        : "memory");
-}
-__device__ __forceinline__ void tma_box3_hint(uint32_t dst, const CUtensorMap *map, uint32_t line, uint32_t row, uint64_t *bar, uint64_t pol) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], [%5], %6;" ::"r"(dst),
-        "l"(map), "r"(0), "r"(line), "r"(row), "r"(smem_u32(bar)), "l"(pol)
-        : "memory");
-}
-__device__ __forceinline__ uint64_t l2_policy_evict_first() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
-__device__ __forceinline__ uint64_t l2_policy_evict_last() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
-// Read-only 16-byte load whose line is kept in L2 in preference to others (small tensors every launch reads again)
-__device__ __forceinline__ float4 ldg_keep(const float4 *p, uint64_t pol) {
-    float4 v;
-    asm volatile("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
-    return v;
-}
-// All threads of the prologue (every warp but the producer) meet here.
-__device__ __forceinline__ void prologue_barrier(uint32_t nthreads) {
-    asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
-}
-// D(16x8, f32) += A(16x16, f16, row) * B(16x8, f16, col)
-__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// D(16x8, s32) += A(16x32, u8, row) * B(32x8, s8, col). Lane (g, t): a0 / a1 = rows g / g + 8, k-slots 4t..4t+3;
-// a2 / a3 = the same rows, k-slots 16+4t..; b0 / b1 = column g, the same two k-slot runs; c as for the f16 form.
-__device__ __forceinline__ void imma16832(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                          uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// (a & b) | c in one instruction; b and c are constants the compiler keeps in registers
-__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-// h - off for both halves (exact: the operands are small integers)
-__device__ __forceinline__ uint32_t hsub2_u32(uint32_t h, __half2 off) {
-    const __half2 r = __hsub2(*reinterpret_cast<const __half2 *>(&h), off);
-    return *reinterpret_cast<const uint32_t *>(&r);
-}
-// The common case of a wait: the phase is already complete. The bounded polling loop stays out of line.
-__device__ __noinline__ bool mbar_wait_slow(uint64_t *bar, uint32_t parity, uint32_t *status) {
-    return mbar_wait_bounded(bar, parity, status);
-}
-// The form the consumer loops use: no exit out of the loop. `dead` (warp-uniform) is set when a wait ran out;
-// from then on the warp waits for nothing any more (its results are void, the status word says so) and the
-// launch still ends.
-__device__ __forceinline__ void mbar_wait_or_die(uint64_t *bar, uint32_t parity, uint32_t *status, bool &dead) {
-    if (dead || mbar_try_wait(bar, parity)) return;
-    dead = !mbar_wait_slow(bar, parity, status);
-}
-// byte K of w as a float without the conversion pipe (the byte under 0x4B000000 is 2^23 + byte)
-template <int K>
-__device__ __forceinline__ float u8f(uint32_t w) {
-    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650u | K)) - 8388608.0f;
-}
-__device__ __forceinline__ uint32_t word_of(const uint4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
 // ---- the activation in shared memory ---------------------------------------------------------
 // Per 256-column block 1024 bytes per layout: f16 hi and lo parts in the order the B operand wants.
@@ -312,10 +196,6 @@ __device__ __forceinline__ int unit_tensor(const TcPhase &a, uint32_t u) {
 // volatile asm statements, which the compiler keeps in program order), so that their latency overlaps.
 // xaddr: this lane's 16-byte B slot of word 0 (lanes that feed no column of B point at 16 zero bytes and
 // use a stride of 0).
-// Byte offset o of a row as the stage holds it: as it is, or in the swizzled 128-byte lines (see kPitch4).
-__device__ __forceinline__ uint32_t q4_row_off(uint32_t o, uint32_t g, bool swz) {
-    return swz ? (o & ~127u) + ((((o >> 4) ^ (g + (o >> 7))) & 7u) << 4) : o;
-}
 // r0: row g of the stage; row g + 8 is 8 * kPitch4 further (the same swizzle: 72 lines further). oh / oa / ob: offsets
 // of the block's header and of the two 16-byte halves of chunk t in the row (q4_row_off).
 __device__ __forceinline__ void q4k_block(uint32_t r0, uint32_t oh, uint32_t oa, uint32_t ob, uint32_t t, uint32_t xaddr,
@@ -512,12 +392,6 @@ __device__ __forceinline__ void q6k_block(uint32_t r0, uint32_t r1, uint32_t t, 
         v += (u8f<3>(sw[r]) - 128.f) * (c[3][2 * r] + c[3][2 * r + 1]);
         (r ? out1 : out0) = dd[r] * v;
     }
-}
-
-// byte K of w, which holds s + 128, as the float s (the byte under 0x4B000000 is 2^23 + 128 + s)
-template <int K>
-__device__ __forceinline__ float s8f(uint32_t w) {
-    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + K)) - 8388736.f;
 }
 
 // Q6_K, integer form: the same loads and the same assembly of the 6-bit quants as q6k_block, but the four bytes

@@ -32,13 +32,13 @@ struct fl_b200_moe {
     const float *router = nullptr;
     const uint8_t *wg = nullptr, *wu = nullptr, *wd = nullptr;
     float *logits = nullptr, *gates = nullptr, *mgates = nullptr, *part = nullptr, *partial = nullptr;
-    uint32_t *ids = nullptr, *lids = nullptr;
+    uint32_t *ids = nullptr, *lids = nullptr, *tickets = nullptr;   // tickets: of the router's blocks, zero between launches
     uint32_t *cnt = nullptr, *tok_list = nullptr, *pair_list = nullptr;   // the pairs grouped by local expert (launch_group_by_expert)
     uint32_t *table = nullptr;                                            // active experts of a grouped launch
     // Used by one call at a time and written before it is read, hence shared by all blocks of a context (their calls are in order
     // on its stream): gate / up outputs and down outputs, planes of `rows` rows each, and the converted activations.
     std::shared_ptr<MoeScratch> scratch;
-    float *g = nullptr, *u = nullptr, *d = nullptr;
+    float *g = nullptr, *u = nullptr, *d = nullptr, *h = nullptr;         // h: silu(gate) * up of every slot of one token
     uint8_t *xq = nullptr;
     uint32_t rows = 0, tgs = 0, planes_gu = 0, planes_d = 0;              // tgs: groups of four columns in xq
     uint8_t *arena = nullptr;                                             // the one allocation that holds the block's own buffers
@@ -53,45 +53,6 @@ struct fl_b200_moe {
 };
 
 namespace {
-
-// Router logits of all tokens in one launch: logits[t][e] = dot(router[e], x[t]); one block per (expert, token).
-// wnorm != nullptr: x is the raw hidden state and the logits are those of RMSNorm(x) * wnorm (fl_op_rmsnorm,
-// src/runtime/decode_params.h:101-106, fused: every block norms the token itself).
-__global__ void __launch_bounds__(128) router_logits_kernel(const float *__restrict__ router, const float *__restrict__ x,
-                                                            float *__restrict__ logits, uint32_t n_embd, uint32_t n_expert,
-                                                            const float *__restrict__ wnorm = nullptr, float eps = 0.f) {
-    __shared__ float red[4];
-    const uint32_t e = blockIdx.x, t = blockIdx.y;
-    const float4 *w = reinterpret_cast<const float4 *>(router + (size_t)e * n_embd);
-    const float4 *v = reinterpret_cast<const float4 *>(x + (size_t)t * n_embd);
-    float inv_rms = 1.f;
-    if (wnorm) {
-        float ss = 0.f;
-        for (uint32_t i = threadIdx.x; i < n_embd / 4; i += 128) {
-            const float4 b = v[i];
-            ss += (b.x * b.x + b.y * b.y) + (b.z * b.z + b.w * b.w);
-        }
-        ss = warp_sum(ss);
-        if ((threadIdx.x & 31u) == 0) red[threadIdx.x >> 5] = ss;
-        __syncthreads();
-        inv_rms = 1.0f / sqrtf(((red[0] + red[1]) + (red[2] + red[3])) / (float)n_embd + eps);
-        __syncthreads();
-    }
-    float acc = 0.f;
-    for (uint32_t i = threadIdx.x; i < n_embd / 4; i += 128) {
-        const float4 a = w[i];
-        float4 b = v[i];
-        if (wnorm) {
-            const float4 g = reinterpret_cast<const float4 *>(wnorm)[i];
-            b.x = b.x * inv_rms * g.x; b.y = b.y * inv_rms * g.y; b.z = b.z * inv_rms * g.z; b.w = b.w * inv_rms * g.w;
-        }
-        acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
-    }
-    acc = warp_sum(acc);
-    if ((threadIdx.x & 31u) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) logits[(size_t)t * n_expert + e] = (red[0] + red[1]) + (red[2] + red[3]);
-}
 
 #define CKM(call)                                                      \
     do {                                                               \
@@ -157,6 +118,7 @@ int fl_b200_moe_create(fl_b200_ctx *ctx, const fl_b200_moe_cfg *cfg, uint32_t ra
     };
     struct Buf { void **p; size_t bytes; };
     const Buf shared[] = {{(void **)&m->g, n_gu * R * F * 4}, {(void **)&m->u, n_gu * R * F * 4}, {(void **)&m->d, m->planes_gu ? n_d * R * E * 4 : 0},
+                          {(void **)&m->h, K * F * 4},
                           {(void **)&m->xq, m->planes_gu ? matmul_tc_nx_scratch_bytes((uint32_t)std::max(E, F), m->tgs, 1) : 0}};
     const size_t need = lay_out(shared, nullptr);
     m->scratch = ctx->moe_scratch.lock();
@@ -169,7 +131,7 @@ int fl_b200_moe_create(fl_b200_ctx *ctx, const fl_b200_moe_cfg *cfg, uint32_t ra
     lay_out(shared, m->scratch->p);
     // One allocation, zero-filled: the per-slot form leaves the part of a slot that is skipped as it was and multiplies it by gate 0.
     const Buf own[] = {
-        {(void **)&m->logits, T * c.n_expert * 4}, {(void **)&m->gates, T * K * 4}, {(void **)&m->mgates, T * K * 4},
+        {(void **)&m->logits, T * c.n_expert * 4}, {(void **)&m->tickets, T * 4}, {(void **)&m->gates, T * K * 4}, {(void **)&m->mgates, T * K * 4},
         {(void **)&m->ids, T * K * 4}, {(void **)&m->lids, T * K * 4}, {(void **)&m->table, (1 + (size_t)m->n_local) * 16},
         {(void **)&m->cnt, (size_t)m->n_local * 4}, {(void **)&m->tok_list, (size_t)m->n_local * T * 4},
         {(void **)&m->pair_list, (size_t)m->n_local * T * 4}, {(void **)&m->part, pairs * E * 4}, {(void **)&m->partial, world > 1 ? T * E * 4 : 0}};
@@ -222,6 +184,14 @@ int fl_b200_moe_set_peers(fl_b200_moe *m, void *const *bufs, uint32_t n) {
     return FL_B200_OK;
 }
 
+static RouterArgs moe_router_args(const fl_b200_moe *m, const float *x, uint32_t n_tok, const float *wnorm, float eps) {
+    RouterArgs r{};
+    r.router = m->router; r.x = x; r.n_embd = m->c.n_embd; r.n_expert = m->c.n_expert; r.wnorm = wnorm; r.eps = eps;
+    r.logits = m->logits; r.tickets = m->tickets; r.ids = m->ids; r.gates = m->gates; r.lids = m->lids; r.mgates = m->mgates;
+    r.n_tok = n_tok; r.top_k = m->c.top_k; r.norm = m->c.norm; r.scale = m->c.scale; r.base = m->base; r.n_local = m->n_local;
+    return r;
+}
+
 // Shapes that the grouped form does not take.
 static bool moe_per_slot(const fl_b200_moe *m) { return m->planes_gu == 0; }
 
@@ -272,9 +242,7 @@ static int moe_enqueue_per_slot(fl_b200_moe *m, const float *x, uint32_t n_tok, 
     const fl_b200_moe_cfg &c = m->c;
     const uint32_t E = c.n_embd, F = c.n_ff, K = c.top_k, NE = c.n_expert;
     const uint64_t stride_gu = (uint64_t)F * row_bytes(c.fmt_gate_up, E), stride_d = (uint64_t)E * row_bytes(c.fmt_down, F);
-    router_logits_kernel<<<dim3(NE, n_tok), 128, 0, s>>>(m->router, x, m->logits, E, NE, wnorm, eps);
-    CKM(cudaGetLastError());
-    CKM(launch_router_sel(m->logits, m->ids, m->gates, n_tok, NE, K, c.norm, c.scale, s, m->lids, m->mgates, m->base, m->n_local));
+    CKM(launch_router(moe_router_args(m, x, n_tok, wnorm, eps), s));
     const uint32_t rows_gu = (uint32_t)(stride_gu / row_bytes(c.fmt_gate_up, E)), rows_d = (uint32_t)(stride_d / row_bytes(c.fmt_down, F));
     static const int kMoePdl = getenv("FLB_MOE_PDL") ? atoi(getenv("FLB_MOE_PDL")) : 1;
     bool first_launch = true;
@@ -328,6 +296,33 @@ static int moe_enqueue_per_slot(fl_b200_moe *m, const float *x, uint32_t n_tok, 
     return FL_B200_OK;
 }
 
+// One token of a decoder step: the experts of all its slots in one launch for gate | up and one for down (matvec_expert.cu).
+static bool moe_one_token(const fl_b200_moe *m) {
+    const fl_b200_moe_cfg &c = m->c;
+    return m->world == 1 && c.top_k <= (uint32_t)m->ctx->sms && matvec_expert_takes(c.fmt_gate_up, c.n_embd, c.n_ff, c.top_k, c.n_expert) &&
+           matvec_expert_takes(c.fmt_down, c.n_ff, c.n_embd, c.top_k, c.n_expert);
+}
+
+static int moe_enqueue_one_token(fl_b200_moe *m, const float *x, float *y, const float *wnorm, float eps, const float *resid) {
+    cudaStream_t s = m->ctx->stream;
+    const fl_b200_moe_cfg &c = m->c;
+    static const int pdl = getenv("FLB_MOE_PDL") ? atoi(getenv("FLB_MOE_PDL")) : 1;
+    RouterArgs r = moe_router_args(m, x, 1, wnorm, eps);
+    r.pdl = pdl;
+    CKM(launch_router(r, s));
+    ExpertArgs e{};
+    e.n_experts = c.n_expert; e.n_slots = c.top_k; e.id = m->lids; e.status = m->ctx->status; e.pdl = pdl;
+    e.fmt = c.fmt_gate_up; e.w[0] = m->wg; e.w[1] = m->wu; e.rows = c.n_ff; e.cols = c.n_embd;
+    // the router starts its dependents after it has waited for what lies in front of it, which wrote x
+    e.x = x; e.wnorm = wnorm; e.eps = eps; e.y = m->h; e.x_ready = 1;
+    CKM(launch_matvec_expert(e, m->ctx->sms, s));
+    e.fmt = c.fmt_down; e.w[0] = m->wd; e.w[1] = nullptr; e.rows = c.n_embd; e.cols = c.n_ff;
+    e.x = m->h; e.x_stride = c.n_ff; e.wnorm = nullptr; e.y = m->part; e.x_ready = 0;
+    CKM(launch_matvec_expert(e, m->ctx->sms, s));
+    CKM(launch_wmerge(m->part, m->mgates, resid, nullptr, y, 1.0f, c.top_k, c.n_embd, c.top_k, s, pdl != 0));
+    return FL_B200_OK;
+}
+
 // the multi-column launches of the block as programmatic dependents of one another (FLB_MOE_PDL=0: plain launches)
 static const int kMoePdlNx = getenv("FLB_MOE_PDL") ? atoi(getenv("FLB_MOE_PDL")) : 1;
 
@@ -340,9 +335,7 @@ static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y,
     const fl_b200_moe_cfg &c = m->c;
     const uint32_t E = c.n_embd, F = c.n_ff, K = c.top_k, NE = c.n_expert, T = c.max_tokens;
     if (per_slot) return moe_enqueue_per_slot(m, x, n_tok, y, wnorm, eps, resid);
-    router_logits_kernel<<<dim3(NE, n_tok), 128, 0, s>>>(m->router, x, m->logits, E, NE, wnorm, eps);
-    CKM(cudaGetLastError());
-    CKM(launch_router_sel(m->logits, m->ids, m->gates, n_tok, NE, K, c.norm, c.scale, s, m->lids, m->mgates, m->base, m->n_local));
+    CKM(launch_router(moe_router_args(m, x, n_tok, wnorm, eps), s));
     CKM(launch_group_by_expert(m->lids, n_tok * K, K, m->n_local, T, m->cnt, m->tok_list, m->pair_list, s, m->table));
     // Every local expert once for up to 16 of the tokens that chose it. The table and the lists live on the device, so the
     // launch sequence is the same for every routing (and can be replayed as a graph).
@@ -391,14 +384,19 @@ int flb::moe_enqueue_tokens(fl_b200_moe *m, const float *x, uint32_t n_tok, floa
     if (n_tok == 0 || n_tok > m->c.max_tokens) return set_err(FL_B200_ERR_ARG, "moe: %u tokens outside 1..%u", n_tok, m->c.max_tokens);
     const fl_b200_moe_cfg &c = m->c;
     if (m->world > 1 && (wnorm || resid)) return set_err(FL_B200_ERR_ARG, "moe: the fused norm / residual form is for one GPU");
-    // One token inside a decoder step: per slot. The one-column kernel walks an expert faster than the multi-column one, which
-    // serves at least four columns (whole Mixtral-8x7B-shape step: 3.62 against 3.69 ms); its activation has 21 bits, relative
-    // error 2.3e-6 against 3e-7 of the grouped form, which is why a block called by itself stays on that (fl_b200_moe_forward).
+    // One token inside a decoder step: the slots' experts through the one-column kernel (whole Mixtral-8x7B-shape step: 2.28 ms;
+    // a launch per slot on the streaming kernel, which stays for the shapes the other does not take, 3.66, grouped 3.69); its
+    // activation has 21 bits, relative error 2.3e-6 against 3e-7 of the grouped form, which is why a block called by itself stays
+    // on that (fl_b200_moe_forward).
     const bool per_slot = moe_per_slot(m) || n_tok == 1;
+    if (n_tok == 1 && wnorm && moe_one_token(m)) {
+        if (n_launch) *n_launch = 4;
+        return moe_enqueue_one_token(m, x, y, wnorm, eps, resid);
+    }
     if (n_launch) {   // as moe_enqueue / moe_enqueue_per_slot enqueue them
         const bool down_streams = matvec_is_streaming(c.fmt_down, c.n_ff) && row_bytes(c.fmt_down, c.n_ff) % 16 == 0;
         const uint32_t passes = (n_tok + kNxMaxTokens - 1) / kNxMaxTokens;
-        *n_launch = (!per_slot ? 3 + 4 * passes + (passes > 1 ? 2 * passes - 1 : 0) + 1 : 2 + n_tok * (c.top_k * (down_streams ? 2u : 3u) + 1)) + (m->world > 1 ? n_tok : 0u);
+        *n_launch = (!per_slot ? 2 + 4 * passes + (passes > 1 ? 2 * passes - 1 : 0) + 1 : 1 + n_tok * (c.top_k * (down_streams ? 2u : 3u) + 1)) + (m->world > 1 ? n_tok : 0u);
     }
     return moe_enqueue(m, x, n_tok, y, per_slot, wnorm, eps, resid);
 }

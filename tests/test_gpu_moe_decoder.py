@@ -18,7 +18,7 @@ MOE_LAYERS = (0, 2)
 NE, K, F = 4, 2, 1024
 
 
-def build_moe_pair(ctx, checker, seed, n_prefill, fmt_down=capi.Q4_K, max_tokens=8):
+def build_moe_pair(ctx, checker, seed, n_prefill, fmt_down=capi.Q4_K, max_tokens=8, fmt_gu=capi.Q4_K, NE=NE, K=K, F=F):
     """build_pair's dense model, then layers MOE_LAYERS get an expert block on both sides (their dense gate / up / down
     stay set on the oracle side and are simply not used there either)."""
     dec, orc = build_pair(ctx, checker, CFG, seed, n_prefill, finalize=False)
@@ -26,13 +26,13 @@ def build_moe_pair(ctx, checker, seed, n_prefill, fmt_down=capi.Q4_K, max_tokens
     for l in MOE_LAYERS:
         rng = synth.rng_for(seed, "L%d.moe" % l)
         E = CFG["n_embd"]
-        wg = synth.q4k_tensor(rng, NE * F, E); wu = synth.q4k_tensor(rng, NE * F, E)
+        wg = synth.quant_tensor(fmt_gu, rng, NE * F, E); wu = synth.quant_tensor(fmt_gu, rng, NE * F, E)
         wd = synth.quant_tensor(fmt_down, rng, NE * E, F)
         wr = rng.standard_normal((NE, E)).astype(np.float32)     # wide logits: no near-ties between experts
-        blk = MoeBlock(ctx, E, F, NE, K, norm=1, scale=1.0, fmt_gate_up=capi.Q4_K, fmt_down=fmt_down, max_tokens=max_tokens)
+        blk = MoeBlock(ctx, E, F, NE, K, norm=1, scale=1.0, fmt_gate_up=fmt_gu, fmt_down=fmt_down, max_tokens=max_tokens)
         blk.set_weights(*(torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (wr, wg, wu, wd)))
         dec.set_layer_moe(l, blk)
-        orc.set_layer_moe(l, NE, K, 1, 1.0, F, wr, capi.Q4_K, wg, wu, fmt_down, wd)
+        orc.set_layer_moe(l, NE, K, 1, 1.0, F, wr, fmt_gu, wg, wu, fmt_down, wd)
         blocks.append(blk)
     torch.cuda.synchronize()
     dec.finalize()
@@ -86,4 +86,29 @@ def test_moe_model_run_and_batch_pass(ctx, checker):
     outs, margins = dec.step_batch([3] + seq[:5])          # teacher-forced inputs: 3, a0 .. a4
     for i, (o, mg) in enumerate(zip(outs, margins)):
         assert o == seq[i] or mg < 1e-2, (i, o, seq[i], mg)
+    dec.close(); orc.close()
+
+
+# one token: all slots' experts in one launch for gate | up and one for down (csrc/matvec_expert.cu). Columns of a part segment, of
+# one, of the most blocks a thread converts at once and of more; one slot, as many slots as experts; units that leave groups and
+# CTAs without work; the last shape is not taken (Q6_K rows of 1024 columns are no whole 16 bytes).
+@pytest.mark.parametrize("fmt_gu,fmt_down,NE,K,F", [
+    (capi.Q4_K, capi.Q4_K, 4, 1, 512), (capi.Q4_K, capi.Q4_K, 8, 3, 2304), (capi.Q6_K, capi.Q6_K, 3, 3, 2048),
+    (capi.Q4_K, capi.Q6_K, 2, 2, 10240), (capi.Q6_K, capi.Q4_K, 4, 2, 9216), (capi.Q4_K, capi.Q4_K, 2, 1, 18432), (capi.Q4_K, capi.Q6_K, 4, 2, 1024)])
+def test_one_token_over_its_experts(ctx, checker, fmt_gu, fmt_down, NE, K, F):
+    dec, orc, blocks = build_moe_pair(ctx, checker, 17, 5, fmt_down, 4, fmt_gu, NE, K, F)
+    tok = 7
+    for step in range(2):
+        want_tok = orc.step(tok)
+        got_tok = dec.step(tok)
+        got, want = dec.logits(), orc.logits()
+        assert np.all(np.isfinite(got)) and ctx.status() == 0
+        assert logits_close(got, want) < LOGIT_TOL
+        if got_tok != want_tok:
+            assert orc.margin() <= 2 * np.max(np.abs(got - want))
+        assert logits_close(dec.tap(0), orc.hidden()) < HIDDEN_TOL
+        ids, gates = blocks[-1].routing(1)
+        assert sorted(ids[0]) == sorted(int(i) for i in np.ctypeslib.as_array(orc.p.flo_llama_moe_ids(orc.h), shape=(K,)))
+        force_kv(ctx, dec, orc, CFG, 5 + step)
+        tok = want_tok
     dec.close(); orc.close()
