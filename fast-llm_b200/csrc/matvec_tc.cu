@@ -18,14 +18,14 @@
 //     lane column accumulates its own sub-block, the sub-block scales / mins are
 //     applied once per super-block in f32, and no shuffle is needed until a row is
 //     complete;
-//   * integer forms (the default for Q4_K and Q6_K; q4k_block_i8, q6k_block_i8): the
+//   * integer forms (the default; q4k_block_i8, q6k_block_i8, q8_0_block_i8): the
 //     quants go in as they are, as unsigned 8-bit operands of m16n8k32 (a masked word
 //     is four weights: one logic operation per four weights for Q4_K), the activation
 //     as fixed point per 32-column sub-block, x = 2^e n with |n| < 2^30, cut into four
 //     signed 8-bit digit planes that are the two B columns of a lane column in two
 //     instructions. Products and sums are exact integers; one huge element costs the
 //     other 31 of its sub-block at most the digits it pushes out of 30 bits;
-//   * f16 forms (FLB_TC_I8=0, and every launch that holds a Q8_0 tensor): the quants
+//   * f16 forms (FLB_TC_I8=0, and launches of Q8_0 beside K-quants): the quants
 //     become f16 values with two logic operations per PAIR of weights (the quant lands
 //     in the mantissa of a constant that an exact f16 subtraction takes off again), the
 //     activation per 256-column block as x = 2^e (hi + lo) with hi, lo f16: 22 bits;
@@ -104,7 +104,7 @@ struct TcPhase {
     int x_mode, accumulate, swiglu;
     uint32_t total_units;
     int use_q4, use_q6;
-    int q4_i8;                     // the phase runs on the integer forms (q4k_block_i8, q6k_block_i8): no Q8_0 tensor in it
+    int q4_i8;                     // the phase runs on the integer forms (q4k_block_i8 and the others): no Q8_0 tensor beside another format in it
     float *xn_out;
 };
 
@@ -126,7 +126,7 @@ struct TcArgs {
 struct TcSmem {
     uint64_t *full, *empty;        // [nslots]
     uint64_t *red_full, *red_empty;   // [2]
-    float *red;                    // [2][groups * 8][16]
+    float *red;                    // [2][groups * 8][16 rows][4 lane columns]
     float *ssq;                    // per-warp sums of squares of the prologue
     uint8_t *zero;                 // 16 zero bytes (the B operand of lanes that feed no column)
     float *xs;                     // [nblk] block scale 2^e
@@ -142,7 +142,7 @@ struct TcSmem {
 // the activation of the current phase. The ring starts at the same offset in every phase.
 __host__ __device__ inline size_t tc_head_bytes(uint32_t nslots, int groups) {
     size_t n = (size_t)nslots * 16 + 32;                  // barriers
-    n += (size_t)2 * groups * kCW * 16 * 4;              // red
+    n += (size_t)2 * groups * kCW * 64 * 4;              // red
     n += 36 * 4 + 16;                                     // ssq, 16 zero bytes
     return (n + 15) & ~(size_t)15;
 }
@@ -165,7 +165,7 @@ __device__ __forceinline__ TcSmem tc_carve(uint8_t *base, uint32_t cols, bool q4
     s.empty = (uint64_t *)p; p += nslots * 8;
     s.red_full = (uint64_t *)p; p += 16;
     s.red_empty = (uint64_t *)p; p += 16;
-    s.red = (float *)p; p += 2 * G * kCW * 16 * 4;
+    s.red = (float *)p; p += 2 * G * kCW * 64 * 4;
     s.ssq = (float *)p; p += 36 * 4;
     s.zero = p;
     p = base + tc_head_bytes(nslots, G);
@@ -268,7 +268,7 @@ __device__ __forceinline__ void q4k_block_i8(uint32_t r0, uint32_t oh, uint32_t 
 #pragma unroll
     for (int j = 4; j < 8; ++j) bx[j] = lds128(xaddr + j * xstride);
     const uint4 h0 = lds128(r0 + oh), h1 = lds128(r1 + oh);
-    int cL[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, cH[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    int cL[2][4], cH[2][4];
     const uint32_t ML = 0x0F0F0F0Fu, MH = 0xF0F0F0F0u;
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
@@ -276,25 +276,28 @@ __device__ __forceinline__ void q4k_block_i8(uint32_t r0, uint32_t oh, uint32_t 
         const uint32_t A1 = m < 2 ? word_of(wa1, 2 * m) : word_of(wb1, 2 * m - 4), B1 = m < 2 ? word_of(wa1, 2 * m + 1) : word_of(wb1, 2 * m - 3);
         const uint32_t l0 = A0 & ML, l1 = A1 & ML, l2 = B0 & ML, l3 = B1 & ML;
         const uint32_t g0 = A0 & MH, g1 = A1 & MH, g2 = B0 & MH, g3 = B1 & MH;
-        imma16832(cL[0], l0, l1, l2, l3, bx[2 * m].x, bx[2 * m].y);
-        imma16832(cH[0], g0, g1, g2, g3, bx[2 * m + 1].x, bx[2 * m + 1].y);
-        imma16832(cL[1], l0, l1, l2, l3, bx[2 * m].z, bx[2 * m].w);
-        imma16832(cH[1], g0, g1, g2, g3, bx[2 * m + 1].z, bx[2 * m + 1].w);
+        if (m == 0) {
+            imma16832_first(cL[0], l0, l1, l2, l3, bx[0].x, bx[0].y);
+            imma16832_first(cH[0], g0, g1, g2, g3, bx[1].x, bx[1].y);
+            imma16832_first(cL[1], l0, l1, l2, l3, bx[0].z, bx[0].w);
+            imma16832_first(cH[1], g0, g1, g2, g3, bx[1].z, bx[1].w);
+        } else {
+            imma16832(cL[0], l0, l1, l2, l3, bx[2 * m].x, bx[2 * m].y);
+            imma16832(cH[0], g0, g1, g2, g3, bx[2 * m + 1].x, bx[2 * m + 1].y);
+            imma16832(cL[1], l0, l1, l2, l3, bx[2 * m].z, bx[2 * m].w);
+            imma16832(cH[1], g0, g1, g2, g3, bx[2 * m + 1].z, bx[2 * m + 1].w);
+        }
     }
-    // 6-bit scales / mins of sub-blocks 2t, 2t+1 (fl_q4k_scale_min, src/runtime/quants.h:121-129), as in q4k_block
-    const uint32_t sh = 16u * (t & 1u);
-    const uint32_t shA = t >= 2 ? sh + 2u : sh, mA = t >= 2 ? 0x3030u : 0x3F3Fu, mE = t >= 2 ? 0x0F0Fu : 0u;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         const uint4 hdr = r ? h1 : h0;
-        const uint32_t sc = ((hdr.y >> shA) & mA) | ((hdr.w >> sh) & mE);
-        const uint32_t mn = ((hdr.z >> shA) & mA) | ((hdr.w >> (sh + 4u)) & mE);
+        const uint32_t sm = q4k_scales(hdr, t);
         const float d = h2f_bits((uint16_t)(hdr.x & 0xFFFFu)), dmin = h2f_bits((uint16_t)(hdr.x >> 16));
         // the four plane sums of a sub-block as one number: two exact integer steps (|.| < 2^28), then f32
         const float tl = fmaf((float)(cL[0][2 * r] * 256 + cL[0][2 * r + 1]), 65536.f, (float)(cL[1][2 * r] * 256 + cL[1][2 * r + 1]));
         const float th = fmaf((float)(cH[0][2 * r] * 256 + cH[0][2 * r + 1]), 65536.f, (float)(cH[1][2 * r] * 256 + cH[1][2 * r + 1]));
-        const float q = u8f<0>(sc) * (xs2.x * tl) + u8f<1>(sc) * (xs2.y * th);   // the sums in the activation's units first
-        const float mm = u8f<0>(mn) * sx.x + u8f<1>(mn) * sx.y;
+        const float q = u8f<0>(sm) * (xs2.x * tl) + u8f<1>(sm) * (xs2.y * th);   // the sums in the activation's units first
+        const float mm = u8f<2>(sm) * sx.x + u8f<3>(sm) * sx.y;
         (r ? out1 : out0) = d * q - dmin * mm;
     }
 }
@@ -464,9 +467,9 @@ __device__ __forceinline__ void q6k_block_i8(uint32_t r0, uint32_t r1, uint32_t 
                           : gq == 2 ? ((a >> 4) & 0x0F0F0F0Fu) | (h & 0x30303030u)
                                     : ((b >> 4) & 0x0F0F0F0Fu) | ((h >> 2) & 0x30303030u);
             }
-        int c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
-        imma16832(c0, q[0][0], q[1][0], q[0][1], q[1][1], bx[gq].x, bx[gq].y);
-        imma16832(c1, q[0][0], q[1][0], q[0][1], q[1][1], bx[gq].z, bx[gq].w);
+        int c0[4], c1[4];
+        imma16832_first(c0, q[0][0], q[1][0], q[0][1], q[1][1], bx[gq].x, bx[gq].y);
+        imma16832_first(c1, q[0][0], q[1][0], q[0][1], q[1][1], bx[gq].z, bx[gq].w);
         imma16832(c0, q[0][2], q[1][2], q[0][3], q[1][3], bx[4 + gq].x, bx[4 + gq].y);
         imma16832(c1, q[0][2], q[1][2], q[0][3], q[1][3], bx[4 + gq].z, bx[4 + gq].w);
 #pragma unroll
@@ -517,6 +520,42 @@ __device__ __forceinline__ void q8_0_block(uint32_t r0, uint32_t r1, uint32_t xa
     }
 }
 
+// Q8_0, integer form: the int8 quants as they are, signed operands of m16n8k32, against the digit planes of q4k_block_i8 (the same
+// image: 64 consecutive columns per lane column, blocks 2 t and 2 t + 1 its two sub-blocks; xs2 their activation scales). No
+// conversion is left: about 110 instructions a lane where the f16 form takes 260 (3B-class 8-bit model: 1147 -> 1046 us a step).
+__device__ __forceinline__ void q8_0_block_i8(uint32_t r0, uint32_t r1, uint32_t xaddr, uint32_t xstride, float2 xs2, float &out0, float &out1) {
+    uint32_t w0[17], w1[17];
+#pragma unroll
+    for (int i = 0; i < 17; ++i) { w0[i] = lds32(r0 + 4 * i); w1[i] = lds32(r1 + 4 * i); }
+    int cA[2][4], cB[2][4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const uint4 xa = lds128(xaddr + 2 * m * xstride), xb = lds128(xaddr + (2 * m + 1) * xstride);
+        const uint32_t a0 = __byte_perm(w0[2 * m], w0[2 * m + 1], 0x5432u), a1 = __byte_perm(w1[2 * m], w1[2 * m + 1], 0x5432u);
+        const uint32_t a2 = __byte_perm(w0[2 * m + 1], w0[2 * m + 2], 0x5432u), a3 = __byte_perm(w1[2 * m + 1], w1[2 * m + 2], 0x5432u);
+        const uint32_t b0 = w0[9 + 2 * m], b1 = w1[9 + 2 * m], b2 = w0[10 + 2 * m], b3 = w1[10 + 2 * m];
+        if (m == 0) {
+            imma16832_ss_first(cA[0], a0, a1, a2, a3, xa.x, xa.y);
+            imma16832_ss_first(cB[0], b0, b1, b2, b3, xb.x, xb.y);
+            imma16832_ss_first(cA[1], a0, a1, a2, a3, xa.z, xa.w);
+            imma16832_ss_first(cB[1], b0, b1, b2, b3, xb.z, xb.w);
+        } else {
+            imma16832_ss(cA[0], a0, a1, a2, a3, xa.x, xa.y);
+            imma16832_ss(cB[0], b0, b1, b2, b3, xb.x, xb.y);
+            imma16832_ss(cA[1], a0, a1, a2, a3, xa.z, xa.w);
+            imma16832_ss(cB[1], b0, b1, b2, b3, xb.z, xb.w);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const uint32_t *w = r ? w1 : w0;
+        const float dA = h2f_bits((uint16_t)(w[0] & 0xFFFFu)), dB = h2f_bits((uint16_t)(w[8] >> 16));
+        const float ta = fmaf((float)(cA[0][2 * r] * 256 + cA[0][2 * r + 1]), 65536.f, (float)(cA[1][2 * r] * 256 + cA[1][2 * r + 1]));
+        const float tb = fmaf((float)(cB[0][2 * r] * 256 + cB[0][2 * r + 1]), 65536.f, (float)(cB[1][2 * r] * 256 + cB[1][2 * r + 1]));
+        (r ? out1 : out0) = dA * (xs2.x * ta) + dB * (xs2.y * tb);
+    }
+}
+
 // ---- grid barrier --------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t *p) {
     uint32_t v;
@@ -557,7 +596,7 @@ __device__ __forceinline__ bool grid_barrier(GridBar *b, uint32_t nblocks, uint3
 // between; the producer does not take part in the barriers: the weights of the next phase are already
 // streaming into the ring while the current phase drains and the next activation is built.
 // F: 0 = every format and form, decided per phase at run time (f16 forms, Q8_0 beside K-quants, several phases); 1 / 2 / 3 / 4 =
-// one phase holding Q4_K tensors only / Q6_K only / both (integer forms) / Q8_0 only (f16 form): what a decode step launches. The specialised
+// one phase holding Q4_K tensors only / Q6_K only / both / Q8_0 only (integer forms): what a decode step launches. The specialised
 // instances carry only their own code (the whole kernel is some 7000 instructions, and a launch that has to fetch its
 // path out of that from L2 starts later) and get their own register allocation.
 // R: 256-column blocks a half-warp of the prologue converts (F != 0: 1 up to 34 blocks = 8704 columns, else 2; the
@@ -657,7 +696,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
     for (int p = 0; p < a.n_phases; ++p) {
         const TcPhase &ph = a.ph[p];
         const uint32_t nblk = ph.cols / 256, nseg = (nblk + 7) / 8;
-        const bool I8 = F ? F != 4 : ph.q4_i8 != 0, UQ4 = F ? (F & 5) != 0 : ph.use_q4 != 0, UQ6 = F ? (F & 2) != 0 : ph.use_q6 != 0;
+        const bool I8 = F ? true : ph.q4_i8 != 0, UQ4 = F ? (F & 5) != 0 : ph.use_q4 != 0, UQ6 = F ? (F & 2) != 0 : ph.use_q6 != 0;
         const TcSmem sm = tc_carve<G>(smem_raw, ph.cols, UQ4, UQ6, I8, S, a.ring_off);
         const uint32_t my_units = blockIdx.x < ph.total_units ? (ph.total_units - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
         const bool late = F == 0 && p > 0;   // the activation was written by the previous phase of this launch: read it past L1
@@ -772,6 +811,12 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                         V[i] = ((uint32_t)__float2int_rn(v[i] * inv_s) + 0x00808080u) ^ 0x00808080u;
                     }
                     const float sum32 = sum + __shfl_xor_sync(0xffffffffu, sum, 1);
+                    float odd = 0.f;   // Q8_0 has no term with the sums, which carry an infinity or a NaN for the other formats
+                    if (F == 4) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) odd = fmaf(v[i], 0.f, odd);
+                        odd += __shfl_xor_sync(0xffffffffu, odd, 1);
+                    }
                     uint32_t P[4][4];   // [plane: 0 = most significant digit][group of four elements]
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
@@ -793,7 +838,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                                 sts64(base + (m0 + mm) * 256u + (pl & 1) * 16u + (pl >> 1) * 8u, P[pl][2 * mm], P[pl][2 * mm + 1]);
                         if ((hl & 1u) == 0) {
                             sm.s4[blk * 8 + (hl >> 1)] = sum32;
-                            sm.xs8[blk * 8 + (hl >> 1)] = __uint_as_float((uint32_t)(127 + e - (h ? 4 : 0)) << 23);
+                            sm.xs8[blk * 8 + (hl >> 1)] = __uint_as_float((uint32_t)(127 + e - (h && F != 4 ? 4 : 0)) << 23) + odd;   // (high nibbles are 16 q)
                         }
                     }
                     if (live && UQ6) {
@@ -843,7 +888,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                 }
                 const float sum32 = sum + __shfl_xor_sync(0xffffffffu, sum, 1);
                 if (live) {
-                    if ((F == 0 || F == 4) && UQ4 && !I8) {
+                    if (F == 0 && UQ4 && !I8) {
                         // columns 16 hl .. 16 hl + 15: chunk c = hl / 4, sub-block half (hl / 2) & 1, words 4 (hl & 1) + j
                         const uint32_t c = hl >> 2, sub = (hl >> 1) & 1u, j0 = 4 * (hl & 1u);
                         const uint32_t base = smem_u32(sm.x4) + blk * 1024u;
@@ -897,9 +942,12 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                 if (!mbar_wait_bounded(&sm.red_full[buf], (kk >> 1) & 1u, a.status)) return;
                 float v = 0.f;
                 if (lane < 16) {
-                    const float *pp = sm.red + buf * kConsumers * 16 + lane;
+                    const float4 *pp = reinterpret_cast<const float4 *>(sm.red + buf * kConsumers * 64) + lane;
 #pragma unroll
-                    for (uint32_t w = 0; w < kConsumers; ++w) v += pp[w * 16];
+                    for (uint32_t w = 0; w < kConsumers; ++w) {
+                        const float4 p = pp[w * 16];
+                        v += (p.x + p.y) + (p.z + p.w);
+                    }
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sm.red_empty[buf]);
@@ -960,11 +1008,11 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                         mbar_wait_or_die(&sm.full[c_slot], c_par, a.status, dead);
                         if (blk < nblk) {
                             const uint32_t r0 = ring + c_slot * a.slot_bytes + ((w >> 2) * 16 + g) * kPitch8 + (w & 3u) * 272u + t * 68u;
+                            const float2 xs2 = *reinterpret_cast<const float2 *>(sm.xs8 + blk * 8 + 2 * t);
                             float o0, o1;
-                            q8_0_block(r0, r0 + 8 * kPitch8, xa4 + blk * xb, xstride, o0, o1);
-                            const float xs = sm.xs[blk];
-                            acc0 = fmaf(xs, o0, acc0);
-                            acc1 = fmaf(xs, o1, acc1);
+                            q8_0_block_i8(r0, r0 + 8 * kPitch8, xa4 + blk * xb, xstride, xs2, o0, o1);
+                            acc0 += o0;
+                            acc1 += o1;
                         }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&sm.empty[c_slot]);
@@ -1067,18 +1115,12 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                         if (c_slot >= S) { c_slot -= S; c_par ^= 1u; }
                     }
                 }
-                // the unit's partial sums of rows g and g + 8 over this warp's lane columns
-                acc0 += __shfl_xor_sync(0xffffffffu, acc0, 1);
-                acc1 += __shfl_xor_sync(0xffffffffu, acc1, 1);
-                acc0 += __shfl_xor_sync(0xffffffffu, acc0, 2);
-                acc1 += __shfl_xor_sync(0xffffffffu, acc1, 2);
+                // the unit's partial sums of rows g and g + 8, one per lane column (the finalizer adds those too)
                 const uint32_t buf = kk & 1u;
                 mbar_wait_or_die(&sm.red_empty[buf], ((kk >> 1) & 1u) ^ 1u, a.status, dead);
-                if (t == 0) {
-                    float *pp = sm.red + (buf * kConsumers + warp) * 16;
-                    pp[g] = acc0;
-                    pp[g + 8] = acc1;
-                }
+                float *pp = sm.red + (buf * kConsumers + warp) * 64 + lane;
+                pp[0] = acc0;
+                pp[32] = acc1;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sm.red_full[buf]);
             }
@@ -1112,8 +1154,8 @@ cudaError_t matvec_tc_init(void) {
 
 // True when the launch can run on the tensor-core kernel: Q4_K / Q6_K / Q8_0 tensors only, whole 256-column
 // blocks, 16-byte aligned rows, no expert indirection and no exchange prologue.
-// Q4_K and Q6_K on the integer forms (q4k_block_i8, q6k_block_i8) unless FLB_TC_I8=0; a launch that holds a Q8_0
-// tensor stays on the f16 forms (Q8_0 reads the f16 image of the activation).
+// The integer forms (q4k_block_i8, q6k_block_i8, q8_0_block_i8) unless FLB_TC_I8=0; a launch of Q8_0 beside another format, or with
+// what only the general instance does, stays on the f16 forms.
 bool tc_q4_i8() {
     static const bool on = !(getenv("FLB_TC_I8") && getenv("FLB_TC_I8")[0] == '0');
     return on;
@@ -1144,7 +1186,7 @@ bool matvec_tc_eligible(const MatvecArgs &a) {
     }
     if (a.swiglu && (a.n_tensors != 2 || a.t[0].rows != a.t[1].rows || a.t[0].fmt != a.t[1].fmt || a.accumulate)) return false;
     const uint32_t slot = q8 ? kSlot8 : q6 ? kSlot6 : kSlot4;
-    return tc_head_bytes(2, groups) + tc_x_bytes(a.cols, q4, q6, !q8 && tc_q4_i8()) + 1024 + 2u * slot <= 227 * 1024 - 1024;
+    return tc_head_bytes(2, groups) + tc_x_bytes(a.cols, q4, q6, tc_q4_i8()) + 1024 + 2u * slot <= 227 * 1024 - 1024;
 }
 
 // One launch of n dependent matvecs (phase i + 1 consumes what phase i writes). n = 1: a plain launch.
@@ -1189,7 +1231,7 @@ cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaS
         ph.x = a.x; ph.x2 = a.x2; ph.wnorm = a.wnorm; ph.eps = a.eps; ph.cols = a.cols; ph.x_mode = a.x_mode;
         ph.accumulate = a.accumulate; ph.swiglu = a.swiglu; ph.total_units = units;
         ph.use_q4 = q4 ? 1 : 0; ph.use_q6 = q6 ? 1 : 0;
-        ph.q4_i8 = (!q8 && tc_q4_i8()) ? 1 : 0;
+        ph.q4_i8 = (tc_q4_i8() && (!q8 || (only8 && n == 1 && tc_special() && a.x_mode != MV_X_SILU_MUL && a.xn_out == nullptr))) ? 1 : 0;
         all8 = all8 && only8;
         ph.xn_out = a.xn_out;
         any6 = any6 || q6;
@@ -1226,7 +1268,7 @@ cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaS
         const bool pdl = args[0].pdl != 0;
         const TcPhase &p0 = k.ph[0];
         // the specialised instances: one phase, integer forms or Q8_0 alone, plain or RMSNorm prologue, no copy of the activation asked for
-        const bool special = n == 1 && (p0.q4_i8 || all8) && tc_special() && p0.x_mode != MV_X_SILU_MUL && p0.xn_out == nullptr;
+        const bool special = n == 1 && p0.q4_i8 && tc_special() && p0.x_mode != MV_X_SILU_MUL && p0.xn_out == nullptr;
         const int f = special ? (all8 ? 4 : (p0.use_q4 ? 1 : 0) | (p0.use_q6 ? 2 : 0)) : 0;
         const bool one = p0.cols / 256 <= 2u * (2 * kCW + 1);   // every half-warp of the prologue converts at most one block
         if (f == 1) return one ? launch_kernel(matvec_tc_kernel<2, 1, 1>, dim3(grid), block, smem, stream, pdl, k)
@@ -1234,7 +1276,7 @@ cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaS
         // Q6_K only: the two-block instance for every width (the one-block instance spills in its consume loop: with 18
         // warps a thread can have 96 registers, five warps share a quarter of the register file)
         if (f == 2) return launch_kernel(matvec_tc_kernel<2, 2, 2>, dim3(grid), block, smem, stream, pdl, k);
-        if (f == 4) return launch_kernel(matvec_tc_kernel<2, 4, 2>, dim3(grid), block, smem, stream, pdl, k);   // (one block: spills)
+        if (f == 4) return launch_kernel(matvec_tc_kernel<2, 4, 2>, dim3(grid), block, smem, stream, pdl, k);   // (one block: 36 bytes of spills; a step of the 3B-class 8-bit model 1136 instead of 1046 us)
         if (f == 3) return one ? launch_kernel(matvec_tc_kernel<2, 3, 1>, dim3(grid), block, smem, stream, pdl, k)
                                : launch_kernel(matvec_tc_kernel<2, 3, 2>, dim3(grid), block, smem, stream, pdl, k);
         return launch_kernel(matvec_tc_kernel<2, 0, 0>, dim3(grid), block, smem, stream, pdl, k);

@@ -510,3 +510,32 @@ def multi_column_case(ctx, checker, fmt, rows, cols, nx):
     ctx.matvec(fmt, wd, rows, cols, xd, yd2, nx=nx, xstride=xstride, ystride=ystride)
     ctx.sync()
     assert np.array_equal(bits(yd2.cpu().numpy()), bits(got))
+
+
+# Q8_0 with one column: the integer form of matvec_tc.cu. Blocks of a part segment, of one and of two rounds of the prologue, rows of
+# a part unit. Products and the sums of a block are exact (the activation to 2^-30 of its block's maximum, two roundings to 24
+# bits); what is left are the roundings of at most 16 f32 sums of the warps and of their chain of 5 segments, each 2^-24 of the
+# running sum: relative 2-norm error below sqrt(25) 2^-24 = 3e-7 for random signs.
+@pytest.mark.parametrize("rows,cols", [(1, 256), (15, 2048), (17, 2304), (33, 3072), (100, 8704), (40, 8960), (64, 17408), (2400, 4096)])
+def test_matvec_q8_0_one_column(ctx, rows, cols):
+    rng = np.random.default_rng(rows + cols)
+    w = torch.from_numpy(synth.quant_tensor(capi.Q8_0, rng, rows, cols)).cuda()
+    f = torch.empty((rows, cols), device="cuda")
+    x = torch.from_numpy(rng.standard_normal(cols).astype(np.float32)).cuda()
+    y = torch.empty(rows, device="cuda")
+    torch.cuda.synchronize()
+    ctx.dequant(capi.Q8_0, w, rows, cols, f)
+    ctx.matvec_assign(capi.Q8_0, w, rows, cols, x, y)
+    ctx.sync()
+    want = f.double() @ x.double()
+    assert float((y.double() - want).norm() / (f.double().abs() @ x.double().abs()).norm()) <= 3e-7
+    if rows > 16:
+        assert float((y.double() - want).norm() / want.norm()) <= 3e-7
+    for bad in (float("inf"), -float("inf"), float("nan")):   # an infinity or a NaN in one block shows in every row
+        z = x.clone()
+        z[cols // 2 + 5] = bad
+        torch.cuda.synchronize()
+        ctx.matvec_assign(capi.Q8_0, w, rows, cols, z, y)
+        ctx.sync()
+        assert not bool(torch.isfinite(y).any())
+    assert ctx.status() == 0

@@ -85,3 +85,17 @@ def test_an_outlier_costs_only_its_own_sub_block():
     assert err[own].max() <= 2.0 ** -30 * abs(x[77])                # 30 bits under the outlier: 1e-5 of a unit element
     other = np.ones(256, bool); other[own] = False
     assert err[other].max() <= 2.0 ** -29 * np.abs(x[other]).max()
+
+
+def test_q8_0_block_dot_from_digit_planes_is_exact():
+    """Signed quants against the digit planes (q8_0_block_i8): the plane sums and their two integer steps stay inside int32 and
+    give the integer dot product, at the extremes too."""
+    rng = np.random.default_rng(4)
+    top = np.full(32, 2 ** 30 - 1, np.int64)
+    for q, n in [(rng.integers(-128, 128, 32), fixed_point(rng.standard_normal(32).astype(np.float32))[1]) for _ in range(200)] + \
+                [(np.full(32, -128), top), (np.full(32, 127), -top), (np.full(32, -128), np.full(32, 0x7F7F80))]:
+        q = q.astype(np.int64)
+        p = [int(np.sum(q * d)) for d in digits_of(n)]
+        hi, lo = p[0] * 256 + p[1], p[2] * 256 + p[3]
+        assert max(abs(hi), abs(lo)) < 2 ** 31
+        assert hi * 65536 + lo == int(np.sum(q * n))
