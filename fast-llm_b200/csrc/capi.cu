@@ -264,12 +264,12 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
             // this call or the one before may be on the tcgen05 form, whose image is another one
             const bool reuse = same_columns && nx <= kNxMaxTokens && tm <= 0;
             if (!reuse) {
-                in.dep_first = pdl == kPdlAfter;
                 e = launch_nx_convert(in, &t, 1, cols, nt, c->xq, kNxTgs, c->stream, pdl != 0);
                 if (e == cudaErrorNotSupported) break;
                 if (e != cudaSuccess) return cuda_err(e, "activation conversion launch");
             }
-            // the matmul overlaps the conversion's launch: it reads weights only until the conversion has completed
+            // the matmul overlaps the conversion: it starts after what lies in front of that has completed, and reads weights only until
+            // the conversion has
             const uint32_t most = !in.tm ? parts : planes ? kMaxPlanes : 1;   // (how many planes a slice leaves then depends on its rows)
             const uint32_t cap = (uint32_t)(kNxPartFloats / ((size_t)most * nt)) & ~15u, slice = most == 1 || rows <= cap ? rows : cap;
             const size_t rb = pitch ? pitch : row_bytes(fmt, cols);

@@ -209,7 +209,6 @@ struct ConvArgs {
     const float *att;              // the columns are attention contexts of heads of 128, added up here from n_splits records
     uint32_t n_splits;             // (attn.cu: [column][head][split][132] = context, maximum, sum)
     int tm;                        // img4 or img6 is the image of matmul_tm.cu
-    int dep_first;                 // see NxIn
 };
 // Device-side table of a grouped launch: word 0 = number of active groups, word 1 = the most token groups of one; then four
 // words per active group: {group, number of columns, token groups in front of it, columns in front of it}.
@@ -227,19 +226,21 @@ __device__ __forceinline__ float4 sum_planes(const float *p, uint32_t n, size_t 
 }
 
 // Four dimensions (4 lane ..) of one head's context from its splits' records (attn_decode_kernel's combine, with all lanes of
-// a warp on one head): the weights from every split's maximum and sum, then the contexts in split order, 16 in flight.
+// a warp on one head): the weights from every split's maximum and sum, then the contexts in split order, 40 in flight: it is bound
+// by the latency of its loads (8 positions, 37 splits, launch to launch: 9.3 us with 16 in flight, three round trips to L2; now 5.8).
 __device__ __forceinline__ float4 combine_records(const float *part, uint32_t S, uint32_t lane) {
     const float m0 = lane < S ? __ldcg(part + (size_t)lane * kAttnRecord + 128) : -INFINITY;
     const float m1 = lane + 32 < S ? __ldcg(part + (size_t)(lane + 32) * kAttnRecord + 128) : -INFINITY;
     const float l0 = lane < S ? __ldcg(part + (size_t)lane * kAttnRecord + 129) : 0.f;
     const float l1 = lane + 32 < S ? __ldcg(part + (size_t)(lane + 32) * kAttnRecord + 129) : 0.f;
+    constexpr int kFlight = 40;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     float w0 = 0.f, w1 = 0.f, L = 1.f;
 #pragma unroll 1
-    for (uint32_t s0 = 0; s0 < S; s0 += 16) {
-        float4 ov[16];
+    for (uint32_t s0 = 0; s0 < S; s0 += kFlight) {
+        float4 ov[kFlight];
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
+        for (int j = 0; j < kFlight; ++j)
             ov[j] = s0 + j < S ? __ldcg(reinterpret_cast<const float4 *>(part + (size_t)(s0 + j) * kAttnRecord) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
         if (s0 == 0) {   // the first contexts are on their way meanwhile
             const float mx = warp_max(fmaxf(m0, m1));
@@ -248,8 +249,9 @@ __device__ __forceinline__ float4 combine_records(const float *part, uint32_t S,
             L = warp_sum(l0 * w0 + l1 * w1);
         }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const float w = __shfl_sync(0xffffffffu, s0 < 32 ? w0 : w1, (s0 + j) & 31u);
+        for (int j = 0; j < kFlight; ++j) {
+            const uint32_t sp = s0 + j;
+            const float w = __shfl_sync(0xffffffffu, sp < 32 ? w0 : w1, sp & 31u);
             acc.x = fmaf(ov[j].x, w, acc.x); acc.y = fmaf(ov[j].y, w, acc.y);
             acc.z = fmaf(ov[j].z, w, acc.z); acc.w = fmaf(ov[j].w, w, acc.w);
         }
@@ -260,18 +262,19 @@ __device__ __forceinline__ float4 combine_records(const float *part, uint32_t S,
 
 // grid (blocks, columns rounded up to groups of four, groups), 64 threads: a block converts 256 values of one column, a thread
 // four consecutive ones. What bounds it is latency (a launch moves well under a megabyte): hence few values per thread, every
-// plane in flight, and as many blocks as there are (block, column) pairs.
+// plane in flight, and as many blocks as there are (block, column) pairs. ATT: the columns are attention contexts (a.att), an instance
+// of its own for the registers of the records in flight (254 against 54).
+template <bool ATT>
 __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     __shared__ float2 half_s[2];   // per warp: maximum, sum of squares
     const uint32_t blk = blockIdx.x, warp = threadIdx.x >> 5;
     const uint32_t pp = blockIdx.y & 3u, i = threadIdx.x, hl = i >> 2, tq = i & 3u;   // column of the group; values 16 hl + 4 tq ..
-    // launched as a programmatic dependent: the launch itself overlaps the tail of the kernel before, whose output
-    // (x, the table) is read only after it has completed
-    if (!a.dep_first) griddep_launch_dependents();
+    // Launched as a programmatic dependent: the launch itself overlaps the tail of the kernel before, whose output (x, the table) is
+    // read only after it has completed. Its own dependent, the matmul, starts when this kernel's loads are back: started at once it
+    // fills its rings, 30 MB of weights, in front of them (pass of 8 positions, 8B shape: 3216 -> 3115 us, gate | up to down 5.3 -> 3.6).
     float4 wn = make_float4(1.f, 1.f, 1.f, 1.f);
     if (a.wnorm) wn = __ldg(reinterpret_cast<const float4 *>(a.wnorm + blk * 256 + 4 * i));   // a constant
     griddep_wait();
-    if (a.dep_first) griddep_launch_dependents();
     uint32_t n_valid = a.P, tg = blockIdx.y >> 2, ntg = (a.P + 3) / 4, tg0 = 0, grp = 0, row0 = 0;
     if (a.table) {
         if (blockIdx.z >= a.table[0]) return;
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
         const size_t at = row * a.xstride + blk * 256 + 4 * i, rat = (size_t)p * a.rstride + blk * 256 + 4 * i;
         float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
         if (a.resid) r = *reinterpret_cast<const float4 *>(a.resid + rat);
-        if (a.att) v = combine_records(a.att + ((size_t)p * (2 * a.nblk) + 2 * blk + warp) * a.n_splits * kAttnRecord, a.n_splits, threadIdx.x & 31u);
+        if (ATT) v = combine_records(a.att + ((size_t)p * (2 * a.nblk) + 2 * blk + warp) * a.n_splits * kAttnRecord, a.n_splits, threadIdx.x & 31u);
         else v = sum_planes(a.x + at, a.n_parts, a.part_stride);
         if (a.x2) {   // fl_op_silu_mul (src/runtime/decode_params.h:267-272)
             const float4 u = sum_planes(a.x2 + at, a.n_parts, a.part_stride);
@@ -302,6 +305,7 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
             v.x *= wn.x; v.y *= wn.y; v.z *= wn.z; v.w *= wn.w;
         }
     }
+    griddep_launch_dependents();
     if (!a.img4 && !a.img6 && !a.img8) return;   // only the sum was asked for
     float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
     amax = warp_max(amax);
@@ -1047,14 +1051,14 @@ cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t
     ConvArgs c{};
     c.x = in.x; c.x2 = in.x2; c.part_stride = in.part_stride; c.resid = in.resid; c.x_out = in.x_out; c.wnorm = in.wnorm;
     c.xstride = in.xstride; c.rstride = in.rstride; c.n_parts = in.n_parts ? in.n_parts : 1; c.P = P; c.nblk = cols / 256;
-    c.tm = in.tm; c.dep_first = in.dep_first;
+    c.tm = in.tm;
     if (in.tm && (q8 || q4 == q6 || in.table)) return cudaErrorNotSupported;
     if (q4) c.img4 = xq;
     if (q6) c.img6 = xq + nx_image_off(FMT_Q6_K, q4, q6, cols, tgs_cap);
     if (q8) c.img8 = xq + nx_image_off(FMT_Q8_0, q4, q6, cols, tgs_cap);
     c.att = in.att; c.n_splits = in.n_splits;
     c.table = in.table; c.col_idx = in.col_idx; c.list_stride = in.list_stride; c.col_off = in.col_off;
-    return launch_kernel(act_convert_nx_kernel, dim3(cols / 256, (P + 3) / 4 * 4, in.table ? in.n_groups : 1), dim3(64), 0, stream, pdl, c);
+    return launch_kernel(in.att ? act_convert_nx_kernel<true> : act_convert_nx_kernel<false>, dim3(cols / 256, (P + 3) / 4 * 4, in.table ? in.n_groups : 1), dim3(64), 0, stream, pdl, c);
 }
 
 cudaError_t launch_nx_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,

@@ -240,7 +240,7 @@ static int moe_enqueue_per_slot(fl_b200_moe *m, const float *x, uint32_t n_tok, 
     fl_b200_ctx *ctx = m->ctx;
     cudaStream_t s = ctx->stream;
     const fl_b200_moe_cfg &c = m->c;
-    const uint32_t E = c.n_embd, F = c.n_ff, K = c.top_k, NE = c.n_expert;
+    const uint32_t E = c.n_embd, F = c.n_ff, K = c.top_k;
     const uint64_t stride_gu = (uint64_t)F * row_bytes(c.fmt_gate_up, E), stride_d = (uint64_t)E * row_bytes(c.fmt_down, F);
     CKM(launch_router(moe_router_args(m, x, n_tok, wnorm, eps), s));
     const uint32_t rows_gu = (uint32_t)(stride_gu / row_bytes(c.fmt_gate_up, E)), rows_d = (uint32_t)(stride_d / row_bytes(c.fmt_down, F));
@@ -333,7 +333,7 @@ static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y,
     fl_b200_ctx *ctx = m->ctx;
     cudaStream_t s = ctx->stream;
     const fl_b200_moe_cfg &c = m->c;
-    const uint32_t E = c.n_embd, F = c.n_ff, K = c.top_k, NE = c.n_expert, T = c.max_tokens;
+    const uint32_t E = c.n_embd, F = c.n_ff, K = c.top_k, T = c.max_tokens;
     if (per_slot) return moe_enqueue_per_slot(m, x, n_tok, y, wnorm, eps, resid);
     CKM(launch_router(moe_router_args(m, x, n_tok, wnorm, eps), s));
     CKM(launch_group_by_expert(m->lids, n_tok * K, K, m->n_local, T, m->cnt, m->tok_list, m->pair_list, s, m->table));
