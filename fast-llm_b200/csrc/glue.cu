@@ -109,11 +109,66 @@ __global__ void __launch_bounds__(kRouterWarps * 32) router_sel_kernel(const flo
     router_select(logits + (size_t)tok * n_expert, w_s[warp], g_s[warp], lane, tok, n_expert, o);
 }
 
+// The table of a grouped multi-column launch (matvec_tc_nx.cu), by one warp: active experts in ascending order, their
+// columns from col_off on (at most P), the groups of four columns in front of them and the columns in front of them.
+__device__ __forceinline__ void nx_table_warp(const uint32_t *cnt, uint32_t n_local, uint32_t col_off, uint32_t P, uint32_t *table) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t n_act = 0, before = 0, most = 0;   // before: groups of four, columns << 16
+    for (uint32_t b = 0; b < n_local; b += 32) {
+        const uint32_t e = b + lane, c = e < n_local ? cnt[e] : 0u;
+        const uint32_t n = c > col_off ? min(c - col_off, P) : 0u, tg = (n + 3) / 4, own = tg | n << 16;
+        uint32_t incl = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += v;
+        }
+        const uint32_t mask = __ballot_sync(0xffffffffu, n != 0), at = before + incl - own;
+        if (n) reinterpret_cast<uint4 *>(table)[1 + n_act + __popc(mask & ((1u << lane) - 1u))] = make_uint4(e, n, at & 0xFFFFu, at >> 16);
+        n_act += __popc(mask);
+        most = max(most, __reduce_max_sync(0xffffffffu, tg));
+        before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) { table[0] = n_act; table[1] = most; }
+}
+
+// One warp: a stable counting sort of the (token, slot) pairs by local expert (within an expert they stay in ascending order).
+// The counts in shared memory (in device memory every expert was a round trip: 3 us for 8 of them).
+__global__ void __launch_bounds__(32) group_by_expert_kernel(const uint32_t *lids, uint32_t n_pairs, uint32_t top_k, uint32_t n_local, uint32_t cap,
+                                                             uint32_t *cnt, uint32_t *tok_list, uint32_t *pair_list, uint32_t *table) {
+    __shared__ uint32_t n_s[256];
+    const uint32_t lane = threadIdx.x;
+    griddep_launch_dependents();
+    griddep_wait();
+    for (uint32_t e = lane; e < n_local; e += 32) n_s[e] = 0;
+    __syncwarp();
+    for (uint32_t b = 0; b < n_pairs; b += 32) {
+        const uint32_t pair = b + lane;
+        const uint32_t e = pair < n_pairs ? __ldcg(lids + pair) : 0xFFFFFFFFu;
+        for (uint32_t x = 0; x < n_local; ++x) {
+            const uint32_t mask = __ballot_sync(0xffffffffu, e == x);
+            if (mask == 0) continue;
+            const uint32_t base = n_s[x];
+            if (e == x) {
+                const uint32_t pos = base + __popc(mask & ((1u << lane) - 1u));
+                if (pos < cap) { tok_list[(size_t)x * cap + pos] = pair / top_k; pair_list[(size_t)x * cap + pos] = pair; }
+            }
+            __syncwarp();
+            if (lane == 0) n_s[x] = min(base + __popc(mask), cap);
+            __syncwarp();
+        }
+    }
+    for (uint32_t e = lane; e < n_local; e += 32) cnt[e] = n_s[e];
+    nx_table_warp(n_s, n_local, 0, kNxMaxTokens, table);
+}
+
 // Router of a block: logits[t][e] = dot(router[e], x[t]), one block per (expert, token), and the selection by the block that is the
 // last of its token. wnorm != nullptr: x is the raw hidden state and the logits are those of RMSNorm(x) * wnorm (fl_op_rmsnorm,
 // src/runtime/decode_params.h:101-106, fused: every block norms the token itself). Bound by latency: the router's rows and the norm
 // weights are requested before the dependency, the selection saves a launch (8 experts of 4096 columns, one token, inside a
-// step: 10.1 us in two launches -> 5.4).
+// step: 10.1 us in two launches -> 5.4; the grouping of several tokens' pairs in here too cost more than its launch, 12.4 us).
+// AFTER: nothing is read before the dependency is met.
+template <bool AFTER>
 __global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
     __shared__ float red[4], w_s[256], g_s[256];
     __shared__ uint32_t last;
@@ -127,9 +182,15 @@ __global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
     for (int k = 0; k < kAhead; ++k) {
         const uint32_t i = threadIdx.x + 128 * k;
         wa[k] = ga[k] = xa[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i < n4) { wa[k] = __ldg(w + i); if (gn) ga[k] = __ldg(gn + i); }
+        if (i < n4 && !AFTER) { wa[k] = __ldg(w + i); if (gn) ga[k] = __ldg(gn + i); }
     }
     griddep_wait();
+    if (AFTER)
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const uint32_t i = threadIdx.x + 128 * k;
+            if (i < n4) { wa[k] = __ldcg(w + i); if (gn) ga[k] = __ldcg(gn + i); }
+        }
     griddep_launch_dependents();   // what starts now may take x for complete (ExpertArgs::x_ready)
 #pragma unroll
     for (int k = 0; k < kAhead; ++k)
@@ -208,15 +269,22 @@ __global__ void wmerge_kernel(const float *__restrict__ parts, const float *__re
 __global__ void wmerge_tokens_kernel(const float *__restrict__ parts, const float *__restrict__ gates, float *y, uint32_t n_parts,
                                      uint32_t n, uint32_t n_planes, size_t plane_stride, const float *resid,
                                      const uint32_t *__restrict__ lids) {
+    griddep_launch_dependents();
+    griddep_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y;
     if (i >= n) return;
     float acc = 0.f;
+#pragma unroll 2
     for (uint32_t q = 0; q < n_parts; ++q) {
         if (lids && lids[(size_t)t * n_parts + q] == kExpertSkip) continue;   // another rank's: gate 0, and no part was made here
         const float *p = parts + ((size_t)t * n_parts + q) * n + i;
-        float v = p[0];
-#pragma unroll 4
-        for (uint32_t s = 1; s < n_planes; ++s) v = __fadd_rn(v, p[s * plane_stride]);
+        float w[kMaxPlanes];   // all planes requested before the first is used
+#pragma unroll
+        for (uint32_t s = 0; s < kMaxPlanes; ++s) w[s] = s < n_planes ? p[s * plane_stride] : 0.f;
+        float v = w[0];
+#pragma unroll
+        for (uint32_t s = 1; s < kMaxPlanes; ++s)
+            if (s < n_planes) v = __fadd_rn(v, w[s]);
         acc = __fadd_rn(acc, __fmul_rn(gates[(size_t)t * n_parts + q], v));
     }
     if (resid) acc = __fadd_rn(resid[(size_t)t * n + i], acc);
@@ -241,58 +309,9 @@ __global__ void __launch_bounds__(256) scatter_rows_kernel(const float *__restri
     *reinterpret_cast<float4 *>(y + (size_t)idx[(size_t)e.x * list_stride + col_off + p] * n + i) = v;
 }
 
-// The table of a grouped multi-column launch (matvec_tc_nx.cu), by one warp: active experts in ascending order, their
-// columns from col_off on (at most P), the groups of four columns in front of them and the columns in front of them.
-__device__ __forceinline__ void nx_table_warp(const uint32_t *cnt, uint32_t n_local, uint32_t col_off, uint32_t P, uint32_t *table) {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t n_act = 0, before = 0, most = 0;   // before: groups of four, columns << 16
-    for (uint32_t b = 0; b < n_local; b += 32) {
-        const uint32_t e = b + lane, c = e < n_local ? cnt[e] : 0u;
-        const uint32_t n = c > col_off ? min(c - col_off, P) : 0u, tg = (n + 3) / 4, own = tg | n << 16;
-        uint32_t incl = own;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= (uint32_t)o) incl += v;
-        }
-        const uint32_t mask = __ballot_sync(0xffffffffu, n != 0), at = before + incl - own;
-        if (n) reinterpret_cast<uint4 *>(table)[1 + n_act + __popc(mask & ((1u << lane) - 1u))] = make_uint4(e, n, at & 0xFFFFu, at >> 16);
-        n_act += __popc(mask);
-        most = max(most, __reduce_max_sync(0xffffffffu, tg));
-        before += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) { table[0] = n_act; table[1] = most; }
-}
 __global__ void __launch_bounds__(32) nx_table_kernel(const uint32_t *__restrict__ cnt, uint32_t n_local, uint32_t col_off, uint32_t P,
                                                       uint32_t *__restrict__ table) {
     nx_table_warp(cnt, n_local, col_off, P, table);
-}
-
-// One warp: a stable counting sort of the pairs by local expert.
-__global__ void __launch_bounds__(32) group_by_expert_kernel(const uint32_t *__restrict__ lids, uint32_t n_pairs, uint32_t top_k,
-                                                             uint32_t n_local, uint32_t cap, uint32_t *__restrict__ cnt,
-                                                             uint32_t *__restrict__ tok_list, uint32_t *__restrict__ pair_list,
-                                                             uint32_t *__restrict__ table) {
-    const uint32_t lane = threadIdx.x;
-    for (uint32_t e = lane; e < n_local; e += 32) cnt[e] = 0;
-    __syncwarp();
-    for (uint32_t b = 0; b < n_pairs; b += 32) {
-        const uint32_t pair = b + lane;
-        const uint32_t e = pair < n_pairs ? lids[pair] : 0xFFFFFFFFu;
-        for (uint32_t x = 0; x < n_local; ++x) {
-            const uint32_t mask = __ballot_sync(0xffffffffu, e == x);
-            if (mask == 0) continue;
-            const uint32_t base = cnt[x];
-            if (e == x) {
-                const uint32_t pos = base + __popc(mask & ((1u << lane) - 1u));
-                if (pos < cap) { tok_list[(size_t)x * cap + pos] = pair / top_k; pair_list[(size_t)x * cap + pos] = pair; }
-            }
-            __syncwarp();
-            if (lane == 0) cnt[x] = min(base + __popc(mask), cap);
-            __syncwarp();
-        }
-    }
-    if (table) nx_table_warp(cnt, n_local, 0, kNxMaxTokens, table);
 }
 
 // fl_op_silu_mul, decode_params.h:267-272: (g / (1 + expf(-g))) * u
@@ -491,7 +510,7 @@ cudaError_t launch_router_sel(const float *logits, uint32_t *ids, float *gates, 
 
 cudaError_t launch_router(const RouterArgs &a, cudaStream_t stream) {
     if (a.n_tok == 0 || a.n_expert == 0 || a.n_expert > 256 || a.top_k == 0 || a.top_k > a.n_expert || a.n_embd % 4) return cudaErrorInvalidValue;
-    return launch_kernel(router_kernel, dim3(a.n_expert, a.n_tok), dim3(128), 0, stream, a.pdl != 0, a);
+    return launch_kernel(a.w_after ? router_kernel<true> : router_kernel<false>, dim3(a.n_expert, a.n_tok), dim3(128), 0, stream, a.pdl != 0, a);
 }
 
 cudaError_t launch_wmerge(const float *parts, const float *gates, const float *add1, const float *add2, float *y,
@@ -501,10 +520,9 @@ cudaError_t launch_wmerge(const float *parts, const float *gates, const float *a
 }
 
 cudaError_t launch_wmerge_tokens(const float *parts, const float *gates, float *y, uint32_t n_parts, uint32_t n, uint32_t n_tok,
-                                 cudaStream_t stream, uint32_t n_planes, size_t plane_stride, const float *resid, const uint32_t *lids) {
+                                 cudaStream_t stream, uint32_t n_planes, size_t plane_stride, const float *resid, const uint32_t *lids, bool pdl) {
     if (n == 0 || n_parts == 0 || n_tok == 0) return cudaErrorInvalidValue;
-    wmerge_tokens_kernel<<<dim3((n + 255) / 256, n_tok), 256, 0, stream>>>(parts, gates, y, n_parts, n, n_planes, plane_stride, resid, lids);
-    return cudaGetLastError();
+    return launch_kernel(wmerge_tokens_kernel, dim3((n + 255) / 256, n_tok), dim3(256), 0, stream, pdl, parts, gates, y, n_parts, n, n_planes, plane_stride, resid, lids);
 }
 
 cudaError_t launch_scatter_rows(const float *x, uint32_t n_planes, size_t plane_stride, const uint32_t *table, const uint32_t *idx,
@@ -515,15 +533,14 @@ cudaError_t launch_scatter_rows(const float *x, uint32_t n_planes, size_t plane_
     return cudaGetLastError();
 }
 
-cudaError_t launch_nx_table(const uint32_t *cnt, uint32_t n_local, uint32_t col_off, uint32_t P, uint32_t *table, cudaStream_t stream) {
-    nx_table_kernel<<<1, 32, 0, stream>>>(cnt, n_local, col_off, P, table);
-    return cudaGetLastError();
+cudaError_t launch_group_by_expert(const uint32_t *lids, uint32_t n_pairs, uint32_t top_k, uint32_t n_local, uint32_t cap,
+                                   uint32_t *cnt, uint32_t *tok_list, uint32_t *pair_list, uint32_t *table, cudaStream_t stream, bool pdl) {
+    if (n_pairs == 0 || top_k == 0 || n_local == 0 || n_local > 256 || cap == 0) return cudaErrorInvalidValue;
+    return launch_kernel(group_by_expert_kernel, dim3(1), dim3(32), 0, stream, pdl, lids, n_pairs, top_k, n_local, cap, cnt, tok_list, pair_list, table);
 }
 
-cudaError_t launch_group_by_expert(const uint32_t *lids, uint32_t n_pairs, uint32_t top_k, uint32_t n_local, uint32_t cap,
-                                   uint32_t *cnt, uint32_t *tok_list, uint32_t *pair_list, cudaStream_t stream, uint32_t *table) {
-    if (n_pairs == 0 || top_k == 0 || n_local == 0 || cap == 0) return cudaErrorInvalidValue;
-    group_by_expert_kernel<<<1, 32, 0, stream>>>(lids, n_pairs, top_k, n_local, cap, cnt, tok_list, pair_list, table);
+cudaError_t launch_nx_table(const uint32_t *cnt, uint32_t n_local, uint32_t col_off, uint32_t P, uint32_t *table, cudaStream_t stream) {
+    nx_table_kernel<<<1, 32, 0, stream>>>(cnt, n_local, col_off, P, table);
     return cudaGetLastError();
 }
 

@@ -137,7 +137,7 @@ struct NxIn {
     // col_idx[expert * list_stride + col_off + p] of x and goes to output row block out_idx[the same]. Without col_idx / out_idx
     // the rows are numbered through, expert by expert in the table's order.
     const uint32_t *table, *col_idx, *out_idx;
-    uint32_t list_stride, col_off, n_groups, n_experts;   // n_groups: upper bound of active experts
+    uint32_t list_stride, col_off, n_groups, n_experts, n_tgs;   // n_groups: upper bound of active experts; n_tgs: of their groups of four columns
     int table_ready;         // 1: the table was complete before the kernel in front of the matmul started
     int tm;                  // 1: launch_nx_convert builds the image of matmul_tm.cu (Q4_K or Q6_K, one format, not grouped)
 };
@@ -302,17 +302,18 @@ struct RouterArgs {
     uint32_t top_k, norm;
     float scale;
     uint32_t base, n_local;
-    int pdl;
+    int pdl, w_after;                  // w_after: with pdl, nothing is read before the dependency is met
 };
 cudaError_t launch_router(const RouterArgs &a, cudaStream_t stream);
+// The (token, slot) pairs of a block, grouped by the local expert they chose (a stable counting sort: within an
+// expert the pairs stay in ascending order): cnt[e] pairs for expert e, their tokens in tok_list[e * cap + i] and
+// their pair indices (token * top_k + slot) in pair_list[e * cap + i]. lids: local expert of every pair or kExpertSkip. The table
+// of a grouped launch over the first 16 of each (launch_nx_table).
+cudaError_t launch_group_by_expert(const uint32_t *lids, uint32_t n_pairs, uint32_t top_k, uint32_t n_local, uint32_t cap,
+                                   uint32_t *cnt, uint32_t *tok_list, uint32_t *pair_list, uint32_t *table, cudaStream_t stream, bool pdl);
 cudaError_t launch_router_sel(const float *logits, uint32_t *ids, float *gates, uint32_t n_tok, uint32_t n_expert, uint32_t top_k,
                               uint32_t norm, float scale, cudaStream_t stream, uint32_t *lids = nullptr,
                               float *mgates = nullptr, uint32_t base = 0, uint32_t n_local = 0);
-// The (token, slot) pairs of a block, grouped by the local expert they chose (a stable counting sort: within an
-// expert the pairs stay in ascending order): cnt[e] pairs for expert e, their tokens in tok_list[e * cap + i] and
-// their pair indices (token * top_k + slot) in pair_list[e * cap + i]. lids: local expert of every pair or kExpertSkip.
-cudaError_t launch_group_by_expert(const uint32_t *lids, uint32_t n_pairs, uint32_t top_k, uint32_t n_local, uint32_t cap,
-                                   uint32_t *cnt, uint32_t *tok_list, uint32_t *pair_list, cudaStream_t stream, uint32_t *table = nullptr);
 // fl_op_wmerge (src/runtime/decode_params.h:274-295).
 cudaError_t launch_wmerge(const float *parts, const float *gates, const float *add1, const float *add2, float *y,
                           float scale, uint32_t n_parts, uint32_t n, uint32_t n_full, cudaStream_t stream, bool pdl = false);
@@ -320,7 +321,7 @@ cudaError_t launch_wmerge(const float *parts, const float *gates, const float *a
 // rounded in the reference's order); a part is the sum of n_planes planes, plane_stride floats apart.
 cudaError_t launch_wmerge_tokens(const float *parts, const float *gates, float *y, uint32_t n_parts, uint32_t n, uint32_t n_tok,
                                  cudaStream_t stream, uint32_t n_planes = 1, size_t plane_stride = 0, const float *resid = nullptr,
-                                 const uint32_t *lids = nullptr);   // lids: slots whose entry is kExpertSkip are left out
+                                 const uint32_t *lids = nullptr, bool pdl = false);   // lids: slots whose entry is kExpertSkip are left out
 // Rows numbered through by a grouped launch's table (row r of x: n_planes planes of n floats, plane_stride apart) to the rows of
 // y that their columns stand for: y[idx[expert * list_stride + col_off + p]] = the sum of the planes. n a multiple of 4.
 cudaError_t launch_scatter_rows(const float *x, uint32_t n_planes, size_t plane_stride, const uint32_t *table, const uint32_t *idx,

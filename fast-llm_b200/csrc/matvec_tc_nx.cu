@@ -260,7 +260,7 @@ __device__ __forceinline__ float4 combine_records(const float *part, uint32_t S,
     return make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
 }
 
-// grid (blocks, columns rounded up to groups of four, groups), 64 threads: a block converts 256 values of one column, a thread
+// grid (blocks, columns rounded up to groups of four: grouped, those of all active experts), 64 threads: a block converts 256 values of one column, a thread
 // four consecutive ones. What bounds it is latency (a launch moves well under a megabyte): hence few values per thread, every
 // plane in flight, and as many blocks as there are (block, column) pairs. ATT: the columns are attention contexts (a.att), an instance
 // of its own for the registers of the records in flight (254 against 54).
@@ -276,12 +276,22 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     if (a.wnorm) wn = __ldg(reinterpret_cast<const float4 *>(a.wnorm + blk * 256 + 4 * i));   // a constant
     griddep_wait();
     uint32_t n_valid = a.P, tg = blockIdx.y >> 2, ntg = (a.P + 3) / 4, tg0 = 0, grp = 0, row0 = 0;
-    if (a.table) {
-        if (blockIdx.z >= a.table[0]) return;
-        const uint4 e = reinterpret_cast<const uint4 *>(a.table)[1 + blockIdx.z];
-        grp = e.x; n_valid = e.y; tg0 = e.z; row0 = e.w;
-        ntg = (n_valid + 3) / 4;
-        if (tg >= ntg) return;
+    if (a.table) {   // the group of four is one of all active experts' together: look its expert up
+        const uint32_t n_act = a.table[0], lane = threadIdx.x & 31u, at = tg;
+        ntg = 0;
+        for (uint32_t b = 0; b < n_act && ntg == 0; b += 32) {
+            uint4 e = make_uint4(0u, 0u, 0u, 0u);
+            if (b + lane < n_act) e = reinterpret_cast<const uint4 *>(a.table)[1 + b + lane];
+            const uint32_t n = (e.y + 3) / 4, mask = __ballot_sync(0xffffffffu, at - e.z < n);
+            if (mask) {
+                const int l = __ffs(mask) - 1;
+                grp = __shfl_sync(0xffffffffu, e.x, l); n_valid = __shfl_sync(0xffffffffu, e.y, l);
+                tg0 = __shfl_sync(0xffffffffu, e.z, l); row0 = __shfl_sync(0xffffffffu, e.w, l);
+                ntg = __shfl_sync(0xffffffffu, n, l);
+            }
+        }
+        if (ntg == 0) return;
+        tg = at - tg0;
     }
     const uint32_t p = 4 * tg + pp;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1053,12 +1063,13 @@ cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t
     c.xstride = in.xstride; c.rstride = in.rstride; c.n_parts = in.n_parts ? in.n_parts : 1; c.P = P; c.nblk = cols / 256;
     c.tm = in.tm;
     if (in.tm && (q8 || q4 == q6 || in.table)) return cudaErrorNotSupported;
+    if (in.table && (in.n_tgs == 0 || in.n_tgs > 16000)) return cudaErrorNotSupported;
     if (q4) c.img4 = xq;
     if (q6) c.img6 = xq + nx_image_off(FMT_Q6_K, q4, q6, cols, tgs_cap);
     if (q8) c.img8 = xq + nx_image_off(FMT_Q8_0, q4, q6, cols, tgs_cap);
     c.att = in.att; c.n_splits = in.n_splits;
     c.table = in.table; c.col_idx = in.col_idx; c.list_stride = in.list_stride; c.col_off = in.col_off;
-    return launch_kernel(in.att ? act_convert_nx_kernel<true> : act_convert_nx_kernel<false>, dim3(cols / 256, (P + 3) / 4 * 4, in.table ? in.n_groups : 1), dim3(64), 0, stream, pdl, c);
+    return launch_kernel(in.att ? act_convert_nx_kernel<true> : act_convert_nx_kernel<false>, dim3(cols / 256, in.table ? 4 * in.n_tgs : (P + 3) / 4 * 4), dim3(64), 0, stream, pdl, c);
 }
 
 cudaError_t launch_nx_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,

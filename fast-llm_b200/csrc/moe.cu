@@ -335,8 +335,10 @@ static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y,
     const fl_b200_moe_cfg &c = m->c;
     const uint32_t E = c.n_embd, F = c.n_ff, K = c.top_k, T = c.max_tokens;
     if (per_slot) return moe_enqueue_per_slot(m, x, n_tok, y, wnorm, eps, resid);
-    CKM(launch_router(moe_router_args(m, x, n_tok, wnorm, eps), s));
-    CKM(launch_group_by_expert(m->lids, n_tok * K, K, m->n_local, T, m->cnt, m->tok_list, m->pair_list, s, m->table));
+    RouterArgs r = moe_router_args(m, x, n_tok, wnorm, eps);
+    r.pdl = kMoePdlNx; r.w_after = wnorm ? 0 : 1;   // (a block called by itself: its router may have been written just before)
+    CKM(launch_router(r, s));
+    CKM(launch_group_by_expert(m->lids, n_tok * K, K, m->n_local, T, m->cnt, m->tok_list, m->pair_list, m->table, s, kMoePdlNx != 0));
     // Every local expert once for up to 16 of the tokens that chose it. The table and the lists live on the device, so the
     // launch sequence is the same for every routing (and can be replayed as a graph).
     const uint32_t P = std::min(n_tok, kNxMaxTokens);   // every pass is cut into the same parts, the last one too
@@ -351,10 +353,11 @@ static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y,
         in.x = x; in.xstride = E; in.wnorm = wnorm; in.eps = eps;
         in.table = m->table; in.col_idx = m->tok_list; in.out_idx = one_pass ? m->pair_list : nullptr; in.list_stride = T; in.col_off = off;
         in.n_groups = std::min(m->n_local, n_tok * K); in.n_experts = m->n_local;
-        // the first conversion is an ordinary dependent of the kernel that wrote the table; every later launch starts after
-        // it did, so that the table is in place for all of them
+        in.n_tgs = std::min(in.n_groups * ((P + 3) / 4), n_tok * K / 4 + in.n_groups);
+        // a conversion starts its dependent after it has waited for the kernel that wrote the table, so that the table is in place for
+        // every matmul
         in.table_ready = kMoePdlNx;
-        CKM(launch_nx_convert(in, gu, 1, E, P, m->xq, m->tgs, s, false));
+        CKM(launch_nx_convert(in, gu, 1, E, P, m->xq, m->tgs, s, kMoePdlNx != 0));
         CKM(launch_nx_matmul(in, gu, 2, E, P, 0, m->xq, m->tgs, ctx->status, ctx->sms, s, kMoePdlNx != 0, true));
         in.x = m->g; in.x2 = m->u; in.xstride = F; in.wnorm = nullptr;
         in.n_parts = parts_gu; in.part_stride = R * F;
@@ -365,7 +368,7 @@ static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y,
     }
     // WMERGE of every token: y[t] = sum_k gate[t][k] * part[t][k], slots of experts held elsewhere left out
     CKM(launch_wmerge_tokens(one_pass ? m->d : m->part, m->mgates, m->world > 1 ? m->partial : y, K, E, n_tok, s, one_pass ? parts_d : 1, R * E,
-                             m->world > 1 ? nullptr : resid, m->world > 1 ? m->lids : nullptr));
+                             m->world > 1 ? nullptr : resid, m->world > 1 ? m->lids : nullptr, kMoePdlNx != 0 && one_pass));
     if (m->world > 1) {
         for (uint32_t t = 0; t < n_tok; ++t) {   // the combine: sum of the ranks' partial outputs, rank order
             AllReduceArgs r{};
