@@ -72,7 +72,7 @@ __device__ __forceinline__ void q4k_block_x21(uint32_t r0, uint32_t oh, uint32_t
 #pragma unroll
     for (int j = 4; j < 8; ++j) bx[j] = lds128(xaddr + j * xstride);
     const uint4 h0 = lds128(r0 + oh), h1 = lds128(r1 + oh);
-    int cL[2][4], cH[2][4];
+    int cL[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, cH[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
     const uint32_t ML = 0x0F0F0F0Fu, MH = 0xF0F0F0F0u;
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
@@ -80,28 +80,25 @@ __device__ __forceinline__ void q4k_block_x21(uint32_t r0, uint32_t oh, uint32_t
         const uint32_t A1 = m < 2 ? word_of(wa1, 2 * m) : word_of(wb1, 2 * m - 4), B1 = m < 2 ? word_of(wa1, 2 * m + 1) : word_of(wb1, 2 * m - 3);
         const uint32_t l0 = A0 & ML, l1 = A1 & ML, l2 = B0 & ML, l3 = B1 & ML;
         const uint32_t g0 = A0 & MH, g1 = A1 & MH, g2 = B0 & MH, g3 = B1 & MH;   // 16 times the quants
-        if (m == 0) {
-            imma16832_first(cL[0], l0, l1, l2, l3, bx[0].x, bx[0].y);
-            imma16832_first(cH[0], g0, g1, g2, g3, bx[1].x, bx[1].y);
-            imma16832_first(cL[1], l0, l1, l2, l3, bx[0].z, bx[0].w);
-            imma16832_first(cH[1], g0, g1, g2, g3, bx[1].z, bx[1].w);
-        } else {
-            imma16832(cL[0], l0, l1, l2, l3, bx[2 * m].x, bx[2 * m].y);
-            imma16832(cH[0], g0, g1, g2, g3, bx[2 * m + 1].x, bx[2 * m + 1].y);
-            imma16832(cL[1], l0, l1, l2, l3, bx[2 * m].z, bx[2 * m].w);
-            imma16832(cH[1], g0, g1, g2, g3, bx[2 * m + 1].z, bx[2 * m + 1].w);
-        }
+        imma16832(cL[0], l0, l1, l2, l3, bx[2 * m].x, bx[2 * m].y);
+        imma16832(cH[0], g0, g1, g2, g3, bx[2 * m + 1].x, bx[2 * m + 1].y);
+        imma16832(cL[1], l0, l1, l2, l3, bx[2 * m].z, bx[2 * m].w);
+        imma16832(cH[1], g0, g1, g2, g3, bx[2 * m + 1].z, bx[2 * m + 1].w);
     }
+    // 6-bit scales / mins of sub-blocks 2t, 2t+1 (fl_q4k_scale_min, src/runtime/quants.h:121-129), as in matvec_tc.cu
+    const uint32_t sh = 16u * (t & 1u);
+    const uint32_t shA = t >= 2 ? sh + 2u : sh, mA = t >= 2 ? 0x3030u : 0x3F3Fu, mE = t >= 2 ? 0x0F0Fu : 0u;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         const uint4 hdr = r ? h1 : h0;
-        const uint32_t sm = q4k_scales(hdr, t);
+        const uint32_t sc = ((hdr.y >> shA) & mA) | ((hdr.w >> sh) & mE);
+        const uint32_t mn = ((hdr.z >> shA) & mA) | ((hdr.w >> (sh + 4u)) & mE);
         const float d = h2f_bits((uint16_t)(hdr.x & 0xFFFFu)), dmin = h2f_bits((uint16_t)(hdr.x >> 16));
         const float fa = (float)whole(cL[0][2 * r], cL[0][2 * r + 1], cL[1][2 * r]);
         // the high nibbles' sums are multiples of 16, and too large for 32 bits before the division
         const float fb = (float)(cH[0][2 * r] * 4096 + cH[0][2 * r + 1] * 16 + (cH[1][2 * r] >> 4));
-        const float q = u8f<0>(sm) * fa + u8f<1>(sm) * fb;
-        const float m = u8f<2>(sm) * sx.x + u8f<3>(sm) * sx.y;
+        const float q = u8f<0>(sc) * fa + u8f<1>(sc) * fb;
+        const float m = u8f<0>(mn) * sx.x + u8f<1>(mn) * sx.y;
         (r ? out1 : out0) = d * q - dmin * m;
     }
 }
@@ -161,9 +158,9 @@ __device__ __forceinline__ void q6k_block_x21(uint32_t r0, uint32_t r1, uint32_t
                         : gq == 2 ? ((a >> 4) & 0x0F0F0F0Fu) | (h & 0x30303030u) : ((b >> 4) & 0x0F0F0F0Fu) | ((h >> 2) & 0x30303030u);
             }
         const uint4 b0 = lds128(xaddr + gq * xstride), b1 = lds128(xaddr + (4 + gq) * xstride);
-        int c0[4], c1[4];
-        imma16832_first(c0, q[0][0], q[1][0], q[0][1], q[1][1], b0.x, b0.y);
-        imma16832_first(c1, q[0][0], q[1][0], q[0][1], q[1][1], b0.z, b0.w);
+        int c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
+        imma16832(c0, q[0][0], q[1][0], q[0][1], q[1][1], b0.x, b0.y);
+        imma16832(c1, q[0][0], q[1][0], q[0][1], q[1][1], b0.z, b0.w);
         imma16832(c0, q[0][2], q[1][2], q[0][3], q[1][3], b1.x, b1.y);
         imma16832(c1, q[0][2], q[1][2], q[0][3], q[1][3], b1.z, b1.w);
 #pragma unroll

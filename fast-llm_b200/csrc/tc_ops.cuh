@@ -97,30 +97,11 @@ __device__ __forceinline__ void imma16832(int (&c)[4], uint32_t a0, uint32_t a1,
                  : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// The same from a zero accumulator (no registers to clear).
-__device__ __forceinline__ void imma16832_first(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
-}
 // Signed weights.
 __device__ __forceinline__ void imma16832_ss(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void imma16832_ss_first(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
-}
-// Q4_K scales (low half) and mins (high half) of sub-blocks 2 t, 2 t + 1, a byte each, from the block's 16-byte header
-// (fl_q4k_scale_min, src/runtime/quants.h:121-129): sub-blocks 0..3 are the low six bits of bytes 0..3 (mins 4..7), 4..7 a
-// nibble of bytes 8..11 under the top two bits of those. Both kinds at once; what depends on t is constant for a lane.
-__device__ __forceinline__ uint32_t q4k_scales(const uint4 &hdr, uint32_t t) {
-    const uint32_t sel = t & 1u ? 0x7632u : 0x5410u, sh = t & 2u, mA = t >= 2 ? 0x30303030u : 0x3F3F3F3Fu, mE = t >= 2 ? 0x0F0F0F0Fu : 0u;
-    const uint32_t a = __byte_perm(hdr.y, hdr.z, sel), e = __byte_perm(hdr.w, hdr.w >> 4, sel);
-    return ((a >> sh) & mA) | (e & mE);
 }
 // (a & b) | c in one instruction; b and c are constants the compiler keeps in registers
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
