@@ -193,8 +193,9 @@ int fl_b200_memset(fl_b200_ctx *c, void *dst, int value, size_t bytes) {
     int cur = -1;
     if (bytes && cudaGetDevice(&cur) == cudaSuccess && cur == c->device && in_device_memory(cur, dst, bytes))
         return cuda_err(launch_fill(dst, value, bytes, c->sms, c->stream, true), "fill launch");
-    CK(cudaMemsetAsync(dst, value, bytes, c->stream));
-    return FL_B200_OK;
+    const cudaError_t e = cudaMemsetAsync(dst, value, bytes, c->stream);
+    if (e != cudaSuccess) cudaGetLastError();   // reported here: the next launch does not report it again
+    return cuda_err(e, "cudaMemsetAsync");
 }
 
 int fl_b200_timer_start(fl_b200_ctx *c) {
@@ -264,6 +265,7 @@ int flb::matmul(fl_b200_ctx *c, int fmt, const void *w, uint32_t rows, uint32_t 
             // this call or the one before may be on the tcgen05 form, whose image is another one
             const bool reuse = same_columns && nx <= kNxMaxTokens && tm <= 0;
             if (!reuse) {
+                in.dep_first = pdl == kPdlAfter;
                 e = launch_nx_convert(in, &t, 1, cols, nt, c->xq, kNxTgs, c->stream, pdl != 0);
                 if (e == cudaErrorNotSupported) break;
                 if (e != cudaSuccess) return cuda_err(e, "activation conversion launch");

@@ -209,6 +209,7 @@ struct ConvArgs {
     const float *att;              // the columns are attention contexts of heads of 128, added up here from n_splits records
     uint32_t n_splits;             // (attn.cu: [column][head][split][132] = context, maximum, sum)
     int tm;                        // img4 or img6 is the image of matmul_tm.cu
+    int dep_first;                 // see NxIn
 };
 // Device-side table of a grouped launch: word 0 = number of active groups, word 1 = the most token groups of one; then four
 // words per active group: {group, number of columns, token groups in front of it, columns in front of it}.
@@ -226,14 +227,14 @@ __device__ __forceinline__ float4 sum_planes(const float *p, uint32_t n, size_t 
 }
 
 // Four dimensions (4 lane ..) of one head's context from its splits' records (attn_decode_kernel's combine, with all lanes of
-// a warp on one head): the weights from every split's maximum and sum, then the contexts in split order, 40 in flight: it is bound
-// by the latency of its loads (8 positions, 37 splits, launch to launch: 9.3 us with 16 in flight, three round trips to L2; now 5.8).
+// a warp on one head): the weights from every split's maximum and sum, then the contexts in split order, kFlight of them in flight: it is
+// bound by the latency of its loads (8 positions, 37 splits, launch to launch: 9.3 us with 16 in flight, three round trips to L2, 5.8 with 40).
+template <int kFlight>
 __device__ __forceinline__ float4 combine_records(const float *part, uint32_t S, uint32_t lane) {
     const float m0 = lane < S ? __ldcg(part + (size_t)lane * kAttnRecord + 128) : -INFINITY;
     const float m1 = lane + 32 < S ? __ldcg(part + (size_t)(lane + 32) * kAttnRecord + 128) : -INFINITY;
     const float l0 = lane < S ? __ldcg(part + (size_t)lane * kAttnRecord + 129) : 0.f;
     const float l1 = lane + 32 < S ? __ldcg(part + (size_t)(lane + 32) * kAttnRecord + 129) : 0.f;
-    constexpr int kFlight = 40;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     float w0 = 0.f, w1 = 0.f, L = 1.f;
 #pragma unroll 1
@@ -260,23 +261,28 @@ __device__ __forceinline__ float4 combine_records(const float *part, uint32_t S,
     return make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
 }
 
-// grid (blocks, columns rounded up to groups of four: grouped, those of all active experts), 64 threads: a block converts 256 values of one column, a thread
-// four consecutive ones. What bounds it is latency (a launch moves well under a megabyte): hence few values per thread, every
-// plane in flight, and as many blocks as there are (block, column) pairs. ATT: the columns are attention contexts (a.att), an instance
-// of its own for the registers of the records in flight (254 against 54).
-template <bool ATT>
+// grid (blocks, columns rounded up to groups of four: grouped, those of all active experts), 64 threads: a block converts 256
+// values of one column, a thread four consecutive ones. What bounds it is latency (a launch moves well under a megabyte): hence few
+// values per thread, every plane in flight, and as many blocks as there are (block, column) pairs. F: records of a head's splits
+// (a.att) in flight, 16 or 40, the latter (254 registers) for those alone. GROUPED: the columns are those of a table. An instance each,
+// since a launch fetches its code from L2 (lookup and records in one instance: passes of the 8B shape 1 % slower). The instance for
+// ungrouped columns keeps the records although few launches have any: without them the compiler takes 54 registers instead of
+// 128 and puts the planes' loads behind one another (6 positions: 1 to 2 % slower); for the thousands of blocks of a grouped launch fewer
+// registers are the better choice (Mixtral-shape block, 16 tokens: 275 against 280 us).
+template <int F, bool GROUPED>
 __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     __shared__ float2 half_s[2];   // per warp: maximum, sum of squares
     const uint32_t blk = blockIdx.x, warp = threadIdx.x >> 5;
     const uint32_t pp = blockIdx.y & 3u, i = threadIdx.x, hl = i >> 2, tq = i & 3u;   // column of the group; values 16 hl + 4 tq ..
-    // Launched as a programmatic dependent: the launch itself overlaps the tail of the kernel before, whose output (x, the table) is
-    // read only after it has completed. Its own dependent, the matmul, starts when this kernel's loads are back: started at once it
-    // fills its rings, 30 MB of weights, in front of them (pass of 8 positions, 8B shape: 3216 -> 3115 us, gate | up to down 5.3 -> 3.6).
+    // launched as a programmatic dependent: the launch itself overlaps the tail of the kernel before, whose output
+    // (x, the table) is read only after it has completed
+    if (!a.dep_first) griddep_launch_dependents();
     float4 wn = make_float4(1.f, 1.f, 1.f, 1.f);
     if (a.wnorm) wn = __ldg(reinterpret_cast<const float4 *>(a.wnorm + blk * 256 + 4 * i));   // a constant
     griddep_wait();
+    if (a.dep_first) griddep_launch_dependents();
     uint32_t n_valid = a.P, tg = blockIdx.y >> 2, ntg = (a.P + 3) / 4, tg0 = 0, grp = 0, row0 = 0;
-    if (a.table) {   // the group of four is one of all active experts' together: look its expert up
+    if (GROUPED) {   // the group of four is one of all active experts' together: look its expert up
         const uint32_t n_act = a.table[0], lane = threadIdx.x & 31u, at = tg;
         ntg = 0;
         for (uint32_t b = 0; b < n_act && ntg == 0; b += 32) {
@@ -297,11 +303,11 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     float ss = 0.f;
     if (p < n_valid) {
-        const size_t row = a.col_idx ? a.col_idx[(size_t)grp * a.list_stride + a.col_off + p] : row0 + p;
+        const size_t row = GROUPED && a.col_idx ? a.col_idx[(size_t)grp * a.list_stride + a.col_off + p] : row0 + p;
         const size_t at = row * a.xstride + blk * 256 + 4 * i, rat = (size_t)p * a.rstride + blk * 256 + 4 * i;
         float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
         if (a.resid) r = *reinterpret_cast<const float4 *>(a.resid + rat);
-        if (ATT) v = combine_records(a.att + ((size_t)p * (2 * a.nblk) + 2 * blk + warp) * a.n_splits * kAttnRecord, a.n_splits, threadIdx.x & 31u);
+        if (!GROUPED && a.att) v = combine_records<F>(a.att + ((size_t)p * (2 * a.nblk) + 2 * blk + warp) * a.n_splits * kAttnRecord, a.n_splits, threadIdx.x & 31u);
         else v = sum_planes(a.x + at, a.n_parts, a.part_stride);
         if (a.x2) {   // fl_op_silu_mul (src/runtime/decode_params.h:267-272)
             const float4 u = sum_planes(a.x2 + at, a.n_parts, a.part_stride);
@@ -315,7 +321,6 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
             v.x *= wn.x; v.y *= wn.y; v.z *= wn.z; v.w *= wn.w;
         }
     }
-    griddep_launch_dependents();
     if (!a.img4 && !a.img6 && !a.img8) return;   // only the sum was asked for
     float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
     amax = warp_max(amax);
@@ -1061,7 +1066,7 @@ cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t
     ConvArgs c{};
     c.x = in.x; c.x2 = in.x2; c.part_stride = in.part_stride; c.resid = in.resid; c.x_out = in.x_out; c.wnorm = in.wnorm;
     c.xstride = in.xstride; c.rstride = in.rstride; c.n_parts = in.n_parts ? in.n_parts : 1; c.P = P; c.nblk = cols / 256;
-    c.tm = in.tm;
+    c.tm = in.tm; c.dep_first = in.dep_first;
     if (in.tm && (q8 || q4 == q6 || in.table)) return cudaErrorNotSupported;
     if (in.table && (in.n_tgs == 0 || in.n_tgs > 16000)) return cudaErrorNotSupported;
     if (q4) c.img4 = xq;
@@ -1069,7 +1074,8 @@ cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t
     if (q8) c.img8 = xq + nx_image_off(FMT_Q8_0, q4, q6, cols, tgs_cap);
     c.att = in.att; c.n_splits = in.n_splits;
     c.table = in.table; c.col_idx = in.col_idx; c.list_stride = in.list_stride; c.col_off = in.col_off;
-    return launch_kernel(in.att ? act_convert_nx_kernel<true> : act_convert_nx_kernel<false>, dim3(cols / 256, in.table ? 4 * in.n_tgs : (P + 3) / 4 * 4), dim3(64), 0, stream, pdl, c);
+    return launch_kernel(in.table ? act_convert_nx_kernel<16, true> : in.att && in.n_splits > 16 ? act_convert_nx_kernel<40, false> : act_convert_nx_kernel<16, false>, dim3(cols / 256, in.table ? 4 * in.n_tgs : (P + 3) / 4 * 4), dim3(64),
+                         0, stream, pdl, c);
 }
 
 cudaError_t launch_nx_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,

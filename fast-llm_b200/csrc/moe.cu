@@ -356,7 +356,7 @@ static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y,
         in.n_tgs = std::min(in.n_groups * ((P + 3) / 4), n_tok * K / 4 + in.n_groups);
         // a conversion starts its dependent after it has waited for the kernel that wrote the table, so that the table is in place for
         // every matmul
-        in.table_ready = kMoePdlNx;
+        in.table_ready = kMoePdlNx; in.dep_first = 1;
         CKM(launch_nx_convert(in, gu, 1, E, P, m->xq, m->tgs, s, kMoePdlNx != 0));
         CKM(launch_nx_matmul(in, gu, 2, E, P, 0, m->xq, m->tgs, ctx->status, ctx->sms, s, kMoePdlNx != 0, true));
         in.x = m->g; in.x2 = m->u; in.xstride = F; in.wnorm = nullptr;
