@@ -804,9 +804,9 @@ static int enqueue_batch_nx(fl_b200_decoder *d, uint32_t m, cudaStream_t s, bool
     auto group = [&](const NxIn &from, const NxTensor *t, int n, uint32_t cols, uint32_t *parts, bool split = true) -> int {
         *parts = matmul_tc_nx_parts(t, n, cols, m, split, b.tm_sms);
         NxIn in = from;
-        in.tm = split && b.tm_sms && matmul_tm_takes(t, n, cols, m, b.tm_sms);
+        in.tm = b.tm_sms && (split ? matmul_tm_takes(t, n, cols, m, b.tm_sms) : matmul_tm_takes_whole(t, n, cols, m, b.tm_sms));
         CK(launch_nx_convert(in, t, n, cols, m, ctx->xq, kNxTgs, s, pdl));
-        if (in.tm) CK(launch_tm_matmul(in, t, n, cols, m, 0, ctx->xq, ctx->status, ctx->sms, s, pdl, true));
+        if (in.tm) CK(launch_tm_matmul(in, t, n, cols, m, 0, ctx->xq, ctx->status, ctx->sms, s, pdl, split));
         else CK(launch_nx_matmul(in, t, n, cols, m, 0, ctx->xq, kNxTgs, ctx->status, ctx->sms, s, pdl, split));
         return FL_B200_OK;
     };
@@ -888,7 +888,7 @@ static int enqueue_batch_nx(fl_b200_decoder *d, uint32_t m, cudaStream_t s, bool
         if (int rc = residual(parts)) return rc;
     }
     const int n = nx_group(d, 0, 4, t, &cols);
-    parts = matmul_tc_nx_parts(t, n, cols, m);
+    parts = matmul_tc_nx_parts(t, n, cols, m, false, b.tm_sms);
     t[0].y = parts > 1 ? b.head : b.logits; t[0].ystride = V; t[0].part_stride = (size_t)m * V;
     if (int rc = group(normed(d->out_norm), t, n, cols, &parts, false)) return rc;
     if (parts > 1) CK(launch_reduce_parts(b.head, (size_t)m * V, parts, b.logits, V, V, m, 0, s, pdl));

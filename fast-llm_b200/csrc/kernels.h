@@ -161,6 +161,7 @@ cudaError_t launch_nx_table(const uint32_t *cnt, uint32_t n_local, uint32_t col_
 // in.tm set and the next conversion or reduction, as launch_nx_matmul. The image of 256 columns takes 8512 bytes up to 8 tokens,
 // else 17024: less than matmul_tc_nx_scratch_bytes provides.
 bool matmul_tm_takes(const NxTensor *t, int n, uint32_t cols, uint32_t P, int sms);   // launches with planes (split) for which it is the faster form
+bool matmul_tm_takes_whole(const NxTensor *t, int n, uint32_t cols, uint32_t P, int sms);   // and without
 uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, bool split, int sms);
 cudaError_t launch_tm_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,
                              uint32_t *status, int sms, cudaStream_t stream, bool pdl, bool split);

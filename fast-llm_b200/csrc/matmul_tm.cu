@@ -766,6 +766,16 @@ bool matmul_tm_takes(const NxTensor *t, int n, uint32_t cols, uint32_t P, int sm
     return P > 1 && tm_plan(t, n, cols, true, sms, p) && p.grid == (uint32_t)sms && p.steps >= (P > 8 ? 3 : 8) * p.grid;
 }
 
+// Whether the head of a pass, whose planes would take a reduction of their own, takes this form, a CTA whole tiles: from 9 columns on,
+// where the other kernel cuts its 4096 columns in two and leaves planes, and from four tiles a CTA on, so that the last round of them is a small
+// part. A pass of 16 positions: 6 layers, 90000 x 2560 Q4_K 657 -> 611 us, 12 positions 622 -> 590, 9 608 -> 581; 100000 x 1536 487 -> 463;
+// 8B shape (128256 x 4096 Q6_K) 3605 -> 3565 (two boxes, with both forms in turn). Up to 8 columns the other kernel walks Q6_K in 131 us, this
+// one's steps would take 165.
+bool matmul_tm_takes_whole(const NxTensor *t, int n, uint32_t cols, uint32_t P, int sms) {
+    TmPlan p;
+    return P > 8 && tm_plan(t, n, cols, false, sms, p) && p.steps >= 4ull * (cols / 256) * sms;
+}
+
 uint32_t matmul_tm_parts(const NxTensor *t, int n, uint32_t cols, bool split, int sms) {
     TmPlan p;
     return tm_plan(t, n, cols, split, sms, p) ? p.parts : 0;

@@ -1053,6 +1053,7 @@ uint32_t matmul_tc_nx_parts(const NxTensor *t, int n, uint32_t cols, uint32_t P,
         fmts[i] = t[i].fmt;
     }
     if (split && tm_sms && matmul_tm_takes(t, n, cols, P, tm_sms)) return matmul_tm_parts(t, n, cols, true, tm_sms);
+    if (!split && tm_sms && matmul_tm_takes_whole(t, n, cols, P, tm_sms)) return 1;
     NxPlan p;
     return nx_plan(fmts, n, cols, (P + 3) / 4, split, p) ? p.parts : 0;
 }
