@@ -105,9 +105,11 @@ __device__ __forceinline__ uint32_t pack_h2(__half lo, __half hi) {
     return (uint32_t)__half_as_ushort(lo) | ((uint32_t)__half_as_ushort(hi) << 16);
 }
 
-// FUSED: RoPE and the append of this token's rows. An instance each, since a launch fetches its code from L2 (1024 keys, 8 KV heads,
-// calls in a row: 6.25 -> 5.50 us; a step of the 8B shape 0.5 % faster).
-template <bool FUSED>
+// MODE 1: with RoPE and the append of this token's rows, 0: without, since a launch fetches its code from L2 (1024 keys, 8 KV heads,
+// calls in a row: 6.25 -> 5.50 us; a step of the 8B shape 0.5 % faster). 2: as the arguments say, for several sequences of a pass, whose
+// positions lie on the device: MODE 0 makes that pass up to 3 % slower (16 sequences: 6 layers in Q8_0 774 -> 787 us, of 1536 columns over 600 keys 459 -> 475, 8B shape
+// 4362 -> 4370).
+template <int MODE>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(const __grid_constant__ AttnArgs a) {
     extern __shared__ uint8_t smem_dyn[];
     AttnSmem &sm = *reinterpret_cast<AttnSmem *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -115,7 +117,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(const __gr
     const uint32_t g = lane >> 2, t = lane & 3u;
     const uint32_t split = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z;
     const uint32_t group = a.n_q_head / a.n_kv_head;   // == kGroup (checked on the host)
-    constexpr bool fused = FUSED;
+    const bool fused = MODE == 2 ? a.rope_k != nullptr : MODE == 1;
     if (tid == 0) trace_min(a.trace, 0);
     griddep_launch_dependents();
     // *pos was written at the end of the previous step (or is kv_len - 1 of a single call): stable here.
@@ -374,7 +376,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(const __gr
         const float inv = 1.0f / L;
         acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
         reinterpret_cast<float4 *>(a.out + hq * kD)[lane] = acc;
-        if (!FUSED && a.lse_out && lane == 0) a.lse_out[hq] = make_float2(mx, L);
+        if (MODE != 1 && a.lse_out && lane == 0) a.lse_out[hq] = make_float2(mx, L);
     }
     if (tid == 0) {
         a.tickets[b * a.n_kv_head + hkv] = 0;   // ready for the next launch
@@ -622,8 +624,9 @@ cudaError_t attn_make_maps(AttnArgs &a) {
 cudaError_t attn_init(void) {
     const cudaError_t e = cudaFuncSetAttribute(attn_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnShSmemBytes);
     if (e != cudaSuccess) return e;
-    if (const cudaError_t r = cudaFuncSetAttribute(attn_decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemBytes)) return r;
-    return cudaFuncSetAttribute(attn_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemBytes);
+    for (auto k : {attn_decode_kernel<0>, attn_decode_kernel<1>, attn_decode_kernel<2>})
+        if (const cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemBytes)) return r;
+    return cudaSuccess;
 }
 
 uint32_t attn_pick_splits(uint32_t n_kv_head, uint32_t batch, uint32_t kv_len, int sms, bool shared_kv) {
@@ -730,7 +733,7 @@ cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t stream) {
     }
     const dim3 grid(a.n_splits, a.n_kv_head, a.batch);
     if (a.rope_k && a.lse_out) return cudaErrorInvalidValue;   // (no caller has both)
-    return launch_kernel(a.rope_k ? attn_decode_kernel<true> : attn_decode_kernel<false>, grid, dim3(kAttnThreads), kAttnSmemBytes, stream, a.pdl != 0, a);
+    return launch_kernel(a.rope_k ? attn_decode_kernel<1> : a.pos && a.batch > 1 ? attn_decode_kernel<2> : attn_decode_kernel<0>, grid, dim3(kAttnThreads), kAttnSmemBytes, stream, a.pdl != 0, a);
 }
 
 } // namespace flb
