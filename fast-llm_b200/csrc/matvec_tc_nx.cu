@@ -264,12 +264,13 @@ __device__ __forceinline__ float4 combine_records(const float *part, uint32_t S,
 // grid (blocks, columns rounded up to groups of four: grouped, those of all active experts), 64 threads: a block converts 256
 // values of one column, a thread four consecutive ones. What bounds it is latency (a launch moves well under a megabyte): hence few
 // values per thread, every plane in flight, and as many blocks as there are (block, column) pairs. F: records of a head's splits
-// (a.att) in flight, 16 or 40, the latter (254 registers) for those alone. GROUPED: the columns are those of a table. An instance each,
+// (a.att) in flight, 16 or 40, the latter (254 registers) for those alone. GROUPED: the columns are those of a table. TM: the image is
+// that of matmul_tm.cu (8B shape, 8 positions 3110 -> 3088 us, 16 sequences 4432 -> 4392). An instance each,
 // since a launch fetches its code from L2 (lookup and records in one instance: passes of the 8B shape 1 % slower). The instance for
 // ungrouped columns keeps the records although few launches have any: without them the compiler takes 54 registers instead of
 // 128 and puts the planes' loads behind one another (6 positions: 1 to 2 % slower); for the thousands of blocks of a grouped launch fewer
 // registers are the better choice (Mixtral-shape block, 16 tokens: 275 against 280 us).
-template <int F, bool GROUPED>
+template <int F, bool GROUPED, bool TM>
 __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     __shared__ float2 half_s[2];   // per warp: maximum, sum of squares
     const uint32_t blk = blockIdx.x, warp = threadIdx.x >> 5;
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     float sum = ((f02.x + g02.x) + (f13.x + g13.x)) + ((f02.y + g02.y) + (f13.y + g13.y));
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);   // over the 32-column sub-block
-    if (a.tm) {
+    if (TM) {
         // Image of a block for NT = 8 or 16 tokens (matmul_tm.cu): a tile per 64 columns of 2 NT rows of 128 bytes (row p the hi parts
         // of token p, row NT + p the lo parts; 16-byte piece j of a row at j ^ (row & 7), the 128-byte swizzle), then the
         // sub-block sums [8][NT], the block scales [NT] and the sums of squares [NT]. Q4_K, piece j: columns 4 j + {0, 2, 1, 3} of
@@ -1075,7 +1076,9 @@ cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t
     if (q8) c.img8 = xq + nx_image_off(FMT_Q8_0, q4, q6, cols, tgs_cap);
     c.att = in.att; c.n_splits = in.n_splits;
     c.table = in.table; c.col_idx = in.col_idx; c.list_stride = in.list_stride; c.col_off = in.col_off;
-    return launch_kernel(in.table ? act_convert_nx_kernel<16, true> : in.att && in.n_splits > 16 ? act_convert_nx_kernel<40, false> : act_convert_nx_kernel<16, false>, dim3(cols / 256, in.table ? 4 * in.n_tgs : (P + 3) / 4 * 4), dim3(64),
+    return launch_kernel(in.table ? act_convert_nx_kernel<16, true, false>
+                         : in.att && in.n_splits > 16 ? (in.tm ? act_convert_nx_kernel<40, false, true> : act_convert_nx_kernel<40, false, false>)
+                         : in.tm ? act_convert_nx_kernel<16, false, true> : act_convert_nx_kernel<16, false, false>, dim3(cols / 256, in.table ? 4 * in.n_tgs : (P + 3) / 4 * 4), dim3(64),
                          0, stream, pdl, c);
 }
 
