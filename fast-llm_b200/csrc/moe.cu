@@ -362,6 +362,10 @@ static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y,
         in.x = m->g; in.x2 = m->u; in.xstride = F; in.wnorm = nullptr;
         in.n_parts = parts_gu; in.part_stride = R * F;
         in.col_idx = in.out_idx;
+        // this conversion releases its dependent at entry: gate | up started after the conversion in front of it had waited, so that table
+        // and weights are in place, and the down matmul's CTAs request weights as those of gate | up leave (2048 x 2048, 4 experts, one
+        // token: 26.7 -> 24.6 us; 4096 x 6144, 16 experts, 12 tokens: 120.9 -> 120.1)
+        in.dep_first = 0;
         CKM(launch_nx_convert(in, &dn, 1, F, P, m->xq, m->tgs, s, kMoePdlNx != 0));
         CKM(launch_nx_matmul(in, &dn, 1, F, P, 0, m->xq, m->tgs, ctx->status, ctx->sms, s, kMoePdlNx != 0, true));
         if (!one_pass) CKM(launch_scatter_rows(m->d, parts_d, R * E, m->table, m->pair_list, T, off, P, in.n_groups, m->part, E, s));

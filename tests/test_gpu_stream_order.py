@@ -6,6 +6,7 @@ import math
 import pytest
 
 from fast_llm_b200 import capi
+from fast_llm_b200.moe import MoeBlock
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -20,6 +21,78 @@ def inputs(fmt, rows, cols, nx, seed):
     for o in at:
         w[:, o:o + 2] = d
     return w.reshape(rows, -1), torch.randn((nx, cols), device="cuda", generator=g)
+
+
+class Writers:
+    """What comes in front of a call here are kernels of the library's own that let the next launch start at their entry, behind a matvec
+    whose last unit runs on one SM: the call's CTAs are on the other SMs before a single byte of its inputs is written."""
+
+    def __init__(self, ctx):
+        self.ctx = ctx
+        units = 2 * ctx.sm_count() + 1
+        self.w, self.x = inputs(capi.Q4_K, 16 * units, 14336, 1, 77)
+        self.y = torch.zeros(16 * units, device="cuda")
+
+    def block(self):
+        self.ctx.matvec_assign(capi.Q4_K, self.w, self.y.numel(), 14336, self.x, self.y)
+
+    def fill(self, t, value):
+        capi._ck(self.ctx.lib.fl_b200_memset(self.ctx._h, C.c_void_p(t.data_ptr()), value, C.c_size_t(t.numel() * t.element_size())))
+
+    def floats(self, source, out):
+        """out = source's weights times its column: random numbers that a matvec of the library writes."""
+        w, x = source
+        self.ctx.matvec_assign(capi.Q4_K, w, out.numel(), 2048, x, out)
+
+    def source(self, n, seed, scale):
+        w, x = inputs(capi.Q4_K, n, 2048, 1, seed)
+        return w, x * scale
+
+    def check(self, write, call, out):
+        """call() after write(0), write(1), write(0), ... without a pause against the same one by one."""
+        want = []
+        for i in range(2):
+            write(i, self.ctx.sync)
+            call()
+            self.ctx.sync()
+            want.append([o.clone() for o in out])
+        torch.cuda.synchronize()
+        assert all(bool(torch.isfinite(o).all()) for w in want for o in w)
+        assert not any(torch.equal(a, b) for a, b in zip(*want))
+        got = []
+        with torch.cuda.stream(torch.cuda.ExternalStream(self.ctx.stream())):
+            for i in range(12):
+                self.block()
+                write(i % 2, lambda: None)
+                call()
+                call()
+                got.append([o.clone() for o in out])
+        torch.cuda.synchronize()
+        for i, g in enumerate(got):
+            assert all(torch.equal(a, b) for a, b in zip(g, want[i % 2])), i
+        assert self.ctx.status() == 0
+
+
+@pytest.mark.parametrize("n_tok,n_expert,top_k,n_ff", [(1, 4, 2, 2048), (4, 4, 2, 2048), (16, 8, 3, 4096), (19, 4, 1, 2048)])   # the last: two passes
+def test_block_written_by_the_kernels_before(ctx, n_tok, n_expert, top_k, n_ff):
+    E, wr = 2048, Writers(ctx)
+    blk = MoeBlock(ctx, E, n_ff, n_expert, top_k, max_tokens=32)
+    gate, up = (torch.zeros((n_expert * n_ff, capi.row_bytes(capi.Q4_K, E)), dtype=torch.uint8, device="cuda") for _ in range(2))
+    down = torch.zeros((n_expert, E, capi.row_bytes(capi.Q4_K, n_ff)), dtype=torch.uint8, device="cuda")
+    router, x, y = torch.zeros((n_expert, E), device="cuda"), torch.zeros((n_tok, E), device="cuda"), torch.zeros((n_tok, E), device="cuda")
+    blk.set_weights(router, gate, up, down)
+    xs, rs = ([wr.source(n, 10 * n + i, 0.01) for i in range(2)] for n in (n_tok * E, n_expert * E))
+    torch.cuda.synchronize()
+
+    def write(i, pause):   # every tensor of the block, the router last
+        steps = [lambda: wr.fill(gate, 0x21 + i), lambda: wr.fill(up, 0x24 - i)]
+        steps += [lambda e=e: wr.fill(down[e], 0x18 + e + 5 * i) for e in range(n_expert)]
+        for s in steps + [lambda: wr.floats(xs[i], x), lambda: wr.floats(rs[i], router)]:
+            s()
+            pause()
+
+    wr.check(write, lambda: blk.forward(x, n_tok, y), [y])
+    blk.close()
 
 
 @pytest.mark.parametrize("fmt", [capi.Q4_K, capi.Q6_K, capi.Q8_0])
