@@ -138,6 +138,7 @@ struct NxIn {
     // the rows are numbered through, expert by expert in the table's order.
     const uint32_t *table, *col_idx, *out_idx;
     uint32_t list_stride, col_off, n_groups, n_experts, n_tgs;   // n_groups: upper bound of active experts; n_tgs: of their groups of four columns
+    uint32_t sms;            // of the device
     int table_ready;         // 1: the table was complete before the kernel in front of the matmul started
     int dep_first;           // 1: the launch after the conversion starts only when what lies in front of the conversion has completed
     int tm;                  // 1: launch_nx_convert builds the image of matmul_tm.cu (Q4_K or Q6_K, one format, not grouped)

@@ -205,7 +205,7 @@ struct ConvArgs {
     uint32_t xstride, rstride, n_parts, P, nblk;
     uint8_t *img4, *img6, *img8;   // images wanted (nullptr: not)
     const uint32_t *table, *col_idx;   // grouped columns (see below)
-    uint32_t list_stride, col_off;
+    uint32_t list_stride, col_off, n_groups;   // n_groups: the table has room for so many
     const float *att;              // the columns are attention contexts of heads of 128, added up here from n_splits records
     uint32_t n_splits;             // (attn.cu: [column][head][split][132] = context, maximum, sum)
     int tm;                        // img4 or img6 is the image of matmul_tm.cu
@@ -286,9 +286,10 @@ __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     if (GROUPED) {   // the group of four is one of all active experts' together: look its expert up
         const uint32_t n_act = a.table[0], lane = threadIdx.x & 31u, at = tg;
         ntg = 0;
-        for (uint32_t b = 0; b < n_act && ntg == 0; b += 32) {
+        for (uint32_t b = 0; b < a.n_groups && ntg == 0; b += 32) {
             uint4 e = make_uint4(0u, 0u, 0u, 0u);
-            if (b + lane < n_act) e = reinterpret_cast<const uint4 *>(a.table)[1 + b + lane];
+            if (b + lane < a.n_groups) e = reinterpret_cast<const uint4 *>(a.table)[1 + b + lane];   // requested together with n_act
+            if (b + lane >= n_act) e.y = 0;
             const uint32_t n = (e.y + 3) / 4, mask = __ballot_sync(0xffffffffu, at - e.z < n);
             if (mask) {
                 const int l = __ffs(mask) - 1;
@@ -1075,11 +1076,17 @@ cudaError_t launch_nx_convert(const NxIn &in, const NxTensor *t, int n, uint32_t
     if (q6) c.img6 = xq + nx_image_off(FMT_Q6_K, q4, q6, cols, tgs_cap);
     if (q8) c.img8 = xq + nx_image_off(FMT_Q8_0, q4, q6, cols, tgs_cap);
     c.att = in.att; c.n_splits = in.n_splits;
-    c.table = in.table; c.col_idx = in.col_idx; c.list_stride = in.list_stride; c.col_off = in.col_off;
+    c.table = in.table; c.col_idx = in.col_idx; c.list_stride = in.list_stride; c.col_off = in.col_off; c.n_groups = in.n_groups;
+    // Grouped, up to eight blocks an SM: each reserves an eighth of the SM's shared memory, so that they spread. They come while the matmul in
+    // front leaves, and without that gather on the first SMs it frees (16 rather than 6 of them for 128 blocks; gate | up's end to the
+    // conversion's, 2048 x 2048, 4 experts, 4 tokens: 4.6 -> 3.2 us; 2048 x 4096, 4 experts, 8 tokens, whole block 51.2 -> 49.2).
+    // More blocks than that take what room there is (4096 x 14336, 16 tokens: 275 us, 280 with eight an SM).
+    const uint32_t blocks = cols / 256 * 4 * in.n_tgs;
+    const size_t reserve = in.table && blocks <= 8u * in.sms ? 24 * 1024 : 0;
     return launch_kernel(in.table ? act_convert_nx_kernel<16, true, false>
                          : in.att && in.n_splits > 16 ? (in.tm ? act_convert_nx_kernel<40, false, true> : act_convert_nx_kernel<40, false, false>)
                          : in.tm ? act_convert_nx_kernel<16, false, true> : act_convert_nx_kernel<16, false, false>, dim3(cols / 256, in.table ? 4 * in.n_tgs : (P + 3) / 4 * 4), dim3(64),
-                         0, stream, pdl, c);
+                         reserve, stream, pdl, c);
 }
 
 cudaError_t launch_nx_matmul(const NxIn &in, const NxTensor *t, int n, uint32_t cols, uint32_t P, int accumulate, const uint8_t *xq,

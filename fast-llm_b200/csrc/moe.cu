@@ -352,7 +352,7 @@ static int moe_enqueue(fl_b200_moe *m, const float *x, uint32_t n_tok, float *y,
         NxIn in{};
         in.x = x; in.xstride = E; in.wnorm = wnorm; in.eps = eps;
         in.table = m->table; in.col_idx = m->tok_list; in.out_idx = one_pass ? m->pair_list : nullptr; in.list_stride = T; in.col_off = off;
-        in.n_groups = std::min(m->n_local, n_tok * K); in.n_experts = m->n_local;
+        in.n_groups = std::min(m->n_local, n_tok * K); in.n_experts = m->n_local; in.sms = ctx->sms;
         in.n_tgs = std::min(in.n_groups * ((P + 3) / 4), n_tok * K / 4 + in.n_groups);
         // a conversion starts its dependent after it has waited for the kernel that wrote the table, so that the table is in place for
         // every matmul

@@ -120,6 +120,7 @@ def test_q4_k_sums_are_not_truncated(ctx, nx):
     (capi.Q4_K, capi.Q4_K, 8, 2, 16, 16), (capi.Q4_K, capi.Q6_K, 16, 1, 3, 16), (capi.Q6_K, capi.Q4_K, 4, 4, 16, 16),
     (capi.Q4_K, capi.Q4_K, 4, 3, 45, 64),    # more tokens per expert than a pass takes
     (capi.Q4_K, capi.Q4_K, 64, 1, 2, 16),    # most experts idle
+    (capi.Q4_K, capi.Q4_K, 48, 6, 16, 16),   # more than 32 at work: the conversion's lookup takes a second round
 ])
 def test_grouped_experts(ctx, fmt_gu, fmt_d, n_expert, top_k, n_tok, max_tokens):
     E, F = 2048, 4096
