@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(const __gr
     const uint32_t group = a.n_q_head / a.n_kv_head;   // == kGroup (checked on the host)
     const bool fused = MODE == 2 ? a.rope_k != nullptr : MODE == 1;
     if (tid == 0) trace_min(a.trace, 0);
-    griddep_launch_dependents();
+    if (MODE != 0 || !a.late) griddep_launch_dependents();
     // *pos was written at the end of the previous step (or is kv_len - 1 of a single call): stable here.
     const uint32_t kv_len = (a.pos ? (uint32_t)a.pos[b * a.pos_stride] + 1u : a.kv_len) + b * a.kv_len_step;
     const uint32_t tiles_total = (kv_len + kTile - 1) / kTile;
@@ -296,6 +296,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(const __gr
         if (tid == 0 && it + kStages < n_tiles) issue(it + kStages);
     }
 
+    if (MODE == 0 && a.late) griddep_launch_dependents();
     // ---- merge the 4 warps' (max, sum, context) and write this split's partial ----
     // o[dt][0] + o[dt][1] = context of head t at dim 16dt + g; o[dt][2] + o[dt][3] at dim 16dt + g + 8.
 #pragma unroll
@@ -416,7 +417,7 @@ __global__ void __launch_bounds__(kShWarps * 32, 2) attn_shared_kernel(const __g
     const uint32_t g = lane >> 2, t = lane & 3u;
     const uint32_t split = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z * kShWarps + warp;
     const uint32_t b_last = min(blockIdx.z * kShWarps + kShWarps, a.batch) - 1;
-    griddep_launch_dependents();
+    if (!a.late) griddep_launch_dependents();
     const uint32_t kv0 = a.pos ? (uint32_t)a.pos[0] + 1u : a.kv_len;
     const uint32_t kv_max = kv0 + b_last * a.kv_len_step;         // keys the CTA's last position attends
     const uint32_t kv_len = kv0 + b * a.kv_len_step;              // ... this warp's
@@ -557,6 +558,7 @@ __global__ void __launch_bounds__(kShWarps * 32, 2) attn_shared_kernel(const __g
         __syncthreads();   // tile fully consumed by all warps: the slot can be refilled
         if (tid == 0 && it + kStages < n_tiles) issue(it + kStages);
     }
+    if (a.late) griddep_launch_dependents();
     if (b > b_last) return;
     float *part = a.part + (((uint64_t)b * a.n_q_head + (uint64_t)hkv * kGroup + t) * a.n_splits + split) * kPartStride;
 #pragma unroll
@@ -718,6 +720,25 @@ size_t attn_static_max_records(void) { return kStaticMaxRecords; }
 uint32_t attn_static_max_tickets(void) { return kStaticMaxTickets; }
 
 bool attn_uses_records(const AttnArgs &a) { return a.shared_kv && !a.per_position && a.batch > 1 && !a.rope_k && a.pos_stride == 0 && a.n_splits <= 64; }
+
+// Calls by themselves as programmatic dependents. A CTA that becomes resident under the launch in front takes a place that one has not
+// filled or has just left, so that a grid smaller than the places there are (two CTAs an SM) can come to lie two on an SM beside idle
+// ones; and where every launch releases the next at its entry, several of them wait on the SMs at once. us as ordinary launches / released
+// at entry / released behind the tiles, for calls in a row:
+//   attn_verify, one KV head, 8 positions over 60000 keys, 63 CTAs: 30.8 / 45.2 / 29.0; attn_decode, 8 KV heads: 1024 keys 8.2 / 5.4 / 5.4; 13 x 20000,
+//   208 CTAs of 157 tiles 158 / 168 / 155; 64 KV heads and sequences over 2048 keys, 10 tiles 14.4 / 14.6 / 12.1. So a launch of one wave releases behind
+//   its tiles; one of several waves at entry, when its last CTAs have started (320 CTAs of one tile 12.3 / 9.1 / 9.5).
+//   Long tiles' lists on a grid with places to spare: 280 CTAs of 94 tiles 132 / 134 / 133, of 188 252 / 269 / 257, 224 of 698 717 / 801 / 831, 288 of 543
+//   833 / 767 / 783: an ordinary launch for more than 128 tiles where the grid leaves more than a twenty-fifth of the places.
+//   Several positions over one cache on more than half the SMs but not all, more than a tile a CTA: ordinary, since the next launch's CTAs pair up either
+//   way (126 CTAs of 15 tiles 32.8 / 31.2 / 45.0, of 4 tiles 14.4 / 17.2 / 15.9).
+void attn_release(AttnArgs &a, int sms) {
+    const bool several = attn_uses_records(a);
+    const uint32_t ctas = a.n_splits * a.n_kv_head * (several ? (a.batch + kShWarps - 1) / kShWarps : a.batch), n = (uint32_t)sms;
+    const uint32_t tiles = (a.kv_len + (a.batch - 1) * a.kv_len_step + kTile - 1) / kTile, per_cta = (tiles + a.n_splits - 1) / a.n_splits;
+    a.late = ctas <= 2 * n;
+    a.pdl = !(25 * ctas < 48 * n && per_cta > 128) && !(several && 2 * ctas > n && ctas <= n && per_cta > 1);
+}
 
 cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t stream) {
     if (a.n_kv_head == 0 || a.n_q_head != a.n_kv_head * kGroup || a.n_splits == 0 || a.batch == 0)

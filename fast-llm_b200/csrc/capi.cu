@@ -406,7 +406,7 @@ static int attn_impl(fl_b200_ctx *c, const float *q, const uint16_t *k, const ui
     a.shared_kv = verify ? 1u : 0u;
     a.scale = scale;
     a.status = c->status;
-    a.pdl = pos_dev ? 0 : 1;   // a programmatic dependent reads *pos before what lies in front has completed; keys and values only after
+    if (!pos_dev) attn_release(a, c->sms);   // (a programmatic dependent reads *pos before what lies in front has completed; keys and values only after)
     const size_t need = attn_part_floats(n_q, batch, a.n_splits) * sizeof(float);
     if (int rc = grow_attn_part(c, need)) return rc;
     a.part = c->attn_part;

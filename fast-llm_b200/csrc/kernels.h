@@ -199,6 +199,7 @@ struct AttnArgs {
     float scale;
     uint32_t *status;
     int pdl;
+    int late;              // dependents are released behind the tiles instead of at entry (attn_release)
     int records_only;      // several positions of one cache (attn_uses_records): leave the splits' records in part, out is not written
     int per_position;      // several positions of one cache, but one CTA per position all the same (attn_few_tiles)
     unsigned long long *trace;   // optional 4-entry timeline record (diagnostics)
@@ -218,6 +219,7 @@ cudaError_t attn_make_maps(AttnArgs &a);
 bool attn_few_tiles(uint32_t n_kv_head, uint32_t batch, uint32_t kv_len);
 bool attn_uses_records(const AttnArgs &a);   // the launch is one of several positions over one cache (attn_shared_kernel)
 cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t stream);
+void attn_release(AttnArgs &a, int sms);     // pdl and late of a call by itself (pos == nullptr), everything else set
 // Same kernel with the split-KV scratch in a fixed file-scope device array
 // (no allocation at call time); cudaErrorMemoryAllocation when the launch needs
 // more than attn_static_max_records() records or attn_static_max_tickets()

@@ -100,6 +100,40 @@ def test_block_written_by_the_kernels_before(ctx, n_tok, n_expert, top_k, n_ff):
     blk.close()
 
 
+# one position and several, with and without the records' sum; CTAs: one, one wave of one tile, of several, more than one wave; several positions on less
+# than half the SMs, on more than half of them (one tile a CTA, several), on all
+@pytest.mark.parametrize("kind,kv,batch,kv_len", [
+    ("decode", 1, 1, 2), ("decode", 2, 1, 1024), ("lse", 1, 3, 20001), ("decode", 8, 16, 1100), ("lse", 8, 40, 64), ("verify", 1, 2, 100),
+    ("verify", 1, 8, 30000), ("verify", 2, 8, 4000), ("verify", 2, 8, 16000), ("verify", 1, 16, 16000), ("verify", 8, 5, 9001)])
+def test_attention_written_by_the_kernels_before(ctx, kind, kv, batch, kv_len):
+    wr, shared = Writers(ctx), kind == "verify"
+    seqs = 1 if shared else batch
+    k, v = (torch.zeros((seqs * kv, kv_len, 128), dtype=torch.float16, device="cuda") for _ in range(2))
+    q, out, lse = (torch.zeros((batch, 4 * kv, n), device="cuda") for n in (128, 128, 2))
+    qs = [wr.source(q.numel(), 5 + i, 0.01) for i in range(2)]
+    half, scale = kv_len // 2, 1.0 / math.sqrt(128)
+    torch.cuda.synchronize()
+
+    def write(i, pause):   # keys and values of the first half of the positions unlike those of the second, per head while there are few
+        steps = [lambda: wr.floats(qs[i], q)]
+        for t, first, rest in ((k, 0x2c + i, 0x30 - i), (v, 0x38 + i, 0x3c - 3 * i)):
+            steps.append(lambda t=t, rest=rest: wr.fill(t, rest))
+            steps += [lambda t=t, h=h, first=first: wr.fill(t[h, :half], first) for h in range(min(seqs * kv, 8))]
+        for s in steps:
+            s()
+            pause()
+
+    def call():
+        if shared:
+            ctx.attn_verify(q, k, v, 4 * kv, kv, 128, kv_len - batch + 1, kv_len, batch, scale, out)
+        elif kind == "lse":
+            ctx.attn_decode_lse(q, k, v, 4 * kv, kv, 128, kv_len, kv_len, batch, scale, out, lse)
+        else:
+            ctx.attn_decode(q, k, v, 4 * kv, kv, 128, kv_len, kv_len, batch, scale, out)
+
+    wr.check(write, call, [out, lse] if kind == "lse" else [out])
+
+
 @pytest.mark.parametrize("fmt", [capi.Q4_K, capi.Q6_K, capi.Q8_0])
 @pytest.mark.parametrize("rows,cols,nx", [(16, 2048, 1), (4096, 4096, 1), (2049, 14336, 1), (4096, 4096, 3), (300, 2048, 16)])
 def test_weights_written_by_the_kernel_before(ctx, fmt, rows, cols, nx):
