@@ -56,6 +56,9 @@ __host__ __device__ constexpr uint32_t pitch_of(int fmt) { return fmt == FMT_Q4_
 // A stage: the rows' bytes, then the step's activation (the operand's four tiles, sub-block sums, block scales, sums of squares).
 template <int F, int T> constexpr uint32_t kSlot = (kRows * pitch_of(F) + T * 1064 + 1023) & ~1023u;
 template <int F, int T> constexpr uint32_t kSlots = (kSmemLimit - head_of(T)) / kSlot<F, T> < kMaxSlots ? (kSmemLimit - head_of(T)) / kSlot<F, T> : kMaxSlots;
+// The unpack groups take the steps in turn. A group that waits for step j has seen the tensor core take step j - 4, hence that and all before it
+// landed: with four slots or more the slot's last stage is one of those, and the parity of its barrier tells the two apart.
+static_assert(kSlots<FMT_Q4_K, 8> >= 4 && kSlots<FMT_Q4_K, 16> >= 4 && kSlots<FMT_Q6_K, 8> >= 4 && kSlots<FMT_Q6_K, 16> >= 4, "slots");
 
 struct TmT {
     float *y;

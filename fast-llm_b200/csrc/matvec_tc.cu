@@ -38,6 +38,7 @@
 // the form that decides everything at run time: see matvec_tc_kernel.
 #include "common.cuh"
 #include "kernels.h"
+#include "ring.h"
 #include "tc_ops.cuh"
 
 #include <cuda.h>
@@ -617,7 +618,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
     if (warp == kProducer) {
         // ---- producer: one bulk copy per row and stage; the weights do not depend on any activation ----
         const TcSmem sm = tc_carve<G>(smem_raw, 256, false, false, false, S, a.ring_off);
-        uint32_t slot = 0, par = 1;   // a fresh barrier passes a wait on parity 1
+        RingTurn<G> turn;
         if (a.w_after) griddep_wait();
         const uint64_t pol = a.l2_hints ? l2_policy_evict_first() : 0ull;
 #pragma unroll 1
@@ -637,8 +638,8 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                 const uint32_t segb = fmt == FMT_Q4_K ? kSeg4 : fmt == FMT_Q6_K ? kSeg6 : kSeg8;
                 const uint32_t row0 = ph.swiglu ? 8 * u : 16 * (u - ph.t[ti].unit0);
                 for (uint32_t seg = 0; seg < nseg; ++seg) {
-                    const uint32_t off = seg * segb;
-                    if (!mbar_wait_bounded(&sm.empty[slot], par, a.status)) return;
+                    const uint32_t off = seg * segb, slot = turn.slot[0];
+                    if (!mbar_wait_bounded(&sm.empty[slot], turn.par[0], a.status)) return;
                     fence_proxy_async_smem();
                     const uint32_t dst = ring + slot * a.slot_bytes;
                     if ((F == 0 || F == 4) && fmt == FMT_Q8_0) {
@@ -671,7 +672,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                             if (ph.swiglu) tma_box2(dst + 8 * segb, &ph.t[1].map, off / 8, row0, &sm.full[slot]);
                         }
                     }
-                    if (++slot == S) { slot = 0; par ^= 1u; }
+                    turn.next(S);
                 }
             }
         }
@@ -680,7 +681,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
 
     uint32_t it_base = 0;    // stages of this CTA in earlier phases
     // consumer warps: the next stage of this warp's group (index over the whole launch), its ring slot and parity
-    uint32_t c_it = (warp / kCW) % G, c_slot = c_it % a.nslots, c_par = 0;
+    uint32_t c_it = (warp / kCW) % G, c_slot = c_it, c_par = 0;
     bool dead = false;       // a bounded wait of this warp ran out
     uint32_t kk = 0;         // units of this CTA so far (all phases): selects the reduction buffer
 #pragma unroll 1
@@ -1007,8 +1008,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                         }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&sm.empty[c_slot]);
-                        c_slot += G;
-                        if (c_slot >= S) { c_slot -= S; c_par ^= 1u; }
+                        ring_next<G>(c_slot, c_par, S);
                     }
                 } else if (is4 && I8) {
 #pragma unroll 1
@@ -1026,8 +1026,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                         }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&sm.empty[c_slot]);
-                        c_slot += G;
-                        if (c_slot >= S) { c_slot -= S; c_par ^= 1u; }
+                        ring_next<G>(c_slot, c_par, S);
                     }
                 } else if (F == 0 && fmt == FMT_Q4_K) {
 #pragma unroll 1
@@ -1045,8 +1044,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                         }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&sm.empty[c_slot]);
-                        c_slot += G;
-                        if (c_slot >= S) { c_slot -= S; c_par ^= 1u; }
+                        ring_next<G>(c_slot, c_par, S);
                     }
                 } else if (F == 0 && fmt == FMT_Q8_0) {
 #pragma unroll 1
@@ -1063,8 +1061,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                         }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&sm.empty[c_slot]);
-                        c_slot += G;
-                        if (c_slot >= S) { c_slot -= S; c_par ^= 1u; }
+                        ring_next<G>(c_slot, c_par, S);
                     }
                 } else if (I8) {
 #pragma unroll 1
@@ -1083,8 +1080,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                         }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&sm.empty[c_slot]);
-                        c_slot += G;
-                        if (c_slot >= S) { c_slot -= S; c_par ^= 1u; }
+                        ring_next<G>(c_slot, c_par, S);
                     }
                 } else if (F == 0) {
 #pragma unroll 1
@@ -1102,8 +1098,7 @@ __global__ void __launch_bounds__((G * kCW + 2) * 32) matvec_tc_kernel(const __g
                         }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&sm.empty[c_slot]);
-                        c_slot += G;
-                        if (c_slot >= S) { c_slot -= S; c_par ^= 1u; }
+                        ring_next<G>(c_slot, c_par, S);
                     }
                 }
                 // the unit's partial sums of rows g and g + 8, one per lane column (the finalizer adds those too)
