@@ -358,7 +358,12 @@ matvec_stream_kernel(const MatvecArgs a, const __grid_constant__ TensorMaps maps
                      const int stages, const int use_q4, const int use_q6) {
     constexpr bool use_q8 = Q8;   // use_q4 is set for Q8_0 launches: they use the Q4_K plane layout
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    if (a.t[0].expert_id != nullptr && *a.t[0].expert_id == kExpertSkip) return;   // not this GPU's expert (see MatvecTensor)
+    if (a.t[0].expert_id != nullptr && *a.t[0].expert_id == kExpertSkip) {   // not this GPU's expert (see MatvecTensor)
+        // A launch that waited for nothing would be over before the one in front of it, and the next one, which waits for this one
+        // alone, would write what that still reads (the gate and up rows of the slot before).
+        griddep_wait();
+        return;
+    }
     const uint32_t nw = blockDim.x >> 5;   // warps of this launch
     const Smem sm = carve(smem_raw, a.cols, use_q4 != 0, use_q6 != 0, stages, nw);   // Q8_0 uses the Q4_K plane layout (use_q4 is set)
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
