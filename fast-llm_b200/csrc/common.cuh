@@ -184,6 +184,13 @@ __device__ __forceinline__ float h2f_bits(uint16_t h) {
     return __half2float(__ushort_as_half(h));
 }
 
+// Larger of the two, NaN where either is (fmaxf drops a NaN).
+__device__ __forceinline__ float fmax_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 #endif // __CUDACC__
 
 // Launch helper: optional programmatic dependent launch (the kernel must call

@@ -531,10 +531,10 @@ matvec_stream_kernel(const MatvecArgs a, const __grid_constant__ TensorMaps maps
         }
         float amax = 0.f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
+        for (int i = 0; i < 16; ++i) amax = fmax_nan(amax, fabsf(v[i]));
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));   // over the half-warp
-        const float s = amax > 0.f ? amax / kFixMax : 1.0f;
+        for (int o = 8; o > 0; o >>= 1) amax = fmax_nan(amax, __shfl_xor_sync(0xffffffffu, amax, o));   // over the half-warp
+        const float s = amax == 0.f ? 1.0f : amax / kFixMax;   // (a NaN among the columns makes the block's sums NaN)
         const float inv_s = 1.0f / s;
         int sum = 0;
         uint32_t pk[3][4] = {{0u, 0u, 0u, 0u}, {0u, 0u, 0u, 0u}, {0u, 0u, 0u, 0u}};   // this lane's 16 columns of each digit plane

@@ -84,6 +84,23 @@ def test_stream_dot_idx_vs_oracle(ctx, checker, fmt, rows, cols):
         ctx.matvec_expert(fmt, wd, rows, cols, idx, stride + 2, xd, yd)   # stride not a whole number of rows
 
 
+@pytest.mark.parametrize("fmt", [capi.Q4_K, capi.Q6_K, capi.Q8_0])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_expert_matvec_hides_no_nan(ctx, fmt, bad):
+    """A NaN or an infinity among the columns reaches every row, as in a sum of products (a quant or a scale of zero makes NaN of it too)."""
+    rows, cols = 64, 4096
+    w = torch.from_numpy(synth.quant_tensor(fmt, np.random.default_rng(3), 2 * rows, cols)).cuda()
+    x = torch.randn(cols, device="cuda")
+    x[1234] = bad
+    eid = torch.ones(1, dtype=torch.int32, device="cuda")
+    y = torch.zeros(rows, device="cuda")
+    torch.cuda.synchronize()
+    ctx.matvec_expert(fmt, w, rows, cols, eid, rows * capi.row_bytes(fmt, cols), x, y)
+    ctx.sync()
+    assert ctx.status() == 0
+    assert not torch.isfinite(y).any()
+
+
 def test_moe_ffn_block_mixtral_shape(ctx, checker):
     """Router -> top-2 experts (gate, up, SiLU*up, down through STREAM_DOT_IDX) -> WMERGE
     with the residual, for 3 tokens; experts Q4_K, router f32 ~ N(0, 0.02) as in the

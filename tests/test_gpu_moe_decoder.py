@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from fast_llm_b200 import capi, synth
+from fast_llm_b200.decoder import Decoder
 from fast_llm_b200.moe import MoeBlock
 from test_gpu_decoder import build_pair, force_kv, logits_close, LOGIT_TOL, HIDDEN_TOL
 
@@ -112,3 +113,52 @@ def test_one_token_over_its_experts(ctx, checker, fmt_gu, fmt_down, NE, K, F):
         force_kv(ctx, dec, orc, CFG, 5 + step)
         tok = want_tok
     dec.close(); orc.close()
+
+
+def gpu_decoder(ctx, E, F, NE, K, fmt_gu, fmt_down, seed, spoil=None):
+    """One layer of attention and experts over random weights, without an oracle. spoil(gate): last change of the gate rows."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+
+    def quants(fmt, rows, cols):
+        n = rows * cols // capi.BLK_ELEMS[fmt]
+        w = torch.randint(0, 256, (n, capi.BLK_BYTES[fmt]), dtype=torch.uint8, device="cuda", generator=gen)
+        d = ((torch.rand(n, device="cuda", generator=gen) * 0.4 + 0.8) / (cols ** 0.5 * 400)).half().view(torch.uint8).reshape(-1, 2)
+        for o in {capi.Q4_K: (0, 2), capi.Q6_K: (208,)}[fmt]:
+            w[:, o:o + 2] = d
+        return w.reshape(rows, -1)
+
+    def norm():
+        return torch.rand(E, device="cuda", generator=gen) * 0.2 + 0.9
+
+    kv = E // 512
+    dec = Decoder(ctx, dict(n_layer=1, n_embd=E, n_head=4 * kv, n_kv_head=kv, head_dim=128, n_ff=512, n_vocab=600, max_kv=64, rope_base=1e4, eps=1e-5))
+    for i, (r, c) in enumerate(((E, E), (E // 4, E), (E // 4, E), (E, E))):
+        dec.set_layer_tensor(0, i, capi.Q4_K, quants(capi.Q4_K, r, c))
+    blk = MoeBlock(ctx, E, F, NE, K, fmt_gate_up=fmt_gu, fmt_down=fmt_down, max_tokens=1)
+    gate = quants(fmt_gu, NE * F, E)
+    if spoil:
+        spoil(gate)
+    blk.set_weights(torch.randn((NE, E), device="cuda", generator=gen), gate, quants(fmt_gu, NE * F, E), quants(fmt_down, NE * E, F))
+    dec.set_layer_moe(0, blk)
+    dec.set_layer_norms(0, norm(), norm())
+    dec.set_global(capi.G_TOK_EMBD, capi.Q4_K, quants(capi.Q4_K, 600, E))
+    dec.set_global(capi.G_OUTPUT, capi.Q4_K, quants(capi.Q4_K, 600, E))
+    dec.set_out_norm(norm())
+    torch.cuda.synchronize()
+    dec.finalize()
+    return dec
+
+
+@pytest.mark.parametrize("fmt", [capi.Q4_K, capi.Q6_K])
+def test_a_token_hides_no_nan(ctx, fmt):
+    """A NaN in one row's result of gate reaches the whole output of the block through down, and the logits."""
+    E, F, NE = 2048, 2048, 4
+
+    def spoil(gate):   # the scale of the first block of row 100 of every expert
+        at = {capi.Q4_K: 0, capi.Q6_K: 208}[fmt]
+        gate.view(NE, F, -1)[:, 100, at:at + 2] = torch.tensor([0x00, 0x7e], dtype=torch.uint8, device="cuda")
+
+    dec = gpu_decoder(ctx, E, F, NE, 2, fmt, fmt, 5, spoil)
+    dec.step(7)
+    assert np.isnan(dec.logits()).all()
+    dec.close()
