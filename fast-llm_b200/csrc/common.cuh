@@ -184,6 +184,9 @@ __device__ __forceinline__ float h2f_bits(uint16_t h) {
     return __half2float(__ushort_as_half(h));
 }
 
+// a b + c d in the two roundings that a compiler free to contract chooses as it likes: for sums whose bits two kernels share.
+__device__ __forceinline__ float dot2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
+
 // Larger of the two, NaN where either is (fmaxf drops a NaN).
 __device__ __forceinline__ float fmax_nan(float a, float b) {
     float r;

@@ -91,7 +91,8 @@ cudaError_t launch_matvec_tc(const MatvecArgs &a, int sms, cudaStream_t stream);
 cudaError_t launch_matvec_tc_chain(const MatvecArgs *args, int n, int sms, cudaStream_t stream);
 cudaError_t matvec_tc_init(void);
 // The experts that one token selected (matvec_expert.cu), slot k's being id[k]: y[k * rows + r] = silu(gate_r . h) * (up_r . h) with
-// h = RMSNorm(x) * wnorm (w[1] set), or y[k * rows + r] = w_r . (x + k * x_stride). Same bits as a streaming launch per slot.
+// h = RMSNorm(x) * wnorm (w[1] set), or y[k * rows + r] = w_r . (x + k * x_stride). The bits of a streaming launch per slot (gate | up: up to
+// 6144 columns).
 struct ExpertArgs {
     int fmt;
     const void *w[2];            // gate and up, or down and nullptr: the experts' rows one behind the other, packed

@@ -208,9 +208,10 @@ __device__ __forceinline__ float q4k_quarter(uint32_t blk, uint32_t c, const XSl
     const float d = h2f_bits((uint16_t)(hdr.x & 0xFFFFu)), dmin = h2f_bits((uint16_t)(hdr.x >> 16));
     // the high-nibble sums are exact multiples of 16: fold the 1/16 into the digit shifts
     const float fb = (float)((b0 << 10) + (b1 << 3) + (b2 >> 4));
-    const float t = u8f<0>(sc) * fix_to_float(a0, a1, a2) + u8f<1>(sc) * fb;
-    const float m = u8f<0>(mn) * sx.x + u8f<1>(mn) * sx.y;
-    return d * t - dmin * m;
+    // (bits shared with matvec_expert.cu, here and for Q6_K)
+    const float t = dot2(u8f<0>(sc), fix_to_float(a0, a1, a2), u8f<1>(sc), fb);
+    const float m = dot2(u8f<0>(mn), sx.x, u8f<1>(mn), sx.y);
+    return dot2(d, t, -dmin, m);
 }
 
 // Q6_K quarter (64 weights: 16 columns of each of the 4 groups of one half).
@@ -258,10 +259,10 @@ __device__ __forceinline__ float q6k_quarter(uint32_t row, uint32_t sbi, uint32_
     const uint32_t sw = __byte_perm(lo, hi, hq ? 0x7531u : 0x6420u) ^ 0x80808080u;
     const float d = h2f_bits((uint16_t)lds16(row + ob + 208));
     // value = d * sc * (q - 32): sum q*x minus 32 * sum x per 16-column group
-    float t = (u8f<0>(sw) - 128.f) * (fix_to_float(acc[0][0], acc[0][1], acc[0][2]) - 32.f * sx.x);
-    t += (u8f<1>(sw) - 128.f) * (fix_to_float(acc[1][0], acc[1][1], acc[1][2]) - 32.f * sx.y);
-    t += (u8f<2>(sw) - 128.f) * (fix_to_float(acc[2][0], acc[2][1], acc[2][2]) - 32.f * sx.z);
-    t += (u8f<3>(sw) - 128.f) * (fix_to_float(acc[3][0], acc[3][1], acc[3][2]) - 32.f * sx.w);
+    float t = dot2(u8f<0>(sw) - 128.f, fix_to_float(acc[0][0], acc[0][1], acc[0][2]) - 32.f * sx.x,
+                   u8f<1>(sw) - 128.f, fix_to_float(acc[1][0], acc[1][1], acc[1][2]) - 32.f * sx.y);
+    t = fmaf(u8f<2>(sw) - 128.f, fix_to_float(acc[2][0], acc[2][1], acc[2][2]) - 32.f * sx.z, t);
+    t = fmaf(u8f<3>(sw) - 128.f, fix_to_float(acc[3][0], acc[3][1], acc[3][2]) - 32.f * sx.w, t);
     return d * t;
 }
 

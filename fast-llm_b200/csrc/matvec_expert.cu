@@ -5,7 +5,8 @@
 // products run on mma.sync.m16n8k32 as in matvec_tc.cu (lane (g, t) holds rows g and g + 8; lane column t accumulates its own
 // sub-blocks). The results are bit for bit those of the dp4a streaming kernel (matvec.cu), one launch per slot, which this
 // replaces where it takes the shape: a model amplifies a difference of 1e-6 in an expert's output to 3e-5 of its logits, since
-// the next block's rounding of the activation is discontinuous. Hence
+// the next block's rounding of the activation is discontinuous. (But for gate | up of more than 6144 columns, whose sum of squares lies on
+// another number of warps: 1 / rms differs in its last bits, the logits by 2e-6.) Hence
 //   * the activation is that kernel's: per 256-column block X = rint(x / s), s = amax / 1040000, sums of X exact in 32 bits. X
 //     is cut into three balanced 8-bit digits (there: 7-bit ones for dp4a), two in the first instruction of a pair and one in the
 //     second; the digit sums are put together in 32-bit integers, the same numbers as there;
@@ -97,9 +98,8 @@ __device__ __forceinline__ void q4k_block_x21(uint32_t r0, uint32_t oh, uint32_t
         const float fa = (float)whole(cL[0][2 * r], cL[0][2 * r + 1], cL[1][2 * r]);
         // the high nibbles' sums are multiples of 16, and too large for 32 bits before the division
         const float fb = (float)(cH[0][2 * r] * 4096 + cH[0][2 * r + 1] * 16 + (cH[1][2 * r] >> 4));
-        const float q = u8f<0>(sc) * fa + u8f<1>(sc) * fb;
-        const float m = u8f<0>(mn) * sx.x + u8f<1>(mn) * sx.y;
-        (r ? out1 : out0) = d * q - dmin * m;
+        const float q = dot2(u8f<0>(sc), fa, u8f<1>(sc), fb), m = dot2(u8f<0>(mn), sx.x, u8f<1>(mn), sx.y);
+        (r ? out1 : out0) = dot2(d, q, -dmin, m);
     }
 }
 
@@ -168,7 +168,7 @@ __device__ __forceinline__ void q6k_block_x21(uint32_t r0, uint32_t r1, uint32_t
             const float f = (float)whole(c0[2 * r], c0[2 * r + 1], c1[2 * r]) - 32.f * sx[gq];
             const float sc = gq == 0 ? s8f<0>(sw[r]) : gq == 1 ? s8f<1>(sw[r]) : gq == 2 ? s8f<2>(sw[r]) : s8f<3>(sw[r]);
             if (gq == 0) { sc0[r] = sc; f0[r] = f; }
-            else v[r] = gq == 1 ? fmaf(sc0[r], f0[r], __fmul_rn(sc, f)) : fmaf(sc, f, v[r]);
+            else v[r] = gq == 1 ? dot2(sc0[r], f0[r], sc, f) : fmaf(sc, f, v[r]);
         }
     }
     out0 = dd[0] * v[0];

@@ -41,6 +41,7 @@ struct fl_b200_moe {
     float *g = nullptr, *u = nullptr, *d = nullptr, *h = nullptr;         // h: silu(gate) * up of every slot of one token
     uint8_t *xq = nullptr;
     uint32_t rows = 0, tgs = 0, planes_gu = 0, planes_d = 0;              // tgs: groups of four columns in xq
+    bool expert_kernel = true;                                            // FLB_MOE_TOKEN=0 when it was created: a decoded token per slot
     uint8_t *arena = nullptr;                                             // the one allocation that holds the block's own buffers
     uint8_t *comm = nullptr;
     uint8_t *peers[kCommMaxRanks] = {};
@@ -80,6 +81,7 @@ int fl_b200_moe_create(fl_b200_ctx *ctx, const fl_b200_moe_cfg *cfg, uint32_t ra
         if (fmt != FL_B200_Q4_K && fmt != FL_B200_Q6_K) return set_err(FL_B200_ERR_ARG, "moe_create: expert format %d (Q4_K or Q6_K)", fmt);
     CKM(cudaSetDevice(ctx->device));
     fl_b200_moe *m = new fl_b200_moe();
+    if (const char *v = getenv("FLB_MOE_TOKEN")) m->expert_kernel = v[0] != '0';
     m->ctx = ctx; m->c = c; m->rank = rank; m->world = world;
     m->n_local = c.n_expert / world;
     m->base = rank * m->n_local;
@@ -299,7 +301,7 @@ static int moe_enqueue_per_slot(fl_b200_moe *m, const float *x, uint32_t n_tok, 
 // One token of a decoder step: the experts of all its slots in one launch for gate | up and one for down (matvec_expert.cu).
 static bool moe_one_token(const fl_b200_moe *m) {
     const fl_b200_moe_cfg &c = m->c;
-    return m->world == 1 && c.top_k <= (uint32_t)m->ctx->sms && matvec_expert_takes(c.fmt_gate_up, c.n_embd, c.n_ff, c.top_k, c.n_expert) &&
+    return m->expert_kernel && m->world == 1 && c.top_k <= (uint32_t)m->ctx->sms && matvec_expert_takes(c.fmt_gate_up, c.n_embd, c.n_ff, c.top_k, c.n_expert) &&
            matvec_expert_takes(c.fmt_down, c.n_ff, c.n_embd, c.top_k, c.n_expert);
 }
 

@@ -162,3 +162,32 @@ def test_a_token_hides_no_nan(ctx, fmt):
     dec.step(7)
     assert np.isnan(dec.logits()).all()
     dec.close()
+
+
+@pytest.mark.parametrize("E,fmt_gu,fmt_down,NE,K,F", [
+    (2048, capi.Q4_K, capi.Q4_K, 4, 1, 512), (2048, capi.Q4_K, capi.Q6_K, 8, 3, 2048), (2048, capi.Q6_K, capi.Q4_K, 3, 3, 2304),
+    (4096, capi.Q4_K, capi.Q4_K, 4, 2, 14336), (4096, capi.Q6_K, capi.Q6_K, 4, 2, 10240), (6144, capi.Q4_K, capi.Q6_K, 2, 2, 4096),
+    (6144, capi.Q6_K, capi.Q4_K, 4, 2, 9216), (8192, capi.Q4_K, capi.Q4_K, 2, 2, 2048)])
+def test_a_token_has_the_bits_of_a_launch_per_slot(ctx, monkeypatch, E, fmt_gu, fmt_down, NE, K, F):
+    """The selected experts in two launches (csrc/matvec_expert.cu) against a launch of the streaming kernel per slot: the same 21-bit
+    activations, exact integer sums and order of f32 sums, hence the same bits, up to 6144 columns of gate and up; above, the sum of squares
+    of the norm is taken in another order (16 units of 2^-24 at most between any two orders of so many warps, the logits 2e-6 measured)."""
+    seen = {}
+    for form in ("1", "0"):
+        monkeypatch.setenv("FLB_MOE_TOKEN", form)
+        dec = gpu_decoder(ctx, E, F, NE, K, fmt_gu, fmt_down, 11)
+        steps, tok = [], 5
+        for _ in range(3):
+            dec.step(tok)
+            steps.append((dec.logits().copy(), dec.tap(0).copy()))
+            tok += 101
+        assert all(np.isfinite(v).all() for s in steps for v in s) and ctx.status() == 0
+        seen[form] = steps, dec.launches_per_step()
+        dec.close()
+    (a, launches), (b, per_slot) = seen["1"], seen["0"]
+    assert per_slot - launches == (1 + 2 * K + 1) - 4    # router, then gate | up and down once or per slot, merge
+    for (la, ha), (lb, hb) in zip(a, b):
+        if E <= 6144:
+            assert np.array_equal(la, lb) and np.array_equal(ha, hb)
+        else:
+            assert np.linalg.norm(la - lb) <= 1e-5 * np.linalg.norm(lb) and np.linalg.norm(ha - hb) <= 1e-5 * np.linalg.norm(hb)
