@@ -25,7 +25,8 @@ def inputs(fmt, rows, cols, nx, seed):
 
 class Writers:
     """What comes in front of a call here are kernels of the library's own that let the next launch start at their entry, behind a matvec
-    whose last unit runs on one SM: the call's CTAs are on the other SMs before a single byte of its inputs is written."""
+    whose last unit runs on one SM: the call's CTAs are on the other SMs before its inputs are written (an attention 8 us before the last
+    of them, a matvec, which finds room only where the writers have left, 1.5 us)."""
 
     def __init__(self, ctx):
         self.ctx = ctx
@@ -33,8 +34,9 @@ class Writers:
         self.w, self.x = inputs(capi.Q4_K, 16 * units, 14336, 1, 77)
         self.y = torch.zeros(16 * units, device="cuda")
 
-    def block(self):
-        self.ctx.matvec_assign(capi.Q4_K, self.w, self.y.numel(), 14336, self.x, self.y)
+    def block(self):   # 14 us each where the call takes 5: the launches behind are all in the stream before these have run
+        for _ in range(16):
+            self.ctx.matvec_assign(capi.Q4_K, self.w, self.y.numel(), 14336, self.x, self.y)
 
     def fill(self, t, value):
         capi._ck(self.ctx.lib.fl_b200_memset(self.ctx._h, C.c_void_p(t.data_ptr()), value, C.c_size_t(t.numel() * t.element_size())))
@@ -132,6 +134,86 @@ def test_attention_written_by_the_kernels_before(ctx, kind, kv, batch, kv_len):
             ctx.attn_decode(q, k, v, 4 * kv, kv, 128, kv_len, kv_len, batch, scale, out)
 
     wr.check(write, call, [out, lse] if kind == "lse" else [out])
+
+
+# bytes that make numbers of a sane size in every format: scales of 0.01 to 0.07, quants and activations alike. A stage and a unit, several
+# units a CTA, more columns than a thread converts at once; planes, slices of columns, two passes over the weights
+@pytest.mark.parametrize("fmt", [capi.Q4_K, capi.Q6_K, capi.Q8_0])
+@pytest.mark.parametrize("rows,cols,nx", [(16, 2048, 1), (4096, 4096, 1), (2049, 14336, 1), (4096, 4096, 3), (300, 2048, 16), (1000, 4096, 19)])
+def test_matvec_written_by_the_kernels_before(ctx, fmt, rows, cols, nx):
+    wr = Writers(ctx)
+    w = torch.zeros((rows, capi.row_bytes(fmt, cols)), dtype=torch.uint8, device="cuda")
+    x, y = torch.zeros((nx, cols), device="cuda"), torch.zeros((nx, rows), device="cuda")
+    xs = [wr.source(nx * cols, 3 + i, 0.01) for i in range(2)]
+    torch.cuda.synchronize()
+
+    few = min(rows // 2, (1 << 20) // w.shape[1])   # a launch small enough to lie on the SMs beside the matvec in front
+
+    def write(i, pause):   # the weights last, the rows of the first units last of all
+        for s in (lambda: wr.floats(xs[i], x), lambda: wr.fill(w, 0x21 + i), lambda: wr.fill(w[:few], 0x2a - i)):
+            s()
+            pause()
+
+    def call():
+        if nx == 1:
+            ctx.matvec_assign(fmt, w, rows, cols, x, y)
+        else:
+            wr.fill(y, 0)
+            ctx.matvec(fmt, w, rows, cols, x, y, nx=nx, xstride=cols, ystride=rows)
+
+    wr.check(write, call, [y])
+
+
+@pytest.mark.parametrize("fmt", [capi.Q4_K, capi.Q6_K, capi.Q8_0])
+def test_pitched_rows_written_by_the_kernels_before(ctx, fmt):
+    rows, cols, wr = 1500, 2304, Writers(ctx)
+    pitch = (capi.row_bytes(fmt, cols) + 15) // 16 * 16 + 16
+    w, x, y = torch.zeros((rows, pitch), dtype=torch.uint8, device="cuda"), torch.zeros(cols, device="cuda"), torch.zeros(rows, device="cuda")
+    xs = [wr.source(cols, 8 + i, 0.01) for i in range(2)]
+    torch.cuda.synchronize()
+
+    def write(i, pause):
+        for s in (lambda: wr.floats(xs[i], x), lambda: wr.fill(w, 0x21 + i), lambda: wr.fill(w[:rows // 3], 0x2a - i)):
+            s()
+            pause()
+
+    wr.check(write, lambda: ctx.matvec_pitched(fmt, w, rows, cols, pitch, x, y), [y])
+
+
+def test_operands_written_on_the_legacy_default_stream(ctx):
+    """The context's stream is a blocking one: a kernel on the legacy default stream lies between the calls in front of it and behind it."""
+    rows = cols = 4096
+    pair = [inputs(capi.Q4_K, rows, cols, 1, s) for s in (1, 2)]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    kv = [tuple(torch.randn(4096 * 128, device="cuda", generator=g).half() for _ in range(2)) for _ in range(2)]
+    w, x, y = torch.empty_like(pair[0][0]), torch.empty_like(pair[0][1]), torch.zeros(rows, device="cuda")
+    k, v = torch.empty_like(kv[0][0]), torch.empty_like(kv[0][1])
+    q, out = torch.randn((1, 4, 128), device="cuda", generator=g), torch.zeros((1, 4, 128), device="cuda")
+
+    def call():
+        ctx.matvec_assign(capi.Q4_K, w, rows, cols, x, y)
+        ctx.attn_decode(q, k, v, 4, 1, 128, 4096, 4096, 1, 0.1, out)
+
+    def write(i):
+        for dst, src in zip((w, x, k, v), pair[i] + kv[i]):
+            dst.copy_(src)
+
+    want = []
+    for i in range(2):
+        write(i)
+        torch.cuda.synchronize()
+        call()
+        ctx.sync()
+        want.append((y.clone(), out.clone()))
+    torch.cuda.synchronize()
+    got = []
+    for i in range(30):   # everything but the calls on the default stream, nothing waited for
+        write(i % 2)
+        call()
+        got.append((y.clone(), out.clone()))
+    torch.cuda.synchronize()
+    assert not torch.equal(want[0][0], want[1][0]) and not torch.equal(want[0][1], want[1][1])
+    assert all(torch.equal(a, b) for i, pair in enumerate(got) for a, b in zip(pair, want[i % 2]))
 
 
 @pytest.mark.parametrize("fmt", [capi.Q4_K, capi.Q6_K, capi.Q8_0])
