@@ -106,9 +106,10 @@ __device__ __forceinline__ uint32_t pack_h2(__half lo, __half hi) {
 }
 
 // MODE 1: with RoPE and the append of this token's rows, 0: without, since a launch fetches its code from L2 (1024 keys, 8 KV heads,
-// calls in a row: 6.25 -> 5.50 us; a step of the 8B shape 0.5 % faster). 2: as the arguments say, for several sequences of a pass, whose
-// positions lie on the device: MODE 0 makes that pass up to 3 % slower (16 sequences: 6 layers in Q8_0 774 -> 787 us, of 1536 columns over 600 keys 459 -> 475, 8B shape
-// 4362 -> 4370).
+// calls in a row: 5.7 -> 5.4 us where the host issues them fast enough, 6.2 either way where it does not; a step of the 8B shape 0.5 % faster). 2: several
+// sequences of a pass, whose positions lie on the device. They have no RoPE here either (rope_k is null): what the branch on it changes is the
+// code around it, 193 registers against 191 in MODE 0, with which the passes take 1 to 3 % longer (16 sequences: 8 layers of the 8B shape 1310 -> 1321 us,
+// 6 layers of 2560 columns in Q8_0 771 -> 787, of 1536 464 -> 475; 5 sequences, 2048 columns 394 -> 405); the cause is not known.
 template <int MODE>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(const __grid_constant__ AttnArgs a) {
     extern __shared__ uint8_t smem_dyn[];
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(const __gr
     const uint32_t g = lane >> 2, t = lane & 3u;
     const uint32_t split = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z;
     const uint32_t group = a.n_q_head / a.n_kv_head;   // == kGroup (checked on the host)
-    const bool fused = MODE == 2 ? a.rope_k != nullptr : MODE == 1;
+    const bool fused = MODE == 2 ? a.rope_k != nullptr : MODE == 1;   // (MODE 2: never)
     if (tid == 0) trace_min(a.trace, 0);
     if (MODE != 0 || !a.late) griddep_launch_dependents();
     // *pos was written at the end of the previous step (or is kv_len - 1 of a single call): stable here.

@@ -278,8 +278,8 @@ static int enqueue_step(fl_b200_decoder *d, cudaStream_t s, uint32_t *n_launch, 
         }
         if (d->moe[l]) {
             // Mixture-of-experts layer: xb = xa + Wo att as usual, then xa = xb + MoE(RMSNorm(xb)). The block's own launches
-            // (router, selection, the selected experts through the expert-indexed matvec, merge) are part of the captured
-            // step; the norm is taken inside the router kernel and the gate | up launches, the residual inside the merge.
+            // (router with its selection, gate | up of the selected experts, their down, merge) are part of the captured
+            // step; the norm is taken inside the router kernel and the gate | up launch, the residual inside the merge.
             MatvecArgs ao = mk_o(l);
             if (mask & K_MATVEC) { if (int rc = do_matvec(ao)) return rc; ++n; }
             if (mask & K_MATVEC) {

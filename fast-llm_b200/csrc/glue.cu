@@ -463,8 +463,6 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ l
     }
 }
 
-} // namespace
-
 // Bound by its launch: a few hundred kilobytes at most in earnest (16 bytes a thread and round).
 __global__ void __launch_bounds__(256) fill_kernel(uint8_t *dst, uint32_t v, size_t bytes, uint32_t head) {
     griddep_launch_dependents();
@@ -478,6 +476,8 @@ __global__ void __launch_bounds__(256) fill_kernel(uint8_t *dst, uint32_t v, siz
         if (tail + threadIdx.x < bytes && threadIdx.x < 16) dst[tail + threadIdx.x] = (uint8_t)v;
     }
 }
+
+} // namespace
 
 cudaError_t launch_fill(void *dst, int value, size_t bytes, int sms, cudaStream_t stream, bool pdl) {
     if (!dst || !bytes) return cudaErrorInvalidValue;

@@ -287,16 +287,13 @@ cudaError_t launch_allreduce_push(const AllReduceArgs &a, cudaStream_t stream, b
 cudaError_t launch_argmax_exchange(const TopExchangeArgs &a, cudaStream_t stream, bool pdl);
 
 // ---- glue.cu ------------------------------------------------------------
-// rows vectors of n floats, `stride` floats apart in x and in y (one weight vector for all).
 // dst[0 .. bytes) = value; dst of any alignment.
 cudaError_t launch_fill(void *dst, int value, size_t bytes, int sms, cudaStream_t stream, bool pdl);
+// rows vectors of n floats, `stride` floats apart in x and in y (one weight vector for all).
 cudaError_t launch_rmsnorm(const float *x, const float *wnorm, float *y, float eps, uint32_t n,
                            cudaStream_t stream, uint32_t rows = 1, uint32_t stride = 0);
 cudaError_t launch_add2(const float *a, const float *b, float *y, uint32_t n, cudaStream_t stream);
-// fl_op_router_sel (src/runtime/decode_params.h:234-265) for n_tok tokens in one launch (one warp per token):
-// softmax over n_expert logits, top_k by weight; logits [n_tok][n_expert], ids / gates [n_tok][top_k]. Expert
-// parallel (lids, mgates != nullptr): also the expert's index among this rank's experts [base, base + n_local)
-// or the skip mark, and the gate or 0.
+// Router of a block in one launch: logits[t][e] = dot(router[e], x[t]), and what launch_router_sel does, by a token's last block.
 struct RouterArgs {
     const float *router, *x, *wnorm;   // [n_expert][n_embd]; [n_tok][n_embd]; optional: the logits are those of RMSNorm(x) * wnorm
     float eps;
@@ -317,6 +314,10 @@ cudaError_t launch_router(const RouterArgs &a, cudaStream_t stream);
 // of a grouped launch over the first 16 of each (launch_nx_table).
 cudaError_t launch_group_by_expert(const uint32_t *lids, uint32_t n_pairs, uint32_t top_k, uint32_t n_local, uint32_t cap,
                                    uint32_t *cnt, uint32_t *tok_list, uint32_t *pair_list, uint32_t *table, cudaStream_t stream, bool pdl);
+// fl_op_router_sel (src/runtime/decode_params.h:234-265) for n_tok tokens in one launch (one warp per token):
+// softmax over n_expert logits, top_k by weight; logits [n_tok][n_expert], ids / gates [n_tok][top_k]. Expert
+// parallel (lids, mgates != nullptr): also the expert's index among this rank's experts [base, base + n_local)
+// or the skip mark, and the gate or 0.
 cudaError_t launch_router_sel(const float *logits, uint32_t *ids, float *gates, uint32_t n_tok, uint32_t n_expert, uint32_t top_k,
                               uint32_t norm, float scale, cudaStream_t stream, uint32_t *lids = nullptr,
                               float *mgates = nullptr, uint32_t base = 0, uint32_t n_local = 0);

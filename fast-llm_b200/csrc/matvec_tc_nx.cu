@@ -267,9 +267,10 @@ __device__ __forceinline__ float4 combine_records(const float *part, uint32_t S,
 // (a.att) in flight, 16 or 40, the latter (254 registers) for those alone. GROUPED: the columns are those of a table. TM: the image is
 // that of matmul_tm.cu (8B shape, 8 positions 3110 -> 3088 us, 16 sequences 4432 -> 4392). An instance each,
 // since a launch fetches its code from L2 (lookup and records in one instance: passes of the 8B shape 1 % slower). The instance for
-// ungrouped columns keeps the records although few launches have any: without them the compiler takes 54 registers instead of
-// 128 and puts the planes' loads behind one another (6 positions: 1 to 2 % slower); for the thousands of blocks of a grouped launch fewer
-// registers are the better choice (Mixtral-shape block, 16 tokens: 275 against 280 us).
+// ungrouped columns keeps the records although few launches have any: with them it takes 128 registers, eight blocks an SM; without, 54, and blocks
+// that become resident while the matmul in front leaves gather on the first SMs it frees (8 positions, 8 layers of the 8B shape 917 -> 943 us,
+// 2048 columns 2.3 % slower). Shared memory reserved for the same eight an SM gives the same time there, but models of 1024 columns in Q8_0 1 to
+// 3 % more; the grouped instance, whose launches can be thousands of blocks, does that (launch_nx_convert).
 template <int F, bool GROUPED, bool TM>
 __global__ void __launch_bounds__(64) act_convert_nx_kernel(const ConvArgs a) {
     __shared__ float2 half_s[2];   // per warp: maximum, sum of squares
