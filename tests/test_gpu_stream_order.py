@@ -287,7 +287,8 @@ def test_cache_written_by_the_kernel_before(ctx, kv_len, batch):
     assert all(torch.equal(o, want[i % 2]) for i, o in enumerate(got))
 
 
-@pytest.mark.parametrize("offset,size", [(0, 1), (0, 16), (1, 15), (3, 14), (15, 1), (7, 4096), (16, 4099), (5, 3_000_001), (0, 64 << 20)])
+@pytest.mark.parametrize("offset,size", [(0, 1), (0, 16), (1, 15), (3, 14), (15, 1), (7, 4096), (16, 4099), (5, 3_000_001), (0, 64 << 20),
+                                         (1, 128 << 20), (1, (128 << 20) + 1)])   # the largest of the library's own kernel, the driver's
 def test_memset_any_range(ctx, offset, size):
     buf = torch.randint(0, 200, (offset + size + 40,), dtype=torch.uint8, device="cuda")
     want = buf.clone()
